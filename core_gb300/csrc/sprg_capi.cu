@@ -62,6 +62,10 @@ struct sprg_ctx {
   DevBuf titems, tcountb;  // triangle patches above the thread-per-vertex size
   DevBuf Lx, pairs, red, eflags;  // MA sweeps: lengths, vertex pairs, reduction scratch, element flags
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
+  // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
+  // egeo_none: there was no memory for them, the kernels compute in place
+  DevBuf egeo;
+  bool egeo_ready = false, egeo_none = false;
   // FP64 recovery on tets: per-mesh QR weights and the listed patches
   DevBuf qw, qwlisted, qwitems, qwcount;
   bool qw_ready = false;
@@ -361,11 +365,36 @@ int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, 
   return check_launch(c, "cached fit");
 }
 
+// the FP64 element records (once per mesh); the kernels that read them take
+// null instead where the device has no memory left for them
+int ensure_elem_records(sprg_ctx* c) {
+  if (c->egeo_ready || c->egeo_none) return SPRG_OK;
+  DevMesh& m = c->m;
+  int rc = ensure(c, c->egeo, sizeof(double) * (size_t)elem_record_planes(m.dim) * m.T);
+  if (rc == SPRG_ENOMEM) {
+    cudaGetLastError();  // the failed allocation is no error of this call
+    c->egeo_none = true;
+    return SPRG_OK;
+  }
+  if (rc) return rc;
+  PB("elem_records_f64");
+  launch_elem_records(m, P<double>(c->egeo), c->stream);
+  PE();
+  c->launches += 1;
+  if ((rc = check_launch(c, "element records"))) return rc;
+  c->egeo_ready = true;
+  return SPRG_OK;
+}
+
+const double* elem_records(sprg_ctx* c) { return c->egeo_ready ? P<double>(c->egeo) : nullptr; }
+
 int step_grad(sprg_ctx* c, int ncin) {
   DevMesh& m = c->m;
   ENSURE(c->ip, sizeof(double) * (size_t)m.T * 3 * ncin);
+  int rc = ensure_elem_records(c);
+  if (rc) return rc;
   PB("grad_ip_f64");
-  launch_grad_ip_f64(m, P<double>(c->f), ncin, P<double>(c->ip), c->stream);
+  launch_grad_ip_f64(m, elem_records(c), P<double>(c->f), ncin, P<double>(c->ip), c->stream);
   PE();
   c->launches += 1;
   c->ip_nc = 3 * ncin;
@@ -694,6 +723,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   // and an adapt iteration changes the patch-size mix little
   c->tw_ready = false;
   c->qw_ready = false;
+  c->egeo_ready = c->egeo_none = false;
   c->vv_ready = false;
   c->cache64.valid = c->cache32.valid = c->cache2d.valid = false;
   c->cache64.w_ready = c->cache32.w_ready = c->cache2d.w_ready = false;
@@ -858,7 +888,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->egeo, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,

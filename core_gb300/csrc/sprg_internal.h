@@ -68,8 +68,15 @@ struct ExpandList {
   int cap;
 };
 
+// ---- FP64 element kernels (sprg_elem_f64.cu) --------------------------
+// per-mesh element records: elem_record_planes(dim) planes of T doubles
+// (J^-1 row-major, D columns a row; det J; the longest edge)
+int elem_record_planes(int dim);
+void launch_elem_records(const DevMesh& m, double* geo, cudaStream_t s);
+// geo: the records, or null to compute them in place
+void launch_grad_ip_f64(const DevMesh& m, const double* geo, const double* f, int ncin, double* ip, cudaStream_t s);
+
 // ---- kernel launchers (sprg_kernels_f64.cu) ---------------------------
-void launch_grad_ip_f64(const DevMesh& m, const double* f, int ncin, double* ip, cudaStream_t s);
 // Triangles (tets recover through launch_qr_weights / launch_recover_w64):
 // xl: patches that need growth; big: patches above the thread-per-vertex
 // size (fitted by the warp path inside this call; its counter must be zero

@@ -89,40 +89,6 @@ __device__ __forceinline__ V3 elem_grad_component(const DevMesh& m, int e, const
 }
 
 // ---------------------------------------------------------------------
-// spr::getGradIPField
-// ---------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_grad_ip(DevMesh m, const double* __restrict__ f, int ncin,
-                                                    double* __restrict__ ip) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.T) return;
-  const int* ev = m.ev + (size_t)e * m.nn;
-  V3 x[4];
-  for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-  M3 J = ref::jacobian(x, m.nn, m.dim);
-  M3 jinv = ref::jacobian_inverse(J, m.dim);
-  V3 lg[4], gg[4];
-  ref::shape_grads(m.dim, lg);
-  for (int a = 0; a < m.nn; ++a) gg[a] = ref::mulv(jinv, lg[a]);
-  if (ncin == 1) {
-    V3 g = ref::scale(gg[0], f[ev[0]]);
-    for (int a = 1; a < m.nn; ++a) g = ref::add(g, ref::scale(gg[a], f[ev[a]]));
-    for (int k = 0; k < 3; ++k) ip[(size_t)e * 3 + k] = g.v[k];
-  } else {
-    M3 g;
-    for (int a = 0; a < m.nn; ++a) {
-      V3 u{{f[3 * (size_t)ev[a]], f[3 * (size_t)ev[a] + 1], f[3 * (size_t)ev[a] + 2]}};
-      for (int r = 0; r < 3; ++r) {
-        V3 rw = ref::scale(u, gg[a].v[r]);
-        if (a == 0) ref::setrow(g, r, rw);
-        else ref::setrow(g, r, ref::add(ref::row(g, r), rw));
-      }
-    }
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c) ip[(size_t)e * 9 + 3 * r + c] = g.m[r][c];
-  }
-}
-
-// ---------------------------------------------------------------------
 // spr::recoverField -- register path: one warp per vertex, RPL rows per
 // lane.  Patches that are too small, rank deficient or larger than 32*RPL
 // rows go to the expansion list.
@@ -2536,10 +2502,6 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
 // ----------------------------------------------------------------------
 // launchers
 // ----------------------------------------------------------------------
-void launch_grad_ip_f64(const DevMesh& m, const double* f, int ncin, double* ip, cudaStream_t s) {
-  if (m.T) k_grad_ip<<<nblk(m.T), kBlock, 0, s>>>(m, f, ncin, ip);
-}
-
 void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, ExpandList xl, ExpandList big,
                         DevStatus* st, cudaStream_t s) {
   (void)st;
