@@ -461,22 +461,24 @@ int step_size(sprg_ctx* c, int mode, double adapt_ratio, double target, double a
   ENSURE(c->size, sizeof(double) * (size_t)m.V);
   ENSURE(c->partials, sizeof(double) * 2 * (size_t)(nb > 0 ? nb : 1));
   ENSURE(c->out3, sizeof(double) * 4);
-  double p = 1, d = m.dim;
-  double gexp = (2 * d) / (2 * p + d);
+  if (!c->edone.p) {
+    ENSURE(c->edone, sizeof(unsigned));
+    CK(cudaMemsetAsync(c->edone.p, 0, sizeof(unsigned), c->stream));
+  }
+  int rc = ensure_elem_records(c);
+  if (rc) return rc;
   PB("error_f64");
-  launch_error_f64(m, P<double>(c->ip), nc, P<double>(c->rec), P<double>(c->err), P<double>(c->partials), nb, gexp,
+  launch_error_f64(m, elem_records(c), P<double>(c->ip), nc, P<double>(c->rec), P<double>(c->err), P<double>(c->esize),
+                   P<double>(c->partials), nb, P<unsigned>(c->edone), mode, adapt_ratio, target, P<double>(c->out3),
                    c->stream);
   PE();
-  PB("size_factor");
-  launch_size_factor(P<double>(c->partials), nb, mode, adapt_ratio, target, m.dim, P<double>(c->out3), c->stream);
-  PE();
   PB("esize_f64");
-  launch_esize_f64(m, P<double>(c->err), P<double>(c->out3), mode, alpha, beta, P<double>(c->esize), c->stream);
+  launch_esize_f64(m, elem_records(c), P<double>(c->out3), mode, alpha, beta, P<double>(c->esize), c->stream);
   PE();
   PB("average_f64");
   launch_average(m, P<double>(c->esize), P<double>(c->size), c->stream);
   PE();
-  c->launches += 4;
+  c->launches += 3;
   c->size_valid = true;
   return check_launch(c, "size field");
 }

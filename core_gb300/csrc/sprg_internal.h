@@ -75,6 +75,18 @@ int elem_record_planes(int dim);
 void launch_elem_records(const DevMesh& m, double* geo, cudaStream_t s);
 // geo: the records, or null to compute them in place
 void launch_grad_ip_f64(const DevMesh& m, const double* geo, const double* f, int ncin, double* ip, cudaStream_t s);
+// per-element errors, their powers in esize (k_error) and deterministic block
+// partials (2 per block, error_blocks(T) blocks); mode 0: SPR, 1: target.
+// done (one unsigned, zero between launches): the last block also computes
+// the size factor into out3, as launch_size_factor does; null: it does not
+void launch_error_f64(const DevMesh& m, const double* geo, const double* ip, int nc, const double* rec, double* err,
+                      double* esize, double* partials, int n_blocks, unsigned* done, int mode, double adapt_ratio,
+                      double target, double* out3, cudaStream_t s);
+int error_blocks(int T);
+// element sizes, in place on the error kernel's esize
+void launch_esize_f64(const DevMesh& m, const double* geo, const double* out3, int mode, double alpha, double beta,
+                      double* esize, cudaStream_t s);
+void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s);
 
 // ---- kernel launchers (sprg_kernels_f64.cu) ---------------------------
 // Triangles (tets recover through launch_qr_weights / launch_recover_w64):
@@ -109,16 +121,9 @@ void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u,
                             const int* wn, DevStatus* st, cudaStream_t s);
 int expand_max_elems();
 int expand_grid();
-// Per-element error terms + deterministic block partials (2 per block).
-void launch_error_f64(const DevMesh& m, const double* ip, int nc, const double* rec, double* err,
-                      double* partials, int n_blocks, double g_exponent, cudaStream_t s);
-int error_blocks(int T);
 // Sum partials in fixed order, compute size factor.  mode 0: SPR; 1: target.
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target,
                         int dim, double* out3, cudaStream_t s);
-void launch_esize_f64(const DevMesh& m, const double* err, const double* out3, int mode, double alpha,
-                      double beta, double* esize, cudaStream_t s);
-void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s);
 void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s);
 void launch_measure_aniso_f64(const DevMesh& m, const double* sizes, const double* frames, double* L,
                               cudaStream_t s);

@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kBlock) k_cached_wsum(DevMesh m, const double*
 }
 
 // ---------------------------------------------------------------------
-// Element error terms (SelfProduct / ElementError, spr/sprEstimateError.cc:98-170)
+// Size factor
 // ---------------------------------------------------------------------
 __device__ __forceinline__ double block_sum(double x, double* sh) {
   x = warp_sum(x);
@@ -696,45 +696,6 @@ __device__ __forceinline__ double block_sum(double x, double* sh) {
   if (threadIdx.x == 0)
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
   return t;
-}
-
-__global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __restrict__ ip, int nc,
-                                                  const double* __restrict__ rec, double* __restrict__ err,
-                                                  double* __restrict__ partials, double g_exponent) {
-  __shared__ double sh[kBlock / 32];
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  double self_term = 0, g_term = 0;
-  if (e < m.T) {
-    const int* ev = m.ev + (size_t)e * m.nn;
-    V3 x[4];
-    for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-    M3 J = ref::jacobian(x, m.nn, m.dim);
-    double dV = ref::jacobian_det(J, m.dim);
-    double w = ref::ip_weight(m.dim);
-    double N[4];
-    ref::ip_shape_values(m.dim, N);
-    double v2[9], v1[9];
-    for (int k = 0; k < nc; ++k) v2[k] = 0;
-    for (int a = 0; a < m.nn; ++a)
-      for (int k = 0; k < nc; ++k) v2[k] += rec[(size_t)ev[a] * nc + k] * N[a];
-    double vv = 0;
-    for (int k = 0; k < nc; ++k) vv += v2[k] * v2[k];
-    self_term = vv * w * dV;
-    for (int k = 0; k < nc; ++k) v1[k] = ip[(size_t)e * nc + k];
-    for (int k = 0; k < nc; ++k) v1[k] -= v2[k];
-    double dd = 0;
-    for (int k = 0; k < nc; ++k) dd += v1[k] * v1[k];
-    double sum = 0;
-    sum += dd * w * dV;
-    err[e] = sum;
-    g_term = pow(sqrt(sum), g_exponent);
-  }
-  double s1 = block_sum(self_term, sh);
-  double s2 = block_sum(g_term, sh);
-  if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = s1;
-    partials[2 * blockIdx.x + 1] = s2;
-  }
 }
 
 // one block: fixed-order reduction of the partials, then the size factor
@@ -780,47 +741,6 @@ __device__ __forceinline__ double edge_measure(const V3& x0, const V3& x1) {
 
 __constant__ int c_tet_edges[6][2] = {{0, 1}, {1, 2}, {2, 0}, {0, 3}, {1, 3}, {2, 3}};
 __constant__ int c_tri_edges[3][2] = {{0, 1}, {1, 2}, {2, 0}};
-
-__global__ void __launch_bounds__(kBlock) k_esize(DevMesh m, const double* __restrict__ err,
-                                                  const double* __restrict__ out3, int mode, double alpha,
-                                                  double beta, double* __restrict__ esize) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.T) return;
-  const int* ev = m.ev + (size_t)e * m.nn;
-  V3 x[4];
-  for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-  double h = 0;
-  for (int i = 0; i < m.ne_el; ++i) {
-    int p = m.dim == 3 ? c_tet_edges[i][0] : c_tri_edges[i][0];
-    int q = m.dim == 3 ? c_tet_edges[i][1] : c_tri_edges[i][1];
-    double l = edge_measure(x[p], x[q]);
-    h = (h < l) ? l : h;
-  }
-  double sf = out3[2];
-  double pp = 1, d = m.dim;
-  if (mode == 0) {
-    double errorNorm = pow(sqrt(err[e]), -(2 / (2 * pp + d)));
-    esize[e] = h * errorNorm * sf;
-  } else {
-    double theta_e = sqrt(err[e]);
-    double r = pow(theta_e, ((-2.0) / (2.0 * 1 + m.dim)));
-    double h_new = sf * r * h;
-    if (h_new < alpha * h) h_new = alpha * h;
-    if (h_new > beta * h) h_new = beta * h;
-    esize[e] = h_new;
-  }
-}
-
-__global__ void __launch_bounds__(kBlock) k_average(DevMesh m, const double* __restrict__ esize,
-                                                    double* __restrict__ size) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= m.V) return;
-  int b = m.a_off[v], e = m.a_off[v + 1];
-  double s = 0;
-  for (int k = b; k < e; ++k) s += esize[m.a_el[k]];
-  s /= (double)(size_t)(e - b);
-  size[v] = s;
-}
 
 // MetricSizeField::measure, 2-point Gauss (ma/maSize.cc:158-214)
 __device__ __forceinline__ double metric_length(const V3& x0, const V3& x1, const double* hv, const double* Rv) {
@@ -2553,13 +2473,6 @@ void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u,
                                                                                 cache_el, woff, w, wn, st);
 }
 
-int error_blocks(int T) { return nblk(T); }
-
-void launch_error_f64(const DevMesh& m, const double* ip, int nc, const double* rec, double* err,
-                      double* partials, int n_blocks, double g_exponent, cudaStream_t s) {
-  if (n_blocks) k_error<<<n_blocks, kBlock, 0, s>>>(m, ip, nc, rec, err, partials, g_exponent);
-}
-
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target, int dim,
                         double* out3, cudaStream_t s) {
   k_size_factor<<<1, kBlock, 0, s>>>(partials, n_blocks, mode, adapt_ratio, target, dim, out3);
@@ -2568,15 +2481,6 @@ void launch_size_factor(const double* partials, int n_blocks, int mode, double a
 void launch_size_factor_batch(const double* partials, BatchView bv, int dim, double* out4, cudaStream_t s) {
   (void)dim;  // p = 1: size_factor = (ratio^2 |eps*|^2 / G)^(1/2) in 2D and 3D
   if (bv.n) k_size_factor_batch<<<bv.n, kBlock, 0, s>>>(partials, bv, out4);
-}
-
-void launch_esize_f64(const DevMesh& m, const double* err, const double* out3, int mode, double alpha, double beta,
-                      double* esize, cudaStream_t s) {
-  if (m.T) k_esize<<<nblk(m.T), kBlock, 0, s>>>(m, err, out3, mode, alpha, beta, esize);
-}
-
-void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s) {
-  if (m.V) k_average<<<nblk(m.V), kBlock, 0, s>>>(m, esize, size);
 }
 
 void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s) {

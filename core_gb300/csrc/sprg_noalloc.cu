@@ -96,10 +96,9 @@ extern "C" int sprg_spr_size_from_recovered_noalloc(int dim, int64_t n_verts, in
   m.p_el = d_vert_elems;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int nb = sprg::error_blocks(m.T);
-  double p = 1, d = dim;
-  sprg::launch_error_f64(m, d_ip, ncomp, d_rec, err, partials, nb, (2 * d) / (2 * p + d), s);
+  sprg::launch_error_f64(m, nullptr, d_ip, ncomp, d_rec, err, esize, partials, nb, nullptr, 0, adapt_ratio, 0, out3, s);
   sprg::launch_size_factor(partials, nb, 0, adapt_ratio, 0, dim, out3, s);
-  sprg::launch_esize_f64(m, err, out3, 0, 0, 0, esize, s);
+  sprg::launch_esize_f64(m, nullptr, out3, 0, 0, 0, esize, s);
   sprg::launch_average(m, esize, d_size, s);
   if (cudaGetLastError() != cudaSuccess) return SPRG_ECUDA;
   if (size_factor_out) {

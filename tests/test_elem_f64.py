@@ -66,3 +66,36 @@ def test_records_follow_a_mesh_update(gpu_lib, oracle_lib):
         c.getGradIPField(u)
         c.update_mesh(m2)
         assert np.array_equal(c.getGradIPField(u), o2.grad_ip(u))
+
+
+@pytest.mark.parametrize("n,nz", [(2, 3), (7, 6), (3, 0), (9, 0), (16, 0)])
+@pytest.mark.parametrize("scale", [1e-160, 1e-70, 1.0, 1e70, 1e140])
+@pytest.mark.parametrize("target", [0, 1000])
+def test_element_sizes_from_errors(gpu_lib, oracle_lib, n, nz, scale, target):
+    """h err^(-1/(D+2)) times the size factor, and the error integral, against
+    extended precision on the errors the pass wrote.  2 ulps for the power and
+    half an ulp for each of the two products after it: 7e-16 relative."""
+    import core_gb300 as cg
+    m, _ = mesh(oracle_lib, n, nz, "plain")
+    ip = np.random.default_rng(5).normal(size=(m.n_elems, 3)) * scale
+    if m.dim == 2:
+        ip[:, 2] = 0.0
+    with cg.Context(m) as c:
+        if target:
+            c.getTargetSPRSizeField(ip, target, 1e-300, 1e300)
+        else:
+            c.getSPRSizeField(ip, 0.1)
+        err = c.debug_read("err", np.float64, m.n_elems).astype(np.longdouble)
+        esize = c.debug_read("esize", np.float64, m.n_elems)
+        out3 = c.debug_read("out3", np.float64, 3)
+    x = m.coords[m.elem_verts]
+    h = np.max([np.linalg.norm(x[:, a] - x[:, b], axis=1) for a in range(m.dim + 1) for b in range(a)], axis=0)
+    ok = err > 1e-290
+    power = err[ok] ** (-1 / np.longdouble(m.dim + 2))
+    want = h[ok].astype(np.longdouble) * power * np.longdouble(out3[2])
+    # h itself is compared as numpy sums it: two more ulps
+    assert np.max(np.abs(esize[ok] - want) / want, initial=0.0) <= 7e-16 + 4.5e-16
+    assert np.all(np.isinf(esize[err == 0])) or target
+    if ok.all():
+        G = np.sum(err ** (np.longdouble(2 * m.dim) / (m.dim + 2) / 2))
+        assert abs(out3[1] - G) <= 1e-13 * G
