@@ -64,8 +64,8 @@ struct sprg_ctx {
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
   // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
   // egeo_none: there was no memory for them, the kernels compute in place
-  DevBuf egeo;
-  bool egeo_ready = false, egeo_none = false;
+  DevBuf egeo, elen64;  // elen64: the edges' lengths
+  bool egeo_ready = false, egeo_none = false, elen64_ready = false, elen64_none = false;
   // FP64 recovery on tets: per-mesh QR weights and the listed patches
   DevBuf qw, qwlisted, qwitems, qwcount;
   bool qw_ready = false;
@@ -494,6 +494,34 @@ int step_measure_iso(sprg_ctx* c) {
   return check_launch(c, "measure");
 }
 
+// the FP64 pass's lengths and mark bitmaps from its size field
+int step_measure_mark(sprg_ctx* c, uint32_t* d_split, uint32_t* d_collapse) {
+  DevMesh& m = c->m;
+  ENSURE(c->L, sizeof(double) * (size_t)m.E);
+  if (!c->elen64_ready && !c->elen64_none) {
+    int rc = ensure(c, c->elen64, sizeof(double) * (size_t)m.E);
+    if (rc == SPRG_ENOMEM) {
+      cudaGetLastError();
+      c->elen64_none = true;
+    } else if (rc) {
+      return rc;
+    } else {
+      PB("edge_records_f64");
+      launch_edge_records(m, P<double>(c->elen64), c->stream);
+      PE();
+      c->launches += 1;
+      c->elen64_ready = true;
+    }
+  }
+  PB("measure_f64");
+  launch_measure_mark_f64(m, c->elen64_ready ? P<double>(c->elen64) : nullptr, P<double>(c->size), P<double>(c->L),
+                          d_split, d_collapse, c->stream);
+  PE();
+  c->launches += 1;
+  c->L_valid = true;
+  return check_launch(c, "measure and mark");
+}
+
 // the pass's integrals and counters, copied into the staging block on the
 // stream (read by info_from_stage after the stream is synchronized)
 int enqueue_info(sprg_ctx* c) {
@@ -725,7 +753,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   // and an adapt iteration changes the patch-size mix little
   c->tw_ready = false;
   c->qw_ready = false;
-  c->egeo_ready = c->egeo_none = false;
+  c->egeo_ready = c->egeo_none = c->elen64_ready = c->elen64_none = false;
   c->vv_ready = false;
   c->cache64.valid = c->cache32.valid = c->cache2d.valid = false;
   c->cache64.w_ready = c->cache32.w_ready = c->cache2d.w_ready = false;
@@ -890,7 +918,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->egeo, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,
@@ -1861,13 +1889,9 @@ static int pass_resident(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uin
   if (c->precision == SPRG_FP32) return pass_fast(c, adapt_ratio, d_split, d_collapse);
   if (c->precision == SPRG_LEARNED) return pass_learned(c, adapt_ratio, d_split, d_collapse);
   if ((rc = reset_status(c)) || (rc = step_grad(c, 1)) || (rc = step_recover(c)) ||
-      (rc = step_size(c, 0, adapt_ratio, 0, 0, 0)) || (rc = step_measure_iso(c)))
+      (rc = step_size(c, 0, adapt_ratio, 0, 0, 0)))
     return rc;
-  PB("mark_bits");
-  launch_mark_bits(c->m.E, P<double>(c->L), d_split, d_collapse, c->stream);
-  PE();
-  c->launches += 1;
-  return check_launch(c, "mark bits");
+  return step_measure_mark(c, d_split, d_collapse);
 }
 
 int sprg_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split_bits,

@@ -7,7 +7,7 @@
 // shape gradients' 0, 1 and -1, sums with 0), and quotients by one common
 // divisor come from its rounded reciprocal with exact residuals.
 #include "sprg_internal.h"
-#include "sprg_refmath.cuh"
+#include "sprg_metric_f64.cuh"
 #include "sprg_reduce.cuh"
 
 namespace sprg {
@@ -34,8 +34,6 @@ __device__ __forceinline__ void load_ids(const int* __restrict__ ev, int e, int*
     for (int a = 0; a < 3; ++a) id[a] = __ldg(ev + 3 * (size_t)e + a);
   }
 }
-
-__device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
 // a / b rounded to nearest, y = 1 / b rounded to nearest: two exact-residual
 // corrections of a y.  The first leaves a faithful quotient, the second
@@ -370,6 +368,68 @@ __global__ void __launch_bounds__(kBlock) k_average(DevMesh m, const double* __r
   size[v] = s;
 }
 
+// ---------------------------------------------------------------------
+// Isotropic edge lengths (ma::makeSizeField(m, size) + measure)
+// ---------------------------------------------------------------------
+// given sizes: the lengths themselves, bitwise
+__global__ void __launch_bounds__(kBlock) k_measure_iso(DevMesh m, const double* __restrict__ size,
+                                                        double* __restrict__ L) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m.E) return;
+  const int2 v = __ldg(reinterpret_cast<const int2*>(m.edv) + e);
+  L[e] = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), __ldg(size + v.x), __ldg(size + v.y));
+}
+
+// per mesh: the edges' Euclidean lengths
+__global__ void __launch_bounds__(kBlock) k_edge_records(DevMesh m, double* __restrict__ len) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m.E) return;
+  const int2 v = __ldg(reinterpret_cast<const int2*>(m.edv) + e);
+  len[e] = ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
+}
+
+// The pass's lengths and marks.  The sizes it computed are good to about
+// 1e-10 of the reference's, so the lengths need no particular rounding:
+// |d| / 2 (1 / h0 + 1 / h1) = |d| (h0 + h1) / (2 h0 h1), about 20 FP64
+// operations with the per-mesh edge lengths against 55.  Lengths within 1e-6
+// of 0.5 or 1.5, and those iso_length hands to the reference's sequence, take
+// iso_length, so every mark is that of the bitwise length.  The comparisons
+// and windows are integer ones on the bits (FP64 comparisons use the FP64
+// pipe).  96^3 box, 6.3M edges: 0.99 ms for the reference's sequence plus
+// 0.03 ms for marking from the stored lengths, 0.24 ms here.
+template <bool REC>
+__global__ void __launch_bounds__(kBlock) k_measure_mark(DevMesh m, const double* __restrict__ len,
+                                                         const double* __restrict__ size, double* __restrict__ L,
+                                                         uint32_t* __restrict__ split,
+                                                         uint32_t* __restrict__ collapse) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  bool sp = false, co = false;
+  if (e < m.E) {
+    const int2 v = __ldg(reinterpret_cast<const int2*>(m.edv) + e);
+    const double sa = __ldg(size + v.x), sb = __ldg(size + v.y);
+    double d;
+    if constexpr (REC) d = __ldcs(len + e);
+    else d = ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
+    double h[2];
+    gauss_sizes(sa, sb, h);
+    double l = 0.5 * ((d * (h[0] + h[1])) / (h[0] * h[1]));
+    const int e0 = __double2hiint(h[0]) >> 20, e1 = __double2hiint(h[1]) >> 20, hl = __double2hiint(l);
+    // hl >> 20 is the biased exponent of a positive length, negative for a
+    // negative one; 0x3ff80000 is 1.5's high word, 0x3fe00000 0.5's
+    if (min(min(e0, e1), hl >> 20) < 623 || max(max(e0, e1), hl >> 20) > 1423 ||
+        (unsigned)(hl - 0x3ff7ffff) < 2u || (unsigned)(hl - 0x3fdfffff) < 2u)
+      l = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), sa, sb);
+    L[e] = l;
+    sp = l > 1.5;
+    co = l < .5;
+  }
+  const unsigned bs = __ballot_sync(0xffffffffu, sp), bc = __ballot_sync(0xffffffffu, co);
+  if ((threadIdx.x & 31) == 0 && e < m.E) {
+    split[e >> 5] = bs;
+    collapse[e >> 5] = bc;
+  }
+}
+
 // blocks of the error kernel: eight per SM, so that a thread takes several
 // elements and the reductions stay a small share
 constexpr int kErrorGrid = 152 * 8;
@@ -424,6 +484,21 @@ void launch_esize_f64(const DevMesh& m, const double* geo, const double* out3, i
 
 void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s) {
   if (m.V) k_average<<<nblk(m.V), kBlock, 0, s>>>(m, esize, size);
+}
+
+void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s) {
+  if (m.E) k_measure_iso<<<nblk(m.E), kBlock, 0, s>>>(m, size, L);
+}
+
+void launch_edge_records(const DevMesh& m, double* len, cudaStream_t s) {
+  if (m.E) k_edge_records<<<nblk(m.E), kBlock, 0, s>>>(m, len);
+}
+
+void launch_measure_mark_f64(const DevMesh& m, const double* len, const double* size, double* L, uint32_t* split,
+                             uint32_t* collapse, cudaStream_t s) {
+  if (!m.E) return;
+  if (len) k_measure_mark<true><<<nblk(m.E), kBlock, 0, s>>>(m, len, size, L, split, collapse);
+  else k_measure_mark<false><<<nblk(m.E), kBlock, 0, s>>>(m, len, size, L, split, collapse);
 }
 
 }  // namespace sprg

@@ -87,6 +87,13 @@ int error_blocks(int T);
 void launch_esize_f64(const DevMesh& m, const double* geo, const double* out3, int mode, double alpha, double beta,
                       double* esize, cudaStream_t s);
 void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s);
+// isotropic lengths of given sizes, bitwise the reference's
+void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s);
+// per-mesh Euclidean edge lengths (E doubles); the pass's lengths (a few ulps,
+// bitwise near 0.5 and 1.5) with the predicate bitmaps, len null: in place
+void launch_edge_records(const DevMesh& m, double* len, cudaStream_t s);
+void launch_measure_mark_f64(const DevMesh& m, const double* len, const double* size, double* L, uint32_t* split,
+                             uint32_t* collapse, cudaStream_t s);
 
 // ---- kernel launchers (sprg_kernels_f64.cu) ---------------------------
 // Triangles (tets recover through launch_qr_weights / launch_recover_w64):
@@ -124,7 +131,6 @@ int expand_grid();
 // Sum partials in fixed order, compute size factor.  mode 0: SPR; 1: target.
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target,
                         int dim, double* out3, cudaStream_t s);
-void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s);
 void launch_measure_aniso_f64(const DevMesh& m, const double* sizes, const double* frames, double* L,
                               cudaStream_t s);
 void launch_mark(int E, const double* L, int which, int* flags, unsigned long long* count, DevStatus* st,

@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "sprg_internal.h"
+#include "sprg_metric_f64.cuh"
 #include "sprg_refmath.cuh"
 #include "sprg_reduce.cuh"
 
@@ -742,41 +743,6 @@ __device__ __forceinline__ double edge_measure(const V3& x0, const V3& x1) {
 __constant__ int c_tet_edges[6][2] = {{0, 1}, {1, 2}, {2, 0}, {0, 3}, {1, 3}, {2, 3}};
 __constant__ int c_tri_edges[3][2] = {{0, 1}, {1, 2}, {2, 0}};
 
-// MetricSizeField::measure, 2-point Gauss (ma/maSize.cc:158-214)
-__device__ __forceinline__ double metric_length(const V3& x0, const V3& x1, const double* hv, const double* Rv) {
-  V3 x[2] = {x0, x1};
-  M3 J = ref::jacobian(x, 2, 1);
-  const double gp[2] = {0.577350269189626, -0.577350269189626};
-  double measurement = 0;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    double N[2];
-    ref::edge_shape_values(gp[p], N);
-    M3 Q = ref::get_transform(hv, Rv, N, 2);
-    double dV2 = ref::jacobian_det(ref::mul(J, Q), 1);
-    measurement += 1 * dV2;
-  }
-  return measurement;
-}
-
-__device__ __forceinline__ void identity9(double* R) {
-  for (int k = 0; k < 9; ++k) R[k] = (k % 4 == 0) ? 1.0 : 0.0;
-}
-
-__global__ void __launch_bounds__(kBlock) k_measure_iso(DevMesh m, const double* __restrict__ size,
-                                                        double* __restrict__ L) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.E) return;
-  int a = m.edv[2 * (size_t)e], b = m.edv[2 * (size_t)e + 1];
-  double hv[6], Rv[18];
-  double sa = size[a], sb = size[b];
-  hv[0] = hv[1] = hv[2] = sa;
-  hv[3] = hv[4] = hv[5] = sb;
-  identity9(Rv);
-  identity9(Rv + 9);
-  L[e] = metric_length(load_xyz(m.xyz, a), load_xyz(m.xyz, b), hv, Rv);
-}
-
 __global__ void __launch_bounds__(kBlock) k_measure_aniso(DevMesh m, const double* __restrict__ sizes,
                                                           const double* __restrict__ frames,
                                                           double* __restrict__ L) {
@@ -1181,10 +1147,7 @@ __global__ void __launch_bounds__(128) k_guard_decide(DevMesh m, const double* _
       if (bad || !(sz[0] == sz[0]) || !(sz[1] == sz[1])) {  // too many elements, or a NaN size
         atomicAdd(unresolved, 1);
       } else {
-        double hv[6] = {sz[0], sz[0], sz[0], sz[1], sz[1], sz[1]}, Rv[18];
-        identity9(Rv);
-        identity9(Rv + 9);
-        double L = metric_length(load_xyz(m.xyz, ab[0]), load_xyz(m.xyz, ab[1]), hv, Rv);
+        double L = iso_length(load_xyz(m.xyz, ab[0]), load_xyz(m.xyz, ab[1]), sz[0], sz[1]);
         uint32_t bit = 1u << (e & 31);
         if (L > 1.5) atomicOr(&split[e >> 5], bit); else atomicAnd(&split[e >> 5], ~bit);
         if (L < .5) atomicOr(&collapse[e >> 5], bit); else atomicAnd(&collapse[e >> 5], ~bit);
@@ -1463,19 +1426,12 @@ __device__ __forceinline__ double pair_length(const DevMesh& m, int kind, int a,
   const V3 xa = load_xyz(m.xyz, a), xb = load_xyz(m.xyz, b);
   if (kind == 0) return edge_measure(xa, xb);
   if (kind == 3) return log_metric_length(xa, xb, logm + 9 * (size_t)a, logm + 9 * (size_t)b, ok);
+  if (kind == 1) return iso_length(xa, xb, size[a], size[b]);
   double hv[6], Rv[18];
-  if (kind == 1) {
-    const double sa = size[a], sb = size[b];
-    hv[0] = hv[1] = hv[2] = sa;
-    hv[3] = hv[4] = hv[5] = sb;
-    identity9(Rv);
-    identity9(Rv + 9);
-  } else {
-    const int vv[2] = {a, b};
-    for (int i = 0; i < 2; ++i) {
-      for (int k = 0; k < 3; ++k) hv[3 * i + k] = sizes[3 * (size_t)vv[i] + k];
-      for (int k = 0; k < 9; ++k) Rv[9 * i + k] = frames[9 * (size_t)vv[i] + k];
-    }
+  const int vv[2] = {a, b};
+  for (int i = 0; i < 2; ++i) {
+    for (int k = 0; k < 3; ++k) hv[3 * i + k] = sizes[3 * (size_t)vv[i] + k];
+    for (int k = 0; k < 9; ++k) Rv[9 * i + k] = frames[9 * (size_t)vv[i] + k];
   }
   return metric_length(xa, xb, hv, Rv);
 }
@@ -2481,10 +2437,6 @@ void launch_size_factor(const double* partials, int n_blocks, int mode, double a
 void launch_size_factor_batch(const double* partials, BatchView bv, int dim, double* out4, cudaStream_t s) {
   (void)dim;  // p = 1: size_factor = (ratio^2 |eps*|^2 / G)^(1/2) in 2D and 3D
   if (bv.n) k_size_factor_batch<<<bv.n, kBlock, 0, s>>>(partials, bv, out4);
-}
-
-void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s) {
-  if (m.E) k_measure_iso<<<nblk(m.E), kBlock, 0, s>>>(m, size, L);
 }
 
 void launch_measure_aniso_f64(const DevMesh& m, const double* sizes, const double* frames, double* L,

@@ -99,3 +99,51 @@ def test_element_sizes_from_errors(gpu_lib, oracle_lib, n, nz, scale, target):
     if ok.all():
         G = np.sum(err ** (np.longdouble(2 * m.dim) / (m.dim + 2) / 2))
         assert abs(out3[1] - G) <= 1e-13 * G
+
+
+@pytest.mark.parametrize("n,nz", [(1, 1), (5, 4), (11, 0)])
+@pytest.mark.parametrize("sizes", ["random", "equal", "tiny", "huge", "odd"])
+def test_iso_lengths_bitwise(gpu_lib, oracle_lib, n, nz, sizes):
+    import core_gb300 as cg
+    m, o = mesh(oracle_lib, n, nz, "plain")
+    s = np.random.default_rng(6).uniform(0.2 / n, 3.0 / n, m.n_verts)
+    if sizes == "equal":
+        s[:] = 1.0 / (1.5 * n)
+    elif sizes == "tiny":
+        s *= 1e-200
+    elif sizes == "huge":
+        s *= 1e200
+    elif sizes == "odd":
+        s[::5] = [0.0, np.inf, np.nan, -s[0], 5e-324][:len(s[::5])] + [s[1]] * max(0, len(s[::5]) - 5)
+    with cg.Context(m) as c:
+        assert np.array_equal(c.measure_edges(s), o.measure(s), equal_nan=True)
+        pairs = m.edge_verts[::-1]
+        assert np.array_equal(c.measure_vertex_pairs(pairs, size=s), o.measure(s)[::-1], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,in_place", [(2, False), (7, False), (7, True)])
+def test_pass_marks_are_those_of_the_bitwise_lengths(gpu_lib, oracle_lib, n, in_place):
+    """The pass's marks against the reference lengths of its own sizes, with
+    the adapt ratio placed so that an edge sits at each threshold; in_place:
+    the last allocation of the first pass, the edge lengths', fails."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m, o = mesh(oracle_lib, n, n, "plain")
+    u = workload.bump_field(m.coords, seed=3)
+    with cg.Context(m) as c:
+        L = np.sort(o.measure(c.estimate_and_mark(u, 0.1)[0]))
+    for threshold in (0.5, 1.5):
+        # sizes are proportional to the ratio: put the median edge on the threshold
+        ratio = 0.1 * L[len(L) // 2] / threshold
+        for k in range(0 if in_place else -1, 100):
+            with cg.Context(m) as c:
+                c.test_hooks(alloc_fail_after=k)
+                try:
+                    size, flags, ns, nc, _ = c.estimate_and_mark(u, ratio)
+                    break
+                except cg.SprgError as e:
+                    assert e.code == 4
+        L1 = o.measure(size)
+        assert np.abs(L1 - threshold).min() < 1e-9
+        assert np.array_equal((flags & 1) != 0, L1 > 1.5) and np.array_equal((flags & 4) != 0, L1 < 0.5)
+        assert (ns, nc) == (int((L1 > 1.5).sum()), int((L1 < 0.5).sum()))
