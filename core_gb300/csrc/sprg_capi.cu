@@ -60,6 +60,11 @@ struct sprg_ctx {
   // scratch
   DevBuf partials, out3, status, count, xitems, xcount, slab, bits;
   DevBuf titems, tcountb;  // triangle patches above the thread-per-vertex size
+  // per mesh: the triangle patches' factors (33 doubles a vertex) and the
+  // lengths of the two lists; tfac_none: no memory, each recovery factors in place
+  DevBuf tqc, trr, tcode, txcount;
+  bool tfac_ready = false, tfac_none = false;
+  int n_tri_big = 0;
   DevBuf Lx, pairs, red, eflags;  // MA sweeps: lengths, vertex pairs, reduction scratch, element flags
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
   // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
@@ -436,18 +441,50 @@ int step_recover(sprg_ctx* c) {
   }
   ENSURE(c->xitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
   ENSURE(c->xcount, sizeof(int));
-  ENSURE(c->titems, sizeof(int) * (size_t)(m.dim == 2 && m.V > 0 ? m.V : 1));
+  ENSURE(c->titems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
   ENSURE(c->tcountb, sizeof(int));
-  CK(cudaMemsetAsync(c->xcount.p, 0, sizeof(int), c->stream));
-  CK(cudaMemsetAsync(c->tcountb.p, 0, sizeof(int), c->stream));
+  ENSURE(c->txcount, sizeof(int));
   ExpandList xl{P<int>(c->xitems), P<int>(c->xcount), m.V};
-  ExpandList big{P<int>(c->titems), P<int>(c->tcountb), m.dim == 2 ? m.V : 0};
+  ExpandList big{P<int>(c->titems), P<int>(c->tcountb), m.V};
+  int rc;
+  if (!c->tfac_ready) {
+    CK(cudaMemsetAsync(c->xcount.p, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->tcountb.p, 0, sizeof(int), c->stream));
+    if (!c->tfac_none) {
+      struct { DevBuf& b; size_t bytes; } need[] = {{c->tqc, sizeof(double) * tri_factor_planes() * (size_t)m.V},
+                                                    {c->trr, sizeof(double) * tri_r_planes() * (size_t)m.V},
+                                                    {c->tcode, (size_t)m.V}};
+      for (auto& n : need) {
+        if (!c->tfac_none && (rc = ensure(c, n.b, n.bytes))) {
+          if (rc != SPRG_ENOMEM) return rc;
+          cudaGetLastError();  // the failed allocation is no error of this call
+          c->tfac_none = true;
+        }
+      }
+    }
+    if (!c->tfac_none) {
+      PB("tri_factor_f64");
+      launch_tri_factor(m, TriFactor{P<double>(c->tqc), P<double>(c->trr), P<unsigned char>(c->tcode)}, xl, big,
+                        c->stream);
+      PE();
+      c->launches += 1;
+      if ((rc = check_launch(c, "triangle factors"))) return rc;
+      CK(cudaMemcpyAsync(c->txcount.p, c->xcount.p, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
+      CK(cudaMemcpyAsync(&c->n_tri_big, c->tcountb.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      c->tfac_ready = true;
+    }
+  } else if (c->n_tri_big) {
+    // the warp path appends its own growth patches behind the factors' ones
+    CK(cudaMemcpyAsync(c->xcount.p, c->txcount.p, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
+  }
+  const TriFactor tf{c->tfac_ready ? P<double>(c->tqc) : nullptr, P<double>(c->trr), P<unsigned char>(c->tcode)};
   PB("recover_f64");
-  launch_recover_f64(m, P<double>(c->ip), nc, P<double>(c->rec), xl, big, P<DevStatus>(c->status), c->stream);
+  launch_recover_f64(m, P<double>(c->ip), nc, P<double>(c->rec), tf, xl, big, !c->tfac_ready || c->n_tri_big > 0,
+                     c->stream);
   PE();
   c->launches += 1;
-  int rc = check_launch(c, "recover");
-  if (rc) return rc;
+  if ((rc = check_launch(c, "recover"))) return rc;
   // patches that need growth: the reference growth order, on the device
   return listed_fits(c, c->cache64, P<double>(c->ip), nullptr, nc, P<double>(c->rec), xl);
 }
@@ -753,6 +790,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   // and an adapt iteration changes the patch-size mix little
   c->tw_ready = false;
   c->qw_ready = false;
+  c->tfac_ready = c->tfac_none = false;
   c->egeo_ready = c->egeo_none = c->elen64_ready = c->elen64_none = false;
   c->vv_ready = false;
   c->cache64.valid = c->cache32.valid = c->cache2d.valid = false;
@@ -918,7 +956,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,

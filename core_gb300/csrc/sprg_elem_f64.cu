@@ -35,18 +35,6 @@ __device__ __forceinline__ void load_ids(const int* __restrict__ ev, int e, int*
   }
 }
 
-// a / b rounded to nearest, y = 1 / b rounded to nearest: two exact-residual
-// corrections of a y.  The first leaves a faithful quotient, the second
-// rounds it correctly (P. Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), given
-// that nothing under- or overflows (the callers' exponent checks).  Five
-// FP64 operations instead of a division each.
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-  double q = a * y;
-  q = fma(fma(-b, q, a), y, q);
-  return fma(fma(-b, q, a), y, q);
-}
-
 // One element's geometry: the rows of J^-1 (D columns each; the third column
 // of a triangle's pseudo-inverse is 0), dV = det J, and the longest edge
 // (apf::measure).  Record planes: J^-1 row-major (3 D planes), dV, h; plane
@@ -101,16 +89,16 @@ __device__ __forceinline__ void tet_record(const V3* x, double* out) {
   double det = m[0][0] * c0.v[0];
   det += m[1][0] * c0.v[1];
   det += m[2][0] * c0.v[2];
-  // an exponent check per quotient: the divisor in [2^-500, 2^500], the
-  // dividend 0 or in [2^-900, 2^500]
-  bool safe = bexp(det) >= 523 && bexp(det) <= 1523;
+  // an exponent check per quotient: the divisor in [2^-400, 2^400], the
+  // dividend 0 or in [2^-500, 2^500]
+  bool safe = bexp(det) >= 623 && bexp(det) <= 1423;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const double c[3] = {c0.v[k], c1.v[k], c2.v[k]};
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       const int ex = bexp(c[r]);
-      safe = safe && ex <= 1523 && (ex >= 123 || c[r] == 0.0);
+      safe = safe && ex <= 1523 && (ex >= 523 || c[r] == 0.0);
     }
   }
   double hh = 0;

@@ -98,10 +98,22 @@ void launch_measure_mark_f64(const DevMesh& m, const double* len, const double* 
 // ---- kernel launchers (sprg_kernels_f64.cu) ---------------------------
 // Triangles (tets recover through launch_qr_weights / launch_recover_w64):
 // xl: patches that need growth; big: patches above the thread-per-vertex
-// size (fitted by the warp path inside this call; its counter must be zero
-// on entry)
-void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, ExpandList xl, ExpandList big,
-                        DevStatus* st, cudaStream_t s);
+// size (fitted by the warp path inside launch_recover_f64, which may add to
+// xl).  The factors of the thread path's patches are per mesh: qc
+// tri_factor_planes() and rr tri_r_planes() planes of V doubles, code V
+// bytes; launch_tri_factor fills them and both lists (counters zero on
+// entry).  qc null: launch_recover_f64 factors in place and fills the lists
+// itself.  any_big: the big list may hold vertices.
+struct TriFactor {
+  double* qc;
+  double* rr;
+  unsigned char* code;
+};
+int tri_factor_planes();
+int tri_r_planes();
+void launch_tri_factor(const DevMesh& m, TriFactor tf, ExpandList xl, ExpandList big, cudaStream_t s);
+void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, TriFactor tf, ExpandList xl,
+                        ExpandList big, bool any_big, cudaStream_t s);
 // Patches on the expansion list: grow as the reference does, then fit.
 // The list length is read on the device (no host round trip).
 // slab: expand_grid() * expand_max_elems() * (4 + nc + 1) doubles.

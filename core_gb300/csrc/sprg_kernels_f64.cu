@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_list(DevMesh m, const double
 
 // ---------------------------------------------------------------------
 // spr::recoverField on triangles -- one thread per vertex for patches of
-// NT..MAXM elements, in the reference's own operation order
+// NT..kTriThreadRows elements, in the reference's own operation order
 // (mth/mthQR.cc:19-160, spr/sprRecoverField.cc:226-353):
 //   get_reflector      column norm from row k down, the 1e-10 rank test,
 //                      v = column + sgn * norm at k, v /= |v|;
@@ -236,30 +236,24 @@ __global__ void __launch_bounds__(kBlock) k_recover_list(DevMesh m, const double
 // are bitwise those of that sequence.  Patches with fewer than NT elements
 // or rank deficient go to the expansion list, larger ones to `big` (the
 // warp path).
+//
+// Q's columns and R depend on the mesh alone: k_tri_factor keeps them (planes
+// over the vertices: entry (r, i) of Q in plane 3 r + i, the upper triangle
+// of R row by row, then the rounded reciprocals of its diagonal) and every
+// recovery starts from them.
 // ---------------------------------------------------------------------
-template <int NC, int MAXM>
-__global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __restrict__ ip,
-                                                     double* __restrict__ rec, ExpandList xl, ExpandList big) {
+constexpr int kTriR = 9;               // planes of R: 6 entries, 3 reciprocals
+constexpr unsigned char kTriPlain = 64;  // flag of a factor that takes plain divisions and sums
+
+template <int MAXM>
+__device__ __forceinline__ bool tri_factor(const DevMesh& m, int beg, int cnt, double Qc[MAXM][3], double* Rr) {
   constexpr int NT = 3;
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= m.V) return;
-  const int beg = m.p_off[v];
-  const int cnt = m.p_off[v + 1] - beg;
-  if (cnt < NT || cnt > MAXM) {
-    const ExpandList& l = cnt < NT ? xl : big;
-    const int slot = atomicAdd(l.count, 1);
-    if (slot < l.cap) l.items[slot] = v;
-    return;
-  }
-  int el[MAXM];
   double R[MAXM][NT];
 #pragma unroll
   for (int i = 0; i < MAXM; ++i) {
-    el[i] = 0;
     R[i][0] = R[i][1] = R[i][2] = 0;
     if (i < cnt) {
-      el[i] = m.p_el[beg + i];
-      const V3 p = elem_ip_point(m, el[i]);
+      const V3 p = elem_ip_point(m, m.p_el[beg + i]);
       R[i][0] = 1.0;
       R[i][1] = p.v[0];
       R[i][2] = p.v[1];
@@ -273,11 +267,7 @@ __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __
     for (int i = k; i < MAXM; ++i)
       if (i < cnt) cn += R[i][k] * R[i][k];
     cn = sqrt(cn);
-    if (cn < 1e-10) {
-      const int slot = atomicAdd(xl.count, 1);
-      if (slot < xl.cap) xl.items[slot] = v;
-      return;
-    }
+    if (cn < 1e-10) return false;
 #pragma unroll
     for (int i = 0; i < MAXM; ++i) H[k][i] = (i >= k && i < cnt) ? R[i][k] : 0.0;
     H[k][k] += ((R[k][k] < 0) ? -1 : 1) * cn;
@@ -301,7 +291,6 @@ __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __
     }
   }
   // the first NT columns of Q, row by row
-  double Qc[MAXM][NT];
 #pragma unroll
   for (int r = 0; r < MAXM; ++r) {
     double q[MAXM];
@@ -320,30 +309,128 @@ __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __
 #pragma unroll
     for (int i = 0; i < NT; ++i) Qc[r][i] = q[i];
   }
-  const V3 xv = load_xyz(m.xyz, v);
-#pragma unroll 1
-  for (int c = 0; c < NC; ++c) {
-    double y[NT] = {0, 0, 0};
+  Rr[0] = R[0][0]; Rr[1] = R[0][1]; Rr[2] = R[0][2];
+  Rr[3] = R[1][1]; Rr[4] = R[1][2]; Rr[5] = R[2][2];
+  return true;
+}
+
+__device__ __forceinline__ void list_append(const ExpandList& l, int v) {
+  const int slot = atomicAdd(l.count, 1);
+  if (slot < l.cap) l.items[slot] = v;
+}
+
+// per mesh: code[v] = the patch size, with kTriPlain where a value is not
+// finite or R's diagonal lies outside [2^-400, 2^400]; 0: listed
+template <int MAXM>
+__global__ void __launch_bounds__(128) k_tri_factor(DevMesh m, double* __restrict__ qc, double* __restrict__ rr,
+                                                    unsigned char* __restrict__ code, ExpandList xl, ExpandList big) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= m.V) return;
+  const int beg = m.p_off[v];
+  const int cnt = m.p_off[v + 1] - beg;
+  double Qc[MAXM][3], R[6];
+  if (cnt < 3 || cnt > MAXM || !tri_factor<MAXM>(m, beg, cnt, Qc, R)) {
+    code[v] = 0;
+    list_append(cnt > MAXM ? big : xl, v);
+    return;
+  }
+  bool plain = false;
 #pragma unroll
-    for (int r = 0; r < MAXM; ++r)
-      if (r < cnt) {
-        const double b = ip[(size_t)el[r] * NC + c];
+  for (int r = 0; r < MAXM; ++r)
+    if (r < cnt)
 #pragma unroll
-        for (int i = 0; i < NT; ++i) y[i] += Qc[r][i] * b;
+      for (int i = 0; i < 3; ++i) {
+        qc[(size_t)(3 * r + i) * m.V + v] = Qc[r][i];
+        plain = plain || bexp(Qc[r][i]) == 0x7ff;
       }
-    double x[NT];
 #pragma unroll
-    for (int ii = 0; ii < NT; ++ii) {
-      const int i = NT - ii - 1;
-      x[i] = y[i];
+  for (int i = 0; i < 6; ++i) {
+    rr[(size_t)i * m.V + v] = R[i];
+    plain = plain || bexp(R[i]) == 0x7ff;
+  }
+  const double diag[3] = {R[0], R[3], R[5]};
 #pragma unroll
-      for (int j = i + 1; j < NT; ++j) x[i] -= R[i][j] * x[j];
-      x[i] /= R[i][i];
+  for (int i = 0; i < 3; ++i) {
+    plain = plain || bexp(diag[i]) < 623 || bexp(diag[i]) > 1423;
+    rr[(size_t)(6 + i) * m.V + v] = __drcp_rn(diag[i]);
+  }
+  code[v] = (unsigned char)(cnt | (plain ? kTriPlain : 0));
+}
+
+// y / R_ii of the back substitution, bitwise the division
+__device__ __forceinline__ double tri_div(double a, double b, double y, bool plain) {
+  const int e = bexp(a);
+  if (plain || e < 523 || e > 1523) return a / b;
+  return quotient(a, b, y);
+}
+
+// The recovery from the factors (CACHED), or with the factors computed in
+// place where there is no memory for them.  Samples that are 0 leave the
+// sums as they are (a planar mesh's z components), and a component whose
+// sums are all 0 is 0.  FP64-rate bound: about 60 operations a component that
+// is not 0; both recoveries of a 1024^2 square's anisotropic pass took
+// 6.65 ms with the QR in every call, 1.30 ms from the factors.
+template <int NC, int MAXM, bool CACHED>
+__global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __restrict__ ip,
+                                                     const double* __restrict__ qc, const double* __restrict__ rr,
+                                                     const unsigned char* __restrict__ code,
+                                                     double* __restrict__ rec, ExpandList xl, ExpandList big) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= m.V) return;
+  const int beg = m.p_off[v];
+  int cnt;
+  bool plain = true;
+  double Qc[CACHED ? 1 : MAXM][3], R[kTriR];
+  if constexpr (CACHED) {
+    const int cd = code[v];
+    if (cd == 0) return;
+    cnt = cd & (kTriPlain - 1);
+    plain = (cd & kTriPlain) != 0;
+#pragma unroll
+    for (int i = 0; i < kTriR; ++i) R[i] = __ldcs(rr + (size_t)i * m.V + v);
+  } else {
+    cnt = m.p_off[v + 1] - beg;
+    if (cnt < 3 || cnt > MAXM || !tri_factor<MAXM>(m, beg, cnt, Qc, R)) {
+      list_append(cnt > MAXM ? big : xl, v);
+      return;
     }
+    R[6] = R[7] = R[8] = 0;
+  }
+  double y[NC][3];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) y[c][0] = y[c][1] = y[c][2] = 0;
+#pragma unroll
+  for (int r = 0; r < MAXM; ++r) {
+    if (r >= cnt) break;
+    const double* b = ip + (size_t)m.p_el[beg + r] * NC;
+    double q[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if constexpr (CACHED) q[i] = __ldcs(qc + (size_t)(3 * r + i) * m.V + v);
+      else q[i] = Qc[r][i];
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double bc = __ldg(b + c);
+      if (plain || (__double_as_longlong(bc) << 1) != 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) y[c][i] += q[i] * bc;
+      }
+    }
+  }
+  const V3 xv = load_xyz(m.xyz, v);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
     double sres = 0;
-    sres += x[0] * 1.0;
-    sres += x[1] * xv.v[0];
-    sres += x[2] * xv.v[1];
+    const long long any = __double_as_longlong(y[c][0]) | __double_as_longlong(y[c][1]) | __double_as_longlong(y[c][2]);
+    if (plain || any != 0) {
+      const double x2 = tri_div(y[c][2], R[5], R[8], plain);
+      const double x1 = tri_div(y[c][1] - R[4] * x2, R[3], R[7], plain);
+      const double x0 = tri_div(y[c][0] - R[1] * x1 - R[2] * x2, R[0], R[6], plain);
+      sres += x0 * 1.0;
+      sres += x1 * xv.v[0];
+      sres += x2 * xv.v[1];
+    }
     rec[(size_t)v * NC + c] = sres;
   }
 }
@@ -2378,20 +2465,27 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
 // ----------------------------------------------------------------------
 // launchers
 // ----------------------------------------------------------------------
-void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, ExpandList xl, ExpandList big,
-                        DevStatus* st, cudaStream_t s) {
-  (void)st;
+int tri_factor_planes() { return 3 * kTriThreadRows; }
+int tri_r_planes() { return kTriR; }
+
+void launch_tri_factor(const DevMesh& m, TriFactor tf, ExpandList xl, ExpandList big, cudaStream_t s) {
+  if (m.V) k_tri_factor<kTriThreadRows><<<(m.V + 127) / 128, 128, 0, s>>>(m, tf.qc, tf.rr, tf.code, xl, big);
+}
+
+void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, TriFactor tf, ExpandList xl,
+                        ExpandList big, bool any_big, cudaStream_t s) {
   if (!m.V || m.dim != 2) return;  // tets recover through the per-mesh QR weights
   // triangles: a thread per vertex up to kTriThreadRows patch elements, then
   // the warp path over the vertices it listed
   const int grid = (m.V + 127) / 128;
   const int lgrid = 152 * 8;
+  auto go = [&](auto kernel) { kernel<<<grid, 128, 0, s>>>(m, ip, tf.qc, tf.rr, tf.code, rec, xl, big); };
   if (nc == 3) {
-    k_recover_tri<3, kTriThreadRows><<<grid, 128, 0, s>>>(m, ip, rec, xl, big);
-    k_recover_list<3, 3, 1><<<lgrid, kBlock, 0, s>>>(m, ip, rec, xl, big);
+    go(tf.qc ? k_recover_tri<3, kTriThreadRows, true> : k_recover_tri<3, kTriThreadRows, false>);
+    if (any_big) k_recover_list<3, 3, 1><<<lgrid, kBlock, 0, s>>>(m, ip, rec, xl, big);
   } else {
-    k_recover_tri<9, kTriThreadRows><<<grid, 128, 0, s>>>(m, ip, rec, xl, big);
-    k_recover_list<3, 9, 1><<<lgrid, kBlock, 0, s>>>(m, ip, rec, xl, big);
+    go(tf.qc ? k_recover_tri<9, kTriThreadRows, true> : k_recover_tri<9, kTriThreadRows, false>);
+    if (any_big) k_recover_list<3, 9, 1><<<lgrid, kBlock, 0, s>>>(m, ip, rec, xl, big);
   }
 }
 

@@ -7,6 +7,19 @@ namespace sprg {
 
 __device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
+// a / b rounded to nearest, y = 1 / b rounded to nearest: two exact-residual
+// corrections of a y.  The first leaves a faithful quotient, the second
+// rounds it correctly (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), given
+// that nothing under- or overflows (the callers check exponents: b in
+// [2^-400, 2^400], a 0 or in [2^-500, 2^500]).  Five FP64 operations instead
+// of a division each.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q, a), y, q);
+}
+
 // 2-point Gauss, the reference's own sequence
 __device__ __forceinline__ double metric_length(const ref::V3& x0, const ref::V3& x1, const double* hv,
                                                 const double* Rv) {

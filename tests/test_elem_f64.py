@@ -16,6 +16,8 @@ def mesh(oracle_lib, n, nz, kind):
         x *= 2.0 ** -172
     elif kind == "huge":      # above 2^500
         x *= 2.0 ** 170
+    elif kind == "edge":      # determinants around 2^-400, cofactors around 2^-267
+        x *= 2.0 ** -132
     elif kind == "stretched":
         x[:, 0] *= 1e-40
         x[:, 1] *= 1e30
@@ -31,7 +33,7 @@ def mesh(oracle_lib, n, nz, kind):
     return m, o
 
 
-MESHES = [(1, 1, "plain"), (5, 4, "plain"), (9, 11, "plain"), (4, 4, "tiny"), (4, 4, "huge"), (4, 3, "stretched"),
+MESHES = [(1, 1, "plain"), (5, 4, "plain"), (9, 11, "plain"), (4, 4, "tiny"), (4, 4, "edge"), (4, 4, "huge"), (4, 3, "stretched"),
           (4, 4, "degenerate"), (3, 3, "inf"), (1, 0, "plain"), (13, 0, "plain"), (6, 0, "tiny"), (6, 0, "degenerate")]
 
 
@@ -147,3 +149,55 @@ def test_pass_marks_are_those_of_the_bitwise_lengths(gpu_lib, oracle_lib, n, in_
         assert np.abs(L1 - threshold).min() < 1e-9
         assert np.array_equal((flags & 1) != 0, L1 > 1.5) and np.array_equal((flags & 4) != 0, L1 < 0.5)
         assert (ns, nc) == (int((L1 > 1.5).sum()), int((L1 < 0.5).sum()))
+
+
+@pytest.mark.parametrize("n,kind", [(2, "plain"), (15, "plain"), (15, "warped"), (6, "tiny"), (6, "huge"), (9, "fan")])
+@pytest.mark.parametrize("nc", [3, 9])
+def test_triangle_recovery_bitwise(gpu_lib, oracle_lib, n, kind, nc):
+    """Patches of 3 to 8 triangles, from the kept factors (twice, the second
+    call on other samples) and factored in place; components that are 0
+    everywhere, zero and infinite samples."""
+    import core_gb300 as cg
+    m, o = mesh(oracle_lib, n, 0, "plain")
+    if kind == "warped":
+        m.coords[:, 2] = np.sin(3 * m.coords[:, 0])
+    elif kind in ("tiny", "huge"):
+        # R's diagonal out of the fast quotients' range for huge; a tiny mesh is rank deficient below 1e-10
+        m.coords *= 2.0 ** (401 if kind == "huge" else -20)
+    elif kind == "fan":  # patches above 8 elements: every triangle of a block shares one vertex
+        ev = m.elem_verts
+        for t in range(20):
+            if 40 not in ev[t]:
+                ev[t][2] = 40
+        m.v2e_off = m.v2e = None
+    if kind == "fan":
+        down = np.unique(np.sort(np.concatenate([m.elem_verts[:, [0, 1]], m.elem_verts[:, [1, 2]], m.elem_verts[:, [0, 2]]]), 1), axis=0)
+        m.edge_verts = np.ascontiguousarray(down, np.int32)
+    else:
+        o.set_coords(m.coords)
+    cnt = np.bincount(m.elem_verts.reshape(-1), minlength=m.n_verts)
+    thread = (cnt >= 3) & (cnt <= 8)
+    rng = np.random.default_rng(8)
+    ips = [rng.normal(size=(m.n_elems, nc)) for _ in range(2)]
+    ips[0][:, 2::3] = 0.0
+    ips[1][::7, 0] = 0.0
+    ips[1][3, 1] = np.inf
+
+    def answers(in_place):
+        with cg.Context(m) as c:
+            if in_place:  # the ninth allocation of the first call is the factors'
+                c.test_hooks(alloc_fail_after=8)
+                with pytest.raises(cg.SprgError):
+                    c.recoverField(ips[0])
+                c.test_hooks()
+            return [c.recoverField(ip) for ip in ips]
+    kept, placed = answers(False), answers(True)
+    for a, b in zip(kept, placed):
+        assert np.array_equal(a, b, equal_nan=True)
+    if kind == "fan":
+        assert cnt.max() > 8
+        return
+    for ip, got in zip(ips, kept):
+        rc, want, _, _ = o.recover(ip)
+        assert rc == 0
+        assert np.array_equal(got[thread], want[thread], equal_nan=True)
