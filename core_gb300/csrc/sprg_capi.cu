@@ -1120,7 +1120,8 @@ int sprg_measure_edges_aniso(sprg_ctx* c, const double* sizes, const double* fra
   ENSURE(c->L, sizeof(double) * (size_t)m.E);
   CK(cudaMemcpyAsync(c->sizes3.p, sizes, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->frames9.p, frames, sizeof(double) * 9 * (size_t)m.V, cudaMemcpyHostToDevice, c->stream));
-  launch_measure_aniso_f64(m, P<double>(c->sizes3), P<double>(c->frames9), P<double>(c->L), c->stream);
+  launch_measure_aniso_f64(m, P<double>(c->sizes3), P<double>(c->frames9), P<double>(c->L), nullptr, nullptr,
+                           c->stream);
   c->launches += 1;
   rc = check_launch(c, "measure aniso");
   if (rc) return rc;
@@ -2517,12 +2518,10 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
                         c->stream);
   PE();
   PB("measure_aniso_f64");
-  launch_measure_aniso_f64(m, P<double>(c->sizes3), P<double>(c->frames9), P<double>(c->L), c->stream);
+  launch_measure_aniso_f64(m, P<double>(c->sizes3), P<double>(c->frames9), P<double>(c->L), d_split_bits,
+                           d_collapse_bits, c->stream);
   PE();
-  PB("mark_bits");
-  launch_mark_bits(m.E, P<double>(c->L), d_split_bits, d_collapse_bits, c->stream);
-  PE();
-  c->launches += 3;
+  c->launches += 2;
   if (d_quality) {
     PB("quality_f64");
     launch_quality_f64(m, nullptr, P<double>(c->sizes3), P<double>(c->frames9), d_quality, c->stream);

@@ -143,12 +143,12 @@ int expand_grid();
 // Sum partials in fixed order, compute size factor.  mode 0: SPR; 1: target.
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target,
                         int dim, double* out3, cudaStream_t s);
-void launch_measure_aniso_f64(const DevMesh& m, const double* sizes, const double* frames, double* L,
-                              cudaStream_t s);
+// split / collapse (optional): the predicate bitmaps of the lengths, bit e of
+// split = L[e] > 1.5, of collapse = L[e] < 0.5
+void launch_measure_aniso_f64(const DevMesh& m, const double* sizes, const double* frames, double* L, uint32_t* split,
+                              uint32_t* collapse, cudaStream_t s);
 void launch_mark(int E, const double* L, int which, int* flags, unsigned long long* count, DevStatus* st,
                  cudaStream_t s);
-// predicate bitmaps: bit e of split = L[e] > 1.5, of collapse = L[e] < 0.5
-void launch_mark_bits(int E, const double* L, uint32_t* split, uint32_t* collapse, cudaStream_t s);
 // markEntities semantics from a predicate bitmap
 void launch_apply_bits(int E, const uint32_t* bits, int which, int* flags, unsigned long long* count,
                        DevStatus* st, cudaStream_t s);

@@ -78,4 +78,106 @@ __device__ __forceinline__ double iso_length(const ref::V3& x0, const ref::V3& x
   return L;
 }
 
+// ---- anisotropic transforms -------------------------------------------
+__device__ __forceinline__ bool all_zero(double a, double b, double c, double d) {
+  return ((__double_as_longlong(a) | __double_as_longlong(b) | __double_as_longlong(c) | __double_as_longlong(d)) << 1) ==
+         0;
+}
+// a size whose reciprocal is an ordinary number (the products with 0 that the
+// transform leaves out are then 0)
+__device__ __forceinline__ bool ordinary(double h) { return (unsigned)(bexp(h) - 523) <= 1000u; }
+
+// AnisoSizeField's Q = orth(R) diag(1/h) (ma/maSize.cc:94-117, 395-412) for an
+// interpolated frame R and ordinary sizes h, bitwise: the products with the
+// diagonal matrix's zeros are left out
+__device__ __forceinline__ ref::M3 transform_of(const double* h, const ref::M3& R) {
+  ref::M3 Q = ref::orthogonalize(R);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double ih = 1 / h[j];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Q.m[i][j] *= ih;
+  }
+  return Q;
+}
+
+// the same where the third row and column are (0, 0, .): the 2 x 2 block q =
+// {Q00, Q01, Q10, Q11}, and the third direction's z (1/h2 not applied)
+__device__ __forceinline__ double planar_transform(double h0, double h1, double a, double b, double c, double d,
+                                                   double* q) {
+  // first column (a, c), second (b, d)
+  const double n0 = sqrt(a * a + c * c);
+  const double r0x = a / n0, r0y = c / n0;
+  const double t = r0x * b + r0y * d;
+  const double x = b - r0x * t, y = d - r0y * t;
+  const double n1 = sqrt(x * x + y * y);
+  const double r1x = x / n1, r1y = y / n1;
+  const double i0 = 1 / h0, i1 = 1 / h1;
+  q[0] = r0x * i0;
+  q[1] = r1x * i1;
+  q[2] = r0y * i0;
+  q[3] = r1y * i1;
+  return r0x * r1y - r0y * r1x;
+}
+
+static __device__ __noinline__ double aniso_length_ref(const ref::V3& x0, const ref::V3& x1, const double* hv,
+                                                       const double* Rv) {
+  return metric_length(x0, x1, hv, Rv);
+}
+
+// AnisoSizeField's length of an edge, bitwise metric_length: half the edge
+// vector is taken once at the end (a power of two), products with the fixed
+// zeros are left out, and an edge and frames in a z = const plane take the
+// 2 x 2 block alone: about 250 FP64 operations, or 390 in space, against 550.
+// Sizes or a length outside the ordinary range take the sequence itself.
+__device__ __forceinline__ double aniso_length(const ref::V3& x0, const ref::V3& x1, const double* hv,
+                                               const double* Rv) {
+  const double gp[2] = {0.577350269189626, -0.577350269189626};
+  const ref::V3 d = ref::sub(x1, x0);
+  bool fine = true;
+  double s[2];
+  if (all_zero(Rv[2], Rv[5], Rv[6], Rv[7]) && all_zero(Rv[11], Rv[14], Rv[15], Rv[16]) && d.v[2] == 0.0) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      double N[2], q[4];
+      ref::edge_shape_values(gp[p], N);
+      const double h0 = hv[0] * N[0] + hv[3] * N[1], h1 = hv[1] * N[0] + hv[4] * N[1],
+                   h2 = hv[2] * N[0] + hv[5] * N[1];
+      fine = fine && ordinary(h0) && ordinary(h1) && ordinary(h2);
+      planar_transform(h0, h1, Rv[0] * N[0] + Rv[9] * N[1], Rv[1] * N[0] + Rv[10] * N[1], Rv[3] * N[0] + Rv[12] * N[1],
+                       Rv[4] * N[0] + Rv[13] * N[1], q);
+      const double a = d.v[0] * q[0] + d.v[1] * q[2], b = d.v[0] * q[1] + d.v[1] * q[3];
+      s[p] = sqrt(a * a + b * b);
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      double N[2], h[3];
+      ref::edge_shape_values(gp[p], N);
+      ref::M3 R;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        h[k] = hv[k] * N[0] + hv[3 + k] * N[1];
+        fine = fine && ordinary(h[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 9; ++k) R.m[k / 3][k % 3] = Rv[k] * N[0] + Rv[9 + k] * N[1];
+      const ref::M3 Q = transform_of(h, R);
+      ref::V3 e;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        double t = d.v[0] * Q.m[0][j];
+        t += d.v[1] * Q.m[1][j];
+        t += d.v[2] * Q.m[2][j];
+        e.v[j] = t;
+      }
+      s[p] = ref::len(e);
+    }
+  }
+  const double L = 0.5 * (s[0] + s[1]);
+  const int el = bexp(L);
+  if (!fine || el < 623 || el > 1423) return aniso_length_ref(x0, x1, hv, Rv);
+  return L;
+}
+
 }  // namespace sprg

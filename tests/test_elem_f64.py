@@ -201,3 +201,48 @@ def test_triangle_recovery_bitwise(gpu_lib, oracle_lib, n, kind, nc):
         rc, want, _, _ = o.recover(ip)
         assert rc == 0
         assert np.array_equal(got[thread], want[thread], equal_nan=True)
+
+
+def metric_of(m, kind, seed=9):
+    """sizes and frames: rotations in the plane (2D) or in space, slightly
+    off orthonormal; odd: sizes and frames the fast forms hand over."""
+    rng = np.random.default_rng(seed)
+    V = m.n_verts
+    sizes = np.exp(rng.uniform(np.log(0.02), np.log(0.4), (V, 3)))
+    if m.dim == 2 and kind != "space":
+        t = rng.uniform(0, np.pi, V)
+        F = np.zeros((V, 3, 3))
+        F[:, 0, 0], F[:, 0, 1], F[:, 1, 0], F[:, 1, 1], F[:, 2, 2] = np.cos(t), -np.sin(t), np.sin(t), np.cos(t), 1.0
+        if kind == "skew":
+            F[:, :2, :2] *= rng.uniform(0.5, 2.0, (V, 2, 2))
+    else:
+        F = np.linalg.qr(rng.normal(size=(V, 3, 3)))[0] * rng.uniform(0.5, 2.0, (V, 1, 1))
+    if kind == "odd":
+        sizes[::6] = 0.0
+        sizes[1::11] = np.inf
+        sizes[2::13] = -sizes[2::13]
+        sizes[3::17] = 5e-324
+        sizes[4::19] = 1e200
+        F[::7] = 0.0
+        F[5::23, 0, 0] = np.nan
+    return sizes, np.ascontiguousarray(F.reshape(V, 9))
+
+
+@pytest.mark.parametrize("n,nz", [(1, 1), (5, 4), (1, 0), (12, 0)])
+@pytest.mark.parametrize("kind", ["plain", "skew", "space", "odd"])
+def test_metric_lengths_and_qualities_bitwise(gpu_lib, oracle_lib, n, nz, kind):
+    import core_gb300 as cg
+    m, o = mesh(oracle_lib, n, nz, "plain")
+    if kind == "skew" and m.dim == 2:
+        m.coords[:, 2] = 0.75  # in a plane, but not z = 0
+        o.set_coords(m.coords)
+    sizes, F = metric_of(m, kind)
+    with cg.Context(m) as c:
+        L = o.measure(sizes=sizes, frames=F)
+        assert np.array_equal(c.measure_edges_aniso(sizes, F), L, equal_nan=True)
+        assert np.array_equal(c.measure_vertex_pairs(m.edge_verts, sizes=sizes, frames=F), L, equal_nan=True)
+        assert np.array_equal(c.measureQuality(sizes=sizes, frames=F), o.quality(sizes=sizes, frames=F), equal_nan=True)
+        iso = np.ascontiguousarray(sizes[:, 0])
+        assert np.array_equal(c.measureQuality(iso), o.quality(iso), equal_nan=True)
+        iso[:] = 0.3  # every vertex alike
+        assert np.array_equal(c.measureQuality(iso), o.quality(iso), equal_nan=True)
