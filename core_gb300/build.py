@@ -23,6 +23,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.pat
 UNITS = {
     "sprg_kernels_f64.cu": ["-fmad=false"],
     "sprg_elem_f64.cu": ["-fmad=false"],
+    "sprg_quality_f64.cu": ["-fmad=false"],
     "sprg_kernels_f32.cu": [],
     "sprg_capi.cu": [],
     "sprg_noalloc.cu": [],

@@ -66,6 +66,7 @@ struct sprg_ctx {
   bool tfac_ready = false, tfac_none = false;
   int n_tri_big = 0;
   DevBuf Lx, pairs, red, eflags;  // MA sweeps: lengths, vertex pairs, reduction scratch, element flags
+  DevBuf vxf, vbad;               // the vertices' metric transforms of the quality kernels
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
   // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
   // egeo_none: there was no memory for them, the kernels compute in place
@@ -615,6 +616,24 @@ int fill_info(sprg_ctx* c, sprg_size_info* info) {
   return info_from_stage(c, info);
 }
 
+// FP64 qualities into q on the context stream; the vertices' transforms need
+// 81 bytes a vertex, without which they are computed per element
+int step_quality(sprg_ctx* c, const double* size, const double* sizes, const double* frames, const double* logm,
+                 double* q) {
+  DevMesh& m = c->m;
+  double* xf = nullptr;
+  if (!size) {
+    int rc = ensure(c, c->vxf, vertex_transform_bytes(m.V));
+    if (rc == SPRG_OK) rc = ensure(c, c->vbad, (size_t)m.V);
+    if (rc == SPRG_OK) xf = P<double>(c->vxf);
+    else if (rc != SPRG_ENOMEM) return rc;
+    else cudaGetLastError();  // the failed allocation is no error of this call
+  }
+  launch_quality_f64(m, size, sizes, frames, logm, xf, P<unsigned char>(c->vbad), q, P<DevStatus>(c->status), c->stream);
+  c->launches += xf ? 2 : 1;
+  return check_launch(c, "quality");
+}
+
 int upload_ip(sprg_ctx* c, const double* ip, int ncomp) {
   if (ncomp != 3 && ncomp != 9) return fail(c, SPRG_EINVAL, "ip field must have 3 or 9 components");
   if (ip) {
@@ -956,7 +975,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,
@@ -1195,9 +1214,7 @@ int sprg_measure_quality(sprg_ctx* c, const double* size, const double* sizes, c
     }
     dsize = P<double>(c->size);
   }
-  launch_quality_f64(m, dsize, dsizes, dframes, P<double>(c->q), c->stream);
-  c->launches += 1;
-  rc = check_launch(c, "quality");
+  rc = step_quality(c, dsize, dsizes, dframes, nullptr, P<double>(c->q));
   if (rc) return rc;
   c->q_valid = true;
   CK(cudaMemcpyAsync(q, c->q.p, sizeof(double) * (size_t)m.T, cudaMemcpyDeviceToHost, c->stream));
@@ -1345,9 +1362,7 @@ int sprg_measure_quality_log_aniso(sprg_ctx* c, const double* sizes, const doubl
   if ((rc = reset_status(c))) return rc;
   if ((rc = size_field_inputs(c, SPRG_SIZE_LOG_ANISO, nullptr, sizes, frames, &ds, &dss, &dff, &dlm))) return rc;
   ENSURE(c->q, sizeof(double) * (size_t)(m.T > 0 ? m.T : 1));
-  launch_quality_f64(m, nullptr, nullptr, nullptr, P<double>(c->q), c->stream, dlm, P<DevStatus>(c->status));
-  c->launches += 1;
-  if ((rc = check_launch(c, "quality log-aniso"))) return rc;
+  if ((rc = step_quality(c, nullptr, nullptr, nullptr, dlm, P<double>(c->q)))) return rc;
   if ((rc = sync_and_status(c))) return rc;
   c->q_valid = true;
   CK(cudaMemcpy(q, c->q.p, sizeof(double) * (size_t)m.T, cudaMemcpyDeviceToHost));
@@ -2524,9 +2539,8 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   c->launches += 2;
   if (d_quality) {
     PB("quality_f64");
-    launch_quality_f64(m, nullptr, P<double>(c->sizes3), P<double>(c->frames9), d_quality, c->stream);
+    if ((rc = step_quality(c, nullptr, P<double>(c->sizes3), P<double>(c->frames9), nullptr, d_quality))) return rc;
     PE();
-    c->launches += 1;
   }
   c->L_valid = true;
   c->size_valid = false;

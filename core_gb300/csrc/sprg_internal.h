@@ -255,8 +255,13 @@ void launch_guard_stage(int stage, const DevMesh& m, const double* u, const doub
                         GuardScratch g, BatchView bv, cudaStream_t s);
 // per-mesh size factors of a batch (SPR mode) from segment partials
 void launch_size_factor_batch(const double* partials, BatchView bv, int dim, double* out4, cudaStream_t s);
+// FP64 qualities (sprg_quality_f64.cu) under the field `size` (isotropic),
+// `sizes` and `frames`, or the log-metrics `logm`; xf / bad:
+// vertex_transform_bytes(V) and V bytes of scratch for the vertices'
+// transforms (null: computed per element), not used for the isotropic field
+size_t vertex_transform_bytes(int V);
 void launch_quality_f64(const DevMesh& m, const double* size, const double* sizes, const double* frames,
-                        double* q, cudaStream_t s, const double* logm = nullptr, DevStatus* st = nullptr);
+                        const double* logm, double* xf, unsigned char* bad, double* q, DevStatus* st, cudaStream_t s);
 // anisotropic metric (sizes V x 3, frames V x 9) from a nodal Hessian (V x 9)
 void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double hmin, double hmax, double* sizes,
                            double* frames, cudaStream_t s);

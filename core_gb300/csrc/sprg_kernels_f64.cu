@@ -827,9 +827,6 @@ __device__ __forceinline__ double edge_measure(const V3& x0, const V3& x1) {
   return r;
 }
 
-__constant__ int c_tet_edges[6][2] = {{0, 1}, {1, 2}, {2, 0}, {0, 3}, {1, 3}, {2, 3}};
-__constant__ int c_tri_edges[3][2] = {{0, 1}, {1, 2}, {2, 0}};
-
 // AnisoSizeField lengths, with the predicate bitmaps where they are asked for.
 // FP64-rate bound: 1.35 ms for the 3.1M edges of a 1024^2 square (2.77 ms with
 // the general 3 x 3 sequence, plus 0.02 ms for marking from the stored lengths).
@@ -987,70 +984,6 @@ __global__ void __launch_bounds__(kBlock) k_apply_marks(int E, const uint32_t* _
   }
   block_count2(counts, ms, counts + 1, mc);
 }
-
-// measureTetQuality / measureTriQuality, useMax = true (ma/maQuality.cc:83-167)
-__device__ __forceinline__ double q_measure(const V3* x, int nn, int edim, const M3& Q) {
-  M3 J = ref::jacobian(x, nn, edim);
-  double w = edim == 3 ? 1.0 / 6.0 : (edim == 2 ? 1.0 / 2.0 : 2.0);
-  double dV2 = ref::jacobian_det(ref::mul(J, Q), edim);
-  double measurement = 0;
-  measurement += w * dV2;
-  return measurement;
-}
-
-template <bool LOG>
-__global__ void __launch_bounds__(kBlock) k_quality(DevMesh m, const double* __restrict__ size,
-                                                    const double* __restrict__ sizes,
-                                                    const double* __restrict__ frames,
-                                                    const double* __restrict__ logm, double* __restrict__ q,
-                                                    DevStatus* st) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.T) return;
-  const int* ev = m.ev + (size_t)e * m.nn;
-  M3 Q;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) Q.m[i][j] = 0;
-  double maxJ = -1.0;
-  for (int i = 0; i < m.nn; ++i) {
-    int v = ev[i];
-    double hv[3], Rv[9], N[1] = {1.0};
-    M3 cQ;
-    if (LOG) {  // LogAnisoSizeField: the vertex's own log-metric
-      bool ok = true;
-      cQ = ref::log_transform(logm + 9 * (size_t)v, N, 1, &ok);
-      if (!ok) set_status(st, SPRG_EEIGEN, e);
-    } else {
-      if (size) { hv[0] = hv[1] = hv[2] = size[v]; identity9(Rv); }
-      else {
-        for (int k = 0; k < 3; ++k) hv[k] = sizes[3 * (size_t)v + k];
-        for (int k = 0; k < 9; ++k) Rv[k] = frames[9 * (size_t)v + k];
-      }
-      cQ = ref::get_transform(hv, Rv, N, 1);
-    }
-    double cJ = ref::jacobian_det(cQ, m.dim);
-    if (cJ > maxJ) { maxJ = cJ; Q = cQ; }
-  }
-  V3 x[4];
-  for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-  double s = 0;
-  for (int i = 0; i < m.ne_el; ++i) {
-    int p = m.dim == 3 ? c_tet_edges[i][0] : c_tri_edges[i][0];
-    int r = m.dim == 3 ? c_tet_edges[i][1] : c_tri_edges[i][1];
-    V3 xe[2] = {x[p], x[r]};
-    double l = q_measure(xe, 2, 1, Q);
-    s += l * l;
-  }
-  double Vm = q_measure(x, m.nn, m.dim, Q);
-  double res;
-  if (m.dim == 3) {
-    if (Vm < 0) res = -15552 * (Vm * Vm) / (s * s * s);
-    else res = 15552 * (Vm * Vm) / (s * s * s);
-  } else {
-    res = 48 * (Vm * Vm) / (s * s);
-  }
-  q[e] = res;
-}
-
 
 // ---------------------------------------------------------------------
 // FP64 guard band of the FP32 path: for each listed edge, recompute the
@@ -2560,13 +2493,6 @@ void launch_apply_marks(int E, const uint32_t* split_bits, const uint32_t* colla
                         unsigned long long* counts, DevStatus* st, const int* skip, cudaStream_t s) {
   if (E)
     k_apply_marks<<<count_grid((E + 3) / 4), kBlock, 0, s>>>(E, split_bits, collapse_bits, flags, counts, st, skip);
-}
-
-void launch_quality_f64(const DevMesh& m, const double* size, const double* sizes, const double* frames, double* q,
-                        cudaStream_t s, const double* logm, DevStatus* st) {
-  if (!m.T) return;
-  if (logm) k_quality<true><<<nblk(m.T), kBlock, 0, s>>>(m, size, sizes, frames, logm, q, st);
-  else k_quality<false><<<nblk(m.T), kBlock, 0, s>>>(m, size, sizes, frames, logm, q, st);
 }
 
 void launch_guard_stage(int stage, const DevMesh& m, const double* u, const double* out3, const int* items,

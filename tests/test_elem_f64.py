@@ -246,3 +246,20 @@ def test_metric_lengths_and_qualities_bitwise(gpu_lib, oracle_lib, n, nz, kind):
         assert np.array_equal(c.measureQuality(iso), o.quality(iso), equal_nan=True)
         iso[:] = 0.3  # every vertex alike
         assert np.array_equal(c.measureQuality(iso), o.quality(iso), equal_nan=True)
+
+
+@pytest.mark.parametrize("n,nz", [(4, 3), (9, 0)])
+def test_qualities_without_the_transform_records(gpu_lib, oracle_lib, n, nz):
+    """The allocation of the vertices' transforms fails: computed per element."""
+    import core_gb300 as cg
+    m, o = mesh(oracle_lib, n, nz, "plain")
+    sizes, F = metric_of(m, "plain")
+    with cg.Context(m) as c:
+        c.test_hooks(alloc_fail_after=3)
+        assert np.array_equal(c.measureQuality(sizes=sizes, frames=F), o.quality(sizes=sizes, frames=F))
+    got = []
+    for after in (4, -1):
+        with cg.Context(m) as c:
+            c.test_hooks(alloc_fail_after=after)
+            got.append(c.measureQualityLog(sizes, F))
+    assert np.array_equal(*got)
