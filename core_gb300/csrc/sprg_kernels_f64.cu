@@ -1417,41 +1417,15 @@ inline int count_grid(long n) { return (int)std::min<long>((n + kBlock - 1) / kB
 // MA sweeps around the marks (ma/maSize.cc:652-690, ma/maShape.cc:132-169,
 // ma/maCoarsen.cc:36-60)
 // ---------------------------------------------------------------------
-// MetricSizeField::measure under LogAnisoSizeField (ma/maSize.cc:158-216,
-// 508-523): two Gauss points, log-metrics of both ends interpolated
-__device__ __forceinline__ double log_metric_length(const V3& x0, const V3& x1, const double* __restrict__ la,
-                                                    const double* __restrict__ lb, bool* ok) {
-  V3 x[2] = {x0, x1};
-  M3 J = ref::jacobian(x, 2, 1);
-  double Mv[18];
-  for (int k = 0; k < 9; ++k) {
-    Mv[k] = la[k];
-    Mv[9 + k] = lb[k];
-  }
-  const double gp[2] = {0.577350269189626, -0.577350269189626};
-  double measurement = 0;
-  for (int p = 0; p < 2; ++p) {
-    double N[2];
-    ref::edge_shape_values(gp[p], N);
-    M3 Q = ref::log_transform(Mv, N, 2, ok);
-    double dV2 = ref::jacobian_det(ref::mul(J, Q), 1);
-    measurement += 1 * dV2;
-  }
-  return measurement;
-}
-
 // length of the vertex pair (a, b) under a size field: kind 0 the identity
 // field (apf::measure of the edge, ma/maSize.cc:54-60), 1 the isotropic
-// user field, 2 the anisotropic one, 3 LogAnisoSizeField (per-vertex
-// log-metrics) -- the same evaluation as the edge measure kernels, for
-// edges that may not exist yet
+// user field, 2 the anisotropic one -- the same evaluation as the edge
+// measure kernels, for edges that may not exist yet
 __device__ __forceinline__ double pair_length(const DevMesh& m, int kind, int a, int b,
                                               const double* __restrict__ size, const double* __restrict__ sizes,
-                                              const double* __restrict__ frames, const double* __restrict__ logm,
-                                              bool* ok) {
+                                              const double* __restrict__ frames) {
   const V3 xa = load_xyz(m.xyz, a), xb = load_xyz(m.xyz, b);
   if (kind == 0) return edge_measure(xa, xb);
-  if (kind == 3) return log_metric_length(xa, xb, logm + 9 * (size_t)a, logm + 9 * (size_t)b, ok);
   if (kind == 1) return iso_length(xa, xb, size[a], size[b]);
   double hv[6], Rv[18];
   const int vv[2] = {a, b};
@@ -1467,14 +1441,27 @@ __global__ void __launch_bounds__(kBlock) k_measure_pairs(DevMesh m, int kind, l
                                                           const int* __restrict__ pairs,
                                                           const double* __restrict__ size,
                                                           const double* __restrict__ sizes,
-                                                          const double* __restrict__ frames,
-                                                          const double* __restrict__ logm, double* __restrict__ L,
-                                                          DevStatus* st) {
+                                                          const double* __restrict__ frames, double* __restrict__ L) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int* ab = pairs ? pairs + 2 * i : m.edv + 2 * i;
+  L[i] = pair_length(m, kind, ab[0], ab[1], size, sizes, frames);
+}
+
+// LogAnisoSizeField, per-vertex log-metrics.  FP64-rate bound by the eigen
+// iterations (0.2 ms for the 92k edges of a 24^3 box, 1.0 ms with the full
+// 3 x 3 iteration in local memory); blocks of two warps, so that a mesh of
+// some thousand edges still spreads evenly over the SMs.
+constexpr int kLogBlock = 64;
+__global__ void __launch_bounds__(kLogBlock) k_measure_log(DevMesh m, long long n, const int* __restrict__ pairs,
+                                                           const double* __restrict__ logm, double* __restrict__ L,
+                                                           DevStatus* st) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int* ab = pairs ? pairs + 2 * i : m.edv + 2 * i;
+  const int a = ab[0], b = ab[1];
   bool ok = true;
-  L[i] = pair_length(m, kind, ab[0], ab[1], size, sizes, frames, logm, &ok);
+  L[i] = log_metric_length(load_xyz(m.xyz, a), load_xyz(m.xyz, b), logm + 9 * (size_t)a, logm + 9 * (size_t)b, &ok);
   if (!ok) set_status(st, SPRG_EEIGEN, (int)i);
 }
 
@@ -2543,9 +2530,11 @@ void launch_xyz_to_fixed(const DevMesh& m, const double* frame, int* xyzq, cudaS
 void launch_measure_pairs(const DevMesh& m, int kind, long long n, const int* pairs, const double* size,
                           const double* sizes, const double* frames, const double* logm, double* L, DevStatus* st,
                           cudaStream_t s) {
-  if (n > 0)
-    k_measure_pairs<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, kind, n, pairs, size, sizes, frames,
-                                                                            logm, L, st);
+  if (n <= 0) return;
+  if (kind == 3)
+    k_measure_log<<<(unsigned)((n + kLogBlock - 1) / kLogBlock), kLogBlock, 0, s>>>(m, n, pairs, logm, L, st);
+  else
+    k_measure_pairs<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, kind, n, pairs, size, sizes, frames, L);
 }
 
 void launch_log_metric(int V, const double* sizes, const double* frames, double* logm, cudaStream_t s) {

@@ -180,4 +180,131 @@ __device__ __forceinline__ double aniso_length(const ref::V3& x0, const ref::V3&
   return L;
 }
 
+// ---- log-interpolated transforms (LogAnisoSizeField) ------------------------
+// |e Q|^2 at one point, e the edge vector and Q = R diag(sqrt(exp(lambda))) of
+// the interpolated log-metric A = R diag(lambda) R^T (a: rows 0 and 1 from
+// the diagonal on, then A22): the squares of e in the eigenvectors' frame
+// weighted with exp(lambda).  The eigenvalues come from mth::eigenQR's own
+// iteration (mth/mthQR.cc:192-297: Hessenberg reduction, Wilkinson shifts,
+// 1e-10 deflation from the bottom, the same failures) in its symmetric
+// tridiagonal form: two rotations a step, applied to e instead of to an
+// accumulated Q.  Same shifts and tests up to rounding; about 95 FP64
+// operations a step against 400 for the full 3 x 3 matrices.
+// Returns eigenQR's status (1 converged).
+__device__ __forceinline__ int log_length2(const double* a, const ref::V3& e, double* out) {
+  double d0 = a[0], d1 = a[3], d2 = a[5], e0 = a[1], e1 = a[4];
+  double w0 = e.v[0], w1 = e.v[1], w2 = e.v[2];
+  if (a[2] != 0.0) {
+    const double n2 = fma(e0, e0, a[2] * a[2]), rn = rsqrt(n2), c = e0 * rn, s = a[2] * rn;
+    const double cs = c * s, df = d2 - d1, t = 2 * cs * e1;
+    e1 = fma(cs, df, (c * c - s * s) * e1);
+    const double sd = s * s * df;
+    d1 += sd + t;
+    d2 -= sd + t;
+    e0 = n2 * rn;
+    const double y = fma(c, w1, s * w2);
+    w2 = fma(c, w2, -s * w1);
+    w1 = y;
+  }
+  int m = 3, status = 0;
+  for (int it = 0; it < 100; ++it) {
+    if (m == 3 && fabs(e1) < 1e-10) m = 2;
+    if (m == 2 && fabs(e0) < 1e-10) m = 1;
+    if (m == 1) {
+      status = 1;
+      break;
+    }
+    const double hi = m == 3 ? d1 : d0, lo = m == 3 ? d2 : d1, b = m == 3 ? e1 : e0;
+    const double sig = (hi - lo) * 0.5, b2 = b * b;
+    const double den = fabs(sig) + sqrt(fma(sig, sig, b2));
+    if (!(den > 1e-10)) {
+      status = -1;
+      break;
+    }
+    const double mu = lo - copysign(b2, sig < 0 ? -1.0 : 1.0) / den;
+    // two rotations; a column shorter than 1e-10 is left alone
+    const double x0 = d0 - mu, x1 = d1 - mu, x2 = d2 - mu;
+    double c0 = 1, s0 = 0, r0 = x0, c1 = 1, s1 = 0;
+    const double n0 = fma(x0, x0, e0 * e0);
+    if (!(n0 < 1e-20)) {
+      const double rn = rsqrt(n0);
+      c0 = x0 * rn;
+      s0 = e0 * rn;
+      r0 = n0 * rn;
+    }
+    const double r01 = fma(c0, e0, s0 * x1), q1 = fma(c0, x1, -s0 * e0), p1 = c0 * e1;
+    double r1 = q1;
+    const double n1 = fma(q1, q1, e1 * e1);
+    if (!(n1 < 1e-20)) {
+      const double rn = rsqrt(n1);
+      c1 = q1 * rn;
+      s1 = e1 * rn;
+      r1 = n1 * rn;
+    }
+    const double r12 = fma(c1, p1, s1 * x2), r22 = fma(c1, x2, -s1 * p1);
+    d0 = fma(r0, c0, r01 * s0) + mu;
+    e0 = r1 * s0;
+    d1 = fma(r1 * c0, c1, r12 * s1) + mu;
+    e1 = r22 * s1;
+    d2 = r22 * c1 + mu;
+    const double y0 = fma(c0, w0, s0 * w1), y1 = fma(c0, w1, -s0 * w0);
+    w0 = y0;
+    w1 = fma(c1, y1, s1 * w2);
+    w2 = fma(c1, w2, -s1 * y1);
+  }
+  *out = w0 * w0 * exp(d0) + w1 * w1 * exp(d1) + w2 * w2 * exp(d2);
+  return status;
+}
+
+// the reference's sequence at one Gauss point
+static __device__ __noinline__ double log_point_ref(const ref::V3& x0, const ref::V3& x1, const double* la,
+                                                    const double* lb, double xi, bool* ok) {
+  const ref::V3 x[2] = {x0, x1};
+  const ref::M3 J = ref::jacobian(x, 2, 1);
+  double Mv[18], N[2];
+  for (int k = 0; k < 9; ++k) {
+    Mv[k] = la[k];
+    Mv[9 + k] = lb[k];
+  }
+  ref::edge_shape_values(xi, N);
+  const ref::M3 Q = ref::log_transform(Mv, N, 2, ok);
+  return ref::jacobian_det(ref::mul(J, Q), 1);
+}
+
+// MetricSizeField::measure under LogAnisoSizeField (ma/maSize.cc:158-216,
+// 508-523): two Gauss points, the ends' log-metrics la, lb interpolated.
+// Entries above 200 in magnitude (sizes beyond e^-100: the absolute deflation
+// test is then near the rounding) or not finite, and a first column the
+// reduction would leave alone (below 1e-10, not 0), take the sequence itself.
+__device__ __forceinline__ double log_metric_length(const ref::V3& x0, const ref::V3& x1,
+                                                    const double* __restrict__ la, const double* __restrict__ lb,
+                                                    bool* ok) {
+  const double gp[2] = {0.577350269189626, -0.577350269189626};
+  const int at[6] = {0, 3, 6, 4, 7, 8};  // the lower triangle by columns
+  const ref::V3 d = ref::sub(x1, x0);
+  double L = 0;
+#pragma unroll 1
+  for (int p = 0; p < 2; ++p) {
+    double N[2], a[6];
+    ref::edge_shape_values(gp[p], N);
+    double big = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      a[k] = la[at[k]] * N[0] + lb[at[k]] * N[1];
+      big = fmax(big, fabs(a[k]));
+    }
+    double s;
+    const double col = fmax(fabs(a[1]), fabs(a[2]));
+    const bool fast = big <= 200.0 && a[0] == a[0] && a[1] == a[1] && a[2] == a[2] && a[3] == a[3] && a[4] == a[4] &&
+                      a[5] == a[5] && (a[2] == 0.0 || col >= 1e-10);
+    if (fast) {
+      if (log_length2(a, d, &s) != 1) *ok = false;
+      L += 0.5 * sqrt(s);
+    } else {
+      L += log_point_ref(x0, x1, la, lb, gp[p], ok);
+    }
+  }
+  return L;
+}
+
 }  // namespace sprg

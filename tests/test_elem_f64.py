@@ -263,3 +263,47 @@ def test_qualities_without_the_transform_records(gpu_lib, oracle_lib, n, nz):
             c.test_hooks(alloc_fail_after=after)
             got.append(c.measureQualityLog(sizes, F))
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("n,nz", [(1, 1), (4, 5), (7, 0)])
+@pytest.mark.parametrize("kind", ["plain", "diagonal", "isotropic", "close", "wide", "outside", "zero", "nan"])
+def test_log_lengths(gpu_lib, oracle_lib, n, nz, kind):
+    """Lengths under the log-interpolated field to 1e-10 (the deflation
+    threshold of the reference's iteration), its failures included: frames
+    along the axes, equal and nearly equal eigenvalues, sizes far apart,
+    entries beyond the fast form's range."""
+    import core_gb300 as cg
+    m, o = mesh(oracle_lib, n, nz, "plain")
+    sizes, F = metric_of(m, "plain")
+    F /= np.linalg.norm(F.reshape(-1, 3, 3)[:, :, :1], axis=1, keepdims=True).reshape(-1, 1)
+    if kind == "diagonal":
+        F = np.tile(np.eye(3).reshape(1, 9), (m.n_verts, 1))
+    elif kind == "isotropic":
+        sizes[:] = sizes[:, :1]
+    elif kind == "close":
+        sizes[:] = 0.1 * (1 + 1e-11 * np.random.default_rng(2).normal(size=sizes.shape))
+    elif kind == "wide":
+        sizes[:, 0] *= 1e-9
+        sizes[:, 1] *= 1e3
+    elif kind == "outside":
+        sizes[::3] *= 1e-60
+    elif kind == "zero":
+        sizes[1] = 0.0
+    elif kind == "nan":
+        F[2, 4] = np.nan
+    rc, want = o.measure_log(sizes, F)
+    with cg.Context(m) as c:
+        if rc:
+            with pytest.raises(cg.SprgError) as e:
+                c.measure_edges_log_aniso(sizes, F)
+            assert e.value.code == 7
+            return
+        got = c.measure_edges_log_aniso(sizes, F)
+        assert np.all(np.isfinite(want)) and kind not in ("zero", "nan")
+        # the deflated entries (up to 1e-10) couple the directions: against
+        # the longest direction's weight at that edge
+        scale = np.linalg.norm(m.coords[m.edge_verts[:, 1]] - m.coords[m.edge_verts[:, 0]], axis=1) / sizes.min()
+        assert np.all(np.abs(got - want) <= 1e-10 * scale)
+        assert np.abs(got - want).max() <= 1e-10 * want.max()
+        L = c.getMaximumEdgeLength(sizes=sizes, frames=F, log=True)
+        assert L == got.max()
