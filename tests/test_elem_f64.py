@@ -307,3 +307,45 @@ def test_log_lengths(gpu_lib, oracle_lib, n, nz, kind):
         assert np.abs(got - want).max() <= 1e-10 * want.max()
         L = c.getMaximumEdgeLength(sizes=sizes, frames=F, log=True)
         assert L == got.max()
+
+
+@pytest.mark.parametrize("k", [5, 31, 32, 33, 64, 65, 127, 128, 129, 200])
+def test_adjacency_ascends_at_every_patch_size(gpu_lib, k):
+    """A fan of k triangles in shuffled order around one vertex: its size is
+    the sum over its elements in ascending order, to the bit."""
+    import core_gb300 as cg
+    from core_gb300.mesh import Mesh
+    rng = np.random.default_rng(k)
+    t = np.arange(k) * 2 * np.pi / k
+    x = np.zeros((k + 1, 3))
+    x[1:, 0], x[1:, 1] = np.cos(t), np.sin(t)
+    x[1:, :2] *= rng.uniform(0.8, 1.2, (k, 1))
+    ring = 1 + np.arange(k)
+    ev = np.stack([np.zeros(k, int), ring, np.roll(ring, -1)], 1)[rng.permutation(k)].astype(np.int32)
+    ed = np.concatenate([np.stack([np.zeros(k, int), ring], 1), np.stack([ring, np.roll(ring, -1)], 1)]).astype(np.int32)
+    ip = rng.normal(size=(k, 3))
+    ip[:, 2] = 0.0
+    with cg.Context(Mesh(2, x, ev, ed)) as c:
+        size, _ = c.getSPRSizeField(ip, 0.1)
+        esize = c.debug_read("esize", np.float64, k)
+    total = 0.0
+    for e in esize:
+        total += e
+    assert size[0] == total / k
+
+
+def test_frame_of_an_updated_mesh(gpu_lib):
+    """The bounding box of an update (block reductions): a mesh moved and
+    stretched by sprg_update_mesh gives a fresh context's FP32 answers."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    a, b = workload.box(11, jitter=0.2, seed=1), workload.box(11, jitter=0.2, seed=2)
+    b.coords = b.coords * np.array([3.0, 0.2, 1.7]) - np.array([5.0, -0.3, 900.0])
+    u = workload.sine_field(a.coords)
+    with cg.Context(a, precision="fp32") as c:
+        c.estimate_and_mark(u, 0.1)
+        c.update_mesh(b)
+        got = c.estimate_and_mark(u, 0.1)
+    with cg.Context(b, precision="fp32") as c:
+        want = c.estimate_and_mark(u, 0.1)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
