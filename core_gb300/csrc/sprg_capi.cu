@@ -352,8 +352,10 @@ int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, 
   ENSURE(pc.n, sizeof(int) * slots);
   ENSURE(pc.el, sizeof(int) * slots * expand_max_elems());
   PB("expand_f64");
-  launch_expand_f64(m, ip, u, nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status), c->stream, P<int>(pc.v),
-                    P<int>(pc.n), P<int>(pc.el));
+  // tets: the growth and its rank tests only, the values follow from the
+  // weights below
+  launch_expand_f64(m, ip, u, m.dim == 3 ? 0 : nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status), c->stream,
+                    P<int>(pc.v), P<int>(pc.n), P<int>(pc.el));
   PE();
   c->launches += 1;
   int rc = check_launch(c, "expand");

@@ -11,7 +11,7 @@ int fast_error_blocks(int T);
 void fast_prep_coords(const DevMesh& m, const double* frame, float4* vrec, cudaStream_t s);
 // once per mesh: per tet {w dV, h_max} (FP32) and {det J, h_max} (FP64), per
 // edge half its length
-// cent: 3 doubles per element, the integration point (once per mesh, read by
+// cent: 3 doubles per element, four times the integration point (once per mesh, read by
 // fast_weights); qmax: one double (as its bits, set here), the largest
 // |cof J|_F^2 / |det J| over the elements
 void fast_geometry(const DevMesh& m, float2* geo, double2* geo64, double* cent, unsigned long long* qmax,

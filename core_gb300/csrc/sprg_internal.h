@@ -119,7 +119,7 @@ void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec,
 // slab: expand_grid() * expand_max_elems() * (4 + nc + 1) doubles.
 // ip may be NULL: the element gradients of u are computed in place (nc 3:
 // u scalar; nc 9: u a VECTOR field, V x 3) -- for the forms that keep no ip
-// field.
+// field.  nc 0: growth and rank tests alone (ip, u and rec unused).
 // cache_* (optional): record each listed vertex's final element set
 // (expand_max_elems() ints per list slot) for launch_cached_fit_f64.
 void launch_expand_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, ExpandList xl,

@@ -272,39 +272,66 @@ __global__ void __launch_bounds__(kBlock) k_fast_geo(DevMesh m, float2* __restri
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int k = 0; k < 3; ++k) e[i][k] = x[i + 1][k] - x[0][k];
-    double det = e[0][0] * (e[1][1] * e[2][2] - e[1][2] * e[2][1]) + e[0][1] * (e[1][2] * e[2][0] - e[1][0] * e[2][2]) +
-                 e[0][2] * (e[1][0] * e[2][1] - e[1][1] * e[2][0]);
-    double h2 = 0;
+    double c[3][3];  // rows of cofactors
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double* p = e[(i + 1) % 3];
+      const double* q = e[(i + 2) % 3];
+      c[i][0] = p[1] * q[2] - p[2] * q[1];
+      c[i][1] = p[2] * q[0] - p[0] * q[2];
+      c[i][2] = p[0] * q[1] - p[1] * q[0];
+    }
+    const double det = e[0][0] * c[0][0] + e[0][1] * c[0][1] + e[0][2] * c[0][2];
+    // the longest edge; squares are not negative, so they order as their bits
+    // (an FP64 maximum would take the FP64 pipe, which bounds this kernel)
+    unsigned long long h2 = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = i + 1; j < 4; ++j) {
-        double dx = x[j][0] - x[i][0], dy = x[j][1] - x[i][1], dz = x[j][2] - x[i][2];
-        h2 = fmax(h2, dx * dx + dy * dy + dz * dz);
+        const double dx = i ? x[j][0] - x[i][0] : e[j - 1][0], dy = i ? x[j][1] - x[i][1] : e[j - 1][1],
+                     dz = i ? x[j][2] - x[i][2] : e[j - 1][2];
+        const unsigned long long b = (unsigned long long)__double_as_longlong(dx * dx + dy * dy + dz * dz);
+        if (b <= 0x7ff0000000000000ull) h2 = b > h2 ? b : h2;  // a NaN does not count
       }
-    const double h = sqrt(h2);
+    const double h = sqrt(__longlong_as_double((long long)h2));
     geo[t] = make_float2((float)(det * (1.0 / 6.0)), (float)h);
     geo64[t] = make_double2(det, h);
-    // the integration point, summed in vertex order as the weights use it
+    // four times the integration point, summed in vertex order as the weights use it
 #pragma unroll
-    for (int k = 0; k < 3; ++k) cent[3 * (size_t)t + k] = 0.25 * (((x[0][k] + x[1][k]) + x[2][k]) + x[3][k]);
+    for (int k = 0; k < 3; ++k) cent[3 * (size_t)t + k] = ((x[0][k] + x[1][k]) + x[2][k]) + x[3][k];
     // |cof(J)|_F^2 / |det J| (= |J^-1|_F^2 |det J|): the element's share of the
     // reference's gradient rounding in the error integral scales with it; the
-    // largest over the mesh, for the rounding-dominance test
+    // largest over the mesh, for the rounding-dominance test (whose threshold
+    // is a factor 256 wide: the reciprocal is good to 2^-40)
     double c2 = 0;
-    for (int i = 0; i < 3; ++i) {
-      const double* a = e[(i + 1) % 3];
-      const double* b = e[(i + 2) % 3];
-      const double c0 = a[1] * b[2] - a[2] * b[1], c1 = a[2] * b[0] - a[0] * b[2], cc = a[0] * b[1] - a[1] * b[0];
-      c2 += c0 * c0 + c1 * c1 + cc * cc;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) c2 += c[i][0] * c[i][0] + c[i][1] * c[i][1] + c[i][2] * c[i][2];
+    const double ad = fabs(det);
+    const int ex = __double2hiint(ad) >> 20;
+    if (ex >= 100 && ex <= 1900) {
+      // 1 / det from the hardware's FP32 reciprocal of its mantissa in [1, 2)
+      // and one Newton step
+      const int hi = __double2hiint(ad), lo = __double2loint(ad);
+      float f = __int_as_float(((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29) | 0x3f800000);
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(f));
+      const int b = __float_as_int(f);
+      double r = __hiloint2double((b >> 3) + (896 << 20) - ((ex - 1023) << 20), b << 29);
+      r = r * (2.0 - ad * r);
+      qv = c2 * r;
+    } else {
+      qv = c2 / ad;  // inf for a flat element
     }
-    qv = c2 / fabs(det);  // inf for a flat element
     if (!(qv == qv)) qv = INFINITY;
   }
+  // non-negative doubles order as their bit patterns
+  unsigned long long qb = (unsigned long long)__double_as_longlong(qv);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) qv = fmax(qv, __shfl_xor_sync(0xffffffffu, qv, o));
-  // non-negative doubles order as their bit patterns (one atomic per warp)
-  if ((threadIdx.x & 31) == 0 && qv > 0) atomicMax(qmax, (unsigned long long)__double_as_longlong(qv));
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, qb, o);
+    qb = y > qb ? y : qb;
+  }
+  if ((threadIdx.x & 31) == 0 && qb > 0) atomicMax(qmax, qb);
 }
 
 __global__ void __launch_bounds__(kBlock) k_fast_elen(DevMesh m, float* __restrict__ half_len) {
@@ -461,39 +488,85 @@ __global__ void __launch_bounds__(kBlock, 4) k_fast_tet(DevMesh m, const float4*
 // depend on the geometry only, so they are computed once per mesh in FP64
 // (normal equations, Cholesky) and stored in patch-CSR order.  Patches with
 // fewer than four elements or a condition estimate above 1e6 are listed for
-// the FP64 reference path (growth + Householder QR) instead.
+// the FP64 reference path (growth + Householder QR) instead.  FP64-rate
+// bound: about 19 operations a patch element and 130 a vertex, 200 us for the
+// 141k vertices of a 51^3 box (283 with 28 and 220).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_fast_weights(DevMesh m, const double* __restrict__ cent,
+// the integration points k0 .. k0 + G - 1 of a patch relative to its vertex
+// (the last one repeated past the end); cent holds four times the point
+template <int G>
+__device__ __forceinline__ void load_points(const double* __restrict__ cent, const int* __restrict__ el, int k0, int cnt,
+                                            double xv, double yv, double zv, double s[G][3]) {
+  int t[G];
+#pragma unroll
+  for (int j = 0; j < G; ++j) t[j] = __ldg(el + min(k0 + j, cnt - 1));
+#pragma unroll
+  for (int j = 0; j < G; ++j) {
+    const double* ce = cent + 3 * (size_t)t[j];
+    s[j][0] = fma(0.25, __ldg(ce), -xv);
+    s[j][1] = fma(0.25, __ldg(ce + 1), -yv);
+    s[j][2] = fma(0.25, __ldg(ce + 2), -zv);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_fast_weights(DevMesh m, const double* __restrict__ cent,
                                                          float* __restrict__ w, double* __restrict__ w64, ExpandList xl,
                                                          int* __restrict__ n_refit, unsigned char* __restrict__ listed) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= m.V) return;
   const int beg = m.p_off[v], cnt = m.p_off[v + 1] - beg;
   const double xv = m.xyz[3 * (size_t)v], yv = m.xyz[3 * (size_t)v + 1], zv = m.xyz[3 * (size_t)v + 2];
-  double a[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const bool enough = cnt >= 4;
+  // moments of the integration points about v; the unit of length is the
+  // distance of the first one: 1 / |s_0| is applied to the sums afterwards, or
+  // to every point where the points' squares could under- or overflow
+  double a[10] = {(double)cnt, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   double inv_h = 0;
-  bool ok = cnt >= 4;
-  for (int k = 0; ok && k < cnt; ++k) {
-    const double* ce = cent + 3 * (size_t)m.p_el[beg + k];
-    double sx = ce[0] - xv, sy = ce[1] - yv, sz = ce[2] - zv;
-    if (k == 0) inv_h = 1.0 / sqrt(sx * sx + sy * sy + sz * sz);
-    sx *= inv_h; sy *= inv_h; sz *= inv_h;
-    a[0] += 1; a[1] += sx; a[2] += sy; a[3] += sz;
-    a[4] += sx * sx; a[5] += sx * sy; a[6] += sx * sz; a[7] += sy * sy; a[8] += sy * sz; a[9] += sz * sz;
+  bool each = false;
+  constexpr int G = 4;  // points fetched together: the id and point gathers of a group overlap
+  for (int k0 = 0; enough && k0 < cnt; k0 += G) {
+    double s[G][3];
+    load_points<G>(cent, m.p_el + beg, k0, cnt, xv, yv, zv, s);
+    if (k0 == 0) {
+      const double s2 = s[0][0] * s[0][0] + s[0][1] * s[0][1] + s[0][2] * s[0][2];
+      inv_h = 1.0 / sqrt(s2);
+      const int ex = (__double2hiint(s2) >> 20) & 0x7ff;
+      each = ex < 723 || ex > 1323;
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      if (k0 + j >= cnt) break;
+      double sx = s[j][0], sy = s[j][1], sz = s[j][2];
+      if (each) {
+        sx *= inv_h; sy *= inv_h; sz *= inv_h;
+      }
+      a[1] += sx; a[2] += sy; a[3] += sz;
+      a[4] += sx * sx; a[5] += sx * sy; a[6] += sx * sz; a[7] += sy * sy; a[8] += sy * sz; a[9] += sz * sz;
+    }
   }
-  double l00 = 0, l10 = 0, l20 = 0, l30 = 0, l11 = 0, l21 = 0, l31 = 0, l22 = 0, l32 = 0, l33 = 0;
-  if (ok) {
-    l00 = sqrt(a[0]);
-    l10 = a[1] / l00; l20 = a[2] / l00; l30 = a[3] / l00;
-    double d1 = a[4] - l10 * l10;
-    l11 = sqrt(fmax(d1, 0.0));
-    l21 = (a[5] - l20 * l10) / l11; l31 = (a[6] - l30 * l10) / l11;
-    double d2 = a[7] - l20 * l20 - l21 * l21;
-    l22 = sqrt(fmax(d2, 0.0));
-    l32 = (a[8] - l30 * l20 - l31 * l21) / l22;
-    double d3 = a[9] - l30 * l30 - l31 * l31 - l32 * l32;
-    l33 = sqrt(fmax(d3, 0.0));
-    double pmin = fmin(fmin(d1, d2), fmin(d3, a[0])), pmax = fmax(fmax(d1, d2), fmax(d3, a[0]));
+  if (!each) {
+    const double i2 = inv_h * inv_h;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) a[i] *= inv_h;
+#pragma unroll
+    for (int i = 4; i < 10; ++i) a[i] *= i2;
+  }
+  // Cholesky with the pivots' inverse roots r_i = 1 / l_ii (the square roots and
+  // divisions of the textbook form took a third of this kernel)
+  double r0 = 0, r1 = 0, r2 = 0, r3 = 0, l10 = 0, l20 = 0, l30 = 0, l21 = 0, l31 = 0, l32 = 0;
+  bool ok = false;
+  if (enough) {
+    r0 = rsqrt(a[0]);
+    l10 = a[1] * r0; l20 = a[2] * r0; l30 = a[3] * r0;
+    const double d1 = a[4] - l10 * l10;
+    r1 = rsqrt(fmax(d1, 0.0));
+    l21 = (a[5] - l20 * l10) * r1; l31 = (a[6] - l30 * l10) * r1;
+    const double d2 = a[7] - l20 * l20 - l21 * l21;
+    r2 = rsqrt(fmax(d2, 0.0));
+    l32 = (a[8] - l30 * l20 - l31 * l21) * r2;
+    const double d3 = a[9] - l30 * l30 - l31 * l31 - l32 * l32;
+    r3 = rsqrt(fmax(d3, 0.0));
+    const double pmin = fmin(fmin(d1, d2), fmin(d3, a[0])), pmax = fmax(fmax(d1, d2), fmax(d3, a[0]));
     ok = (pmin > 0) && (pmax <= 1e6 * pmin);
   }
   listed[v] = ok ? 0 : 1;
@@ -504,20 +577,30 @@ __global__ void __launch_bounds__(kBlock) k_fast_weights(DevMesh m, const double
     return;
   }
   // row q = e_0^T (L L^T)^{-1}: solve L y = e_0, then L^T q = y
-  double y0 = 1.0 / l00;
-  double y1 = (-l10 * y0) / l11;
-  double y2 = (-l20 * y0 - l21 * y1) / l22;
-  double y3 = (-l30 * y0 - l31 * y1 - l32 * y2) / l33;
-  double q3 = y3 / l33;
-  double q2 = (y2 - l32 * q3) / l22;
-  double q1 = (y1 - l21 * q2 - l31 * q3) / l11;
-  double q0 = (y0 - l10 * q1 - l20 * q2 - l30 * q3) / l00;
-  for (int k = 0; k < cnt; ++k) {
-    const double* ce = cent + 3 * (size_t)m.p_el[beg + k];
-    double sx = (ce[0] - xv) * inv_h, sy = (ce[1] - yv) * inv_h, sz = (ce[2] - zv) * inv_h;
-    const double wk = q0 + q1 * sx + q2 * sy + q3 * sz;
-    w[beg + k] = (float)wk;
-    w64[beg + k] = wk;
+  const double y1 = (-l10 * r0) * r1;
+  const double y2 = (-l20 * r0 - l21 * y1) * r2;
+  const double y3 = (-l30 * r0 - l31 * y1 - l32 * y2) * r3;
+  double q3 = y3 * r3;
+  double q2 = (y2 - l32 * q3) * r2;
+  double q1 = (y1 - l21 * q2 - l31 * q3) * r1;
+  const double q0 = (r0 - l10 * q1 - l20 * q2 - l30 * q3) * r0;
+  if (!each) {
+    q1 *= inv_h; q2 *= inv_h; q3 *= inv_h;
+  }
+  for (int k0 = 0; k0 < cnt; k0 += G) {
+    double s[G][3];
+    load_points<G>(cent, m.p_el + beg, k0, cnt, xv, yv, zv, s);
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      if (k0 + j >= cnt) break;
+      double sx = s[j][0], sy = s[j][1], sz = s[j][2];
+      if (each) {
+        sx *= inv_h; sy *= inv_h; sz *= inv_h;
+      }
+      const double wk = q0 + q1 * sx + q2 * sy + q3 * sz;
+      w[beg + k0 + j] = (float)wk;
+      w64[beg + k0 + j] = wk;
+    }
   }
 }
 
@@ -1194,7 +1277,7 @@ void fast_tet(const DevMesh& m, const float4* vrec, const double* u, float gscal
 
 void fast_weights(const DevMesh& m, const double* cent, float* w, double* w64, ExpandList xl, int* n_refit,
                   unsigned char* listed, cudaStream_t s) {
-  if (m.V) k_fast_weights<<<nblk(m.V), kBlock, 0, s>>>(m, cent, w, w64, xl, n_refit, listed);
+  if (m.V) k_fast_weights<<<nblk(m.V, 128), 128, 0, s>>>(m, cent, w, w64, xl, n_refit, listed);
 }
 
 
