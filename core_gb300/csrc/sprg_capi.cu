@@ -53,6 +53,10 @@ struct sprg_ctx {
   DevMesh m{};
   // mesh
   DevBuf xyz, xyzq, ev, edv, poff, pel, aoff, ael, tmp;
+  // sprg_update_mesh: the arrays of the mesh before the last update, into which
+  // the next one builds (given back when an allocation fails), and its staging
+  DevBuf sxyz, sev, sedv, ustage, ubad;
+  bool updating = false;  // an update is filling the spare arrays
   // fields
   DevBuf f, ip, rec, err, esize, size, L, flags, q, sizes3, frames9;
   int ip_nc = 0;
@@ -83,6 +87,7 @@ struct sprg_ctx {
   // FP32 path buffers
   DevBuf crec, vrec, rec32, q32, sz2, fcnt, guard, tetd, wts, w64, listed, geo, geo64, elen, fitems;
   DevBuf gstamp, gfit, grec;  // guard pipeline scratch
+  bool gstamp_ready = false;
   DevBuf tnext;               // work counter of the tet kernel
   DevBuf edone;               // blocks of the error kernel done (zero between passes)
   // learned form
@@ -193,6 +198,12 @@ int cuda_fail(sprg_ctx* c, cudaError_t e, const char* where) {
     if (e_ != cudaSuccess) return cuda_fail(c, e_, #call);    \
   } while (0)
 
+void release(DevBuf& b) {
+  if (b.p) cudaFree(b.p);
+  b.p = nullptr;
+  b.bytes = 0;
+}
+
 // grow-only device buffer
 int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -203,15 +214,25 @@ int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   b.p = nullptr;
   b.bytes = 0;
   cudaError_t e = cudaMalloc(&b.p, bytes);
-  if (e != cudaSuccess) return cuda_fail(c, e, "cudaMalloc");
+  if (e == cudaErrorMemoryAllocation) {
+    // the spare mesh arrays are only kept while there is room for them
+    bool freed = false;
+    for (DevBuf* sp : {&c->sxyz, &c->sev, &c->sedv, &c->ustage})
+      if (sp != &b && sp->p && !c->updating) {
+        release(*sp);
+        freed = true;
+      }
+    if (freed) {
+      cudaGetLastError();
+      e = cudaMalloc(&b.p, bytes);
+    }
+  }
+  if (e != cudaSuccess) {
+    b.p = nullptr;
+    return cuda_fail(c, e, "cudaMalloc");
+  }
   b.bytes = bytes;
   return SPRG_OK;
-}
-
-void release(DevBuf& b) {
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.bytes = 0;
 }
 
 template <class T>
@@ -818,8 +839,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   c->cache64.w_ready = c->cache32.w_ready = c->cache2d.w_ready = false;
   c->batch_n = 0;
   c->batch_nseg = 0;
-  // stamps are zeroed when (re)allocated at the next guard pass
-  release(c->gstamp);
+  c->gstamp_ready = false;  // zeroed again at the next guard pass
   if (c->graph_exec) {
     cudaGraphExecDestroy(c->graph_exec);
     c->graph_exec = nullptr;
@@ -862,81 +882,100 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   if (rc) return rc;
   c->launches = 0;
   CK(cudaStreamSynchronize(c->stream));
-  // ---- the new arrays: kept rows copied, listed rows scattered
-  DevBuf nxyz, nev, nedv, ids, vals, bad;
-  auto cleanup = [&]() {
-    release(nxyz); release(nev); release(nedv); release(ids); release(vals); release(bad);
+  // ---- the new arrays, in the spare buffers: kept rows copied, listed rows
+  // scattered from one staging buffer (each kind its own part, so that
+  // nothing waits in between)
+  struct Updating {
+    sprg_ctx* c;
+    explicit Updating(sprg_ctx* x) : c(x) { c->updating = true; }
+    ~Updating() { c->updating = false; }
   };
-#define CKU(call)                                                  \
-  do {                                                             \
-    cudaError_t e_ = (call);                                       \
-    if (e_ != cudaSuccess) { cleanup(); return cuda_fail(c, e_, #call); } \
-  } while (0)
-#define ENSUREU(buf, bytes)                                        \
-  do {                                                             \
-    int rc_ = ensure(c, (buf), (bytes));                           \
-    if (rc_) { cleanup(); return rc_; }                            \
-  } while (0)
-  ENSUREU(nxyz, sizeof(double) * 3 * (size_t)V1);
-  ENSUREU(nev, sizeof(int) * (size_t)(T1 * nn));
-  ENSUREU(nedv, sizeof(int) * 2 * (size_t)E1);
-  const int64_t kv = V1 < m.V ? V1 : m.V, kt = T1 < m.T ? T1 : m.T, ke = E1 < m.E ? E1 : m.E;
-  CKU(cudaMemcpyAsync(nxyz.p, c->xyz.p, sizeof(double) * 3 * (size_t)kv, cudaMemcpyDeviceToDevice, c->stream));
-  CKU(cudaMemcpyAsync(nev.p, c->ev.p, sizeof(int) * (size_t)(kt * nn), cudaMemcpyDeviceToDevice, c->stream));
-  CKU(cudaMemcpyAsync(nedv.p, c->edv.p, sizeof(int) * 2 * (size_t)ke, cudaMemcpyDeviceToDevice, c->stream));
-  const int64_t maxrows = std::max(d->n_vert_rows, std::max(d->n_elem_rows, d->n_edge_rows));
-  ENSUREU(ids, sizeof(int) * (size_t)(maxrows > 0 ? maxrows : 1));
-  ENSUREU(vals, sizeof(double) * 3 * (size_t)(maxrows > 0 ? maxrows : 1) + sizeof(int) * (size_t)(maxrows * nn));
-  ENSUREU(bad, sizeof(unsigned long long));
-  auto scatter_i32 = [&](int64_t n, const int32_t* hid, const int32_t* hval, int width, int* dst) -> int {
-    if (!n) return SPRG_OK;
-    CKU(cudaMemcpyAsync(ids.p, hid, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    CKU(cudaMemcpyAsync(vals.p, hval, sizeof(int) * (size_t)(n * width), cudaMemcpyHostToDevice, c->stream));
-    launch_scatter_rows_i32(n, width, P<int>(ids), P<int>(vals), dst, c->stream);
-    CKU(cudaStreamSynchronize(c->stream));  // the staging buffers are reused
-    return SPRG_OK;
+  {
+    Updating in_progress(c);
+    ENSURE(c->sxyz, sizeof(double) * 3 * (size_t)V1);
+    ENSURE(c->sev, sizeof(int) * (size_t)(T1 * nn));
+    ENSURE(c->sedv, sizeof(int) * 2 * (size_t)E1);
+    const int64_t kv = V1 < m.V ? V1 : m.V, kt = T1 < m.T ? T1 : m.T, ke = E1 < m.E ? E1 : m.E;
+    const size_t nv = (size_t)d->n_vert_rows, nt = (size_t)d->n_elem_rows, ne = (size_t)d->n_edge_rows;
+    // coordinates first (8-byte values), then the ids and the integer rows
+    ENSURE(c->ustage, sizeof(double) * 3 * nv + sizeof(int) * (nv + nt * (1 + nn) + ne * 3));
+    ENSURE(c->ubad, sizeof(unsigned long long));
+    ENSURE(c->red, sizeof(double) * (size_t)(sum_partials_count() + 4));
+    double* sx = P<double>(c->ustage);
+    int* vi = reinterpret_cast<int*>(sx + 3 * nv);
+    int* ti = vi + nv;
+    int* tv = ti + nt;
+    int* ei = tv + nt * nn;
+    int* ed = ei + ne;
+    CK(cudaMemcpyAsync(c->sxyz.p, c->xyz.p, sizeof(double) * 3 * (size_t)kv, cudaMemcpyDeviceToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->sev.p, c->ev.p, sizeof(int) * (size_t)(kt * nn), cudaMemcpyDeviceToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->sedv.p, c->edv.p, sizeof(int) * 2 * (size_t)ke, cudaMemcpyDeviceToDevice, c->stream));
+    auto put = [&](void* dst, const void* src, size_t bytes) {
+      return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
+    };
+    CK(put(sx, d->coords, sizeof(double) * 3 * nv));
+    CK(put(vi, d->vert_ids, sizeof(int) * nv));
+    CK(put(ti, d->elem_ids, sizeof(int) * nt));
+    CK(put(tv, d->elem_verts, sizeof(int) * nt * nn));
+    CK(put(ei, d->edge_ids, sizeof(int) * ne));
+    CK(put(ed, d->edge_verts, sizeof(int) * ne * 2));
+    launch_scatter_rows_f64((long long)nv, 3, vi, sx, P<double>(c->sxyz), c->stream);
+    launch_scatter_rows_i32((long long)nt, nn, ti, tv, P<int>(c->sev), c->stream);
+    launch_scatter_rows_i32((long long)ne, 2, ei, ed, P<int>(c->sedv), c->stream);
+    // kept rows may name vertices beyond a smaller vertex count
+    CK(cudaMemsetAsync(c->ubad.p, 0, sizeof(unsigned long long), c->stream));
+    launch_count_out_of_range(T1 * nn, P<int>(c->sev), (int)V1, P<unsigned long long>(c->ubad), c->stream);
+    launch_count_out_of_range(2 * E1, P<int>(c->sedv), (int)V1, P<unsigned long long>(c->ubad), c->stream);
+    launch_bbox((int)V1, P<double>(c->sxyz), P<unsigned long long>(c->red), c->stream);
+  }
+  unsigned long long nbad = 0, keys[6];
+  CK(cudaMemcpyAsync(&nbad, c->ubad.p, sizeof nbad, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(keys, c->red.p, sizeof keys, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));  // the caller's rows are read, too
+  if ((rc = check_launch(c, "mesh update"))) return rc;
+  if (nbad) return fail(c, SPRG_EINVAL, "kept elements or edges name vertices beyond the new vertex count");
+  // room for what derives from the arrays, so that nothing can fail once the
+  // old mesh is gone
+  const size_t nel = (size_t)(T1 * nn);
+  struct Grow {
+    DevBuf& b;
+    size_t bytes;
+    DevBuf fresh;
   };
-  if (d->n_vert_rows) {
-    CKU(cudaMemcpyAsync(ids.p, d->vert_ids, sizeof(int) * (size_t)d->n_vert_rows, cudaMemcpyHostToDevice, c->stream));
-    CKU(cudaMemcpyAsync(vals.p, d->coords, sizeof(double) * 3 * (size_t)d->n_vert_rows, cudaMemcpyHostToDevice,
-                        c->stream));
-    launch_scatter_rows_f64(d->n_vert_rows, 3, P<int>(ids), P<double>(vals), P<double>(nxyz), c->stream);
-    CKU(cudaStreamSynchronize(c->stream));
+  std::vector<Grow> grow;
+  grow.push_back({c->xyzq, sizeof(int) * 4 * (size_t)V1, {}});
+  grow.push_back({c->poff, sizeof(int) * ((size_t)V1 + 1), {}});
+  grow.push_back({c->pel, sizeof(int) * nel, {}});
+  grow.push_back({c->tmp, sizeof(int) * (size_t)V1, {}});
+  if (d->vert_elem_offsets) {
+    grow.push_back({c->aoff, sizeof(int) * ((size_t)V1 + 1), {}});
+    grow.push_back({c->ael, sizeof(int) * nel, {}});
   }
-  if ((rc = scatter_i32(d->n_elem_rows, d->elem_ids, d->elem_verts, nn, P<int>(nev)))) return rc;
-  if ((rc = scatter_i32(d->n_edge_rows, d->edge_ids, d->edge_verts, 2, P<int>(nedv)))) return rc;
-  // kept rows may name vertices beyond a smaller vertex count
-  CKU(cudaMemsetAsync(bad.p, 0, sizeof(unsigned long long), c->stream));
-  launch_count_out_of_range(T1 * nn, P<int>(nev), (int)V1, P<unsigned long long>(bad), c->stream);
-  launch_count_out_of_range(2 * E1, P<int>(nedv), (int)V1, P<unsigned long long>(bad), c->stream);
-  unsigned long long nbad = 0;
-  CKU(cudaMemcpyAsync(&nbad, bad.p, sizeof nbad, cudaMemcpyDeviceToHost, c->stream));
-  CKU(cudaStreamSynchronize(c->stream));
-  if (nbad) {
-    cleanup();
-    return fail(c, SPRG_EINVAL, "kept elements or edges name vertices beyond the new vertex count");
+  c->updating = true;
+  for (auto& g : grow)
+    if (g.b.bytes < g.bytes && (rc = ensure(c, g.fresh, g.bytes))) break;
+  c->updating = false;
+  if (rc) {
+    for (auto& g : grow) release(g.fresh);
+    return rc;
   }
+  for (auto& g : grow)
+    if (g.fresh.p) {
+      std::swap(g.b, g.fresh);
+      release(g.fresh);
+    }
   // ---- swap in, rebuild what derives from the arrays
-  release(c->xyz); release(c->ev); release(c->edv);
-  c->xyz = nxyz; c->ev = nev; c->edv = nedv;
-  nxyz = DevBuf{}; nev = DevBuf{}; nedv = DevBuf{};
-  cleanup();
-#undef CKU
-#undef ENSUREU
+  invalidate_mesh_state(c);
+  std::swap(c->xyz, c->sxyz);
+  std::swap(c->ev, c->sev);
+  std::swap(c->edv, c->sedv);
   m.V = (int)V1;
   m.T = (int)T1;
   m.E = (int)E1;
   m.xyz = P<double>(c->xyz);
   m.ev = P<int>(c->ev);
   m.edv = P<int>(c->edv);
-  const size_t nel = (size_t)m.T * nn;
-  ENSURE(c->xyzq, sizeof(int) * 4 * (size_t)m.V);
   m.xyzq = P<int>(c->xyzq);
-  ENSURE(c->red, sizeof(double) * (size_t)(sum_partials_count() + 4));
-  launch_bbox(m.V, m.xyz, P<unsigned long long>(c->red), c->stream);
-  unsigned long long keys[6];
-  CK(cudaMemcpyAsync(keys, c->red.p, sizeof keys, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   double lo[3], hi[3];
   for (int k = 0; k < 3; ++k) {
     lo[k] = key_to_double(keys[k]);
@@ -944,12 +983,7 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   }
   set_frame(c, lo, hi);
   launch_xyz_to_fixed(m, c->frame, P<int>(c->xyzq), c->stream);
-  ENSURE(c->poff, sizeof(int) * ((size_t)m.V + 1));
-  ENSURE(c->pel, sizeof(int) * nel);
-  ENSURE(c->tmp, sizeof(int) * (size_t)m.V);
   if (d->vert_elem_offsets) {
-    ENSURE(c->aoff, sizeof(int) * ((size_t)m.V + 1));
-    ENSURE(c->ael, sizeof(int) * nel);
     CK(cudaMemcpyAsync(c->aoff.p, d->vert_elem_offsets, sizeof(int) * ((size_t)m.V + 1), cudaMemcpyHostToDevice,
                        c->stream));
     CK(cudaMemcpyAsync(c->ael.p, d->vert_elems, sizeof(int) * nel, cudaMemcpyHostToDevice, c->stream));
@@ -968,8 +1002,7 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   m.p_el = P<int>(c->pel);
   c->launches += 5;
   if ((rc = check_launch(c, "mesh update"))) return rc;
-  CK(cudaStreamSynchronize(c->stream));
-  invalidate_mesh_state(c);
+  if (d->vert_elem_offsets) CK(cudaStreamSynchronize(c->stream));  // the caller's CSR is read
   return SPRG_OK;
 }
 
@@ -977,7 +1010,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,
@@ -1817,12 +1850,11 @@ static int pass_fast(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_
   fast_measure(m, P<float>(c->elen), P<float2>(c->sz2), d_split, d_collapse, P<int>(c->guard), P<int>(c->fcnt) + 1,
                sprg_ctx::kGuardCap, sprg_ctx::kGuardRel, c->stream);
   PE();
-  if (!c->gstamp.p) {  // V stamps (zero) and the stamp-id counter (one)
+  if (!c->gstamp_ready) {  // V stamps (zero) and the stamp-id counter, which starts at 0x01010101 (any id above 0)
     ENSURE(c->gstamp, sizeof(int) * ((size_t)m.V + 1));
     CK(cudaMemsetAsync(c->gstamp.p, 0, sizeof(int) * (size_t)m.V, c->stream));
-    const int one = 1;
-    CK(cudaMemcpyAsync(P<int>(c->gstamp) + m.V, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    CK(cudaMemsetAsync(P<int>(c->gstamp) + m.V, 1, sizeof(int), c->stream));
+    c->gstamp_ready = true;
   }
   ENSURE(c->gfit, sizeof(int) * ((size_t)m.V + 1));
   ENSURE(c->grec, 3 * sizeof(double) * (size_t)m.V);

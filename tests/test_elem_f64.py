@@ -349,3 +349,32 @@ def test_frame_of_an_updated_mesh(gpu_lib):
     with cg.Context(b, precision="fp32") as c:
         want = c.estimate_and_mark(u, 0.1)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "learned"])
+def test_updates_in_a_row(gpu_lib, precision):
+    """Growing, shrinking and moving back and forth through the spare arrays,
+    with a pass after each, a failed allocation in between; every pass equals
+    a fresh context's."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    meshes = [workload.box(n, jitter=0.2, seed=s) for n, s in ((5, 1), (7, 2), (5, 3), (4, 4), (7, 5), (9, 6), (5, 1))]
+    want = []
+    for m in meshes:
+        with cg.Context(m, precision=precision) as c:
+            want.append(c.estimate_and_mark(workload.sine_field(m.coords), 0.1)[:2])
+    with cg.Context(meshes[0], precision=precision) as c:
+        for i, m in enumerate(meshes):
+            if i:
+                if m.n_verts > max(x.n_verts for x in meshes[:i]):
+                    c.test_hooks(alloc_fail_after=4)
+                    with pytest.raises(cg.SprgError) as e:
+                        c.update_mesh(m)
+                    assert e.value.code == 4
+                    c.test_hooks()
+                    old = meshes[i - 1]
+                    got = c.estimate_and_mark(workload.sine_field(old.coords), 0.1)
+                    assert np.array_equal(got[0], want[i - 1][0]) and np.array_equal(got[1], want[i - 1][1])
+                c.update_mesh(m)
+            got = c.estimate_and_mark(workload.sine_field(m.coords), 0.1)
+            assert np.array_equal(got[0], want[i][0]) and np.array_equal(got[1], want[i][1])
