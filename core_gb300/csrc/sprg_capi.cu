@@ -89,6 +89,7 @@ struct sprg_ctx {
   DevBuf gstamp, gfit, grec;  // guard pipeline scratch
   bool gstamp_ready = false;
   DevBuf tnext;               // work counter of the tet kernel
+  DevBuf umaxp;               // the field's largest value per block of the prep kernel
   DevBuf edone;               // blocks of the error kernel done (zero between passes)
   // learned form
   DevBuf hess;  // nodal Hessian upload (sprg_hessian_metric)
@@ -217,7 +218,7 @@ int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (e == cudaErrorMemoryAllocation) {
     // the spare mesh arrays are only kept while there is room for them
     bool freed = false;
-    for (DevBuf* sp : {&c->sxyz, &c->sev, &c->sedv, &c->ustage})
+    for (DevBuf* sp : {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage})
       if (sp != &b && sp->p && !c->updating) {
         release(*sp);
         freed = true;
@@ -344,6 +345,35 @@ int ensure_cache_weights(sprg_ctx* c, PatchCache& pc) {
   return SPRG_OK;
 }
 
+// The growth of the listed patches (once per mesh), their final element sets
+// into the cache; triangles also take their fits from it (ip or u, nc, rec64).
+// known: the list's length, or -1 to read it back.
+int grow_patches(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, int nc, double* rec64, ExpandList xl,
+                 int known) {
+  int xc = known;
+  if (known < 0) {
+    CK(cudaMemcpyAsync(&xc, xl.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
+  if (xc > xl.cap) xc = xl.cap;
+  size_t slots = (size_t)(xc > 0 ? xc : 1);
+  ENSURE(pc.v, sizeof(int) * slots);
+  ENSURE(pc.n, sizeof(int) * slots);
+  ENSURE(pc.el, sizeof(int) * slots * expand_max_elems());
+  PB("expand_f64");
+  // tets: the growth and its rank tests only, the values follow from the
+  // weights
+  launch_expand_f64(c->m, ip, u, c->m.dim == 3 ? 0 : nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status),
+                    c->stream, P<int>(pc.v), P<int>(pc.n), P<int>(pc.el));
+  PE();
+  c->launches += 1;
+  int rc = check_launch(c, "expand");
+  if (rc) return rc;
+  pc.count = xc;
+  pc.valid = true;
+  return SPRG_OK;
+}
+
 int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, int nc, double* rec64, ExpandList xl,
                 cudaStream_t on = nullptr) {
   DevMesh& m = c->m;
@@ -364,25 +394,8 @@ int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, 
     c->launches += 1;
     return check_launch(c, "cached fit");
   }
-  int xc = 0;
-  CK(cudaMemcpyAsync(&xc, xl.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  if (xc > xl.cap) xc = xl.cap;
-  size_t slots = (size_t)(xc > 0 ? xc : 1);
-  ENSURE(pc.v, sizeof(int) * slots);
-  ENSURE(pc.n, sizeof(int) * slots);
-  ENSURE(pc.el, sizeof(int) * slots * expand_max_elems());
-  PB("expand_f64");
-  // tets: the growth and its rank tests only, the values follow from the
-  // weights below
-  launch_expand_f64(m, ip, u, m.dim == 3 ? 0 : nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status), c->stream,
-                    P<int>(pc.v), P<int>(pc.n), P<int>(pc.el));
-  PE();
-  c->launches += 1;
-  int rc = check_launch(c, "expand");
+  int rc = grow_patches(c, pc, ip, u, nc, rec64, xl, -1);
   if (rc) return rc;
-  pc.count = xc;
-  pc.valid = true;
   if (m.dim != 3) return SPRG_OK;
   // tets: this pass already takes the weighted sums, so every pass gives the
   // same bits for the listed patches
@@ -417,13 +430,13 @@ int ensure_elem_records(sprg_ctx* c) {
 
 const double* elem_records(sprg_ctx* c) { return c->egeo_ready ? P<double>(c->egeo) : nullptr; }
 
-int step_grad(sprg_ctx* c, int ncin) {
+int step_grad(sprg_ctx* c, const double* f, int ncin) {
   DevMesh& m = c->m;
   ENSURE(c->ip, sizeof(double) * (size_t)m.T * 3 * ncin);
   int rc = ensure_elem_records(c);
   if (rc) return rc;
   PB("grad_ip_f64");
-  launch_grad_ip_f64(m, elem_records(c), P<double>(c->f), ncin, P<double>(c->ip), c->stream);
+  launch_grad_ip_f64(m, elem_records(c), f, ncin, P<double>(c->ip), c->stream);
   PE();
   c->launches += 1;
   c->ip_nc = 3 * ncin;
@@ -1010,7 +1023,7 @@ int sprg_destroy(sprg_ctx* c) {
   if (!c) return SPRG_OK;
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
-  DevBuf* bufs[] = {&c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
+  DevBuf* bufs[] = {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,
@@ -1081,7 +1094,7 @@ int sprg_get_grad_ip_field(sprg_ctx* c, const double* f, int ncomp_in, int order
   CK(cudaMemcpyAsync(c->f.p, f, sizeof(double) * (size_t)m.V * ncomp_in, cudaMemcpyHostToDevice, c->stream));
   int saved = c->precision;
   c->precision = SPRG_FP64;  // the explicit ip field is always the FP64 one
-  rc = step_grad(c, ncomp_in);
+  rc = step_grad(c, P<double>(c->f), ncomp_in);
   c->precision = saved;
   if (rc) return rc;
   if (ip_out)
@@ -1507,7 +1520,7 @@ static int fast_setup(sprg_ctx* c, ExpandList xl) {
 // the listed patches' FP64 fits: the first pass grows the patches (and
 // caches them) in order; later passes run the cached fits on the side
 // stream, joined by the caller before the results are used
-static int listed_fork(sprg_ctx* c, ExpandList xl, bool* forked) {
+static int listed_fork(sprg_ctx* c, const double* d_u, ExpandList xl, bool* forked) {
   *forked = false;
   if (!c->cache32.valid) return SPRG_OK;
   int wrc = ensure_cache_weights(c, c->cache32);
@@ -1519,19 +1532,19 @@ static int listed_fork(sprg_ctx* c, ExpandList xl, bool* forked) {
   }
   CK(cudaEventRecord(c->fork, c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork, 0));
-  int rc = listed_fits(c, c->cache32, nullptr, P<double>(c->f), 3, P<double>(c->rec), xl, c->side);
+  int rc = listed_fits(c, c->cache32, nullptr, d_u, 3, P<double>(c->rec), xl, c->side);
   if (rc) return rc;
   CK(cudaEventRecord(c->join, c->side));
   *forked = true;
   return SPRG_OK;
 }
 
-static int listed_join(sprg_ctx* c, ExpandList xl, bool forked) {
+static int listed_join(sprg_ctx* c, const double* d_u, ExpandList xl, bool forked) {
   if (forked) {
     CK(cudaStreamWaitEvent(c->stream, c->join, 0));
     return SPRG_OK;
   }
-  return listed_fits(c, c->cache32, nullptr, P<double>(c->f), 3, P<double>(c->rec), xl);
+  return listed_fits(c, c->cache32, nullptr, d_u, 3, P<double>(c->rec), xl);
 }
 
 // patch-size bins of the non-listed vertices (stable: ascending ids within a
@@ -1643,7 +1656,8 @@ static int build_tiles(sprg_ctx* c, int only = -1) {
   return SPRG_OK;
 }
 
-static void run_tiles(sprg_ctx* c, float4* rec32) {
+static void run_tiles(sprg_ctx* c, float4* rec32, bool reset) {
+  if (reset) cudaMemsetAsync(c->bnext.p, 0, sizeof(int), c->stream);
   fast_recover_tiles(c->m, P<float>(c->wts), sliced_view(c), P<uint4>(c->tetd), rec32, P<int>(c->bverts),
                      P<int4>(c->btiles), c->n_tiles, c->tile_mode < 0 ? -1 : c->tile_mode, P<int>(c->bnext),
                      c->n_sms * c->grid_per_sm, c->stream);
@@ -1658,7 +1672,7 @@ static float time_tiles(sprg_ctx* c, float4* rec32, int only) {
   float best = 1e30f;
   for (int r = 0; r < 3; ++r) {
     cudaEventRecord(e0, c->stream);
-    run_tiles(c, rec32);
+    run_tiles(c, rec32, true);
     cudaEventRecord(e1, c->stream);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -1761,7 +1775,7 @@ static int autotune(sprg_ctx* c, float4* rec32) {
 
 // FP32 pass: packed double-float records, FP32 fits and sweeps, FP64
 // reference path for ill-conditioned or growing patches (sprg_kernels_f32.cu).
-static int pass_fast(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
+static int pass_fast(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
   DevMesh& m = c->m;
   int rc;
   if (m.dim != 3)
@@ -1787,26 +1801,31 @@ static int pass_fast(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_
   ENSURE(c->guard, sizeof(int) * (size_t)sprg_ctx::kGuardCap);
   ENSURE(c->partials, sizeof(double) * 2 * (size_t)(nb > 0 ? nb : 1));
   ENSURE(c->out3, sizeof(double) * 4 * (size_t)(bv.n > 0 ? bv.n : 1));
-  if ((rc = reset_status(c))) return rc;
+  ENSURE(c->umaxp, sizeof(int) * (size_t)fast_prep_blocks(m.V));
+  ENSURE(c->bnext, sizeof(int));
+  ENSURE(c->gfit, sizeof(int) * ((size_t)m.V + 1));
+  ENSURE(c->grec, 3 * sizeof(double) * (size_t)m.V);
   // fcnt: [0] refit patches, [1] guard edges, [3] listed patches,
-  // [4] unresolved guard edges, [5] rounding dominance (max |u| as float
-  // bits from the prep kernel, then 0 / 1 from the error kernel's last
-  // block) (0, 3 per mesh; 1, 4, 5 per pass)
+  // [4] unresolved guard edges, [5] rounding dominance (0 / 1 from the error
+  // kernel's last block) (0, 3 per mesh; 1, 4, 5 per pass)
   ExpandList xl{P<int>(c->fitems), P<int>(c->fcnt) + 3, m.V};
   float4* vrec = P<float4>(c->vrec);
   float4* rec32 = P<float4>(c->rec32);
   if ((rc = fast_setup(c, xl))) return rc;
-  // the FP64 fits of the listed patches depend on the field only: once their
-  // patches are cached they run on the side stream, beside the FP32 phases
-  bool fork = false;
-  if ((rc = listed_fork(c, xl, &fork))) return rc;
-  CK(cudaMemsetAsync(P<int>(c->fcnt) + 1, 0, sizeof(int), c->stream));
-  CK(cudaMemsetAsync(P<int>(c->fcnt) + 4, 0, 2 * sizeof(int), c->stream));
+  PatchCache& pc = c->cache32;
+  if (!pc.valid) {  // once per mesh: the listed patches' growth and FP64 weights
+    if ((rc = reset_status(c)) || (rc = grow_patches(c, pc, nullptr, nullptr, 3, nullptr, xl, c->n_listed))) return rc;
+  }
+  if ((rc = ensure_cache_weights(c, pc))) return rc;
+  const ListedSums ls{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
+                      P<double>(pc.w), P<int>(pc.wn), P<double>(c->rec), rec32, P<DevStatus>(c->status)};
+  const PassCounters counters{{P<int>(c->status), P<int>(c->status) + 1, P<int>(c->fcnt) + 1, P<int>(c->fcnt) + 4,
+                               P<int>(c->tnext), P<int>(c->bnext), P<int>(c->gfit)}};
   PB("prep_f32");
-  fast_prep(m, P<double>(c->f), P<float4>(c->crec), vrec, P<int>(c->fcnt) + 5, c->stream);
+  fast_prep(m, d_u, P<float4>(c->crec), vrec, P<int>(c->umaxp), counters, c->stream);
   PE();
   PB("tet_f32");
-  fast_tet(m, vrec, P<double>(c->f), (float)c->frame[3], P<uint4>(c->tetd), P<int>(c->tnext), c->stream);
+  fast_tet(m, vrec, d_u, (float)c->frame[3], P<uint4>(c->tetd), P<int>(c->tnext), ls, c->stream);
   PE();
   if (!c->bins_ready) {
     PB("setup_bins");
@@ -1814,19 +1833,19 @@ static int pass_fast(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_
     if ((rc = build_tiles(c))) return rc;
     PE();
   }
-  if (c->autotune && !c->tuned && (rc = autotune(c, rec32))) return rc;
+  bool tuned_now = false;
+  if (c->autotune && !c->tuned) {
+    if ((rc = autotune(c, rec32))) return rc;
+    tuned_now = true;  // the timed launches left the tile counter behind
+  }
   PB("recover_f32");
-  run_tiles(c, rec32);
-  PE();
-  if ((rc = listed_join(c, xl, fork))) return rc;
-  PB("merge_f64");
-  fast_merge_ref(xl, P<double>(c->rec), rec32, c->stream);
+  run_tiles(c, rec32, tuned_now);
   PE();
   // one mesh: the error kernel's last block also computes the size factor
   PB("error_f32");
   fast_error(m, P<uint4>(c->tetd), P<float2>(c->geo), rec32, P<float2>(c->q32), P<double>(c->partials), nb,
              bv.n ? P<int2>(c->bseg) : nullptr, bv.n ? nullptr : P<unsigned>(c->edone), adapt_ratio,
-             P<double>(c->out3), P<int>(c->fcnt) + 5, P<unsigned long long>(c->qmax), c->stream);
+             P<double>(c->out3), P<int>(c->umaxp), P<int>(c->fcnt) + 5, P<unsigned long long>(c->qmax), c->stream);
   PE();
   if (bv.n) {
     PB("size_factor");
@@ -1856,19 +1875,17 @@ static int pass_fast(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_
     CK(cudaMemsetAsync(P<int>(c->gstamp) + m.V, 1, sizeof(int), c->stream));
     c->gstamp_ready = true;
   }
-  ENSURE(c->gfit, sizeof(int) * ((size_t)m.V + 1));
-  ENSURE(c->grec, 3 * sizeof(double) * (size_t)m.V);
   GuardScratch gs{P<int>(c->gstamp), P<int>(c->gstamp) + m.V, P<int>(c->gfit) + 1,   P<int>(c->gfit),
                   m.V,               P<double>(c->grec), P<double>(c->w64),           P<unsigned char>(c->listed),
                   P<double>(c->rec), P<double2>(c->geo64)};
   static const char* const kGuardNames[kGuardStages] = {"guard_collect", "guard_fit", "guard_decide"};
   for (int stage = 0; stage < kGuardStages; ++stage) {
     PB(kGuardNames[stage]);
-    launch_guard_stage(stage, m, P<double>(c->f), P<double>(c->out3), P<int>(c->guard), P<int>(c->fcnt) + 1,
+    launch_guard_stage(stage, m, d_u, P<double>(c->out3), P<int>(c->guard), P<int>(c->fcnt) + 1,
                        sprg_ctx::kGuardCap, d_split, d_collapse, P<int>(c->fcnt) + 4, gs, bv, c->stream);
     PE();
   }
-  c->launches += (bv.n ? 8 : 7) + kGuardStages;  // FP32-path and guard kernels (listed_fits counts its own)
+  c->launches += (bv.n ? 7 : 6) + kGuardStages;  // FP32-path and guard kernels
   c->size_valid = false;  // the FP64 size buffer is filled on demand
   c->L_valid = false;
   return check_launch(c, "fast pass");
@@ -1897,7 +1914,7 @@ static void learned_records(sprg_ctx* c, const double* d_u) {
 
 // Learned pass: network recovery with plain-SPR fallback, FP32 sweeps
 // (sprg_learned.cu).
-static int pass_learned(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
+static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
   DevMesh& m = c->m;
   int rc;
   if (!c->have_mlp) return fail(c, SPRG_ESTATE, "learned form: no network parameters (sprg_set_mlp_params)");
@@ -1934,20 +1951,20 @@ static int pass_learned(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint
     c->vv_ready = true;
   }
   bool fork = false;
-  if ((rc = listed_fork(c, xl, &fork))) return rc;
+  if ((rc = listed_fork(c, d_u, xl, &fork))) return rc;
   LearnMesh lm{P<int>(c->vvoff), P<int>(c->vv), P<unsigned char>(c->listed), P<unsigned char>(c->vtile)};
   float4* vr = P<float4>(c->vr16);
   float4* rec = P<float4>(c->rec16);
   CK(cudaMemsetAsync(c->fbcount.p, 0, sizeof(int), c->stream));
   PB("prep_l");
-  learned_records(c, P<double>(c->f));
+  learned_records(c, d_u);
   PE();
   PB("mlp_l");
   CK(cudaMemsetAsync(c->mlp_err.p, 0, sizeof(int), c->stream));  // a wait that ran out is reported once
   learned_infer(m, lm, vr, P<float>(c->lsc), c->mlp_packed.p, rec, P<int>(c->fbitems), P<int>(c->fbcount), c->z_max,
                 c->use_mlp, c->max_degree, c->stall_polls, P<int>(c->mlp_err), c->stream);
   PE();
-  if ((rc = listed_join(c, xl, fork))) return rc;
+  if ((rc = listed_join(c, d_u, xl, fork))) return rc;
   PB("fallback_l");
   learned_fallback(m, lm, vr, P<float>(c->lsc), P<float>(c->wts), P<double>(c->rec), P<int>(c->fbitems),
                    P<int>(c->fbcount), m.V, rec, c->stream);
@@ -1970,13 +1987,14 @@ static int pass_learned(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint
   return check_launch(c, "learned pass");
 }
 
-static int pass_resident(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
+// the pass on a device field (read in place, in stream order)
+static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
   int rc;
   if (c->batch_n && c->precision != SPRG_FP32)
     return fail(c, SPRG_EINVAL, "a batch of meshes runs in SPRG_FP32 (per-mesh size factors)");
-  if (c->precision == SPRG_FP32) return pass_fast(c, adapt_ratio, d_split, d_collapse);
-  if (c->precision == SPRG_LEARNED) return pass_learned(c, adapt_ratio, d_split, d_collapse);
-  if ((rc = reset_status(c)) || (rc = step_grad(c, 1)) || (rc = step_recover(c)) ||
+  if (c->precision == SPRG_FP32) return pass_fast(c, d_u, adapt_ratio, d_split, d_collapse);
+  if (c->precision == SPRG_LEARNED) return pass_learned(c, d_u, adapt_ratio, d_split, d_collapse);
+  if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = step_recover(c)) ||
       (rc = step_size(c, 0, adapt_ratio, 0, 0, 0)))
     return rc;
   return step_measure_mark(c, d_split, d_collapse);
@@ -1989,9 +2007,7 @@ int sprg_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double adapt
   int rc = set_device(c);
   if (rc) return rc;
   c->launches = 0;
-  ENSURE(c->f, sizeof(double) * (size_t)c->m.V);
-  CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)c->m.V, cudaMemcpyDeviceToDevice, c->stream));
-  return pass_resident(c, adapt_ratio, d_split_bits, d_collapse_bits);
+  return pass_resident(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits);
 }
 
 int sprg_rounding_dominated(sprg_ctx* c, int* out) {
@@ -2011,19 +2027,19 @@ int sprg_rounding_dominated(sprg_ctx* c, int* out) {
 // two calls with a key, a captured graph from the third on
 static int e2e_pass(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
   const int call = c->e2e_calls++;
-  if (c->prof || c->e2e_off) return pass_resident(c, adapt_ratio, d_split, d_collapse);
+  if (c->prof || c->e2e_off) return pass_resident(c, P<double>(c->f), adapt_ratio, d_split, d_collapse);
   if (c->e2e_exec) {
     CK(cudaGraphLaunch(c->e2e_exec, c->stream));
     c->launches += c->e2e_launches;
     return SPRG_OK;
   }
-  if (call < 2) return pass_resident(c, adapt_ratio, d_split, d_collapse);
+  if (call < 2) return pass_resident(c, P<double>(c->f), adapt_ratio, d_split, d_collapse);
   const int64_t before = c->launches;
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
   int rc = SPRG_OK;
   if (e == cudaSuccess) {
-    rc = pass_resident(c, adapt_ratio, d_split, d_collapse);
+    rc = pass_resident(c, P<double>(c->f), adapt_ratio, d_split, d_collapse);
     e = cudaStreamEndCapture(c->stream, &graph);
     if (rc == SPRG_OK && e == cudaSuccess && graph) e = cudaGraphInstantiate(&c->e2e_exec, graph, 0);
   }
@@ -2039,7 +2055,7 @@ static int e2e_pass(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t
   c->e2e_exec = nullptr;
   c->e2e_off = true;
   c->launches = before;
-  return pass_resident(c, adapt_ratio, d_split, d_collapse);
+  return pass_resident(c, P<double>(c->f), adapt_ratio, d_split, d_collapse);
 }
 
 int sprg_estimate_and_mark(sprg_ctx* c, const double* u, double adapt_ratio, double* size_out, int32_t* flags,
@@ -2484,9 +2500,9 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
     if ((rc = hessian_operator_2d(c))) return rc;
     H = P<double>(c->rec9);
   } else {  // tets: the FP64 gradients and recoveries
-    if ((rc = step_grad(c, 1)) || (rc = step_recover(c))) return rc;
+    if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = step_recover(c))) return rc;
     CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
-    if ((rc = step_grad(c, 3)) || (rc = step_recover(c))) return rc;
+    if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = step_recover(c))) return rc;
     H = P<double>(c->rec);
   }
   ENSURE(c->met32, sizeof(float) * 12 * (size_t)(m.V > 0 ? m.V : 1));
@@ -2559,9 +2575,9 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
   if (c->precision == SPRG_FP32) return aniso_pass_mixed(c, eps, h_min, h_max, d_split_bits, d_collapse_bits, d_quality);
   // recovered gradient, then the recovered gradient of it (nodal Hessian)
-  if ((rc = step_grad(c, 1)) || (rc = step_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = step_recover(c))) return rc;
   CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
-  if ((rc = step_grad(c, 3)) || (rc = step_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = step_recover(c))) return rc;
   PB("hessian_metric");
   launch_hessian_metric(m, P<double>(c->rec), eps, h_min, h_max, P<double>(c->sizes3), P<double>(c->frames9),
                         c->stream);

@@ -16,22 +16,41 @@ void fast_prep_coords(const DevMesh& m, const double* frame, float4* vrec, cudaS
 // |cof J|_F^2 / |det J| over the elements
 void fast_geometry(const DevMesh& m, float2* geo, double2* geo64, double* cent, unsigned long long* qmax,
                    float* half_len, cudaStream_t s);
+// device words the pass's first kernel clears for the kernels after it
+struct PassCounters {
+  static constexpr int kCount = 7;
+  int* p[kCount];
+};
 // the pass's vertex records: coordinate records with the field pair (u_hi,
-// u_lo); umax_bits (zeroed by the caller): max |u_hi| as float bits
-void fast_prep(const DevMesh& m, const double* u, const float4* crec, float4* vrec, int* umax_bits, cudaStream_t s);
-// per tet: gradient value (3 floats) and packed correction (1 word)
+// u_lo); umax_part: max |u_hi| per block as float bits (fast_prep_blocks ints)
+int fast_prep_blocks(int V);
+void fast_prep(const DevMesh& m, const double* u, const float4* crec, float4* vrec, int* umax_part,
+               const PassCounters& pc, cudaStream_t s);
+// the listed patches' FP64 sums (n patches; patch it: vertex v[it], elements
+// el + it stride, wn[it] weights at w + woff[it], or -1: SPRG_EPATCH), into
+// rec64 (V x 3) and rec32 (32-byte records)
+struct ListedSums {
+  int n, stride;
+  const int* v;
+  const int* el;
+  const long long* woff;
+  const double* w;
+  const int* wn;
+  double* rec64;
+  float4* rec32;
+  DevStatus* st;
+};
+// per tet: gradient value (3 floats) and packed correction (1 word); also the
+// listed patches' sums
 // gscale = the frame's s (gradients in the mesh's coordinates); u: the FP64
-// field, read for the ill-conditioned tets solved in FP64
-// next_chunk: one device int (the kernel's work counter, cleared here)
+// field, read for the ill-conditioned tets solved in FP64 and the listed sums
+// next_chunk: one device int (the kernel's work counter, zero on entry)
 void fast_tet(const DevMesh& m, const float4* vrec, const double* u, float gscale, uint4* td, int* next_chunk,
-              cudaStream_t s);
+              const ListedSums& ls, cudaStream_t s);
 // once per mesh: SPR weights in patch-CSR order (FP32 for the pass, FP64 for
 // the guard), listed patches
 void fast_weights(const DevMesh& m, const double* cent, float* w, double* w64, ExpandList xl, int* n_refit,
                   unsigned char* listed, cudaStream_t s);
-// recovered value per vertex as a 32-byte record {s0, s1, s2, r0}, {r1, r2,
-// 0, 0}: the FP32 value and its FP32 remainder (listed vertices: from rec64)
-void fast_merge_ref(ExpandList xl, const double* rec64, float4* rec32, cudaStream_t s);
 // patch-size class per vertex: 0 (<= 8 elements), 1 (<= 16), 2 (<= 32), 3, 4 = listed
 void fast_patch_class(const DevMesh& m, const unsigned char* listed, unsigned char* cls, cudaStream_t s);
 // the bins' vertex order on the device: per-block class counts (4 ints per
@@ -61,20 +80,22 @@ void fast_slice_fill(const DevMesh& m, const BinSlices& bs, const int* verts, co
 // taken from a counter by a persistent grid; lanes 1, 2, 4 per vertex over
 // the patch-CSR lists, or 0: one per vertex over the sliced copy (tiles then
 // start on a slice); every tiling gives the same bits.  mode: the lane count
-// of every tile (a kernel for that mode alone), or -1 for mixed tiles
+// of every tile (a kernel for that mode alone), or -1 for mixed tiles; next:
+// the work counter, zero on entry.  Recovered values: 32-byte records {s0, s1,
+// s2, r0}, {r1, r2, 0, 0}, the FP32 value and its FP32 remainder
 void fast_recover_tiles(const DevMesh& m, const float* w, SlicedPatches sp, const uint4* td, float4* rec,
                         const int* verts, const int4* tiles, int n_tiles, int mode, int* next, int grid,
                         cudaStream_t s);
 // q: (h_max err^(-1/5), its relative error bound) per tet
 // seg (batch): one element range per block, nb = number of segments
 // done (one unsigned, zero between passes) and out3: the last block also
-// computes the size factor (one mesh; pass null for a batch); n_round (max
-// |u| from fast_prep) is replaced by the last block with 1 when the
-// reference's FP64 rounding of its IP gradients (bounded with qmax from
+// computes the size factor (one mesh; pass null for a batch) and sets n_round
+// to 1 when the reference's FP64 rounding of its IP gradients (bounded with
+// the field's largest value, umax_part from fast_prep, and qmax from
 // fast_geometry) could move the error integral by 1e-7 of it, else 0
 void fast_error(const DevMesh& m, const uint4* td, const float2* geo, const float4* rec, float2* q, double* partials,
-                int nb, const int2* seg, unsigned* done, double adapt_ratio, double* out3, int* n_round,
-                const unsigned long long* qmax, cudaStream_t s);
+                int nb, const int2* seg, unsigned* done, double adapt_ratio, double* out3, const int* umax_part,
+                int* n_round, const unsigned long long* qmax, cudaStream_t s);
 // sz2: (size, its relative error bound) per vertex
 void fast_average(const DevMesh& m, const float2* q, const double* out3, float2* sz2, BatchView bv, cudaStream_t s);
 void fast_measure(const DevMesh& m, const float* half_len, const float2* sz2, uint32_t* split, uint32_t* collapse,

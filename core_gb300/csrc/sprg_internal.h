@@ -239,7 +239,7 @@ struct GuardScratch {
   int* stamp;      // V ints, persistent (de-duplication stamps)
   int* stamp_id;   // device counter: this pass's stamp id (starts at 1; the decide stage bumps it)
   int* fit_items;  // fit_cap ints
-  int* fit_count;
+  int* fit_count;  // zero before the first stage
   int fit_cap;
   double* rec64;   // V x 3 doubles (FP64 recovered values of collected vertices)
   const double* w64;            // FP64 SPR weights in patch-CSR order

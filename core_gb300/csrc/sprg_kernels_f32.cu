@@ -38,6 +38,8 @@
 //   measure   thread per edge: metric length, split/collapse bitmaps, and the
 //             list of edges whose distance to 0.5 / 1.5 is within the error
 //             bound (re-decided in FP64 by the guard kernels)
+#include <algorithm>
+
 #include "sprg_fast.h"
 #include "sprg_ld.cuh"
 #include "sprg_reduce.cuh"
@@ -225,32 +227,49 @@ __device__ __forceinline__ float2 split_pair(double w) {
 
 // the pass's vertex records: the per-mesh coordinate records with the field
 // pair in the fourth slots, {x,y,z,u}_hi, {x,y,z,u}_lo (one sector per vertex)
-// (also the field's largest |u| in FP32, for the rounding-dominance test:
-// one atomic per block)
+// (also the field's largest |u| in FP32 per block, for the rounding-dominance
+// test in the error kernel's last block, and the pass's counters, which every
+// later kernel of the pass finds zero: six memsets of a few bytes were a third
+// of a small mesh's launches)
 __global__ void __launch_bounds__(kBlock) k_prep(int V, const double* __restrict__ u, const float4* __restrict__ crec,
-                                                 float4* __restrict__ vrec, int* __restrict__ umax_bits) {
+                                                 float4* __restrict__ vrec, int* __restrict__ umax_part,
+                                                 PassCounters pc) {
+  if (blockIdx.x == 0 && threadIdx.x < PassCounters::kCount) *pc.p[threadIdx.x] = 0;
   // |u_hi| as float bits: non-negative floats order as their bit patterns,
   // a NaN (sign cleared) above +inf, so an integer max keeps it
   int um = 0;
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < V) {
-    const float2 p = split_pair(__ldg(u + v));
-    float4 h = ld4(crec + 2 * (size_t)v), l = ld4(crec + 2 * (size_t)v + 1);
-    h.w = p.x;
-    l.w = p.y;
-    vrec[2 * (size_t)v] = h;
-    vrec[2 * (size_t)v + 1] = l;
-    um = __float_as_int(p.x) & 0x7fffffff;
-  }
+  constexpr int U = 4;  // vertices a thread loads before it stores any
+  const long step = (long)gridDim.x * blockDim.x;
+  for (long v0 = blockIdx.x * (long)blockDim.x + threadIdx.x; v0 < V; v0 += U * step) {
+    double w[U];
+    float4 h[U], l[U];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) um = max(um, __shfl_xor_sync(0xffffffffu, um, o));
+    for (int j = 0; j < U; ++j) {
+      const long v = min(v0 + j * step, (long)V - 1);
+      w[j] = __ldg(u + v);
+      h[j] = ld4(crec + 2 * (size_t)v);
+      l[j] = ld4(crec + 2 * (size_t)v + 1);
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const long v = v0 + j * step;
+      if (v >= V) break;
+      const float2 p = split_pair(w[j]);
+      h[j].w = p.x;
+      l[j].w = p.y;
+      vrec[2 * (size_t)v] = h[j];
+      vrec[2 * (size_t)v + 1] = l[j];
+      um = max(um, __float_as_int(p.x) & 0x7fffffff);
+    }
+  }
+  um = __reduce_max_sync(0xffffffffu, um);
   __shared__ int sw[kBlock / 32];
   if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = um;
   __syncthreads();
   if (threadIdx.x == 0) {
     int b = sw[0];
     for (int i = 1; i < kBlock / 32; ++i) b = max(b, sw[i]);
-    if (b != 0) atomicMax(umax_bits, b);
+    umax_part[blockIdx.x] = b;
   }
 }
 
@@ -376,13 +395,12 @@ __device__ __forceinline__ TetData load_tet(const float4* __restrict__ vr, int4 
 // ---------------------------------------------------------------------------
 // tet: gradient value and packed correction
 // ---------------------------------------------------------------------------
-// Blocks take chunks of kTetChunk x blockDim elements from a counter (so a
-// kernel running beside this one, such as the listed patches' FP64 fits on
-// the side stream, only delays the chunks of the blocks it displaces); in a
-// chunk each thread loads the next element's vertex ids before working on
-// the current one, so only the record gathers (mostly L2 hits) stay on the
-// dependent chain.
-constexpr int kTetChunk = 8;
+// Blocks take chunks from a counter: first the listed patches' FP64 sums, a
+// warp each (the pass's longest chains, and they read the field only), then
+// `per` x blockDim elements at a time; in a chunk each thread loads the next
+// element's vertex ids before working on the current one, so only the record
+// gathers (mostly L2 hits) stay on the dependent chain.
+constexpr int kTetChunk = 8;  // the largest `per`; smaller where the chunks would not fill the grid
 
 // The gradient of an ill-conditioned tet from the mesh's FP64 coordinates and
 // field: J g = du solved with FP64 cofactors (the FP64 path's arithmetic,
@@ -419,17 +437,86 @@ __device__ __noinline__ uint4 tet_grad_f64(const double* __restrict__ xyz, const
                     pack_corr(s[0], s[1], s[2], r[0], r[1], r[2]));
 }
 
-__global__ void __launch_bounds__(kBlock, 4) k_fast_tet(DevMesh m, const float4* __restrict__ vr, const double* __restrict__ u,
-                                                        float gscale, uint4* __restrict__ td, int* __restrict__ next_chunk) {
+// rec(v) = sum_i w_i g_i over a listed vertex's grown patch (its FP64 weights
+// from the reference's QR, FP64 gradients of the field), by one warp: lanes over
+// the elements, fixed reduction tree.  Stored in FP64 for the guard and as the
+// 32-byte record of the other vertices.  These sums ran in a kernel of their
+// own beside this one, joined by two events and merged by a third kernel: on a
+// small mesh that chain was the pass's critical path.
+__device__ __noinline__ void listed_sum(const DevMesh& m, const double* __restrict__ u, const ListedSums& ls, int it) {
+  const int lane = threadIdx.x & 31;
+  const int v = ls.v[it], n = ls.wn[it];
+  if (n < 0) {
+    if (lane == 0 && atomicCAS(&ls.st->code, 0, SPRG_EPATCH) == 0) ls.st->where = v;
+    return;
+  }
+  const int* el = ls.el + (size_t)it * ls.stride;
+  const double* wi = ls.w + ls.woff[it];
+  double acc[3] = {0, 0, 0};
+  for (int i = lane; i < n; i += 32) {
+    const int4 tv = __ldg(reinterpret_cast<const int4*>(m.ev) + el[i]);
+    const int id[4] = {tv.x, tv.y, tv.z, tv.w};
+    double x[4][3], e[3][3], du[3];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) x[a][k] = __ldg(m.xyz + 3 * (size_t)id[a] + k);
+    const double u0 = __ldg(u + id[0]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      du[a] = __ldg(u + id[a + 1]) - u0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) e[a][k] = x[a + 1][k] - x[0][k];
+    }
+    double cf[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double* p = e[(a + 1) % 3];
+      const double* q = e[(a + 2) % 3];
+      cf[a][0] = p[1] * q[2] - p[2] * q[1];
+      cf[a][1] = p[2] * q[0] - p[0] * q[2];
+      cf[a][2] = p[0] * q[1] - p[1] * q[0];
+    }
+    const double wk = wi[i] / (e[0][0] * cf[0][0] + e[0][1] * cf[0][1] + e[0][2] * cf[0][2]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc[k] += wk * (cf[0][k] * du[0] + cf[1][k] * du[1] + cf[2][k] * du[2]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+  if (lane == 0) {
+    float h[3], l[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      ls.rec64[3 * (size_t)v + k] = acc[k];
+      h[k] = (float)acc[k];
+      l[k] = (float)(acc[k] - (double)h[k]);
+    }
+    ls.rec32[2 * (size_t)v] = make_float4(h[0], h[1], h[2], l[0]);
+    ls.rec32[2 * (size_t)v + 1] = make_float4(l[1], l[2], 0.f, 0.f);
+  }
+}
+
+__global__ void __launch_bounds__(kBlock, 4)
+    k_fast_tet(const __grid_constant__ DevMesh m, const float4* __restrict__ vr, const double* __restrict__ u, float gscale,
+               uint4* __restrict__ td, int* __restrict__ next_chunk, int per, const __grid_constant__ ListedSums ls) {
   const int4* __restrict__ ev4 = reinterpret_cast<const int4*>(m.ev);
+  const int n_lc = (ls.n + kBlock / 32 - 1) / (kBlock / 32);
   __shared__ int chunk;
   for (;;) {
     if (threadIdx.x == 0) chunk = atomicAdd(next_chunk, 1);
     __syncthreads();
-    const long t0 = (long)chunk * (kTetChunk * kBlock);
+    const int c = chunk;
     __syncthreads();
+    if (c < n_lc) {
+      const int it = c * (kBlock / 32) + (threadIdx.x >> 5);
+      if (it < ls.n) listed_sum(m, u, ls, it);
+      continue;
+    }
+    const long t0 = (long)(c - n_lc) * (per * kBlock);
     if (t0 >= m.T) break;  // every thread of the block leaves here together
-    const int t_end = (int)min((long)m.T, t0 + kTetChunk * kBlock);
+    const int t_end = (int)min((long)m.T, t0 + per * kBlock);
     int t = (int)t0 + threadIdx.x;
     int4 next = t < t_end ? __ldg(ev4 + t) : make_int4(0, 0, 0, 0);
     for (; t < t_end; t += kBlock) {
@@ -872,19 +959,6 @@ __global__ void __launch_bounds__(kBinBlock) k_bin_scatter(int V, const unsigned
   }
 }
 
-// listed vertices take the FP64 reference result, as value + remainder
-__global__ void k_merge_ref(const int* __restrict__ items, const int* __restrict__ count, int cap,
-                            const double* __restrict__ rec64, float4* __restrict__ rec) {
-  int n = min(*count, cap);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int v = items[i];
-    double a = rec64[3 * (size_t)v], b = rec64[3 * (size_t)v + 1], c = rec64[3 * (size_t)v + 2];
-    float ah = (float)a, bh = (float)b, ch = (float)c;
-    rec[2 * (size_t)v] = make_float4(ah, bh, ch, (float)(a - ah));
-    rec[2 * (size_t)v + 1] = make_float4((float)(b - bh), (float)(c - ch), 0.f, 0.f);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // error: thread per tet, grid-stride over a fixed grid
 // ---------------------------------------------------------------------------
@@ -922,7 +996,8 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
                                                        const float4* __restrict__ rec, float2* __restrict__ q,
                                                        double* __restrict__ partials, const int2* __restrict__ seg,
                                                        unsigned* __restrict__ done, double adapt_ratio, int dim,
-                                                       double* __restrict__ out3, int* __restrict__ n_round,
+                                                       double* __restrict__ out3, const int* __restrict__ umax_part,
+                                                       int n_umax, int* __restrict__ n_round,
                                                        const unsigned long long* __restrict__ qmax) {
   __shared__ double sh[2][kBlock / 32];
   PairSum self{0.f, 0.f}, gsum{0.f, 0.f};
@@ -1039,6 +1114,13 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
   if (!last) return;
   __threadfence();  // every block's partials are visible to the last one
   __shared__ double shr[kBlock / 32];
+  __shared__ int umax;
+  if (threadIdx.x == 0) umax = 0;
+  __syncthreads();
+  int um = 0;
+  for (int i = threadIdx.x; i < n_umax; i += kBlock) um = max(um, __ldg(umax_part + i));
+  um = __reduce_max_sync(0xffffffffu, um);
+  if ((threadIdx.x & 31) == 0) atomicMax(&umax, um);
   rd_size_factor(partials, gridDim.x, 0, adapt_ratio, 0.0, dim, out3, shr);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1053,8 +1135,8 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
     // field, one offset far above its variation): 1 here, else 0.  (max|u|
     // from the prep kernel, the largest |cof|^2 / |det| once per mesh.)
     const double G = out3[1];
-    const double um = (double)__int_as_float(*n_round);
-    const double en = 0x1p-84 / 6.0 * um * um * __longlong_as_double((long long)*qmax);
+    const double uf = (double)__int_as_float(umax);
+    const double en = 0x1p-84 / 6.0 * uf * uf * __longlong_as_double((long long)*qmax);
     const double worst = (double)m.T * pow(en, 0.6);
     *n_round = (!(worst <= 1e-7 * G) || !(G > 0.0)) ? 1 : 0;
   }
@@ -1233,17 +1315,16 @@ int error_grid() {
 }
 
 // the tet kernel runs one full wave of resident blocks as well
-int tet_grid(int T) {
+int tet_wave() {
   static int grid = 0;
   if (!grid) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fast_tet, kBlock, 0);
-    grid = (sms > 0 ? sms : 152) * (per_sm > 0 ? per_sm : 5);
+    grid = (sms > 0 ? sms : 152) * (per_sm > 0 ? per_sm : 4);
   }
-  const int nb = (int)((T + (long)kTetChunk * kBlock - 1) / ((long)kTetChunk * kBlock));
-  return nb < grid ? nb : grid;
+  return grid;
 }
 
 }  // namespace
@@ -1264,15 +1345,20 @@ void fast_geometry(const DevMesh& m, float2* geo, double2* geo64, double* cent, 
   if (m.E) k_fast_elen<<<nblk(m.E), kBlock, 0, s>>>(m, half_len);
 }
 
-void fast_prep(const DevMesh& m, const double* u, const float4* crec, float4* vrec, int* umax_bits, cudaStream_t s) {
-  if (m.V) k_prep<<<nblk(m.V), kBlock, 0, s>>>(m.V, u, crec, vrec, umax_bits);
+int fast_prep_blocks(int V) { return std::min(nblk(V), 152 * 8); }
+
+void fast_prep(const DevMesh& m, const double* u, const float4* crec, float4* vrec, int* umax_part,
+               const PassCounters& pc, cudaStream_t s) {
+  if (m.V) k_prep<<<fast_prep_blocks(m.V), kBlock, 0, s>>>(m.V, u, crec, vrec, umax_part, pc);
 }
 
 void fast_tet(const DevMesh& m, const float4* vrec, const double* u, float gscale, uint4* td, int* next_chunk,
-              cudaStream_t s) {
+              const ListedSums& ls, cudaStream_t s) {
   if (!m.T) return;
-  cudaMemsetAsync(next_chunk, 0, sizeof(int), s);
-  k_fast_tet<<<tet_grid(m.T), kBlock, 0, s>>>(m, vrec, u, gscale, td, next_chunk);
+  const long wave = tet_wave();
+  const int per = (int)std::max(1L, std::min((long)kTetChunk, (long)m.T / (wave * kBlock)));
+  const long chunks = ((long)m.T + (long)per * kBlock - 1) / ((long)per * kBlock) + (ls.n + kBlock / 32 - 1) / (kBlock / 32);
+  k_fast_tet<<<(int)std::min(wave, chunks), kBlock, 0, s>>>(m, vrec, u, gscale, td, next_chunk, per, ls);
 }
 
 void fast_weights(const DevMesh& m, const double* cent, float* w, double* w64, ExpandList xl, int* n_refit,
@@ -1298,8 +1384,8 @@ void fast_bin_scatter(int V, const unsigned char* cls, const int* offs, int* ord
 void fast_recover_tiles(const DevMesh& m, const float* w, SlicedPatches sp, const uint4* td, float4* rec,
                         const int* verts, const int4* tiles, int n_tiles, int mode, int* next, int grid,
                         cudaStream_t s) {
-  cudaMemsetAsync(next, 0, sizeof(int), s);
   if (!n_tiles) return;
+  grid = std::min(grid, n_tiles);
   switch (mode) {
     case 0: k_fast_recover_tiles<0><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
     case 1: k_fast_recover_tiles<1><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
@@ -1318,16 +1404,12 @@ void fast_slice_fill(const DevMesh& m, const BinSlices& bs, const int* verts, co
   if (bs.start[4]) k_slice_fill<<<nblk(bs.start[4]), kBlock, 0, s>>>(m, bs, verts, w, off, sel, sw);
 }
 
-void fast_merge_ref(ExpandList xl, const double* rec64, float4* rec, cudaStream_t s) {
-  k_merge_ref<<<152, 256, 0, s>>>(xl.items, xl.count, xl.cap, rec64, rec);
-}
-
 void fast_error(const DevMesh& m, const uint4* td, const float2* geo, const float4* rec, float2* q, double* partials,
-                int nb, const int2* seg, unsigned* done, double adapt_ratio, double* out3, int* n_round,
-                const unsigned long long* qmax, cudaStream_t s) {
+                int nb, const int2* seg, unsigned* done, double adapt_ratio, double* out3, const int* umax_part,
+                int* n_round, const unsigned long long* qmax, cudaStream_t s) {
   if (nb)
-    k_fast_error<<<nb, kBlock, 0, s>>>(m, td, geo, rec, q, partials, seg, done, adapt_ratio, m.dim, out3, n_round,
-                                       qmax);
+    k_fast_error<<<nb, kBlock, 0, s>>>(m, td, geo, rec, q, partials, seg, done, adapt_ratio, m.dim, out3, umax_part,
+                                       fast_prep_blocks(m.V), n_round, qmax);
 }
 
 void fast_average(const DevMesh& m, const float2* q, const double* out3, float2* sz2, BatchView bv, cudaStream_t s) {

@@ -2556,7 +2556,6 @@ void launch_guard_stage(int stage, const DevMesh& m, const double* u, const doub
                         GuardScratch g, BatchView bv, cudaStream_t s) {
   switch (stage) {
     case 0:
-      cudaMemsetAsync(g.fit_count, 0, sizeof(int), s);
       k_guard_collect<<<152 * 4, 256, 0, s>>>(m, items, count, cap, g.stamp_id, g.stamp, g.fit_items, g.fit_count,
                                           g.fit_cap, unresolved);
       break;
