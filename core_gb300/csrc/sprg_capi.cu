@@ -1992,6 +1992,11 @@ static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uin
   int rc;
   if (c->batch_n && c->precision != SPRG_FP32)
     return fail(c, SPRG_EINVAL, "a batch of meshes runs in SPRG_FP32 (per-mesh size factors)");
+  {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(c->stream, &cap));
+    c->m.early = c->m.T <= (cap == cudaStreamCaptureStatusActive ? 2 << 20 : 6 << 20);
+  }
   if (c->precision == SPRG_FP32) return pass_fast(c, d_u, adapt_ratio, d_split, d_collapse);
   if (c->precision == SPRG_LEARNED) return pass_learned(c, d_u, adapt_ratio, d_split, d_collapse);
   if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = step_recover(c)) ||

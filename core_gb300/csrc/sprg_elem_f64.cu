@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __res
                                                   double* __restrict__ err, double* __restrict__ esize,
                                                   double* __restrict__ partials, unsigned* __restrict__ done, int mode,
                                                   double adapt_ratio, double target, double* __restrict__ out3) {
+  after_previous(geo, ip, rec);
   __shared__ double sh[kBlock / 32];
   double self_sum = 0, g_sum = 0;
   double N[4];
@@ -322,6 +323,7 @@ template <int D, bool REC>
 __global__ void __launch_bounds__(kBlock) k_esize(DevMesh m, const double* __restrict__ geo,
                                                   const double* __restrict__ out3, int mode, double alpha, double beta,
                                                   double* __restrict__ esize) {
+  after_previous(geo, out3);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.T) return;
   const double sf = out3[2];
@@ -347,6 +349,7 @@ __global__ void __launch_bounds__(kBlock) k_esize(DevMesh m, const double* __res
 
 __global__ void __launch_bounds__(kBlock) k_average(DevMesh m, const double* __restrict__ esize,
                                                     double* __restrict__ size) {
+  after_previous(esize);
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= m.V) return;
   int b = m.a_off[v], e = m.a_off[v + 1];
@@ -390,6 +393,7 @@ __global__ void __launch_bounds__(kBlock) k_measure_mark(DevMesh m, const double
                                                          const double* __restrict__ size, double* __restrict__ L,
                                                          uint32_t* __restrict__ split,
                                                          uint32_t* __restrict__ collapse) {
+  after_previous(len, size);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   bool sp = false, co = false;
   if (e < m.E) {
@@ -451,7 +455,7 @@ void launch_error_f64(const DevMesh& m, const double* geo, const double* ip, int
                       double target, double* out3, cudaStream_t s) {
   if (!n_blocks) return;
   auto go = [&](auto kernel) {
-    kernel<<<n_blocks, kBlock, 0, s>>>(m, geo, ip, rec, err, esize, partials, done, mode, adapt_ratio, target, out3);
+    launch_after(m.early, kernel, n_blocks, kBlock, s, m, geo, ip, rec, err, esize, partials, done, mode, adapt_ratio, target, out3);
   };
   if (m.dim == 3) {
     if (nc == 3) go(geo ? k_error<3, 3, true> : k_error<3, 3, false>);
@@ -465,13 +469,13 @@ void launch_error_f64(const DevMesh& m, const double* geo, const double* ip, int
 void launch_esize_f64(const DevMesh& m, const double* geo, const double* out3, int mode, double alpha, double beta,
                       double* esize, cudaStream_t s) {
   if (!m.T) return;
-  auto go = [&](auto kernel) { kernel<<<nblk(m.T), kBlock, 0, s>>>(m, geo, out3, mode, alpha, beta, esize); };
+  auto go = [&](auto kernel) { launch_after(m.early, kernel, nblk(m.T), kBlock, s, m, geo, out3, mode, alpha, beta, esize); };
   if (m.dim == 3) go(geo ? k_esize<3, true> : k_esize<3, false>);
   else go(geo ? k_esize<2, true> : k_esize<2, false>);
 }
 
 void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s) {
-  if (m.V) k_average<<<nblk(m.V), kBlock, 0, s>>>(m, esize, size);
+  if (m.V) launch_after(m.early, k_average, nblk(m.V), kBlock, s, m, esize, size);
 }
 
 void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s) {
@@ -485,8 +489,7 @@ void launch_edge_records(const DevMesh& m, double* len, cudaStream_t s) {
 void launch_measure_mark_f64(const DevMesh& m, const double* len, const double* size, double* L, uint32_t* split,
                              uint32_t* collapse, cudaStream_t s) {
   if (!m.E) return;
-  if (len) k_measure_mark<true><<<nblk(m.E), kBlock, 0, s>>>(m, len, size, L, split, collapse);
-  else k_measure_mark<false><<<nblk(m.E), kBlock, 0, s>>>(m, len, size, L, split, collapse);
+  launch_after(m.early, len ? k_measure_mark<true> : k_measure_mark<false>, nblk(m.E), kBlock, s, m, len, size, L, split, collapse);
 }
 
 }  // namespace sprg

@@ -23,6 +23,7 @@ struct DevMesh {
   const int* p_el;
   const int* a_off;    // V + 1, averaging CSR (reference getAdjacent order)
   const int* a_el;
+  bool early;          // launches of this pass: see launch_after
 };
 
 // A batch of independent meshes flattened into one context (disjoint union,
@@ -52,6 +53,43 @@ __device__ __forceinline__ int batch_mesh(const BatchView& b, int v) {
 // the size factor that applies at vertex v
 __device__ __forceinline__ double batch_sf(const BatchView& b, const double* out3, int v) {
   return b.n ? out3[4 * batch_mesh(b, v) + 2] : out3[2];
+}
+
+// Programmatic dependent launch: a kernel launched with launch_after may be set
+// up while the kernel before it on the stream drains; it calls
+// after_previous() before it reads anything a kernel before it wrote.  On a
+// small mesh the launch gaps are as long as the kernels.  The first statement
+// lets the kernel after this one be set up in turn (once every block of this
+// one has started), the second waits until the one before is complete and
+// its writes are visible; both do nothing in an ordinary launch.
+// early (DevMesh::early, set per pass): whether to.  Direct passes gain 18 us
+// at 3k tets and 11 us at 6M (the host's launches and the kernels' set-up
+// overlap), passes being captured into a graph 4 us at 3k, 2 at 1.6M and
+// nothing at 3M; at 13M tets both are slower by 40 to 58 us (the waiting
+// blocks take the slots that the tail of the kernel before would fill), so
+// the lines lie at 6M and 2M tets.
+// The kernel's inputs that a kernel before it (back to the last ordinary launch)
+// wrote go through it: a pointer to const with __restrict__ is memory that does not change during the kernel, so the
+// compiler may move its loads above the wait; values that come out of an asm
+// behind it cannot be used earlier.
+template <class... P>
+__device__ __forceinline__ void after_previous(P&... p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (void)(([&] { asm volatile("" : "+l"(p)::"memory"); }(), 0) + ... + 0);
+}
+template <class... P, class... A>
+inline void launch_after(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 // Device status word written by kernels (first error wins).

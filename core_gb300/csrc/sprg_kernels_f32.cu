@@ -501,6 +501,7 @@ __device__ __noinline__ void listed_sum(const DevMesh& m, const double* __restri
 __global__ void __launch_bounds__(kBlock, 4)
     k_fast_tet(const __grid_constant__ DevMesh m, const float4* __restrict__ vr, const double* __restrict__ u, float gscale,
                uint4* __restrict__ td, int* __restrict__ next_chunk, int per, const __grid_constant__ ListedSums ls) {
+  after_previous(vr);
   const int4* __restrict__ ev4 = reinterpret_cast<const int4*>(m.ev);
   const int n_lc = (ls.n + kBlock / 32 - 1) / (kBlock / 32);
   __shared__ int chunk;
@@ -853,6 +854,7 @@ __global__ void __launch_bounds__(kBlock, MODE <= 0 ? 4 : 5)
     k_fast_recover_tiles(DevMesh m, const float* __restrict__ w, SlicedPatches sp, const uint4* __restrict__ td,
                          float4* __restrict__ rec, const int* __restrict__ verts, const int4* __restrict__ tiles,
                          int n_tiles, int* __restrict__ next) {
+  after_previous(td);
   __shared__ int cur;
   for (;;) {
     if (threadIdx.x == 0) cur = atomicAdd(next, 1);
@@ -999,6 +1001,7 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
                                                        double* __restrict__ out3, const int* __restrict__ umax_part,
                                                        int n_umax, int* __restrict__ n_round,
                                                        const unsigned long long* __restrict__ qmax) {
+  after_previous(td, rec, umax_part);
   __shared__ double sh[2][kBlock / 32];
   PairSum self{0.f, 0.f}, gsum{0.f, 0.f};
   int t_beg = blockIdx.x * blockDim.x + threadIdx.x, t_end = m.T, t_step = gridDim.x * blockDim.x;
@@ -1148,6 +1151,7 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
 __global__ void __launch_bounds__(kBlock) k_fast_average(DevMesh m, const float2* __restrict__ q,
                                                          const double* __restrict__ out3, float2* __restrict__ sz2,
                                                          BatchView bv) {
+  after_previous(q, out3);
   // kGroup lanes per vertex; each lane sums every kGroup-th entry with a
   // compensated sum, the lane sums are combined in a fixed order.  The
   // size's relative error bound is the q-weighted mean of the element
@@ -1224,6 +1228,7 @@ __global__ void __launch_bounds__(kBlock) k_fast_measure(DevMesh m, const float*
                                                          uint32_t* __restrict__ collapse, int* __restrict__ guard_items,
                                                          int* __restrict__ guard_count, int guard_cap,
                                                          float guard_rel) {
+  after_previous(sz2);
   const int lane = threadIdx.x & 31;
   const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const int e0 = (int)(warp * 128) + lane;
@@ -1358,7 +1363,7 @@ void fast_tet(const DevMesh& m, const float4* vrec, const double* u, float gscal
   const long wave = tet_wave();
   const int per = (int)std::max(1L, std::min((long)kTetChunk, (long)m.T / (wave * kBlock)));
   const long chunks = ((long)m.T + (long)per * kBlock - 1) / ((long)per * kBlock) + (ls.n + kBlock / 32 - 1) / (kBlock / 32);
-  k_fast_tet<<<(int)std::min(wave, chunks), kBlock, 0, s>>>(m, vrec, u, gscale, td, next_chunk, per, ls);
+  launch_after(m.early, k_fast_tet, (int)std::min(wave, chunks), kBlock, s, m, vrec, u, gscale, td, next_chunk, per, ls);
 }
 
 void fast_weights(const DevMesh& m, const double* cent, float* w, double* w64, ExpandList xl, int* n_refit,
@@ -1386,12 +1391,13 @@ void fast_recover_tiles(const DevMesh& m, const float* w, SlicedPatches sp, cons
                         cudaStream_t s) {
   if (!n_tiles) return;
   grid = std::min(grid, n_tiles);
+  auto go = [&](auto kernel) { launch_after(m.early, kernel, grid, kBlock, s, m, w, sp, td, rec, verts, tiles, n_tiles, next); };
   switch (mode) {
-    case 0: k_fast_recover_tiles<0><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
-    case 1: k_fast_recover_tiles<1><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
-    case 2: k_fast_recover_tiles<2><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
-    case 4: k_fast_recover_tiles<4><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next); break;
-    default: k_fast_recover_tiles<-1><<<grid, kBlock, 0, s>>>(m, w, sp, td, rec, verts, tiles, n_tiles, next);
+    case 0: go(k_fast_recover_tiles<0>); break;
+    case 1: go(k_fast_recover_tiles<1>); break;
+    case 2: go(k_fast_recover_tiles<2>); break;
+    case 4: go(k_fast_recover_tiles<4>); break;
+    default: go(k_fast_recover_tiles<-1>);
   }
 }
 
@@ -1408,19 +1414,19 @@ void fast_error(const DevMesh& m, const uint4* td, const float2* geo, const floa
                 int nb, const int2* seg, unsigned* done, double adapt_ratio, double* out3, const int* umax_part,
                 int* n_round, const unsigned long long* qmax, cudaStream_t s) {
   if (nb)
-    k_fast_error<<<nb, kBlock, 0, s>>>(m, td, geo, rec, q, partials, seg, done, adapt_ratio, m.dim, out3, umax_part,
-                                       fast_prep_blocks(m.V), n_round, qmax);
+    launch_after(m.early, k_fast_error, nb, kBlock, s, m, td, geo, rec, q, partials, seg, done, adapt_ratio, m.dim, out3,
+                 umax_part, fast_prep_blocks(m.V), n_round, qmax);
 }
 
 void fast_average(const DevMesh& m, const float2* q, const double* out3, float2* sz2, BatchView bv, cudaStream_t s) {
-  if (m.V) k_fast_average<<<nblk((long)m.V * kGroup), kBlock, 0, s>>>(m, q, out3, sz2, bv);
+  if (m.V) launch_after(m.early, k_fast_average, nblk((long)m.V * kGroup), kBlock, s, m, q, out3, sz2, bv);
 }
 
 void fast_measure(const DevMesh& m, const float* half_len, const float2* sz2, uint32_t* split, uint32_t* collapse,
                   int* guard_items, int* guard_count, int guard_cap, float guard_rel, cudaStream_t s) {
   if (m.E)
-    k_fast_measure<<<nblk((m.E + 3) / 4), kBlock, 0, s>>>(m, half_len, sz2, split, collapse, guard_items, guard_count,
-                                                          guard_cap, guard_rel);
+    launch_after(m.early, k_fast_measure, nblk((m.E + 3) / 4), kBlock, s, m, half_len, sz2, split, collapse, guard_items,
+                 guard_count, guard_cap, guard_rel);
 }
 
 void fast_size_to_f64(int V, const float2* sz2, double* s64, cudaStream_t s) {

@@ -740,6 +740,7 @@ __global__ void __launch_bounds__(kBlock) k_cached_wsum(DevMesh m, const double*
                                                         const long long* __restrict__ woff,
                                                         const double* __restrict__ w, const int* __restrict__ wn,
                                                         DevStatus* st) {
+  after_previous(ip, u, cache_v, cache_el, woff, w, wn);
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (blockDim.x >> 5);
   for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < n_cached; it += nwarps) {
@@ -1051,6 +1052,7 @@ __global__ void k_guard_collect(DevMesh m, const int* __restrict__ items, const 
                                 const int* __restrict__ stamp_id_ptr, int* __restrict__ stamp,
                                 int* __restrict__ fit_items,
                                 int* __restrict__ fit_count, int fit_cap, int* __restrict__ unresolved) {
+  after_previous(items, count, stamp_id_ptr);
   // warp per (edge, end): lanes over the end's elements in rounds of 32
   const int n = min(*count, cap);
   const int stamp_id = *stamp_id_ptr;
@@ -1083,6 +1085,7 @@ __global__ void k_guard_collect(DevMesh m, const int* __restrict__ items, const 
 // patches take their FP64 reference (QR, grown patch) result
 __global__ void k_guard_fit(DevMesh m, const double* __restrict__ u, const int* __restrict__ fit_items,
                             const int* __restrict__ fit_count, int fit_cap, GuardScratch g) {
+  after_previous(fit_items, fit_count);
   const int n = min(*fit_count, fit_cap);
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (blockDim.x >> 5);
@@ -1122,6 +1125,7 @@ __global__ void __launch_bounds__(128) k_guard_decide(DevMesh m, const double* _
                                                       const int* __restrict__ items, const int* __restrict__ count,
                                                       int cap, uint32_t* split, uint32_t* collapse,
                                                       int* __restrict__ unresolved, BatchView bv) {
+  after_previous(out3, items, count);
   // the stamp id of the next guard pass (the collect stage of this one is
   // done): a device counter, so a pass replayed from a CUDA graph still
   // de-duplicates with a fresh id; 0, the stamps' initial value, is skipped
@@ -2439,6 +2443,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
                                                         const double* __restrict__ w,
                                                         const unsigned char* __restrict__ listed,
                                                         double* __restrict__ rec) {
+  after_previous(ip, w, listed);
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= m.V || listed[v]) return;
   const int beg = m.p_off[v], end = m.p_off[v + 1];
@@ -2514,8 +2519,8 @@ void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u,
                             const int* cache_v, const int* cache_el, const long long* woff, const double* w,
                             const int* wn, DevStatus* st, cudaStream_t s) {
   if (n_cached > 0)
-    k_cached_wsum<<<std::min(nblk((long)n_cached * 32), 152 * 8), kBlock, 0, s>>>(m, ip, u, nc, rec, n_cached, cache_v,
-                                                                                cache_el, woff, w, wn, st);
+    launch_after(m.early, k_cached_wsum, std::min(nblk((long)n_cached * 32), 152 * 8), kBlock, s, m, ip, u, nc, rec, n_cached,
+                 cache_v, cache_el, woff, w, wn, st);
 }
 
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target, int dim,
@@ -2556,14 +2561,14 @@ void launch_guard_stage(int stage, const DevMesh& m, const double* u, const doub
                         GuardScratch g, BatchView bv, cudaStream_t s) {
   switch (stage) {
     case 0:
-      k_guard_collect<<<152 * 4, 256, 0, s>>>(m, items, count, cap, g.stamp_id, g.stamp, g.fit_items, g.fit_count,
-                                          g.fit_cap, unresolved);
+      launch_after(m.early, k_guard_collect, 152 * 4, 256, s, m, items, count, cap, g.stamp_id, g.stamp, g.fit_items, g.fit_count,
+                   g.fit_cap, unresolved);
       break;
     case 1:
-      k_guard_fit<<<152 * 8, 256, 0, s>>>(m, u, g.fit_items, g.fit_count, g.fit_cap, g);
+      launch_after(m.early, k_guard_fit, 152 * 8, 256, s, m, u, g.fit_items, g.fit_count, g.fit_cap, g);
       break;
     default:
-      k_guard_decide<<<152 * 4, 128, 0, s>>>(m, u, out3, g, items, count, cap, split, collapse, unresolved, bv);
+      launch_after(m.early, k_guard_decide, 152 * 4, 128, s, m, u, out3, g, items, count, cap, split, collapse, unresolved, bv);
   }
 }
 
@@ -2734,8 +2739,7 @@ void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, Expan
 void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
                         double* rec, cudaStream_t s) {
   if (!m.V) return;
-  if (nc == 3) k_recover_w64<3><<<nblk(m.V), kBlock, 0, s>>>(m, ip, w, listed, rec);
-  else k_recover_w64<9><<<nblk(m.V), kBlock, 0, s>>>(m, ip, w, listed, rec);
+  launch_after(m.early, nc == 3 ? k_recover_w64<3> : k_recover_w64<9>, nblk(m.V), kBlock, s, m, ip, w, listed, rec);
 }
 
 }  // namespace sprg

@@ -378,3 +378,48 @@ def test_updates_in_a_row(gpu_lib, precision):
                 c.update_mesh(m)
             got = c.estimate_and_mark(workload.sine_field(m.coords), 0.1)
             assert np.array_equal(got[0], want[i][0]) and np.array_equal(got[1], want[i][1])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "learned"])
+@pytest.mark.parametrize("n", [2, 8, 23])
+@pytest.mark.parametrize("graph", [False, True])
+def test_resident_passes_back_to_back(gpu_lib, precision, n, graph):
+    """Sixty passes enqueued without a wait, the field changing between them on
+    the same stream: each pass's marks are those of a fresh context (the
+    kernels of a pass are launched while the ones before them drain)."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m = workload.box(n, jitter=0.2, seed=2)
+    E, ratio = m.n_edges, 1.28 / n
+    nw = (E + 31) // 32
+    us = [workload.bump_field(m.coords, seed=s) for s in (1, 2, 3)]
+    want = []
+    for u in us:
+        with cg.Context(m, precision=precision) as c:
+            want.append(c.estimate_and_mark(u, ratio)[1])
+    stream = torch.cuda.Stream()
+    with cg.Context(m, precision=precision) as c, torch.cuda.stream(stream):
+        c.set_stream(stream.cuda_stream)
+        fields = torch.from_numpy(np.stack(us)).cuda()
+        d_u = fields[0].clone()
+        bits = torch.zeros((2, nw), dtype=torch.int32, device="cuda")
+        ptrs = (d_u.data_ptr(), ratio, bits[0].data_ptr(), bits[1].data_ptr())
+        if graph:
+            c.graph_capture(*ptrs)
+        kept = []
+        for i in range(60):
+            d_u.copy_(fields[i % 3])
+            if graph:
+                c.graph_replay()
+            else:
+                c.estimate_and_mark_resident(*ptrs)
+            kept.append(bits.clone())
+        stream.synchronize()
+        c.set_stream(0)
+    e = np.arange(E)
+    for i, b in enumerate(kept):
+        b = b.cpu().numpy().view(np.uint32)
+        flags = want[i % 3]
+        assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, flags & 1), i
+        assert np.array_equal((b[1][e >> 5] >> (e & 31)) & 1, (flags >> 2) & 1), i
