@@ -314,11 +314,12 @@ void prof_end(sprg_ctx* c) {
 
 // Listed patches: grow them on the first pass (recording the final element
 // sets), afterwards one QR fit per cached set.
-// Tets: once a patch cache exists, the QR of each cached patch runs once
-// (per mesh) into weights, and later passes take weighted sums.  Runs on
+// Once a patch cache exists, the QR of each cached patch runs once (per mesh)
+// into weights, and the passes on tets and the mixed one on triangles take
+// weighted sums.  Runs on
 // the context stream (it reads the patch sizes back).
 int ensure_cache_weights(sprg_ctx* c, PatchCache& pc) {
-  if (!pc.valid || pc.w_ready || c->m.dim != 3 || pc.count <= 0) return SPRG_OK;
+  if (!pc.valid || pc.w_ready || pc.count <= 0) return SPRG_OK;
   std::vector<int> n((size_t)pc.count);
   CK(cudaMemcpyAsync(n.data(), pc.n.p, sizeof(int) * n.size(), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -378,7 +379,7 @@ int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, 
                 cudaStream_t on = nullptr) {
   DevMesh& m = c->m;
   if (pc.valid) {
-    if (!on) {
+    if (!on && m.dim == 3) {
       int rc = ensure_cache_weights(c, pc);
       if (rc) return rc;
     }
@@ -1026,7 +1027,7 @@ int sprg_destroy(sprg_ctx* c) {
   DevBuf* bufs[] = {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
-                    &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->agitems, &c->agcount,
+                    &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->cache2d.woff, &c->cache2d.w, &c->cache2d.wn, &c->agitems, &c->agcount,
                     &c->crec,  &c->vrec,    &c->rec32, &c->q32, &c->sz2,  &c->fcnt,   &c->guard, &c->tetd,
                     &c->wts,   &c->w64,     &c->listed, &c->geo, &c->geo64, &c->elen, &c->fitems, &c->gstamp, &c->gfit, &c->grec, &c->tnext, &c->edone,
                     &c->hess, &c->pcls, &c->bverts, &c->btiles, &c->bnext, &c->bvoff, &c->bseg, &c->bsegoff, &c->bratios, &c->vvoff, &c->vv, &c->vtile, &c->vr16, &c->rec16,
@@ -2447,9 +2448,10 @@ int sprg_hessian_metric(sprg_ctx* c, const double* hessian, double eps, double h
 
 // The mixed-precision pass's nodal Hessian on triangles: per mesh, the
 // patch weights and the recovery-of-gradient operator K (FP64); per pass
-// rec1 = K u and H = K rec1, the listed patches (growth or more than the
-// weights' patch size) by the FP64 slab fits with in-place gradients.
-static int hessian_operator_2d(sprg_ctx* c) {
+// rec1 = K u and H = K rec1 with the metric records of H, the listed patches
+// (growth or more than the weights' patch size) by their grown patches'
+// FP64 weights.
+static int hessian_operator_2d(sprg_ctx* c, double eps, double h_min, double h_max) {
   DevMesh& m = c->m;
   int rc;
   const int ks = tri_operator_slots();
@@ -2479,18 +2481,22 @@ static int hessian_operator_2d(sprg_ctx* c) {
   ENSURE(c->rec, sizeof(double) * 3 * (size_t)m.V);
   ENSURE(c->rec9, sizeof(double) * 9 * (size_t)m.V);
   ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + 9 + 1));
+  PatchCache& pc = c->cache2d;
+  if (!pc.valid && (rc = grow_patches(c, pc, nullptr, nullptr, 0, nullptr, lst, -1))) return rc;
+  if ((rc = ensure_cache_weights(c, pc))) return rc;
+  const TriListed ls{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
+                     P<double>(pc.w), P<int>(pc.wn), P<DevStatus>(c->status)};
   PB("recover_grad_op_f64");
-  launch_apply_operator(m.V, 1, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
-                        P<int>(c->klen), P<double>(c->f), P<double>(c->rec), c->stream);
+  launch_apply_operator(m, 1, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
+                        P<int>(c->klen), P<double>(c->f), P<double>(c->rec), ls, 0, 0, 0, nullptr, nullptr, c->stream);
   PE();
-  c->launches += 1;
-  if ((rc = listed_fits(c, c->cache2d, nullptr, P<double>(c->f), 3, P<double>(c->rec), lst))) return rc;
-  PB("recover_grad_op_f64");
-  launch_apply_operator(m.V, 3, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
-                        P<int>(c->klen), P<double>(c->rec), P<double>(c->rec9), c->stream);
+  PB("hessian_metric_op_f64");
+  launch_apply_operator(m, 3, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
+                        P<int>(c->klen), P<double>(c->rec), P<double>(c->rec9), ls, eps, h_min, h_max, P<float>(c->met32),
+                        c->qrec32.p, c->stream);
   PE();
-  c->launches += 1;
-  return listed_fits(c, c->cache2d, nullptr, P<double>(c->rec), 9, P<double>(c->rec9), lst);
+  c->launches += 2;
+  return check_launch(c, "triangle operator");
 }
 
 // the mixed-precision anisotropic pass (SPRG_FP32): FP64 nodal Hessian
@@ -2501,8 +2507,10 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
   DevMesh& m = c->m;
   int rc;
   const double* H;
+  ENSURE(c->met32, sizeof(float) * 12 * (size_t)(m.V > 0 ? m.V : 1));
+  ENSURE(c->qrec32, (size_t)quality_rec_bytes() * (size_t)(m.V > 0 ? m.V : 1));
   if (m.dim == 2) {
-    if ((rc = hessian_operator_2d(c))) return rc;
+    if ((rc = hessian_operator_2d(c, eps, h_min, h_max))) return rc;
     H = P<double>(c->rec9);
   } else {  // tets: the FP64 gradients and recoveries
     if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = step_recover(c))) return rc;
@@ -2510,8 +2518,6 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
     if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = step_recover(c))) return rc;
     H = P<double>(c->rec);
   }
-  ENSURE(c->met32, sizeof(float) * 12 * (size_t)(m.V > 0 ? m.V : 1));
-  ENSURE(c->qrec32, (size_t)quality_rec_bytes() * (size_t)(m.V > 0 ? m.V : 1));
   if (!c->crec_ready) {  // the coordinate records of the edge and element Jacobians (per mesh)
     ENSURE(c->crec, 32 * (size_t)(m.V > 0 ? m.V : 1));
     fast_prep_coords(m, c->frame, P<float4>(c->crec), c->stream);
@@ -2521,16 +2527,12 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
   ENSURE(c->agitems, sizeof(int) * (size_t)(m.E > 0 ? m.E : 1));
   ENSURE(c->agcount, sizeof(int));
   CK(cudaMemsetAsync(c->agcount.p, 0, sizeof(int), c->stream));
-  // triangles: the FP32 records straight from the Hessian, and the FP64
-  // metric rebuilt only where the guard and the quality's tie-breaks need
-  // it; tets: the FP64 metric, then its FP32 records
+  // triangles: the FP32 records came with the Hessian, and the FP64 metric is
+  // rebuilt only where the guard and the quality's tie-breaks need it; tets:
+  // the FP64 metric, then its FP32 records
   const double* sizes64 = nullptr;
   const double* frames64 = nullptr;
-  if (m.dim == 2) {
-    PB("metric_f32");
-    launch_metric_mixed2d(m.V, H, eps, h_min, h_max, P<float>(c->met32), c->qrec32.p, c->stream);
-    PE();
-  } else {
+  if (m.dim == 3) {
     PB("hessian_metric");
     launch_hessian_metric(m, H, eps, h_min, h_max, P<double>(c->sizes3), P<double>(c->frames9), c->stream);
     PE();

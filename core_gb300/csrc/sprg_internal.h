@@ -167,7 +167,7 @@ void launch_expand_f64(const DevMesh& m, const double* ip, const double* u, int 
 void launch_cached_fit_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
                            const int* cache_v, const int* cache_n, const int* cache_el, double* slab, DevStatus* st,
                            cudaStream_t s);
-// Tets: per-mesh weights of the cached patches (w = Q1 R^-T t from the fit's
+// Per-mesh weights of the cached patches (w = Q1 R^-T t from the fit's
 // QR; woff: each patch's offset into w, wn: its size or -1 where the rank
 // test fails) and the per-pass weighted sums that replace the fits
 void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_v, const int* cache_n,
@@ -244,21 +244,30 @@ void launch_measure_guard_f64(const DevMesh& m, const double* sizes, const doubl
 void launch_quality_aniso_f32(const DevMesh& m, const void* qrec, const float4* crec, double frame_scale,
                               const double* sizes, const double* frames, const double* H, double eps, double hmin,
                               double hmax, double* cj64, int* tie_items, int* tie_count, double* q, cudaStream_t s);
-// triangles: FP32 metric records (12 floats) and quality records straight
-// from the Hessian (FP64 decisions, FP32 magnitudes)
-void launch_metric_mixed2d(int V, const double* H, double eps, double hmin, double hmax, float* out, void* qrec,
-                           cudaStream_t s);
 // Triangle recovery-of-gradient operator (per mesh, FP64): K_va over the
 // patch vertices, tri_operator_slots() slots per vertex (kidx ints, kval 3
-// doubles each, klen counts; patches that are not fans are added to the
-// listed set); applied to a scalar (ncin 1 -> V x 3) or a
-// VECTOR field (ncin 3 -> V x 9) at the covered (not listed) vertices
+// doubles each, a plane of V per slot; klen counts; patches that are not fans
+// are added to the listed set)
 int tri_operator_slots();
 // kc: components per operator slot, 3, or 2 for a mesh in the z = 0 plane
 void launch_tri_operator(const DevMesh& m, int kc, const double* w, unsigned char* listed, ExpandList lst, int* kidx,
                          double* kval, int* klen, cudaStream_t s);
-void launch_apply_operator(int V, int ncin, int kc, const unsigned char* listed, const int* kidx, const double* kval,
-                           const int* klen, const double* f, double* out, cudaStream_t s);
+// applied to a scalar (ncin 1 -> V x 3) or a VECTOR field (ncin 3 -> V x 9, and
+// from that Hessian the FP32 metric records, 12 floats in met, and quality
+// records: FP64 decisions, FP32 magnitudes) at every vertex, the listed ones
+// through their patches' weights
+struct TriListed {
+  int n, stride;
+  const int* v;
+  const int* el;
+  const long long* woff;
+  const double* w;
+  const int* wn;
+  DevStatus* st;
+};
+void launch_apply_operator(const DevMesh& m, int ncin, int kc, const unsigned char* listed, const int* kidx,
+                           const double* kval, const int* klen, const double* f, double* out, const TriListed& ls,
+                           double eps, double hmin, double hmax, float* met, void* qrec, cudaStream_t s);
 // incremental mesh update: dst[ids[r] * width + j] = vals[r * width + j];
 // the coordinates' bounding box as order keys (3 minima, 3 maxima)
 void launch_scatter_rows_f64(long long n, int width, const int* ids, const double* vals, double* dst, cudaStream_t s);

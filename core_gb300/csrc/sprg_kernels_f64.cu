@@ -642,19 +642,20 @@ __global__ void __launch_bounds__(32) k_cached_fit(DevMesh m, const double* __re
   }
 }
 
-// Tets: the cached patches' fits are linear in the samples as well.  Per mesh,
+// The cached patches' fits are linear in the samples as well.  Per mesh,
 // the fit's Householder QR (slab_fit's reflectors and 1e-10 rank test) of the
-// rows [1, x_ip, y_ip, z_ip] gives w = Q1 R^-T t (t = [1, x_v, y_v, z_v]),
+// rows [1, x_ip, y_ip(, z_ip)] gives w = Q1 R^-T t (t = [1, x_v, y_v(, z_v)]),
 // and every pass recovers rec(v) = sum_i w_i b_i.  Warp per cached patch;
 // rows (4 geometry columns, then the 4 reflectors) in shared memory up to
 // kExpandSmemRows elements, else in the block's slab.  wn[it] = the patch
 // size, or -1 where the rank test fails (the fit's SPRG_EPATCH).
+template <int NT>
 __global__ void __launch_bounds__(32) k_cached_weights(DevMesh m, int n_cached, const int* __restrict__ cache_v,
                                                        const int* __restrict__ cache_n,
                                                        const int* __restrict__ cache_el,
                                                        const long long* __restrict__ woff, double* __restrict__ w,
                                                        int* __restrict__ wn, double* slab) {
-  constexpr int NT = 4, LD = 2 * NT;
+  constexpr int LD = 2 * NT;
   __shared__ double srows[kExpandSmemRows * 8];
   const int lane = threadIdx.x & 31;
   double* grows = slab + (size_t)blockIdx.x * kExpandMaxElems * LD;
@@ -669,7 +670,8 @@ __global__ void __launch_bounds__(32) k_cached_weights(DevMesh m, int n_cached, 
     for (int i = lane; i < n; i += 32) {
       const V3 p = elem_ip_point(m, S[i]);
       double* rw = rows + (size_t)i * LD;
-      rw[0] = 1.0; rw[1] = p.v[0]; rw[2] = p.v[1]; rw[3] = p.v[2];
+      rw[0] = 1.0; rw[1] = p.v[0]; rw[2] = p.v[1];
+      if (NT == 4) rw[NT - 1] = p.v[2];
     }
     __syncwarp();
     bool ok = true;
@@ -1830,17 +1832,14 @@ __device__ __forceinline__ float d_to_f32_scaled(double x, int e) {
 // results, inside the FP32 measure's bound.  The sign test runs on the
 // unnormalised FP64 direction (the normalisation by a positive length keeps
 // signs and zeros).
-__global__ void __launch_bounds__(kBlock) k_metric_mixed2d(int V, const double* __restrict__ H, double eps,
-                                                           double hmin, double hmax, float* __restrict__ out,
-                                                           QualityRec* __restrict__ qrec) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= V) return;
-  const double* h = H + 9 * (size_t)v;
+__device__ __forceinline__ void metric_mixed_vertex(double h00, double h01, double h10, double h11, double eps,
+                                                    double hmin, double hmax, float* __restrict__ met,
+                                                    QualityRec* __restrict__ qrec) {
   // the same power-of-two prescaling as hessian_metric_vertex, so every
   // decision below sees that function's values
-  const double b0 = 0.5 * (h[1] + h[3]);
-  const int es = hessian_scale_exp(max(max(dbexp(h[0]), dbexp(h[4])), dbexp(b0)));
-  double a = h[0], b = b0, c = h[4];
+  const double b0 = 0.5 * (h01 + h10);
+  const int es = hessian_scale_exp(max(max(dbexp(h00), dbexp(h11)), dbexp(b0)));
+  double a = h00, b = b0, c = h11;
   if (es) {
     a = times_pow2(a, -es);
     b = times_pow2(b, -es);
@@ -1892,10 +1891,10 @@ __global__ void __launch_bounds__(kBlock) k_metric_mixed2d(int V, const double* 
     l2 = times_pow2(l2, es);
   }
   const float o[12] = {size_f32(l1), size_f32(l2), hmaxf, xf, -yf, 0.f, yf, xf, 0.f, 0.f, 0.f, 1.f};
-  store_met(out + 12 * (size_t)v, o);
+  store_met(met, o);
   float Q[3][3];
   transform_f32(o, o + 3, Q);
-  store_qrec(qrec + v, Q, det_f32(Q, 2));
+  store_qrec(qrec, Q, det_f32(Q, 2));
 }
 
 // AnisoSizeField measure in FP32 with a relative error bound.  Per Gauss
@@ -2190,8 +2189,9 @@ __global__ void __launch_bounds__(kBlock) k_quality_ties(DevMesh m, const Qualit
 // only.  It is built once per mesh (FP64) and the two recoveries of the
 // Hessian workload become two sparse products with it.  kOpSlots slots per
 // vertex (a fan of up to kTriThreadRows triangles touches at most
-// kTriThreadRows + 2 vertices); a patch touching more is listed for the
-// FP64 slab fit instead.
+// kTriThreadRows + 2 vertices), slot s of every vertex in one plane, so that a
+// warp reads whole lines; a patch touching more is listed, and takes the
+// weighted sum over its (grown) patch instead.
 constexpr int kOpSlots = kTriThreadRows + 2;
 // KC: components stored per slot, 3, or 2 on a mesh in the z = 0 plane
 // (there the z component of every element gradient is exactly zero)
@@ -2240,52 +2240,139 @@ __global__ void __launch_bounds__(kBlock) k_tri_operator(DevMesh m, const double
   }
   klen[v] = n;
   for (int s = 0; s < n; ++s) {
-    kidx[(size_t)v * kOpSlots + s] = ids[s];
-    for (int c = 0; c < KC; ++c) kval[((size_t)v * kOpSlots + s) * KC + c] = acc[s][c];
+    kidx[(size_t)s * m.V + v] = ids[s];
+    for (int c = 0; c < KC; ++c) kval[((size_t)s * m.V + v) * KC + c] = acc[s][c];
   }
 }
 
-// out (V x 3 NCIN) = K f (f: V x NCIN) at the covered vertices; row r of a
-// MATRIX value is the recovered gradient of component r.  KC = 2 (mesh in
-// the z = 0 plane): K's z components, and the z components of a gradient
-// input, are zero, so only the x / y products are formed and the z entries
-// of the output are zero.
-template <int NCIN, int KC>
-__global__ void __launch_bounds__(kBlock) k_apply_operator(int V, const unsigned char* __restrict__ listed,
+// The listed patches of a triangle mesh (n patches; patch it: vertex v[it],
+// elements el + it stride, wn[it] weights at w + woff[it], or -1: SPRG_EPATCH):
+// sum_i w_i grad f over the patch by one warp, lanes over the elements, fixed
+// reduction tree; every lane gets the sums (row r of a VECTOR field's MATRIX
+// value in acc[3 r ..]).  false: no weights.
+template <int NCIN>
+__device__ __noinline__ bool tri_listed_sum(const DevMesh& m, const double* __restrict__ f, const TriListed& ls, int it,
+                                            double* acc) {
+  const int lane = threadIdx.x & 31;
+  const int n = ls.wn[it];
+  for (int k = 0; k < 3 * NCIN; ++k) acc[k] = 0;
+  if (n < 0) {
+    if (lane == 0) set_status(ls.st, SPRG_EPATCH, ls.v[it]);
+    return false;
+  }
+  const int* el = ls.el + (size_t)it * ls.stride;
+  const double* wi = ls.w + ls.woff[it];
+  for (int i = lane; i < n; i += 32) {
+    const int* ev = m.ev + 3 * (size_t)el[i];
+    V3 x[3];
+    for (int a = 0; a < 3; ++a) x[a] = load_xyz(m.xyz, ev[a]);
+    const M3 jinv = ref::jacobian_inverse(ref::jacobian(x, 3, 2), 2);
+    const double wk = wi[i];
+    for (int r = 0; r < NCIN; ++r) {
+      const double f0 = f[(size_t)ev[0] * NCIN + r];
+      const double d1 = f[(size_t)ev[1] * NCIN + r] - f0, d2 = f[(size_t)ev[2] * NCIN + r] - f0;
+      for (int c = 0; c < 3; ++c) acc[3 * r + c] += wk * (jinv.m[c][0] * d1 + jinv.m[c][1] * d2);
+    }
+  }
+  for (int k = 0; k < 3 * NCIN; ++k) acc[k] = warp_sum(acc[k]);
+  return true;
+}
+
+// out (V x 3 NCIN) = K f (f: V x NCIN) at every vertex; row r of a MATRIX value
+// is the recovered gradient of component r.  KC = 2 (mesh in the z = 0
+// plane): K's z components, and the z components of a gradient input, are
+// zero, so only the x / y products are formed and the z entries of the output
+// are zero.  METRIC: also the FP32 metric and quality records of the value (a
+// Hessian), which is then not read back.  The first blocks take the listed
+// vertices, a warp each; the others' values go through shared memory, so that
+// they leave as whole lines.  The Hessian is FP64-rate bound (86 % of that
+// pipe), the gradient waits on its gathers.  2501^2 square: 240 us for the
+// gradient, 770 us for the Hessian with its records, against 652 us for both
+// with strided slots and values, 118 us of fits behind them and 422 us for
+// the records from the stored Hessian.
+struct MetricOut {
+  double eps, hmin, hmax;
+  float* met;
+  QualityRec* qrec;
+};
+template <int NCIN, int KC, bool METRIC>
+__global__ void __launch_bounds__(kBlock, METRIC ? 4 : 5) k_apply_operator(DevMesh m, const unsigned char* __restrict__ listed,
                                                            const int* __restrict__ kidx,
                                                            const double* __restrict__ kval,
                                                            const int* __restrict__ klen, const double* __restrict__ f,
-                                                           double* __restrict__ out) {
+                                                           double* __restrict__ out, int n_list_blocks,
+                                                           const __grid_constant__ TriListed ls, MetricOut mo) {
   constexpr int NR = (KC == 2 && NCIN == 3) ? 2 : NCIN;  // input components that can be nonzero
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= V || listed[v]) return;
-  const int n = klen[v];
+  constexpr int NO = 3 * NCIN;
+  const int V = m.V;
+  if ((int)blockIdx.x < n_list_blocks) {
+    const int it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (it >= ls.n) return;
+    const int v = ls.v[it];
+    double acc[NO];
+    if (!tri_listed_sum<NCIN>(m, f, ls, it, acc)) return;
+    if (lane == 0) {
+      for (int k = 0; k < NO; ++k) out[(size_t)v * NO + k] = acc[k];
+      if constexpr (METRIC)
+        metric_mixed_vertex(acc[0], acc[1], acc[3], acc[4], mo.eps, mo.hmin, mo.hmax, mo.met + 12 * (size_t)v,
+                            mo.qrec + v);
+    }
+    return;
+  }
+  __shared__ double sh[kBlock * NO];
+  __shared__ bool own[kBlock];
+  const int v0 = (blockIdx.x - n_list_blocks) * kBlock, v = v0 + threadIdx.x;
+  const bool mine = v < V && !listed[v];
   double acc[NCIN][3];
 #pragma unroll
   for (int r = 0; r < NCIN; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0;
-  for (int s = 0; s < n; ++s) {
-    const size_t slot = (size_t)v * kOpSlots + s;
-    const int a = kidx[slot];
-    double k[KC];
-    if (KC == 2) {  // one 16-byte load per slot
-      const double2 kk = __ldg(reinterpret_cast<const double2*>(kval) + slot);
-      k[0] = kk.x;
-      k[KC - 1] = kk.y;
-    } else {
+  const int n = mine ? __ldg(klen + v) : 0;
+  // slots in groups whose ids, coefficients and gathers are all in flight
+  // together (ids past the end: the vertex itself, coefficients 0 skipped)
+  constexpr int G = KC == 2 ? 4 : 2;
+#pragma unroll 1
+  for (int s0 = 0; s0 < n; s0 += G) {
+    int a[G];
+    double k[G][KC];
 #pragma unroll
-      for (int c = 0; c < KC; ++c) k[c] = kval[KC * slot + c];
+    for (int j = 0; j < G; ++j) a[j] = s0 + j < n ? __ldcs(kidx + (size_t)(s0 + j) * V + v) : v;
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+      const size_t slot = (size_t)min(s0 + j, n - 1) * V + v;
+      if (KC == 2) {  // one 16-byte load per slot
+        const double2 kk = __ldcs(reinterpret_cast<const double2*>(kval) + slot);
+        k[j][0] = kk.x;
+        k[j][KC - 1] = kk.y;
+      } else {
+#pragma unroll
+        for (int c = 0; c < KC; ++c) k[j][c] = __ldcs(kval + KC * slot + c);
+      }
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-      const double fa = f[(size_t)a * NCIN + r];
+      double fa[G];
 #pragma unroll
-      for (int c = 0; c < KC; ++c) acc[r][c] = fma(k[c], fa, acc[r][c]);
+      for (int j = 0; j < G; ++j) fa[j] = __ldg(f + (size_t)a[j] * NCIN + r);
+#pragma unroll
+      for (int j = 0; j < G; ++j)
+        if (s0 + j < n)
+#pragma unroll
+          for (int c = 0; c < KC; ++c) acc[r][c] = fma(k[j][c], fa[j], acc[r][c]);
     }
   }
 #pragma unroll
   for (int r = 0; r < NCIN; ++r)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[(size_t)v * 3 * NCIN + 3 * r + c] = acc[r][c];
+    for (int c = 0; c < 3; ++c) sh[NO * threadIdx.x + 3 * r + c] = acc[r][c];
+  own[threadIdx.x] = mine;
+  __syncthreads();
+  const int nv = min(kBlock, V - v0);
+  for (int i = threadIdx.x; i < NO * nv; i += kBlock)
+    if (own[i / NO]) out[(size_t)v0 * NO + i] = sh[i];
+  if constexpr (METRIC)
+    if (mine)
+      metric_mixed_vertex(acc[0][0], acc[0][1], acc[NCIN > 1][0], acc[NCIN > 1][1], mo.eps, mo.hmin, mo.hmax,
+                          mo.met + 12 * (size_t)v, mo.qrec + v);
 }
 
 // ---------------------------------------------------------------------
@@ -2510,9 +2597,10 @@ void launch_cached_fit_f64(const DevMesh& m, const double* ip, const double* u, 
 void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_v, const int* cache_n,
                                const int* cache_el, const long long* woff, double* w, int* wn, double* slab,
                                cudaStream_t s) {
-  if (n_cached > 0)
-    k_cached_weights<<<n_cached < kExpandGrid ? n_cached : kExpandGrid, 32, 0, s>>>(m, n_cached, cache_v, cache_n,
-                                                                                   cache_el, woff, w, wn, slab);
+  if (n_cached <= 0) return;
+  const int g = n_cached < kExpandGrid ? n_cached : kExpandGrid;
+  if (m.dim == 3) k_cached_weights<4><<<g, 32, 0, s>>>(m, n_cached, cache_v, cache_n, cache_el, woff, w, wn, slab);
+  else k_cached_weights<3><<<g, 32, 0, s>>>(m, n_cached, cache_v, cache_n, cache_el, woff, w, wn, slab);
 }
 
 void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
@@ -2663,11 +2751,6 @@ void launch_measure_guard_f64(const DevMesh& m, const double* sizes, const doubl
   k_measure_guard_f64<<<152 * 4, kBlock, 0, s>>>(m, src, guard, gcount, gcap, split, collapse);
 }
 
-void launch_metric_mixed2d(int V, const double* H, double eps, double hmin, double hmax, float* out, void* qrec,
-                           cudaStream_t s) {
-  if (V) k_metric_mixed2d<<<nblk(V), kBlock, 0, s>>>(V, H, eps, hmin, hmax, out, static_cast<QualityRec*>(qrec));
-}
-
 int quality_rec_bytes() { return (int)sizeof(QualityRec); }
 
 void launch_quality_aniso_f32(const DevMesh& m, const void* qrec, const float4* crec, double frame_scale,
@@ -2692,17 +2775,17 @@ void launch_tri_operator(const DevMesh& m, int kc, const double* w, unsigned cha
   else k_tri_operator<3><<<nblk(m.V), kBlock, 0, s>>>(m, w, listed, lst, kidx, kval, klen);
 }
 
-void launch_apply_operator(int V, int ncin, int kc, const unsigned char* listed, const int* kidx, const double* kval,
-                           const int* klen, const double* f, double* out, cudaStream_t s) {
-  if (!V) return;
-  const int g = nblk(V);
-  if (kc == 2) {
-    if (ncin == 1) k_apply_operator<1, 2><<<g, kBlock, 0, s>>>(V, listed, kidx, kval, klen, f, out);
-    else k_apply_operator<3, 2><<<g, kBlock, 0, s>>>(V, listed, kidx, kval, klen, f, out);
-  } else {
-    if (ncin == 1) k_apply_operator<1, 3><<<g, kBlock, 0, s>>>(V, listed, kidx, kval, klen, f, out);
-    else k_apply_operator<3, 3><<<g, kBlock, 0, s>>>(V, listed, kidx, kval, klen, f, out);
-  }
+void launch_apply_operator(const DevMesh& m, int ncin, int kc, const unsigned char* listed, const int* kidx,
+                           const double* kval, const int* klen, const double* f, double* out, const TriListed& ls,
+                           double eps, double hmin, double hmax, float* met, void* qrec, cudaStream_t s) {
+  if (!m.V) return;
+  const int nl = nblk((long)ls.n * 32);
+  const MetricOut mo{eps, hmin, hmax, met, static_cast<QualityRec*>(qrec)};
+  auto go = [&](auto kernel) {
+    kernel<<<nl + nblk(m.V), kBlock, 0, s>>>(m, listed, kidx, kval, klen, f, out, nl, ls, mo);
+  };
+  if (ncin == 1) go(kc == 2 ? k_apply_operator<1, 2, false> : k_apply_operator<1, 3, false>);
+  else go(kc == 2 ? k_apply_operator<3, 2, true> : k_apply_operator<3, 3, true>);
 }
 
 void launch_scatter_rows_f64(long long n, int width, const int* ids, const double* vals, double* dst, cudaStream_t s) {
