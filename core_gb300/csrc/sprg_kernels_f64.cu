@@ -2524,7 +2524,9 @@ __global__ void __launch_bounds__(kBlock) k_qr_weights(DevMesh m, double* __rest
   if (lane == 0) listed[v] = 0;
 }
 
-// FP64 recovery from the weights: thread per vertex, NC components
+// FP64 recovery from the weights: thread per vertex, NC components (fused
+// multiply-adds: the sum's order is this method's own, and the FP64 pipe, at
+// 73 % with separate products and sums, bounds the kernel)
 template <int NC>
 __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double* __restrict__ ip,
                                                         const double* __restrict__ w,
@@ -2541,7 +2543,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
     const double wk = w[k];
     const double* b = ip + (size_t)m.p_el[k] * NC;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] += wk * b[c];
+    for (int c = 0; c < NC; ++c) acc[c] = fma(wk, b[c], acc[c]);
   }
 #pragma unroll
   for (int c = 0; c < NC; ++c) rec[(size_t)v * NC + c] = acc[c];
