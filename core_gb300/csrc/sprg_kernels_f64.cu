@@ -364,41 +364,17 @@ __device__ __forceinline__ double tri_div(double a, double b, double y, bool pla
   return quotient(a, b, y);
 }
 
-// The recovery from the factors (CACHED), or with the factors computed in
-// place where there is no memory for them.  Samples that are 0 leave the
-// sums as they are (a planar mesh's z components), and a component whose
-// sums are all 0 is 0.  FP64-rate bound: about 60 operations a component that
-// is not 0; both recoveries of a 1024^2 square's anisotropic pass took
-// 6.65 ms with the QR in every call, 1.30 ms from the factors.
-template <int NC, int MAXM, bool CACHED>
-__global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __restrict__ ip,
-                                                     const double* __restrict__ qc, const double* __restrict__ rr,
-                                                     const unsigned char* __restrict__ code,
-                                                     double* __restrict__ rec, ExpandList xl, ExpandList big) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= m.V) return;
-  const int beg = m.p_off[v];
-  int cnt;
-  bool plain = true;
-  double Qc[CACHED ? 1 : MAXM][3], R[kTriR];
-  if constexpr (CACHED) {
-    const int cd = code[v];
-    if (cd == 0) return;
-    cnt = cd & (kTriPlain - 1);
-    plain = (cd & kTriPlain) != 0;
+// the recovery of one vertex.  FLAT: the samples' z components (NC = 3), or z
+// row and column (NC = 9), are all 0, and so are their values
+template <int NC, int MAXM, bool CACHED, bool FLAT>
+__device__ __forceinline__ void recover_tri_vertex(const DevMesh& m, int v, int beg, int cnt, bool plain,
+                                                   const double* __restrict__ ip, const double* __restrict__ qc,
+                                                   const double (*Qc)[3], const double* R, double* __restrict__ rec) {
+  constexpr int NW = FLAT ? (NC == 9 ? 4 : 2) : NC;  // components worked on
+  auto comp = [](int c) { return FLAT && c > 1 ? c + 1 : c; };  // 0, 1(, 3, 4)
+  double y[NW][3];
 #pragma unroll
-    for (int i = 0; i < kTriR; ++i) R[i] = __ldcs(rr + (size_t)i * m.V + v);
-  } else {
-    cnt = m.p_off[v + 1] - beg;
-    if (cnt < 3 || cnt > MAXM || !tri_factor<MAXM>(m, beg, cnt, Qc, R)) {
-      list_append(cnt > MAXM ? big : xl, v);
-      return;
-    }
-    R[6] = R[7] = R[8] = 0;
-  }
-  double y[NC][3];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) y[c][0] = y[c][1] = y[c][2] = 0;
+  for (int c = 0; c < NW; ++c) y[c][0] = y[c][1] = y[c][2] = 0;
 #pragma unroll
   for (int r = 0; r < MAXM; ++r) {
     if (r >= cnt) break;
@@ -410,28 +386,74 @@ __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __
       else q[i] = Qc[r][i];
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double bc = __ldg(b + c);
-      if (plain || (__double_as_longlong(bc) << 1) != 0) {
+    for (int c = 0; c < NW; ++c) {
+      const double bc = __ldg(b + comp(c));
 #pragma unroll
-        for (int i = 0; i < 3; ++i) y[c][i] += q[i] * bc;
-      }
+      for (int i = 0; i < 3; ++i) y[c][i] += q[i] * bc;
     }
   }
   const V3 xv = load_xyz(m.xyz, v);
+  double* o = rec + (size_t)v * NC;
+  if (FLAT)
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
+    for (int c = 0; c < NC; ++c)
+      if (c == 2 || c > 4) o[c] = 0.0;
+#pragma unroll
+  for (int c = 0; c < NW; ++c) {
+    const double x2 = tri_div(y[c][2], R[5], R[8], plain);
+    const double x1 = tri_div(y[c][1] - R[4] * x2, R[3], R[7], plain);
+    const double x0 = tri_div(y[c][0] - R[1] * x1 - R[2] * x2, R[0], R[6], plain);
     double sres = 0;
-    const long long any = __double_as_longlong(y[c][0]) | __double_as_longlong(y[c][1]) | __double_as_longlong(y[c][2]);
-    if (plain || any != 0) {
-      const double x2 = tri_div(y[c][2], R[5], R[8], plain);
-      const double x1 = tri_div(y[c][1] - R[4] * x2, R[3], R[7], plain);
-      const double x0 = tri_div(y[c][0] - R[1] * x1 - R[2] * x2, R[0], R[6], plain);
-      sres += x0 * 1.0;
-      sres += x1 * xv.v[0];
-      sres += x2 * xv.v[1];
+    sres += x0 * 1.0;
+    sres += x1 * xv.v[0];
+    sres += x2 * xv.v[1];
+    o[comp(c)] = sres;
+  }
+}
+
+// The recovery from the factors (CACHED), or with the factors computed in
+// place where there is no memory for them.  Patches whose samples lie in the
+// plane leave the z components out (a branch around the whole recovery: a
+// test per sample becomes predicates, which take the FP64 pipe all the
+// same).  FP64-rate bound: about 63 operations a component; both recoveries of a
+// 1024^2 square's anisotropic pass took 6.65 ms with the QR in every call,
+// 1.30 ms from the factors, 0.74 ms without the z components.
+template <int NC, int MAXM, bool CACHED>
+__global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __restrict__ ip,
+                                                     const double* __restrict__ qc, const double* __restrict__ rr,
+                                                     const unsigned char* __restrict__ code,
+                                                     double* __restrict__ rec, ExpandList xl, ExpandList big) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= m.V) return;
+  const int beg = m.p_off[v];
+  double R[kTriR];
+  if constexpr (CACHED) {
+    const int cd = code[v];
+    if (cd == 0) return;
+    const int cnt = cd & (kTriPlain - 1);
+    const bool plain = (cd & kTriPlain) != 0;
+    long long z = 0;  // the z components' bits
+    for (int r = 0; r < cnt; ++r) {
+      const double* b = ip + (size_t)m.p_el[beg + r] * NC;
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (c == 2 || c > 4) z |= __double_as_longlong(__ldg(b + c));
     }
-    rec[(size_t)v * NC + c] = sres;
+#pragma unroll
+    for (int i = 0; i < kTriR; ++i) R[i] = __ldcs(rr + (size_t)i * m.V + v);
+    if (!plain && (z << 1) == 0)
+      recover_tri_vertex<NC, MAXM, true, true>(m, v, beg, cnt, false, ip, qc, nullptr, R, rec);
+    else
+      recover_tri_vertex<NC, MAXM, true, false>(m, v, beg, cnt, plain, ip, qc, nullptr, R, rec);
+  } else {
+    const int cnt = m.p_off[v + 1] - beg;
+    double Qc[MAXM][3];
+    if (cnt < 3 || cnt > MAXM || !tri_factor<MAXM>(m, beg, cnt, Qc, R)) {
+      list_append(cnt > MAXM ? big : xl, v);
+      return;
+    }
+    R[6] = R[7] = R[8] = 0;
+    recover_tri_vertex<NC, MAXM, false, false>(m, v, beg, cnt, true, ip, qc, Qc, R, rec);
   }
 }
 

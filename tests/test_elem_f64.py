@@ -178,8 +178,9 @@ def test_triangle_recovery_bitwise(gpu_lib, oracle_lib, n, kind, nc):
     cnt = np.bincount(m.elem_verts.reshape(-1), minlength=m.n_verts)
     thread = (cnt >= 3) & (cnt <= 8)
     rng = np.random.default_rng(8)
-    ips = [rng.normal(size=(m.n_elems, nc)) for _ in range(2)]
+    ips = [rng.normal(size=(m.n_elems, nc)) for _ in range(3)]
     ips[0][:, 2::3] = 0.0
+    ips[2][:, [c for c in range(nc) if c == 2 or c > 4]] = 0.0  # a planar mesh's gradients
     ips[1][::7, 0] = 0.0
     ips[1][3, 1] = np.inf
 
