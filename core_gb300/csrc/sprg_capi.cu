@@ -347,10 +347,9 @@ int ensure_cache_weights(sprg_ctx* c, PatchCache& pc) {
 }
 
 // The growth of the listed patches (once per mesh), their final element sets
-// into the cache; triangles also take their fits from it (ip or u, nc, rec64).
+// into the cache (with nc > 0 also this pass's fits of ip into rec64).
 // known: the list's length, or -1 to read it back.
-int grow_patches(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, int nc, double* rec64, ExpandList xl,
-                 int known) {
+int grow_patches(sprg_ctx* c, PatchCache& pc, const double* ip, int nc, double* rec64, ExpandList xl, int known) {
   int xc = known;
   if (known < 0) {
     CK(cudaMemcpyAsync(&xc, xl.count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -362,10 +361,8 @@ int grow_patches(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u,
   ENSURE(pc.n, sizeof(int) * slots);
   ENSURE(pc.el, sizeof(int) * slots * expand_max_elems());
   PB("expand_f64");
-  // tets: the growth and its rank tests only, the values follow from the
-  // weights
-  launch_expand_f64(c->m, ip, u, c->m.dim == 3 ? 0 : nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status),
-                    c->stream, P<int>(pc.v), P<int>(pc.n), P<int>(pc.el));
+  launch_expand_f64(c->m, ip, nc, rec64, xl, P<double>(c->slab), P<DevStatus>(c->status), c->stream, P<int>(pc.v),
+                    P<int>(pc.n), P<int>(pc.el));
   PE();
   c->launches += 1;
   int rc = check_launch(c, "expand");
@@ -375,35 +372,27 @@ int grow_patches(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u,
   return SPRG_OK;
 }
 
-int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, const double* u, int nc, double* rec64, ExpandList xl,
-                cudaStream_t on = nullptr) {
-  DevMesh& m = c->m;
-  if (pc.valid) {
-    if (!on && m.dim == 3) {
-      int rc = ensure_cache_weights(c, pc);
-      if (rc) return rc;
-    }
-    cudaStream_t s = on ? on : c->stream;
-    if (!on) PB("cached_fit_f64");
-    if (pc.w_ready)
-      launch_cached_wsum_f64(m, ip, u, nc, rec64, pc.count, P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
-                             P<double>(pc.w), P<int>(pc.wn), P<DevStatus>(c->status), s);
-    else
-      launch_cached_fit_f64(m, ip, u, nc, rec64, pc.count, P<int>(pc.v), P<int>(pc.n), P<int>(pc.el),
-                            P<double>(c->slab), P<DevStatus>(c->status), s);
-    if (!on) PE();
-    c->launches += 1;
-    return check_launch(c, "cached fit");
-  }
-  int rc = grow_patches(c, pc, ip, u, nc, rec64, xl, -1);
-  if (rc) return rc;
-  if (m.dim != 3) return SPRG_OK;
-  // tets: this pass already takes the weighted sums, so every pass gives the
-  // same bits for the listed patches
-  if ((rc = ensure_cache_weights(c, pc))) return rc;
-  if (!pc.w_ready) return SPRG_OK;
-  launch_cached_wsum_f64(m, ip, u, nc, rec64, pc.count, P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
-                         P<double>(pc.w), P<int>(pc.wn), P<DevStatus>(c->status), c->stream);
+// the listed patches' growth and FP64 weights (once per mesh)
+int ensure_listed(sprg_ctx* c, PatchCache& pc, ExpandList xl, int known) {
+  int rc = SPRG_OK;
+  if (!pc.valid && (rc = grow_patches(c, pc, nullptr, 0, nullptr, xl, known))) return rc;
+  return ensure_cache_weights(c, pc);
+}
+
+// their weights for the recovery kernels (none of them: n = 0)
+PatchWeights patch_weights(sprg_ctx* c, PatchCache& pc) {
+  return PatchWeights{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v),  P<int>(pc.el),
+                      P<long long>(pc.woff),     P<double>(pc.w),    P<int>(pc.wn), P<DevStatus>(c->status)};
+}
+
+// triangles with patches on the warp path: the listed vertices' QR fits, which
+// the first pass takes with the growth
+int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, int nc, double* rec64, ExpandList xl) {
+  if (!pc.valid) return grow_patches(c, pc, ip, nc, rec64, xl, -1);
+  PB("cached_fit_f64");
+  launch_cached_fit_f64(c->m, ip, nc, rec64, pc.count, P<int>(pc.v), P<int>(pc.n), P<int>(pc.el), P<double>(c->slab),
+                        P<DevStatus>(c->status), c->stream);
+  PE();
   c->launches += 1;
   return check_launch(c, "cached fit");
 }
@@ -468,14 +457,15 @@ int step_recover(sprg_ctx* c) {
       if (rc) return rc;
       c->qw_ready = true;
     }
+    PatchCache& pc = c->cache64;
+    int rc;
+    if ((rc = ensure_listed(c, pc, lst, -1))) return rc;
     PB("recover_f64");
-    launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->qw), P<unsigned char>(c->qwlisted), P<double>(c->rec),
-                       c->stream);
+    launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->qw), P<unsigned char>(c->qwlisted), patch_weights(c, pc),
+                       P<double>(c->rec), c->stream);
     PE();
     c->launches += 1;
-    int rc = check_launch(c, "recover");
-    if (rc) return rc;
-    return listed_fits(c, c->cache64, P<double>(c->ip), nullptr, nc, P<double>(c->rec), lst);
+    return check_launch(c, "recover");
   }
   ENSURE(c->xitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
   ENSURE(c->xcount, sizeof(int));
@@ -517,14 +507,21 @@ int step_recover(sprg_ctx* c) {
     CK(cudaMemcpyAsync(c->xcount.p, c->txcount.p, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
   }
   const TriFactor tf{c->tfac_ready ? P<double>(c->tqc) : nullptr, P<double>(c->trr), P<unsigned char>(c->tcode)};
+  // with the lists complete (no patch on the warp path, which may add to
+  // them), the growth patches too are weighted sums inside the recovery
+  PatchCache& pc = c->cache64;
+  const bool complete = c->tfac_ready && !c->n_tri_big;
+  if (complete && (rc = ensure_listed(c, pc, xl, -1))) return rc;
+  const PatchWeights none{};
   PB("recover_f64");
   launch_recover_f64(m, P<double>(c->ip), nc, P<double>(c->rec), tf, xl, big, !c->tfac_ready || c->n_tri_big > 0,
-                     c->stream);
+                     complete ? patch_weights(c, pc) : none, c->stream);
   PE();
   c->launches += 1;
   if ((rc = check_launch(c, "recover"))) return rc;
+  if (complete) return SPRG_OK;
   // patches that need growth: the reference growth order, on the device
-  return listed_fits(c, c->cache64, P<double>(c->ip), nullptr, nc, P<double>(c->rec), xl);
+  return listed_fits(c, c->cache64, P<double>(c->ip), nc, P<double>(c->rec), xl);
 }
 
 int step_size(sprg_ctx* c, int mode, double adapt_ratio, double target, double alpha, double beta) {
@@ -1518,14 +1515,11 @@ static int fast_setup(sprg_ctx* c, ExpandList xl) {
   return SPRG_OK;
 }
 
-// the listed patches' FP64 fits: the first pass grows the patches (and
-// caches them) in order; later passes run the cached fits on the side
-// stream, joined by the caller before the results are used
-static int listed_fork(sprg_ctx* c, const double* d_u, ExpandList xl, bool* forked) {
-  *forked = false;
-  if (!c->cache32.valid) return SPRG_OK;
-  int wrc = ensure_cache_weights(c, c->cache32);
-  if (wrc) return wrc;
+// the learned form's listed patches: their FP64 sums on the side stream,
+// joined by the caller before the results are used
+static int listed_fork(sprg_ctx* c, const double* d_u, ExpandList xl) {
+  int rc = ensure_listed(c, c->cache32, xl, c->n_listed);
+  if (rc) return rc;
   if (!c->side) {
     CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
@@ -1533,19 +1527,11 @@ static int listed_fork(sprg_ctx* c, const double* d_u, ExpandList xl, bool* fork
   }
   CK(cudaEventRecord(c->fork, c->stream));
   CK(cudaStreamWaitEvent(c->side, c->fork, 0));
-  int rc = listed_fits(c, c->cache32, nullptr, d_u, 3, P<double>(c->rec), xl, c->side);
-  if (rc) return rc;
+  launch_cached_wsum_f64(c->m, d_u, patch_weights(c, c->cache32), P<double>(c->rec), c->side);
+  c->launches += 1;
+  if ((rc = check_launch(c, "listed sums"))) return rc;
   CK(cudaEventRecord(c->join, c->side));
-  *forked = true;
   return SPRG_OK;
-}
-
-static int listed_join(sprg_ctx* c, const double* d_u, ExpandList xl, bool forked) {
-  if (forked) {
-    CK(cudaStreamWaitEvent(c->stream, c->join, 0));
-    return SPRG_OK;
-  }
-  return listed_fits(c, c->cache32, nullptr, d_u, 3, P<double>(c->rec), xl);
 }
 
 // patch-size bins of the non-listed vertices (stable: ascending ids within a
@@ -1814,12 +1800,9 @@ static int pass_fast(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_
   float4* rec32 = P<float4>(c->rec32);
   if ((rc = fast_setup(c, xl))) return rc;
   PatchCache& pc = c->cache32;
-  if (!pc.valid) {  // once per mesh: the listed patches' growth and FP64 weights
-    if ((rc = reset_status(c)) || (rc = grow_patches(c, pc, nullptr, nullptr, 3, nullptr, xl, c->n_listed))) return rc;
-  }
-  if ((rc = ensure_cache_weights(c, pc))) return rc;
-  const ListedSums ls{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
-                      P<double>(pc.w), P<int>(pc.wn), P<double>(c->rec), rec32, P<DevStatus>(c->status)};
+  if (!pc.valid && (rc = reset_status(c))) return rc;
+  if ((rc = ensure_listed(c, pc, xl, c->n_listed))) return rc;
+  const ListedSums ls{patch_weights(c, pc), P<double>(c->rec), rec32};
   const PassCounters counters{{P<int>(c->status), P<int>(c->status) + 1, P<int>(c->fcnt) + 1, P<int>(c->fcnt) + 4,
                                P<int>(c->tnext), P<int>(c->bnext), P<int>(c->gfit)}};
   PB("prep_f32");
@@ -1951,8 +1934,7 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
     if ((rc = check_launch(c, "vertex adjacency"))) return rc;
     c->vv_ready = true;
   }
-  bool fork = false;
-  if ((rc = listed_fork(c, d_u, xl, &fork))) return rc;
+  if ((rc = listed_fork(c, d_u, xl))) return rc;
   LearnMesh lm{P<int>(c->vvoff), P<int>(c->vv), P<unsigned char>(c->listed), P<unsigned char>(c->vtile)};
   float4* vr = P<float4>(c->vr16);
   float4* rec = P<float4>(c->rec16);
@@ -1965,7 +1947,7 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
   learned_infer(m, lm, vr, P<float>(c->lsc), c->mlp_packed.p, rec, P<int>(c->fbitems), P<int>(c->fbcount), c->z_max,
                 c->use_mlp, c->max_degree, c->stall_polls, P<int>(c->mlp_err), c->stream);
   PE();
-  if ((rc = listed_join(c, d_u, xl, fork))) return rc;
+  CK(cudaStreamWaitEvent(c->stream, c->join, 0));
   PB("fallback_l");
   learned_fallback(m, lm, vr, P<float>(c->lsc), P<float>(c->wts), P<double>(c->rec), P<int>(c->fbitems),
                    P<int>(c->fbcount), m.V, rec, c->stream);
@@ -2482,10 +2464,8 @@ static int hessian_operator_2d(sprg_ctx* c, double eps, double h_min, double h_m
   ENSURE(c->rec9, sizeof(double) * 9 * (size_t)m.V);
   ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + 9 + 1));
   PatchCache& pc = c->cache2d;
-  if (!pc.valid && (rc = grow_patches(c, pc, nullptr, nullptr, 0, nullptr, lst, -1))) return rc;
-  if ((rc = ensure_cache_weights(c, pc))) return rc;
-  const TriListed ls{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v), P<int>(pc.el), P<long long>(pc.woff),
-                     P<double>(pc.w), P<int>(pc.wn), P<DevStatus>(c->status)};
+  if ((rc = ensure_listed(c, pc, lst, -1))) return rc;
+  const PatchWeights ls = patch_weights(c, pc);
   PB("recover_grad_op_f64");
   launch_apply_operator(m, 1, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
                         P<int>(c->klen), P<double>(c->f), P<double>(c->rec), ls, 0, 0, 0, nullptr, nullptr, c->stream);

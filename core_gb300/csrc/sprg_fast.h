@@ -26,19 +26,11 @@ struct PassCounters {
 int fast_prep_blocks(int V);
 void fast_prep(const DevMesh& m, const double* u, const float4* crec, float4* vrec, int* umax_part,
                const PassCounters& pc, cudaStream_t s);
-// the listed patches' FP64 sums (n patches; patch it: vertex v[it], elements
-// el + it stride, wn[it] weights at w + woff[it], or -1: SPRG_EPATCH), into
-// rec64 (V x 3) and rec32 (32-byte records)
+// the listed patches' FP64 sums, into rec64 (V x 3) and rec32 (32-byte records)
 struct ListedSums {
-  int n, stride;
-  const int* v;
-  const int* el;
-  const long long* woff;
-  const double* w;
-  const int* wn;
+  PatchWeights pw;
   double* rec64;
   float4* rec32;
-  DevStatus* st;
 };
 // per tet: gradient value (3 floats) and packed correction (1 word); also the
 // listed patches' sums

@@ -98,6 +98,19 @@ struct DevStatus {
   int where;       // entity index that raised it
 };
 
+// The listed patches' per-mesh FP64 weights: n patches; patch it: vertex v[it],
+// elements el + it stride, wn[it] weights at w + woff[it], or -1 where the
+// growth or the rank test failed (SPRG_EPATCH in st)
+struct PatchWeights {
+  int n, stride;
+  const int* v;
+  const int* el;
+  const long long* woff;
+  const double* w;
+  const int* wn;
+  DevStatus* st;
+};
+
 // Expansion work list for patches that need growth or are too large for the
 // register path.
 struct ExpandList {
@@ -150,32 +163,29 @@ struct TriFactor {
 int tri_factor_planes();
 int tri_r_planes();
 void launch_tri_factor(const DevMesh& m, TriFactor tf, ExpandList xl, ExpandList big, cudaStream_t s);
+// pw: the listed patches (n = 0: left to the caller)
 void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, TriFactor tf, ExpandList xl,
-                        ExpandList big, bool any_big, cudaStream_t s);
+                        ExpandList big, bool any_big, const PatchWeights& pw, cudaStream_t s);
 // Patches on the expansion list: grow as the reference does, then fit.
 // The list length is read on the device (no host round trip).
 // slab: expand_grid() * expand_max_elems() * (4 + nc + 1) doubles.
-// ip may be NULL: the element gradients of u are computed in place (nc 3:
-// u scalar; nc 9: u a VECTOR field, V x 3) -- for the forms that keep no ip
-// field.  nc 0: growth and rank tests alone (ip, u and rec unused).
+// nc 0: growth and rank tests alone (ip and rec unused).
 // cache_* (optional): record each listed vertex's final element set
-// (expand_max_elems() ints per list slot) for launch_cached_fit_f64.
-void launch_expand_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, ExpandList xl,
-                       double* slab, DevStatus* st, cudaStream_t s, int* cache_v = nullptr, int* cache_n = nullptr,
+// (expand_max_elems() ints per list slot).
+void launch_expand_f64(const DevMesh& m, const double* ip, int nc, double* rec, ExpandList xl, double* slab,
+                       DevStatus* st, cudaStream_t s, int* cache_v = nullptr, int* cache_n = nullptr,
                        int* cache_el = nullptr);
-// One QR fit per cached listed vertex (patch growth depends on geometry only).
-void launch_cached_fit_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
-                           const int* cache_v, const int* cache_n, const int* cache_el, double* slab, DevStatus* st,
-                           cudaStream_t s);
+// Triangles with patches on the warp path: one QR fit per cached listed vertex
+// (patch growth depends on geometry only).
+void launch_cached_fit_f64(const DevMesh& m, const double* ip, int nc, double* rec, int n_cached, const int* cache_v,
+                           const int* cache_n, const int* cache_el, double* slab, DevStatus* st, cudaStream_t s);
 // Per-mesh weights of the cached patches (w = Q1 R^-T t from the fit's
 // QR; woff: each patch's offset into w, wn: its size or -1 where the rank
-// test fails) and the per-pass weighted sums that replace the fits
+// test fails); tets: the per-pass weighted sums of the gradients of u
 void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_v, const int* cache_n,
                                const int* cache_el, const long long* woff, double* w, int* wn, double* slab,
                                cudaStream_t s);
-void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
-                            const int* cache_v, const int* cache_el, const long long* woff, const double* w,
-                            const int* wn, DevStatus* st, cudaStream_t s);
+void launch_cached_wsum_f64(const DevMesh& m, const double* u, const PatchWeights& pw, double* rec, cudaStream_t s);
 int expand_max_elems();
 int expand_grid();
 // Sum partials in fixed order, compute size factor.  mode 0: SPR; 1: target.
@@ -256,17 +266,8 @@ void launch_tri_operator(const DevMesh& m, int kc, const double* w, unsigned cha
 // from that Hessian the FP32 metric records, 12 floats in met, and quality
 // records: FP64 decisions, FP32 magnitudes) at every vertex, the listed ones
 // through their patches' weights
-struct TriListed {
-  int n, stride;
-  const int* v;
-  const int* el;
-  const long long* woff;
-  const double* w;
-  const int* wn;
-  DevStatus* st;
-};
 void launch_apply_operator(const DevMesh& m, int ncin, int kc, const unsigned char* listed, const int* kidx,
-                           const double* kval, const int* klen, const double* f, double* out, const TriListed& ls,
+                           const double* kval, const int* klen, const double* f, double* out, const PatchWeights& ls,
                            double eps, double hmin, double hmax, float* met, void* qrec, cudaStream_t s);
 // incremental mesh update: dst[ids[r] * width + j] = vals[r * width + j];
 // the coordinates' bounding box as order keys (3 minima, 3 maxima)
@@ -277,10 +278,11 @@ void launch_bbox(int V, const double* xyz, unsigned long long* keys, cudaStream_
 void launch_count_out_of_range(long long n, const int* a, int limit, unsigned long long* bad, cudaStream_t s);
 double key_to_double(unsigned long long k);
 // FP64 SPR weights of tet patches (per mesh, the reference's QR; listed
-// patches in lst) and the FP64 recovery from them (listed vertices skipped)
+// patches in lst) and the FP64 recovery from them
 void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, ExpandList lst, cudaStream_t s);
+// (the listed ones through pw)
 void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
-                        double* rec, cudaStream_t s);
+                        const PatchWeights& pw, double* rec, cudaStream_t s);
 // FP64 guard band of the FP32 path: re-decide the listed edges' bits.
 struct GuardScratch {
   int* stamp;      // V ints, persistent (de-duplication stamps)

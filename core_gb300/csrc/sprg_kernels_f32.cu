@@ -445,13 +445,14 @@ __device__ __noinline__ uint4 tet_grad_f64(const double* __restrict__ xyz, const
 // small mesh that chain was the pass's critical path.
 __device__ __noinline__ void listed_sum(const DevMesh& m, const double* __restrict__ u, const ListedSums& ls, int it) {
   const int lane = threadIdx.x & 31;
-  const int v = ls.v[it], n = ls.wn[it];
+  const PatchWeights& pw = ls.pw;
+  const int v = pw.v[it], n = pw.wn[it];
   if (n < 0) {
-    if (lane == 0 && atomicCAS(&ls.st->code, 0, SPRG_EPATCH) == 0) ls.st->where = v;
+    if (lane == 0 && atomicCAS(&pw.st->code, 0, SPRG_EPATCH) == 0) pw.st->where = v;
     return;
   }
-  const int* el = ls.el + (size_t)it * ls.stride;
-  const double* wi = ls.w + ls.woff[it];
+  const int* el = pw.el + (size_t)it * pw.stride;
+  const double* wi = pw.w + pw.woff[it];
   double acc[3] = {0, 0, 0};
   for (int i = lane; i < n; i += 32) {
     const int4 tv = __ldg(reinterpret_cast<const int4*>(m.ev) + el[i]);
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(kBlock, 4)
                uint4* __restrict__ td, int* __restrict__ next_chunk, int per, const __grid_constant__ ListedSums ls) {
   after_previous(vr);
   const int4* __restrict__ ev4 = reinterpret_cast<const int4*>(m.ev);
-  const int n_lc = (ls.n + kBlock / 32 - 1) / (kBlock / 32);
+  const int n_lc = (ls.pw.n + kBlock / 32 - 1) / (kBlock / 32);
   __shared__ int chunk;
   for (;;) {
     if (threadIdx.x == 0) chunk = atomicAdd(next_chunk, 1);
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(kBlock, 4)
     __syncthreads();
     if (c < n_lc) {
       const int it = c * (kBlock / 32) + (threadIdx.x >> 5);
-      if (it < ls.n) listed_sum(m, u, ls, it);
+      if (it < ls.pw.n) listed_sum(m, u, ls, it);
       continue;
     }
     const long t0 = (long)(c - n_lc) * (per * kBlock);
@@ -1362,7 +1363,7 @@ void fast_tet(const DevMesh& m, const float4* vrec, const double* u, float gscal
   if (!m.T) return;
   const long wave = tet_wave();
   const int per = (int)std::max(1L, std::min((long)kTetChunk, (long)m.T / (wave * kBlock)));
-  const long chunks = ((long)m.T + (long)per * kBlock - 1) / ((long)per * kBlock) + (ls.n + kBlock / 32 - 1) / (kBlock / 32);
+  const long chunks = ((long)m.T + (long)per * kBlock - 1) / ((long)per * kBlock) + (ls.pw.n + kBlock / 32 - 1) / (kBlock / 32);
   launch_after(m.early, k_fast_tet, (int)std::min(wave, chunks), kBlock, s, m, vrec, u, gscale, td, next_chunk, per, ls);
 }
 

@@ -73,22 +73,6 @@ __device__ __forceinline__ V3 elem_grad_scalar(const DevMesh& m, int e, const do
   return g;
 }
 
-// gradient of component r of a P1 field stored with stride `stride` (a
-// VECTOR field's row r of the MATRIX ip value), same operation order
-__device__ __forceinline__ V3 elem_grad_component(const DevMesh& m, int e, const double* __restrict__ f, int stride,
-                                                  int r) {
-  const int* ev = m.ev + (size_t)e * m.nn;
-  V3 x[4];
-  for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-  M3 J = ref::jacobian(x, m.nn, m.dim);
-  M3 jinv = ref::jacobian_inverse(J, m.dim);
-  V3 lg[4];
-  ref::shape_grads(m.dim, lg);
-  V3 g = ref::scale(ref::mulv(jinv, lg[0]), f[(size_t)ev[0] * stride + r]);
-  for (int a = 1; a < m.nn; ++a) g = ref::add(g, ref::scale(ref::mulv(jinv, lg[a]), f[(size_t)ev[a] * stride + r]));
-  return g;
-}
-
 // ---------------------------------------------------------------------
 // spr::recoverField -- register path: one warp per vertex, RPL rows per
 // lane.  Patches that are too small, rank deficient or larger than 32*RPL
@@ -364,6 +348,37 @@ __device__ __forceinline__ double tri_div(double a, double b, double y, bool pla
   return quotient(a, b, y);
 }
 
+// A listed patch's sum_i w_i b_i of the samples, by one warp: lanes over the
+// elements, fixed reduction tree.  The recovery kernels' first blocks run these
+// beside the other vertices (a launch of their own took 10 us of latency, the
+// triangles' QR fits 46).
+template <int NC>
+__device__ __noinline__ void listed_ip_sum(const double* __restrict__ ip, const PatchWeights& pw, int it,
+                                           double* __restrict__ rec) {
+  const int lane = threadIdx.x & 31;
+  const int v = pw.v[it], n = pw.wn[it];
+  if (n < 0) {
+    if (lane == 0) set_status(pw.st, SPRG_EPATCH, v);
+    return;
+  }
+  const int* el = pw.el + (size_t)it * pw.stride;
+  const double* w = pw.w + pw.woff[it];
+  double acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0;
+  for (int i = lane; i < n; i += 32) {
+    const double* b = ip + (size_t)el[i] * NC;
+    const double wk = w[i];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] += wk * b[c];
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const double a = warp_sum(acc[c]);
+    if (lane == 0) rec[(size_t)v * NC + c] = a;
+  }
+}
+
 // the recovery of one vertex.  FLAT: the samples' z components (NC = 3), or z
 // row and column (NC = 9), are all 0, and so are their values
 template <int NC, int MAXM, bool CACHED, bool FLAT>
@@ -422,8 +437,14 @@ template <int NC, int MAXM, bool CACHED>
 __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __restrict__ ip,
                                                      const double* __restrict__ qc, const double* __restrict__ rr,
                                                      const unsigned char* __restrict__ code,
-                                                     double* __restrict__ rec, ExpandList xl, ExpandList big) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+                                                     double* __restrict__ rec, ExpandList xl, ExpandList big,
+                                                     int n_list_blocks, const __grid_constant__ PatchWeights pw) {
+  if ((int)blockIdx.x < n_list_blocks) {
+    const int it = blockIdx.x * (128 / 32) + (threadIdx.x >> 5);
+    if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
+    return;
+  }
+  const int v = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
   if (v >= m.V) return;
   const int beg = m.p_off[v];
   double R[kTriR];
@@ -487,8 +508,8 @@ __device__ void warp_sort_set(int* S, int n, int* tmp) {
 // QR fit over the element set S (sorted).  Returns false if rank deficient.
 // rows: n x (NT + nc + 1) doubles; the last column holds the reflector.
 // nc = 0: the rank test alone, nothing is written.
-__device__ bool slab_fit(const DevMesh& m, const int* S, int n, const double* __restrict__ ip,
-                         const double* __restrict__ u, int nc, double* rows, int v, double* rec) {
+__device__ bool slab_fit(const DevMesh& m, const int* S, int n, const double* __restrict__ ip, int nc, double* rows,
+                         int v, double* rec) {
   const int lane = threadIdx.x & 31;
   const int NT = m.dim == 3 ? 4 : 3;
   const int W = NT + nc;
@@ -500,18 +521,7 @@ __device__ bool slab_fit(const DevMesh& m, const int* S, int n, const double* __
     double* rw = rows + (size_t)i * LD;
     rw[0] = 1.0; rw[1] = p.v[0]; rw[2] = p.v[1];
     if (NT == 4) rw[3] = p.v[2];
-    if (nc == 0) continue;
-    if (ip) {
-      for (int c = 0; c < nc; ++c) rw[NT + c] = ip[(size_t)el * nc + c];
-    } else if (nc == 3) {  // no resident ip field: the gradient of the scalar field u
-      V3 g = elem_grad_scalar(m, el, u);
-      for (int c = 0; c < 3; ++c) rw[NT + c] = g.v[c];
-    } else {  // ... or of the VECTOR field u (V x 3): MATRIX rows, row r = grad u_r
-      for (int r = 0; r < 3; ++r) {
-        V3 g = elem_grad_component(m, el, u, 3, r);
-        for (int c = 0; c < 3; ++c) rw[NT + 3 * r + c] = g.v[c];
-      }
-    }
+    for (int c = 0; c < nc; ++c) rw[NT + c] = ip[(size_t)el * nc + c];
   }
   __syncwarp();
   for (int k = 0; k < NT; ++k) {
@@ -556,8 +566,7 @@ __device__ bool slab_fit(const DevMesh& m, const int* S, int n, const double* __
   return true;
 }
 
-__global__ void __launch_bounds__(32) k_expand(DevMesh m, const double* __restrict__ ip,
-                                               const double* __restrict__ u, int nc,
+__global__ void __launch_bounds__(32) k_expand(DevMesh m, const double* __restrict__ ip, int nc,
                                                double* __restrict__ rec, const int* __restrict__ items,
                                                const int* __restrict__ n_items_ptr, int cap, double* slab,
                                                DevStatus* st, int* cache_v, int* cache_n, int* cache_el) {
@@ -596,7 +605,7 @@ __global__ void __launch_bounds__(32) k_expand(DevMesh m, const double* __restri
       int n0 = nS;
       warp_sort_set(S, n0, tmp);
       double* rows = (n0 * (NT + nc + 1) <= kExpandSmemRows * 8) ? srows : grows;
-      if (slab_fit(m, S, n0, ip, u, nc, rows, v, rec)) { done = true; break; }
+      if (slab_fit(m, S, n0, ip, nc, rows, v, rec)) { done = true; break; }
       for (int i = lane; i < n0; i += 32) old[i] = S[i];
       __syncwarp();
       for (int sd = m.dim - 1; sd >= 0 && !done; --sd) {
@@ -624,7 +633,7 @@ __global__ void __launch_bounds__(32) k_expand(DevMesh m, const double* __restri
         int n1 = nS;
         warp_sort_set(S, n1, tmp);
         double* rows1 = (n1 * (NT + nc + 1) <= kExpandSmemRows * 8) ? srows : grows;
-        if (slab_fit(m, S, n1, ip, u, nc, rows1, v, rec)) { done = true; break; }
+        if (slab_fit(m, S, n1, ip, nc, rows1, v, rec)) { done = true; break; }
       }
       if (!done && !failed && !(nS > n0)) failed = true;  // "all hope is lost"
     }
@@ -644,7 +653,7 @@ __global__ void __launch_bounds__(32) k_expand(DevMesh m, const double* __restri
 // Later passes: the listed vertices' final patches come from the cache; one
 // QR fit each, no growth rounds.
 __global__ void __launch_bounds__(32) k_cached_fit(DevMesh m, const double* __restrict__ ip,
-                                                   const double* __restrict__ u, int nc, double* __restrict__ rec,
+                                                   int nc, double* __restrict__ rec,
                                                    int n_cached, const int* __restrict__ cache_v,
                                                    const int* __restrict__ cache_n, const int* __restrict__ cache_el,
                                                    double* slab, DevStatus* st) {
@@ -658,7 +667,7 @@ __global__ void __launch_bounds__(32) k_cached_fit(DevMesh m, const double* __re
       continue;
     }
     double* rows = (n * (NT + nc + 1) <= kExpandSmemRows * 8) ? srows : grows;
-    if (!slab_fit(m, cache_el + (size_t)it * kExpandMaxElems, n, ip, u, nc, rows, v, rec) && threadIdx.x == 0)
+    if (!slab_fit(m, cache_el + (size_t)it * kExpandMaxElems, n, ip, nc, rows, v, rec) && threadIdx.x == 0)
       set_status(st, SPRG_EPATCH, v);
     __syncwarp();
   }
@@ -753,47 +762,29 @@ __global__ void __launch_bounds__(32) k_cached_weights(DevMesh m, int n_cached, 
   }
 }
 
-// rec(v) = sum_i w_i b_i over a cached patch, warp per patch (lanes over the
-// elements, fixed reduction tree); b_i = the element's IP value, or the
-// gradient of the scalar field (nc = 3) / of the vector field (nc = 9)
-__global__ void __launch_bounds__(kBlock) k_cached_wsum(DevMesh m, const double* __restrict__ ip,
-                                                        const double* __restrict__ u, int nc,
-                                                        double* __restrict__ rec, int n_cached,
-                                                        const int* __restrict__ cache_v,
-                                                        const int* __restrict__ cache_el,
-                                                        const long long* __restrict__ woff,
-                                                        const double* __restrict__ w, const int* __restrict__ wn,
-                                                        DevStatus* st) {
-  after_previous(ip, u, cache_v, cache_el, woff, w, wn);
+// rec(v) = sum_i w_i grad u over a cached tet patch, warp per patch (lanes over
+// the elements, fixed reduction tree): the learned form's listed vertices
+__global__ void __launch_bounds__(kBlock) k_cached_wsum(DevMesh m, const double* __restrict__ u,
+                                                        double* __restrict__ rec,
+                                                        const __grid_constant__ PatchWeights pw) {
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * (blockDim.x >> 5);
-  for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < n_cached; it += nwarps) {
-    const int v = cache_v[it], n = wn[it];
+  for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < pw.n; it += nwarps) {
+    const int v = pw.v[it], n = pw.wn[it];
     if (n < 0) {
-      if (lane == 0) set_status(st, SPRG_EPATCH, v);
+      if (lane == 0) set_status(pw.st, SPRG_EPATCH, v);
       continue;
     }
-    const int* S = cache_el + (size_t)it * kExpandMaxElems;
-    const double* wi = w + woff[it];
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const int* S = pw.el + (size_t)it * pw.stride;
+    const double* wi = pw.w + pw.woff[it];
+    double acc[3] = {0, 0, 0};
     for (int i = lane; i < n; i += 32) {
-      const int el = S[i];
-      const double wk = wi[i];
-      if (ip) {
-        for (int c = 0; c < nc; ++c) acc[c] += wk * ip[(size_t)el * nc + c];
-      } else if (nc == 3) {
-        const V3 g = elem_grad_scalar(m, el, u);
-        for (int c = 0; c < 3; ++c) acc[c] += wk * g.v[c];
-      } else {
-        for (int r = 0; r < 3; ++r) {
-          const V3 g = elem_grad_component(m, el, u, 3, r);
-          for (int c = 0; c < 3; ++c) acc[3 * r + c] += wk * g.v[c];
-        }
-      }
+      const V3 g = elem_grad_scalar(m, S[i], u);
+      for (int c = 0; c < 3; ++c) acc[c] += wi[i] * g.v[c];
     }
-    for (int c = 0; c < nc; ++c) {
+    for (int c = 0; c < 3; ++c) {
       const double a = warp_sum(acc[c]);
-      if (lane == 0) rec[(size_t)v * nc + c] = a;
+      if (lane == 0) rec[(size_t)v * 3 + c] = a;
     }
   }
 }
@@ -2267,13 +2258,11 @@ __global__ void __launch_bounds__(kBlock) k_tri_operator(DevMesh m, const double
   }
 }
 
-// The listed patches of a triangle mesh (n patches; patch it: vertex v[it],
-// elements el + it stride, wn[it] weights at w + woff[it], or -1: SPRG_EPATCH):
-// sum_i w_i grad f over the patch by one warp, lanes over the elements, fixed
-// reduction tree; every lane gets the sums (row r of a VECTOR field's MATRIX
-// value in acc[3 r ..]).  false: no weights.
+// A listed patch of a triangle mesh: sum_i w_i grad f over it by one warp, lanes
+// over the elements, fixed reduction tree; every lane gets the sums (row r of
+// a VECTOR field's MATRIX value in acc[3 r ..]).  false: no weights.
 template <int NCIN>
-__device__ __noinline__ bool tri_listed_sum(const DevMesh& m, const double* __restrict__ f, const TriListed& ls, int it,
+__device__ __noinline__ bool tri_listed_sum(const DevMesh& m, const double* __restrict__ f, const PatchWeights& ls, int it,
                                             double* acc) {
   const int lane = threadIdx.x & 31;
   const int n = ls.wn[it];
@@ -2323,7 +2312,7 @@ __global__ void __launch_bounds__(kBlock, METRIC ? 4 : 5) k_apply_operator(DevMe
                                                            const double* __restrict__ kval,
                                                            const int* __restrict__ klen, const double* __restrict__ f,
                                                            double* __restrict__ out, int n_list_blocks,
-                                                           const __grid_constant__ TriListed ls, MetricOut mo) {
+                                                           const __grid_constant__ PatchWeights ls, MetricOut mo) {
   constexpr int NR = (KC == 2 && NCIN == 3) ? 2 : NCIN;  // input components that can be nonzero
   constexpr int NO = 3 * NCIN;
   const int V = m.V;
@@ -2553,9 +2542,15 @@ template <int NC>
 __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double* __restrict__ ip,
                                                         const double* __restrict__ w,
                                                         const unsigned char* __restrict__ listed,
+                                                        int n_list_blocks, const __grid_constant__ PatchWeights pw,
                                                         double* __restrict__ rec) {
   after_previous(ip, w, listed);
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((int)blockIdx.x < n_list_blocks) {
+    const int it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
+    return;
+  }
+  const int v = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
   if (v >= m.V || listed[v]) return;
   const int beg = m.p_off[v], end = m.p_off[v + 1];
   double acc[NC];
@@ -2584,13 +2579,13 @@ void launch_tri_factor(const DevMesh& m, TriFactor tf, ExpandList xl, ExpandList
 }
 
 void launch_recover_f64(const DevMesh& m, const double* ip, int nc, double* rec, TriFactor tf, ExpandList xl,
-                        ExpandList big, bool any_big, cudaStream_t s) {
+                        ExpandList big, bool any_big, const PatchWeights& pw, cudaStream_t s) {
   if (!m.V || m.dim != 2) return;  // tets recover through the per-mesh QR weights
   // triangles: a thread per vertex up to kTriThreadRows patch elements, then
   // the warp path over the vertices it listed
-  const int grid = (m.V + 127) / 128;
+  const int nl = (pw.n + 3) / 4, grid = nl + (m.V + 127) / 128;
   const int lgrid = 152 * 8;
-  auto go = [&](auto kernel) { kernel<<<grid, 128, 0, s>>>(m, ip, tf.qc, tf.rr, tf.code, rec, xl, big); };
+  auto go = [&](auto kernel) { kernel<<<grid, 128, 0, s>>>(m, ip, tf.qc, tf.rr, tf.code, rec, xl, big, nl, pw); };
   if (nc == 3) {
     go(tf.qc ? k_recover_tri<3, kTriThreadRows, true> : k_recover_tri<3, kTriThreadRows, false>);
     if (any_big) k_recover_list<3, 3, 1><<<lgrid, kBlock, 0, s>>>(m, ip, rec, xl, big);
@@ -2604,17 +2599,17 @@ int expand_max_elems() { return kExpandMaxElems; }
 
 int expand_grid() { return kExpandGrid; }
 
-void launch_expand_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, ExpandList xl,
+void launch_expand_f64(const DevMesh& m, const double* ip, int nc, double* rec, ExpandList xl,
                        double* slab, DevStatus* st, cudaStream_t s, int* cache_v, int* cache_n, int* cache_el) {
-  k_expand<<<kExpandGrid, 32, 0, s>>>(m, ip, u, nc, rec, xl.items, xl.count, xl.cap, slab, st, cache_v, cache_n,
+  k_expand<<<kExpandGrid, 32, 0, s>>>(m, ip, nc, rec, xl.items, xl.count, xl.cap, slab, st, cache_v, cache_n,
                                       cache_el);
 }
 
-void launch_cached_fit_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
+void launch_cached_fit_f64(const DevMesh& m, const double* ip, int nc, double* rec, int n_cached,
                            const int* cache_v, const int* cache_n, const int* cache_el, double* slab, DevStatus* st,
                            cudaStream_t s) {
   if (n_cached > 0)
-    k_cached_fit<<<n_cached < kExpandGrid ? n_cached : kExpandGrid, 32, 0, s>>>(m, ip, u, nc, rec, n_cached, cache_v,
+    k_cached_fit<<<n_cached < kExpandGrid ? n_cached : kExpandGrid, 32, 0, s>>>(m, ip, nc, rec, n_cached, cache_v,
                                                                                 cache_n, cache_el, slab, st);
 }
 
@@ -2627,12 +2622,8 @@ void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_
   else k_cached_weights<3><<<g, 32, 0, s>>>(m, n_cached, cache_v, cache_n, cache_el, woff, w, wn, slab);
 }
 
-void launch_cached_wsum_f64(const DevMesh& m, const double* ip, const double* u, int nc, double* rec, int n_cached,
-                            const int* cache_v, const int* cache_el, const long long* woff, const double* w,
-                            const int* wn, DevStatus* st, cudaStream_t s) {
-  if (n_cached > 0)
-    launch_after(m.early, k_cached_wsum, std::min(nblk((long)n_cached * 32), 152 * 8), kBlock, s, m, ip, u, nc, rec, n_cached,
-                 cache_v, cache_el, woff, w, wn, st);
+void launch_cached_wsum_f64(const DevMesh& m, const double* u, const PatchWeights& pw, double* rec, cudaStream_t s) {
+  if (pw.n > 0) k_cached_wsum<<<std::min(nblk((long)pw.n * 32), 152 * 8), kBlock, 0, s>>>(m, u, rec, pw);
 }
 
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target, int dim,
@@ -2800,7 +2791,7 @@ void launch_tri_operator(const DevMesh& m, int kc, const double* w, unsigned cha
 }
 
 void launch_apply_operator(const DevMesh& m, int ncin, int kc, const unsigned char* listed, const int* kidx,
-                           const double* kval, const int* klen, const double* f, double* out, const TriListed& ls,
+                           const double* kval, const int* klen, const double* f, double* out, const PatchWeights& ls,
                            double eps, double hmin, double hmax, float* met, void* qrec, cudaStream_t s) {
   if (!m.V) return;
   const int nl = nblk((long)ls.n * 32);
@@ -2844,9 +2835,11 @@ void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, Expan
 }
 
 void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
-                        double* rec, cudaStream_t s) {
+                        const PatchWeights& pw, double* rec, cudaStream_t s) {
   if (!m.V) return;
-  launch_after(m.early, nc == 3 ? k_recover_w64<3> : k_recover_w64<9>, nblk(m.V), kBlock, s, m, ip, w, listed, rec);
+  const int nl = nblk((long)pw.n * 32);
+  launch_after(m.early, nc == 3 ? k_recover_w64<3> : k_recover_w64<9>, nl + nblk(m.V), kBlock, s, m, ip, w, listed, nl,
+               pw, rec);
 }
 
 }  // namespace sprg

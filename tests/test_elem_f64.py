@@ -194,7 +194,10 @@ def test_triangle_recovery_bitwise(gpu_lib, oracle_lib, n, kind, nc):
             return [c.recoverField(ip) for ip in ips]
     kept, placed = answers(False), answers(True)
     for a, b in zip(kept, placed):
-        assert np.array_equal(a, b, equal_nan=True)
+        assert np.array_equal(a[thread], b[thread], equal_nan=True)
+        # the grown patches: weighted sums with the factors kept, QR fits without
+        fin = np.isfinite(a).all(axis=1) & np.isfinite(b).all(axis=1)
+        assert np.abs(a[fin] - b[fin]).max() <= 1e-10 * np.abs(b[fin]).max()
     if kind == "fan":
         assert cnt.max() > 8
         return
