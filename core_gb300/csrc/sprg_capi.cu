@@ -130,10 +130,6 @@ struct sprg_ctx {
   float z_max = 8.f;
   int stall_polls = 0;      // test hook: network-kernel wait on a barrier nothing completes (0: off)
   int alloc_fail_in = -1;   // test hook: device allocations left before one fails (-1: off)
-  // side stream for the FP64 fits of listed patches, forked from and joined
-  // back into the pass's stream
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
   // copy stream of the host entry point: the flags upload and (FP32) the size
   // download run beside the pass
   cudaStream_t copy = nullptr;
@@ -1045,14 +1041,8 @@ int sprg_destroy(sprg_ctx* c) {
   for (auto& e : c->e2e_ev)
     if (e) cudaEventDestroy(e);
   if (c->stage) cudaFreeHost(c->stage);
-  if (c->side) {
-    cudaStreamSynchronize(c->side);
-    cudaStreamDestroy(c->side);
-  }
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->e2e_exec) cudaGraphExecDestroy(c->e2e_exec);
-  if (c->fork) cudaEventDestroy(c->fork);
-  if (c->join) cudaEventDestroy(c->join);
   if (c->own) cudaStreamDestroy(c->own);
   delete c;
   return SPRG_OK;
@@ -1515,25 +1505,6 @@ static int fast_setup(sprg_ctx* c, ExpandList xl) {
   return SPRG_OK;
 }
 
-// the learned form's listed patches: their FP64 sums on the side stream,
-// joined by the caller before the results are used
-static int listed_fork(sprg_ctx* c, const double* d_u, ExpandList xl) {
-  int rc = ensure_listed(c, c->cache32, xl, c->n_listed);
-  if (rc) return rc;
-  if (!c->side) {
-    CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
-  }
-  CK(cudaEventRecord(c->fork, c->stream));
-  CK(cudaStreamWaitEvent(c->side, c->fork, 0));
-  launch_cached_wsum_f64(c->m, d_u, patch_weights(c, c->cache32), P<double>(c->rec), c->side);
-  c->launches += 1;
-  if ((rc = check_launch(c, "listed sums"))) return rc;
-  CK(cudaEventRecord(c->join, c->side));
-  return SPRG_OK;
-}
-
 // patch-size bins of the non-listed vertices (stable: ascending ids within a
 // bin), once per mesh
 // the sliced copy of the patch lists over the bins (after the bins and the
@@ -1891,9 +1862,8 @@ static int learned_scratch(sprg_ctx* c) {
 // 2^-30 / s: the coordinate records' difference scale
 static float learned_cs(const sprg_ctx* c) { return (float)(std::ldexp(1.0, -30) / c->frame[3]); }
 
-static void learned_records(sprg_ctx* c, const double* d_u) {
-  learned_prep(c->m, d_u, learned_cs(c), P<double>(c->lrange), P<unsigned>(c->ldone), P<float>(c->lsc),
-               P<float4>(c->vr16), c->stream);
+static void learned_range_of(sprg_ctx* c, const double* d_u, const LearnCounters& lc) {
+  learned_range(c->m, d_u, learned_cs(c), P<double>(c->lrange), P<unsigned>(c->ldone), P<float>(c->lsc), lc, c->stream);
 }
 
 // Learned pass: network recovery with plain-SPR fallback, FP32 sweeps
@@ -1917,8 +1887,12 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
   ENSURE(c->fbitems, sizeof(int) * (size_t)m.V);
   ENSURE(c->fbcount, sizeof(int));
   ENSURE(c->mlp_err, sizeof(int));
+  if (!c->edone.p) {
+    ENSURE(c->edone, sizeof(unsigned));
+    CK(cudaMemsetAsync(c->edone.p, 0, sizeof(unsigned), c->stream));
+  }
   if ((rc = learned_scratch(c))) return rc;
-  if ((rc = reset_status(c))) return rc;
+  if (!c->cache32.valid && (rc = reset_status(c))) return rc;
   ExpandList xl{P<int>(c->fitems), P<int>(c->fcnt) + 3, m.V};
   if ((rc = fast_setup(c, xl))) return rc;
   if (!c->vv_ready) {
@@ -1934,29 +1908,27 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
     if ((rc = check_launch(c, "vertex adjacency"))) return rc;
     c->vv_ready = true;
   }
-  if ((rc = listed_fork(c, d_u, xl))) return rc;
+  if ((rc = ensure_listed(c, c->cache32, xl, c->n_listed))) return rc;
   LearnMesh lm{P<int>(c->vvoff), P<int>(c->vv), P<unsigned char>(c->listed), P<unsigned char>(c->vtile)};
   float4* vr = P<float4>(c->vr16);
   float4* rec = P<float4>(c->rec16);
-  CK(cudaMemsetAsync(c->fbcount.p, 0, sizeof(int), c->stream));
   PB("prep_l");
-  learned_records(c, d_u);
+  // the range kernel also clears the status, the fallback count and the
+  // network's error word (a wait that ran out is reported once)
+  learned_range_of(c, d_u, LearnCounters{{P<int>(c->status), P<int>(c->status) + 1, P<int>(c->fbcount), P<int>(c->mlp_err)}});
+  learned_prep(m, d_u, P<double>(c->lrange), vr, patch_weights(c, c->cache32), P<double>(c->rec), c->stream);
   PE();
   PB("mlp_l");
-  CK(cudaMemsetAsync(c->mlp_err.p, 0, sizeof(int), c->stream));  // a wait that ran out is reported once
   learned_infer(m, lm, vr, P<float>(c->lsc), c->mlp_packed.p, rec, P<int>(c->fbitems), P<int>(c->fbcount), c->z_max,
                 c->use_mlp, c->max_degree, c->stall_polls, P<int>(c->mlp_err), c->stream);
   PE();
-  CK(cudaStreamWaitEvent(c->stream, c->join, 0));
   PB("fallback_l");
   learned_fallback(m, lm, vr, P<float>(c->lsc), P<float>(c->wts), P<double>(c->rec), P<int>(c->fbitems),
                    P<int>(c->fbcount), m.V, rec, c->stream);
   PE();
   PB("error_l");
-  learned_error(m, rec, P<float>(c->lsc), P<float2>(c->geo), P<float>(c->ql), P<double>(c->partials), nb, c->stream);
-  PE();
-  PB("size_factor");
-  launch_size_factor(P<double>(c->partials), nb, 0, adapt_ratio, 0, m.dim, P<double>(c->out3), c->stream);
+  learned_error(m, rec, P<float>(c->lsc), P<float2>(c->geo), P<float>(c->ql), P<double>(c->partials), nb,
+                P<unsigned>(c->edone), adapt_ratio, P<double>(c->out3), c->stream);
   PE();
   PB("average_l");
   learned_average(m, P<float>(c->ql), P<double>(c->out3), P<float>(c->sizel), c->stream);
@@ -1964,7 +1936,7 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
   PB("measure_l");
   learned_measure(m, P<float>(c->elen), P<float>(c->sizel), d_split, d_collapse, c->stream);
   PE();
-  c->launches += 8;  // range, prep, network, fallback, error, size factor, average, measure
+  c->launches += 7;  // range, prep, network, fallback, error, average, measure
   c->size_valid = false;
   c->L_valid = false;
   return check_launch(c, "learned pass");
@@ -1978,7 +1950,7 @@ static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uin
   {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->stream, &cap));
-    c->m.early = c->m.T <= (cap == cudaStreamCaptureStatusActive ? 2 << 20 : 6 << 20);
+    c->m.early = c->m.T <= (cap == cudaStreamCaptureStatusActive ? 1 << 20 : 3 << 20);
   }
   if (c->precision == SPRG_FP32) return pass_fast(c, d_u, adapt_ratio, d_split, d_collapse);
   if (c->precision == SPRG_LEARNED) return pass_learned(c, d_u, adapt_ratio, d_split, d_collapse);
@@ -2377,7 +2349,9 @@ int sprg_learned_features(sprg_ctx* c, const double* d_u, uint16_t* d_x, float* 
     c->vv_ready = true;
   }
   LearnMesh lm{P<int>(c->vvoff), P<int>(c->vv), P<unsigned char>(c->listed), P<unsigned char>(c->vtile)};
-  learned_records(c, d_u);
+  int* st = P<int>(c->status);  // cleared as a pass would
+  learned_range_of(c, d_u, LearnCounters{{st, st + 1, st, st}});
+  learned_prep(m, d_u, P<double>(c->lrange), P<float4>(c->vr16), PatchWeights{}, nullptr, c->stream);
   learned_features(m, lm, P<float4>(c->vr16), P<float>(c->lsc), d_x, d_aux, c->stream);
   CK(cudaStreamSynchronize(c->stream));
   return check_launch(c, "learned features");

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
+#include <utility>
 
 #include "spr_gb300.h"
 
@@ -62,16 +63,16 @@ __device__ __forceinline__ double batch_sf(const BatchView& b, const double* out
 // lets the kernel after this one be set up in turn (once every block of this
 // one has started), the second waits until the one before is complete and
 // its writes are visible; both do nothing in an ordinary launch.
-// early (DevMesh::early, set per pass): whether to.  Direct passes gain 18 us
-// at 3k tets and 11 us at 6M (the host's launches and the kernels' set-up
-// overlap), passes being captured into a graph 4 us at 3k, 2 at 1.6M and
-// nothing at 3M; at 13M tets both are slower by 40 to 58 us (the waiting
-// blocks take the slots that the tail of the kernel before would fill), so
-// the lines lie at 6M and 2M tets.
+// early (DevMesh::early, set per pass): whether to.  Direct passes gain 14 to
+// 18 us at 3k tets (FP32, learned, FP64), 13 at 1.6M and 7 at 3.1M (the host's
+// launches and the kernels' set-up overlap), passes being captured into a
+// graph 4 us at 3k and nothing from 0.5M; at 5.3M tets both lose 30 to 50 of
+// about 300 us (waiting blocks take the slots that the tail of the kernel
+// before would fill), so the lines lie at 3M and 1M tets.
 // The kernel's inputs that a kernel before it (back to the last ordinary launch)
-// wrote go through it: a pointer to const with __restrict__ is memory that does not change during the kernel, so the
-// compiler may move its loads above the wait; values that come out of an asm
-// behind it cannot be used earlier.
+// wrote go through it: a pointer to const with __restrict__ is memory that does
+// not change during the kernel, so the compiler may move its loads above the
+// wait; values that come out of an asm behind it cannot be used earlier.
 template <class... P>
 __device__ __forceinline__ void after_previous(P&... p) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -79,10 +80,12 @@ __device__ __forceinline__ void after_previous(P&... p) {
   (void)(([&] { asm volatile("" : "+l"(p)::"memory"); }(), 0) + ... + 0);
 }
 template <class... P, class... A>
-inline void launch_after(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+inline void launch_after_smem(bool early, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                              A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -90,6 +93,10 @@ inline void launch_after(bool early, void (*kernel)(P...), int grid, int block, 
   cfg.attrs = at;
   cfg.numAttrs = early ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline void launch_after(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t s, A&&... args) {
+  launch_after_smem(early, kernel, grid, block, 0, s, std::forward<A>(args)...);
 }
 
 // Device status word written by kernels (first error wins).
@@ -181,11 +188,10 @@ void launch_cached_fit_f64(const DevMesh& m, const double* ip, int nc, double* r
                            const int* cache_n, const int* cache_el, double* slab, DevStatus* st, cudaStream_t s);
 // Per-mesh weights of the cached patches (w = Q1 R^-T t from the fit's
 // QR; woff: each patch's offset into w, wn: its size or -1 where the rank
-// test fails); tets: the per-pass weighted sums of the gradients of u
+// test fails)
 void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_v, const int* cache_n,
                                const int* cache_el, const long long* woff, double* w, int* wn, double* slab,
                                cudaStream_t s);
-void launch_cached_wsum_f64(const DevMesh& m, const double* u, const PatchWeights& pw, double* rec, cudaStream_t s);
 int expand_max_elems();
 int expand_grid();
 // Sum partials in fixed order, compute size factor.  mode 0: SPR; 1: target.

@@ -42,6 +42,7 @@
 
 #include "sprg_fast.h"
 #include "sprg_ld.cuh"
+#include "sprg_listed.cuh"
 #include "sprg_reduce.cuh"
 
 namespace sprg {
@@ -437,66 +438,23 @@ __device__ __noinline__ uint4 tet_grad_f64(const double* __restrict__ xyz, const
                     pack_corr(s[0], s[1], s[2], r[0], r[1], r[2]));
 }
 
-// rec(v) = sum_i w_i g_i over a listed vertex's grown patch (its FP64 weights
-// from the reference's QR, FP64 gradients of the field), by one warp: lanes over
-// the elements, fixed reduction tree.  Stored in FP64 for the guard and as the
+// a listed vertex's recovered gradient, stored in FP64 for the guard and as the
 // 32-byte record of the other vertices.  These sums ran in a kernel of their
 // own beside this one, joined by two events and merged by a third kernel: on a
 // small mesh that chain was the pass's critical path.
 __device__ __noinline__ void listed_sum(const DevMesh& m, const double* __restrict__ u, const ListedSums& ls, int it) {
-  const int lane = threadIdx.x & 31;
-  const PatchWeights& pw = ls.pw;
-  const int v = pw.v[it], n = pw.wn[it];
-  if (n < 0) {
-    if (lane == 0 && atomicCAS(&pw.st->code, 0, SPRG_EPATCH) == 0) pw.st->where = v;
-    return;
+  double acc[3];
+  if (!listed_grad_sum(m, u, ls.pw, it, acc) || (threadIdx.x & 31) != 0) return;
+  const int v = ls.pw.v[it];
+  float h[3], l[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    ls.rec64[3 * (size_t)v + k] = acc[k];
+    h[k] = (float)acc[k];
+    l[k] = (float)(acc[k] - (double)h[k]);
   }
-  const int* el = pw.el + (size_t)it * pw.stride;
-  const double* wi = pw.w + pw.woff[it];
-  double acc[3] = {0, 0, 0};
-  for (int i = lane; i < n; i += 32) {
-    const int4 tv = __ldg(reinterpret_cast<const int4*>(m.ev) + el[i]);
-    const int id[4] = {tv.x, tv.y, tv.z, tv.w};
-    double x[4][3], e[3][3], du[3];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) x[a][k] = __ldg(m.xyz + 3 * (size_t)id[a] + k);
-    const double u0 = __ldg(u + id[0]);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      du[a] = __ldg(u + id[a + 1]) - u0;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) e[a][k] = x[a + 1][k] - x[0][k];
-    }
-    double cf[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double* p = e[(a + 1) % 3];
-      const double* q = e[(a + 2) % 3];
-      cf[a][0] = p[1] * q[2] - p[2] * q[1];
-      cf[a][1] = p[2] * q[0] - p[0] * q[2];
-      cf[a][2] = p[0] * q[1] - p[1] * q[0];
-    }
-    const double wk = wi[i] / (e[0][0] * cf[0][0] + e[0][1] * cf[0][1] + e[0][2] * cf[0][2]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) acc[k] += wk * (cf[0][k] * du[0] + cf[1][k] * du[1] + cf[2][k] * du[2]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (lane == 0) {
-    float h[3], l[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      ls.rec64[3 * (size_t)v + k] = acc[k];
-      h[k] = (float)acc[k];
-      l[k] = (float)(acc[k] - (double)h[k]);
-    }
-    ls.rec32[2 * (size_t)v] = make_float4(h[0], h[1], h[2], l[0]);
-    ls.rec32[2 * (size_t)v + 1] = make_float4(l[1], l[2], 0.f, 0.f);
-  }
+  ls.rec32[2 * (size_t)v] = make_float4(h[0], h[1], h[2], l[0]);
+  ls.rec32[2 * (size_t)v + 1] = make_float4(l[1], l[2], 0.f, 0.f);
 }
 
 __global__ void __launch_bounds__(kBlock, 4)

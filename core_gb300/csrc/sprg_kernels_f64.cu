@@ -58,21 +58,6 @@ __device__ __forceinline__ V3 elem_ip_point(const DevMesh& m, int e) {
   return p;
 }
 
-// gradient of a scalar P1 field at the order-1 integration point of e
-// (ScalarElement::grad, apf/apfScalarElement.cc:18)
-__device__ __forceinline__ V3 elem_grad_scalar(const DevMesh& m, int e, const double* __restrict__ f) {
-  const int* ev = m.ev + (size_t)e * m.nn;
-  V3 x[4];
-  for (int a = 0; a < m.nn; ++a) x[a] = load_xyz(m.xyz, ev[a]);
-  M3 J = ref::jacobian(x, m.nn, m.dim);
-  M3 jinv = ref::jacobian_inverse(J, m.dim);
-  V3 lg[4];
-  ref::shape_grads(m.dim, lg);
-  V3 g = ref::scale(ref::mulv(jinv, lg[0]), f[ev[0]]);
-  for (int a = 1; a < m.nn; ++a) g = ref::add(g, ref::scale(ref::mulv(jinv, lg[a]), f[ev[a]]));
-  return g;
-}
-
 // ---------------------------------------------------------------------
 // spr::recoverField -- register path: one warp per vertex, RPL rows per
 // lane.  Patches that are too small, rank deficient or larger than 32*RPL
@@ -759,33 +744,6 @@ __global__ void __launch_bounds__(32) k_cached_weights(DevMesh m, int n_cached, 
     }
     if (lane == 0) wn[it] = n;
     __syncwarp();
-  }
-}
-
-// rec(v) = sum_i w_i grad u over a cached tet patch, warp per patch (lanes over
-// the elements, fixed reduction tree): the learned form's listed vertices
-__global__ void __launch_bounds__(kBlock) k_cached_wsum(DevMesh m, const double* __restrict__ u,
-                                                        double* __restrict__ rec,
-                                                        const __grid_constant__ PatchWeights pw) {
-  const int lane = threadIdx.x & 31;
-  const int nwarps = gridDim.x * (blockDim.x >> 5);
-  for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < pw.n; it += nwarps) {
-    const int v = pw.v[it], n = pw.wn[it];
-    if (n < 0) {
-      if (lane == 0) set_status(pw.st, SPRG_EPATCH, v);
-      continue;
-    }
-    const int* S = pw.el + (size_t)it * pw.stride;
-    const double* wi = pw.w + pw.woff[it];
-    double acc[3] = {0, 0, 0};
-    for (int i = lane; i < n; i += 32) {
-      const V3 g = elem_grad_scalar(m, S[i], u);
-      for (int c = 0; c < 3; ++c) acc[c] += wi[i] * g.v[c];
-    }
-    for (int c = 0; c < 3; ++c) {
-      const double a = warp_sum(acc[c]);
-      if (lane == 0) rec[(size_t)v * 3 + c] = a;
-    }
   }
 }
 
@@ -2620,10 +2578,6 @@ void launch_cached_weights_f64(const DevMesh& m, int n_cached, const int* cache_
   const int g = n_cached < kExpandGrid ? n_cached : kExpandGrid;
   if (m.dim == 3) k_cached_weights<4><<<g, 32, 0, s>>>(m, n_cached, cache_v, cache_n, cache_el, woff, w, wn, slab);
   else k_cached_weights<3><<<g, 32, 0, s>>>(m, n_cached, cache_v, cache_n, cache_el, woff, w, wn, slab);
-}
-
-void launch_cached_wsum_f64(const DevMesh& m, const double* u, const PatchWeights& pw, double* rec, cudaStream_t s) {
-  if (pw.n > 0) k_cached_wsum<<<std::min(nblk((long)pw.n * 32), 152 * 8), kBlock, 0, s>>>(m, u, rec, pw);
 }
 
 void launch_size_factor(const double* partials, int n_blocks, int mode, double adapt_ratio, double target, int dim,

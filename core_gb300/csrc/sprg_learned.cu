@@ -25,7 +25,9 @@
 #include <cub/cub.cuh>
 
 #include "sprg_ld.cuh"
+#include "sprg_listed.cuh"
 #include "sprg_learned.h"
+#include "sprg_reduce.cuh"
 
 namespace sprg {
 namespace {
@@ -89,39 +91,48 @@ __global__ void k_v2v_sort(int V, const int* __restrict__ off, int* __restrict__
 // at 160^3 through the element gradients and the neighbour fit; exact
 // differences take it to the FP32 arithmetic's level.)
 // ---------------------------------------------------------------------------
-constexpr int kRangeGrid = 1216;
+constexpr int kRangeGrid = 304;
 
 __device__ __forceinline__ float qdiff(float a, float b, float scale) {
   return __int2float_rn(__float_as_int(a) - __float_as_int(b)) * scale;
 }
 
-// (min, max, any non-finite) of a block's values, in every thread of warp 0
+// finite doubles as keys that order as the values do, and back
+__device__ __forceinline__ unsigned long long range_key(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double range_value(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
+
+// (min, max, any non-finite) of a block's keys, in every thread of warp 0
 // after the call (order-independent reductions)
-__device__ __forceinline__ void range_block(double& lo, double& hi, int& bad) {
-  __shared__ double sh[3][kBlock / 32];
+__device__ __forceinline__ void range_block(unsigned long long& lo, unsigned long long& hi, int& bad) {
+  __shared__ unsigned long long sh[2][kBlock / 32];
+  __shared__ int shb[kBlock / 32];
+  auto reduce = [&]() {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-  }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
+      lo = a < lo ? a : lo;
+      hi = b > hi ? b : hi;
+    }
+    bad = __any_sync(0xffffffffu, bad);
+  };
+  reduce();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) {
     sh[0][w] = lo;
     sh[1][w] = hi;
-    sh[2][w] = bad;
+    shb[w] = bad;
   }
   __syncthreads();
   if (w == 0) {
-    lo = lane < kBlock / 32 ? sh[0][lane] : INFINITY;
-    hi = lane < kBlock / 32 ? sh[1][lane] : -INFINITY;
-    bad = lane < kBlock / 32 ? (sh[2][lane] != 0.0) : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-      bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-    }
+    lo = lane < kBlock / 32 ? sh[0][lane] : ~0ull;
+    hi = lane < kBlock / 32 ? sh[1][lane] : 0ull;
+    bad = lane < kBlock / 32 ? shb[lane] : 0;
+    reduce();
   }
   __syncthreads();  // sh is reused by the caller's next call
 }
@@ -129,65 +140,90 @@ __device__ __forceinline__ void range_block(double& lo, double& hi, int& bad) {
 // the field's range by blocks (min, max, any non-finite value), four
 // independent loads in flight per thread, reduced by the last block to
 // finish: range[3 kRangeGrid ..] = {u_min, K} with s_u 2^30 = 2^K, lsc =
-// {cs, cu}; a NaN
-// or infinite value makes cu NaN, so every difference of the pass is NaN
-// (as FP64 gives NaN sizes for such a field)
+// {cs, cu}; a NaN or infinite value makes cu NaN, so every difference of the
+// pass is NaN (as FP64 gives NaN sizes for such a field).  The comparisons
+// are integer ones: minima and maxima of doubles take the FP64 pipe (with
+// the record kernel 37 us at the 0.9M vertices of a 96^3 box, 26 here).  Two
+// blocks per SM: 1216 cost the last block 7 us more in partials, and other
+// streams' passes find free SMs.  Also clears the pass's counters.
 __global__ void __launch_bounds__(kBlock) k_lrange(int V, const double* __restrict__ u, float cs,
                                                    double* __restrict__ range, unsigned* __restrict__ done,
-                                                   float* __restrict__ lsc) {
-  double lo = INFINITY, hi = -INFINITY;
+                                                   float* __restrict__ lsc, LearnCounters lc) {
+  if (blockIdx.x == 0 && threadIdx.x < LearnCounters::kCount) *lc.p[threadIdx.x] = 0;
+  unsigned long long lo = ~0ull, hi = 0ull;
   int bad = 0;
-  const int stride = gridDim.x * blockDim.x;
-  for (int v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < V; v0 += 4 * stride) {
+  const long stride = (long)gridDim.x * blockDim.x;
+  for (long v0 = blockIdx.x * (long)blockDim.x + threadIdx.x; v0 < V; v0 += 4 * stride) {
     double x[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = v0 + i * stride < V ? __ldg(u + v0 + i * stride) : 0.0;
+    for (int i = 0; i < 4; ++i) x[i] = __ldg(u + min(v0 + i * stride, (long)V - 1));  // past the end: the last one again
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (v0 + i * stride >= V) continue;
-      if (isfinite(x[i])) {
-        lo = fmin(lo, x[i]);
-        hi = fmax(hi, x[i]);
+      if (((__double2hiint(x[i]) >> 20) & 0x7ff) != 0x7ff) {
+        const unsigned long long k = range_key(x[i]);
+        lo = k < lo ? k : lo;
+        hi = k > hi ? k : hi;
       } else {
         bad = 1;
       }
     }
   }
   range_block(lo, hi, bad);
+  unsigned long long* part = reinterpret_cast<unsigned long long*>(range);
   __shared__ bool last;
   if (threadIdx.x == 0) {
-    range[3 * blockIdx.x] = lo;
-    range[3 * blockIdx.x + 1] = hi;
-    range[3 * blockIdx.x + 2] = bad;
+    part[3 * blockIdx.x] = lo;
+    part[3 * blockIdx.x + 1] = hi;
+    part[3 * blockIdx.x + 2] = (unsigned long long)bad;
     __threadfence();
     last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  lo = INFINITY;
-  hi = -INFINITY;
+  lo = ~0ull;
+  hi = 0ull;
   bad = 0;
   for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-    lo = fmin(lo, range[3 * b]);
-    hi = fmax(hi, range[3 * b + 1]);
-    bad |= range[3 * b + 2] != 0.0;
+    const unsigned long long l = __ldcg(part + 3 * b), h = __ldcg(part + 3 * b + 1);
+    lo = l < lo ? l : lo;
+    hi = h > hi ? h : hi;
+    bad |= __ldcg(part + 3 * b + 2) != 0;
   }
   range_block(lo, hi, bad);
   if (threadIdx.x != 0) return;
   int e = 0;  // s_u = 2^-e: 1 for a constant field
-  if (!bad && hi > lo) frexp(hi - lo, &e);  // hi - lo = m 2^e, m in [1/2, 1)
-  range[3 * kRangeGrid] = bad ? 0.0 : lo;
+  const double l = lo <= hi ? range_value(lo) : INFINITY, h = lo <= hi ? range_value(hi) : -INFINITY;
+  if (!bad && h > l) frexp(h - l, &e);  // h - l = m 2^e, m in [1/2, 1)
+  range[3 * kRangeGrid] = bad ? 0.0 : l;
   range[3 * kRangeGrid + 1] = 30 - e;
   lsc[0] = cs;
   lsc[1] = bad ? __int_as_float(0x7fc00000) : (float)ldexp(1.0, e - 30);
   *done = 0;
 }
 
-__global__ void __launch_bounds__(kBlock) k_lprep(int V, const double* __restrict__ u, const int4* __restrict__ xyzq,
-                                                  const double* __restrict__ range, float4* __restrict__ vr) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= V) return;
+__device__ __noinline__ void listed_sum64(const DevMesh& m, const double* __restrict__ u, const PatchWeights& pw, int it,
+                                          double* __restrict__ rec64) {
+  double acc[3];
+  if (listed_grad_sum(m, u, pw, it, acc) && (threadIdx.x & 31) == 0)
+    for (int k = 0; k < 3; ++k) rec64[3 * (size_t)pw.v[it] + k] = acc[k];
+}
+
+// the vertex records; the first blocks take the listed patches' FP64 sums, a
+// warp each (on a stream beside the network kernel they had to wait for it:
+// its blocks hold every register)
+__global__ void __launch_bounds__(kBlock) k_lprep(const __grid_constant__ DevMesh m, const double* __restrict__ u,
+                                                  const int4* __restrict__ xyzq, const double* __restrict__ range,
+                                                  float4* __restrict__ vr, int n_list_blocks,
+                                                  const __grid_constant__ PatchWeights pw, double* __restrict__ rec64) {
+  after_previous(u, range);
+  if ((int)blockIdx.x < n_list_blocks) {
+    const int it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    if (it < pw.n) listed_sum64(m, u, pw, it, rec64);
+    return;
+  }
+  const int v = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
+  if (v >= m.V) return;
   const double umin = range[3 * kRangeGrid];
   const int K = (int)range[3 * kRangeGrid + 1];  // s_u 2^30 = 2^K
   const int4 p = __ldg(xyzq + v);
@@ -583,6 +619,7 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
   }
   tc_fence_before();
   __syncthreads();
+  after_previous(vr, lsc);  // the weights and the table are set up while the records are made
   tc_fence_after();
   const uint32_t tbase = *tslot;
   const int ntiles = (V + 127) / 128;
@@ -790,6 +827,7 @@ __global__ void k_lfallback(DevMesh m, LearnMesh lm, const float4* __restrict__ 
                             const float* __restrict__ w,
                             const double* __restrict__ rec64, const int* __restrict__ items,
                             const int* __restrict__ count, int cap, float4* __restrict__ rec16) {
+  after_previous(vr, lsc, rec64, items, count);
   const int n = min(*count, cap);
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
@@ -835,7 +873,10 @@ __global__ void k_lfallback(DevMesh m, LearnMesh lm, const float4* __restrict__ 
 // are the per-mesh element geometry
 __global__ void __launch_bounds__(kBlock) k_lerror(DevMesh m, const float4* __restrict__ rec,
                                                    const float* __restrict__ lsc, const float2* __restrict__ geo,
-                                                   float* __restrict__ q, double* __restrict__ partials) {
+                                                   float* __restrict__ q, double* __restrict__ partials,
+                                                   unsigned* __restrict__ done, double adapt_ratio,
+                                                   double* __restrict__ out3) {
+  after_previous(rec, lsc);
   __shared__ double sh[2][kBlock / 32];
   const float cs = __ldg(lsc), cu = __ldg(lsc + 1);
   float self = 0.f, gsum = 0.f;
@@ -897,10 +938,22 @@ __global__ void __launch_bounds__(kBlock) k_lerror(DevMesh m, const float4* __re
     partials[2 * blockIdx.x] = a;
     partials[2 * blockIdx.x + 1] = b;
   }
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's partials before its count
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double shr[kBlock / 32];
+  rd_size_factor(partials, gridDim.x, 0, adapt_ratio, 0.0, m.dim, out3, shr);
+  if (threadIdx.x == 0) *done = 0;
 }
 
 __global__ void __launch_bounds__(kBlock) k_laverage(DevMesh m, const float* __restrict__ q,
                                                      const double* __restrict__ out3, float* __restrict__ size) {
+  after_previous(q, out3);
   // two lanes per vertex (as the FP32 path's average: 4 lanes were slower)
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const int v = gid >> 1, gl = gid & 1;
@@ -926,6 +979,7 @@ __global__ void __launch_bounds__(kBlock) k_laverage(DevMesh m, const float* __r
 __global__ void __launch_bounds__(kBlock) k_lmeasure(DevMesh m, const float* __restrict__ half_len,
                                                      const float* __restrict__ size, uint32_t* __restrict__ split,
                                                      uint32_t* __restrict__ collapse) {
+  after_previous(size);
   const int lane = threadIdx.x & 31;
   const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   // four edges per thread (e, e + 32, e + 64, e + 96 within the warp's
@@ -1266,11 +1320,17 @@ void learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned c
 
 size_t learned_range_bytes() { return sizeof(double) * (3 * kRangeGrid + 2); }
 
-void learned_prep(const DevMesh& m, const double* u, float cs, double* range, unsigned* done, float* lsc,
-                  float4* vr16, cudaStream_t s) {
+void learned_range(const DevMesh& m, const double* u, float cs, double* range, unsigned* done, float* lsc,
+                   const LearnCounters& lc, cudaStream_t s) {
+  if (m.V) k_lrange<<<std::min(nblk(m.V), kRangeGrid), kBlock, 0, s>>>(m.V, u, cs, range, done, lsc, lc);
+}
+
+void learned_prep(const DevMesh& m, const double* u, const double* range, float4* vr16, const PatchWeights& pw,
+                  double* rec64, cudaStream_t s) {
   if (!m.V) return;
-  k_lrange<<<std::min(nblk(m.V), kRangeGrid), kBlock, 0, s>>>(m.V, u, cs, range, done, lsc);
-  k_lprep<<<nblk(m.V), kBlock, 0, s>>>(m.V, u, reinterpret_cast<const int4*>(m.xyzq), range, vr16);
+  const int nl = (pw.n + kBlock / 32 - 1) / (kBlock / 32);
+  launch_after(m.early, k_lprep, nl + nblk(m.V), kBlock, s, m, u, reinterpret_cast<const int4*>(m.xyzq), range, vr16, nl,
+               pw, rec64);
 }
 
 void learned_features(const DevMesh& m, const LearnMesh& lm, const float4* vr16, const float* lsc, uint16_t* x,
@@ -1289,19 +1349,19 @@ void learned_infer(const DevMesh& m, const LearnMesh& lm, const float4* vr16, co
   const int ntiles = (m.V + 127) / 128;
   if (max_degree <= kMlpSlots / 2) {
     const int grid = std::min(infer_grid<64>(), ntiles);
-    k_mlp_infer<64><<<grid, kInferThreads, InferSmem<64>::kTotal, s>>>(
-        m.V, lm, vr16, lsc, static_cast<const uint4*>(packed), rec16, fb_items, fb_count, z_max, use_mlp, stall_polls, err);
+    launch_after_smem(
+        m.early, k_mlp_infer<64>, grid, kInferThreads, InferSmem<64>::kTotal, s, m.V, lm, vr16, lsc, static_cast<const uint4*>(packed), rec16, fb_items, fb_count, z_max, use_mlp, stall_polls, err);
   } else {
     const int grid = std::min(infer_grid<128>(), ntiles);
-    k_mlp_infer<128><<<grid, kInferThreads, InferSmem<128>::kTotal, s>>>(
-        m.V, lm, vr16, lsc, static_cast<const uint4*>(packed), rec16, fb_items, fb_count, z_max, use_mlp, stall_polls, err);
+    launch_after_smem(
+        m.early, k_mlp_infer<128>, grid, kInferThreads, InferSmem<128>::kTotal, s, m.V, lm, vr16, lsc, static_cast<const uint4*>(packed), rec16, fb_items, fb_count, z_max, use_mlp, stall_polls, err);
   }
 }
 
 void learned_fallback(const DevMesh& m, const LearnMesh& lm, const float4* vr16, const float* lsc, const float* w,
                       const double* rec64, const int* fb_items, const int* fb_count, int fb_cap, float4* rec16,
                       cudaStream_t s) {
-  k_lfallback<<<152 * 4, 256, 0, s>>>(m, lm, vr16, lsc, w, rec64, fb_items, fb_count, fb_cap, rec16);
+  launch_after(m.early, k_lfallback, 152 * 4, 256, s, m, lm, vr16, lsc, w, rec64, fb_items, fb_count, fb_cap, rec16);
 }
 
 int learned_error_blocks(int T) {
@@ -1310,17 +1370,18 @@ int learned_error_blocks(int T) {
 }
 
 void learned_error(const DevMesh& m, const float4* rec, const float* lsc, const float2* geo, float* q, double* partials,
-                   int nb, cudaStream_t s) {
-  if (nb) k_lerror<<<nb, kBlock, 0, s>>>(m, rec, lsc, geo, q, partials);
+                   int nb, unsigned* done, double adapt_ratio, double* out3, cudaStream_t s) {
+  if (nb)
+    launch_after(m.early, k_lerror, nb, kBlock, s, m, rec, lsc, geo, q, partials, done, adapt_ratio, out3);
 }
 
 void learned_average(const DevMesh& m, const float* q, const double* out3, float* size, cudaStream_t s) {
-  if (m.V) k_laverage<<<nblk(2L * m.V), kBlock, 0, s>>>(m, q, out3, size);
+  if (m.V) launch_after(m.early, k_laverage, nblk(2L * m.V), kBlock, s, m, q, out3, size);
 }
 
 void learned_measure(const DevMesh& m, const float* half_len, const float* size, uint32_t* split, uint32_t* collapse,
                      cudaStream_t s) {
-  if (m.E) k_lmeasure<<<nblk((m.E + 3) / 4), kBlock, 0, s>>>(m, half_len, size, split, collapse);
+  if (m.E) launch_after(m.early, k_lmeasure, nblk((m.E + 3) / 4), kBlock, s, m, half_len, size, split, collapse);
 }
 
 void learned_size_to_f64(int V, const float* s32, double* s64, cudaStream_t s) {

@@ -38,13 +38,22 @@ struct LearnMesh {
 // the per-tile degree flags (ceil(V / 128) bytes) and the largest degree
 void learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned char* tile_half, int* max_deg,
                        cudaStream_t s);
-// fixed-point vertex records {X, Y, Z, U} (16 bytes): the coordinates from
-// m.xyzq, the field on the pass's range.  range: learned_range_bytes() of
+// device words the pass's first kernel clears for the kernels after it
+struct LearnCounters {
+  static constexpr int kCount = 4;
+  int* p[kCount];
+};
+// the field's range and the difference scales.  range: learned_range_bytes() of
 // scratch, done: one device counter (zero before the first call, left zero),
 // lsc: the two difference scales {cs, cu} (cs = 2^-30 / the frame's s)
 size_t learned_range_bytes();
-void learned_prep(const DevMesh& m, const double* u, float cs, double* range, unsigned* done, float* lsc,
-                  float4* vr16, cudaStream_t s);
+void learned_range(const DevMesh& m, const double* u, float cs, double* range, unsigned* done, float* lsc,
+                   const LearnCounters& lc, cudaStream_t s);
+// fixed-point vertex records {X, Y, Z, U} (16 bytes): the coordinates from
+// m.xyzq, the field on the pass's range; also the listed patches' FP64 sums into
+// rec64 (V x 3)
+void learned_prep(const DevMesh& m, const double* u, const double* range, float4* vr16, const PatchWeights& pw,
+                  double* rec64, cudaStream_t s);
 // features for training: x [V][128] BF16 (row-major), aux [V][5]
 void learned_features(const DevMesh& m, const LearnMesh& lm, const float4* vr16, const float* lsc, uint16_t* x,
                       float* aux, cudaStream_t s);
@@ -68,9 +77,10 @@ void learned_fallback(const DevMesh& m, const LearnMesh& lm, const float4* vr16,
 int learned_error_blocks(int T);
 // rec: one 32-byte record per vertex {X, Y, Z, U}, {eps*, 0} (written by the
 // network and fallback kernels); w dV and h_max from the per-mesh element
-// geometry (geo)
+// geometry (geo); the last block also computes the size factor into out3
+// (done: one unsigned, zero between passes)
 void learned_error(const DevMesh& m, const float4* rec, const float* lsc, const float2* geo, float* q, double* partials,
-                   int nb, cudaStream_t s);
+                   int nb, unsigned* done, double adapt_ratio, double* out3, cudaStream_t s);
 void learned_average(const DevMesh& m, const float* q, const double* out3, float* size, cudaStream_t s);
 void learned_measure(const DevMesh& m, const float* half_len, const float* size, uint32_t* split, uint32_t* collapse,
                      cudaStream_t s);

@@ -39,13 +39,12 @@ __device__ __forceinline__ void rd_size_factor(const double* partials, int nb, i
   const double snorm = rd_block_sum(a, sh);
   const double gsum = rd_block_sum(g, sh);
   if (threadIdx.x == 0) {
-    const double p = 1;
     double sf;
     if (mode == 0) {
       const double esn = sqrt(snorm);
       const double aa = adapt_ratio * adapt_ratio * esn * esn;
       const double b = aa / gsum;
-      sf = pow(b, 1.0 / (2.0 * p));
+      sf = sqrt(b);  // pow(b, 1 / (2 p)), p = 1
     } else {
       sf = pow((gsum / target), (1.0 / dim));
     }
