@@ -1820,10 +1820,6 @@ static int pass_fast(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_
     else
       CK(cudaEventRecord(c->size_ready, c->stream));
   }
-  PB("measure_f32");
-  fast_measure(m, P<float>(c->elen), P<float2>(c->sz2), d_split, d_collapse, P<int>(c->guard), P<int>(c->fcnt) + 1,
-               sprg_ctx::kGuardCap, sprg_ctx::kGuardRel, c->stream);
-  PE();
   if (!c->gstamp_ready) {  // V stamps (zero) and the stamp-id counter, which starts at 0x01010101 (any id above 0)
     ENSURE(c->gstamp, sizeof(int) * ((size_t)m.V + 1));
     CK(cudaMemsetAsync(c->gstamp.p, 0, sizeof(int) * (size_t)m.V, c->stream));
@@ -1833,7 +1829,11 @@ static int pass_fast(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_
   GuardScratch gs{P<int>(c->gstamp), P<int>(c->gstamp) + m.V, P<int>(c->gfit) + 1,   P<int>(c->gfit),
                   m.V,               P<double>(c->grec), P<double>(c->w64),           P<unsigned char>(c->listed),
                   P<double>(c->rec), P<double2>(c->geo64)};
-  static const char* const kGuardNames[kGuardStages] = {"guard_collect", "guard_fit", "guard_decide"};
+  PB("measure_f32");
+  fast_measure(m, P<float>(c->elen), P<float2>(c->sz2), d_split, d_collapse, P<int>(c->guard), P<int>(c->fcnt) + 1,
+               sprg_ctx::kGuardCap, sprg_ctx::kGuardRel, gs, P<int>(c->fcnt) + 4, c->stream);
+  PE();
+  static const char* const kGuardNames[kGuardStages] = {"guard_fit", "guard_decide"};
   for (int stage = 0; stage < kGuardStages; ++stage) {
     PB(kGuardNames[stage]);
     launch_guard_stage(stage, m, d_u, P<double>(c->out3), P<int>(c->guard), P<int>(c->fcnt) + 1,

@@ -214,48 +214,6 @@ __global__ void __launch_bounds__(kBlock) k_grad_ip(DevMesh m, const double* __r
 // Element errors (SelfProduct / ElementError, spr/sprEstimateError.cc:98-170)
 // and the powers of them the size field takes.
 // ---------------------------------------------------------------------
-// err to the exponents the size field needs in D dimensions (p = 1):
-//   q = (sqrt err)^(-2 / (2 + D))  = err^(-1/(D+2))
-//   g = (sqrt err)^(2 D / (2 + D)) = err q^2
-// Reduced to err = 2^(P k) m with m in [1, 2^P), P = D + 2: the hardware
-// log2 / exp2 give m^(-1/P) to 2^-21, one step of the cubically convergent
-// Householder iteration on 1 - m r^P squares that twice over, 2^-k goes into
-// the exponent.  9 FP64 operations, within 2 ulps; pow(sqrt(err)) took about
-// 110 for each of the two.  Zero, subnormal, negative and not finite errors
-// take the sequence itself.
-template <int D>
-__device__ __noinline__ void error_powers_ref(double err, double* q, double* g) {
-  const double t = sqrt(err), p = 1, d = D;
-  *q = pow(t, -(2 / (2 * p + d)));
-  *g = pow(t, (2 * d) / (2 * p + d));
-}
-
-template <int D>
-__device__ __forceinline__ void error_powers(double err, double& q, double& g) {
-  constexpr int P = D + 2;
-  const int hi = __double2hiint(err), lo = __double2loint(err);
-  if (hi < 0x00100000 || hi >= 0x7ff00000) {
-    error_powers_ref<D>(err, &q, &g);
-    return;
-  }
-  const int e = (hi >> 20) - 1023;
-  const int k = (e + 300 * P) / P - 300;  // floor(e / P)
-  const int r = e - P * k, mant = hi & 0xfffff;
-  const double m = __hiloint2double(mant | ((r + 1023) << 20), lo);
-  float l, sf = __int_as_float((mant << 3) | (int)((unsigned)lo >> 29) | ((r + 127) << 23));
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(sf));
-  l *= -1.0f / P;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(sf) : "f"(l));
-  const int b = __float_as_int(sf);
-  const double r0 = __hiloint2double((b >> 3) + (896 << 20), b << 29);
-  const double r2 = r0 * r0, r4 = r2 * r2;
-  const double h = fma(-m, P == 5 ? r4 * r0 : r4, 1.0);
-  const double c = P == 5 ? fma(h, 3.0 / 25.0, 0.2) : fma(h, 5.0 / 32.0, 0.25);
-  const double y = fma(r0 * h, c, r0);
-  q = __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y));
-  g = err * (q * q);
-}
-
 // Per element: err = |eps - eps*(IP)|^2 w dV, and in
 // esize h err^(-1/(D+2)) (mode 0; the size factor follows in k_esize) or the
 // power alone (mode 1).  The two integrals are summed per thread over a fixed
@@ -270,7 +228,7 @@ __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __res
                                                   double* __restrict__ partials, unsigned* __restrict__ done, int mode,
                                                   double adapt_ratio, double target, double* __restrict__ out3) {
   after_previous(geo, ip, rec);
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * (kBlock / 32)];
   double self_sum = 0, g_sum = 0;
   double N[4];
   ref::ip_shape_values(D, N);
@@ -317,8 +275,8 @@ __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __res
     esize[e] = mode == 0 ? h * q : q;
   }
   if (D == 3) self_sum *= 0.0625;
-  const double s1 = rd_block_sum(self_sum, sh);
-  const double s2 = rd_block_sum(g_sum, sh);
+  double s1 = self_sum, s2 = g_sum;
+  rd_block_sum2(s1, s2, sh);
   if (threadIdx.x == 0) {
     partials[2 * blockIdx.x] = s1;
     partials[2 * blockIdx.x + 1] = s2;

@@ -91,7 +91,8 @@ void fast_error(const DevMesh& m, const uint4* td, const float2* geo, const floa
 // sz2: (size, its relative error bound) per vertex
 void fast_average(const DevMesh& m, const float2* q, const double* out3, float2* sz2, BatchView bv, cudaStream_t s);
 void fast_measure(const DevMesh& m, const float* half_len, const float2* sz2, uint32_t* split, uint32_t* collapse,
-                  int* guard_items, int* guard_count, int guard_cap, float guard_rel, cudaStream_t s);
+                  int* guard_items, int* guard_count, int guard_cap, float guard_rel, const GuardScratch& gs,
+                  int* unresolved, cudaStream_t s);
 void fast_size_to_f64(int V, const float2* sz2, double* s64, cudaStream_t s);
 
 }  // namespace sprg

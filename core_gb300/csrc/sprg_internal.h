@@ -294,7 +294,7 @@ struct GuardScratch {
   int* stamp;      // V ints, persistent (de-duplication stamps)
   int* stamp_id;   // device counter: this pass's stamp id (starts at 1; the decide stage bumps it)
   int* fit_items;  // fit_cap ints
-  int* fit_count;  // zero before the first stage
+  int* fit_count;  // zero before the measure kernel
   int fit_cap;
   double* rec64;   // V x 3 doubles (FP64 recovered values of collected vertices)
   const double* w64;            // FP64 SPR weights in patch-CSR order
@@ -302,9 +302,10 @@ struct GuardScratch {
   const double* rec_ref;        // their FP64 reference results (V x 3)
   const double2* geo64;         // per element {det J, h_max} in FP64
 };
-// unresolved[0]: edges left to the FP32 decision.  Three stages in order:
-// 0 collect vertices, 1 fits, 2 decide.
-constexpr int kGuardStages = 3;
+// unresolved[0]: edges left to the FP32 decision.  After the measure kernel,
+// which collects the vertices, two stages in order: 0 fits, 1 decide.
+constexpr int kGuardMaxTets = 96;  // elements around one end vertex
+constexpr int kGuardStages = 2;
 void launch_guard_stage(int stage, const DevMesh& m, const double* u, const double* out3, const int* items,
                         const int* count, int cap, uint32_t* split, uint32_t* collapse, int* unresolved,
                         GuardScratch g, BatchView bv, cudaStream_t s);

@@ -1075,31 +1075,36 @@ __global__ void __launch_bounds__(kBlock) k_fast_error(DevMesh m, const uint4* _
   __syncthreads();
   if (!last) return;
   __threadfence();  // every block's partials are visible to the last one
-  __shared__ double shr[kBlock / 32];
+  __shared__ double shr[2 * (kBlock / 32)];
   __shared__ int umax;
+  __shared__ double worst;
   if (threadIdx.x == 0) umax = 0;
   __syncthreads();
   int um = 0;
   for (int i = threadIdx.x; i < n_umax; i += kBlock) um = max(um, __ldg(umax_part + i));
   um = __reduce_max_sync(0xffffffffu, um);
   if ((threadIdx.x & 31) == 0) atomicMax(&umax, um);
-  rd_size_factor(partials, gridDim.x, 0, adapt_ratio, 0.0, dim, out3, shr);
+  rd_size_factor(partials, gridDim.x, 0, adapt_ratio, 0.0, dim, out3, shr);  // (its barrier follows the atomics)
+  // The reference forms an IP gradient as sum u_i grad N_i in FP64, whose
+  // rounding is about 2^-50 max|u| |J^-1|_F; 256 times that would give an
+  // element error (2^-42 max|u| |J^-1|_F)^2 |det J| / 6 = 2^-84 / 6 max|u|^2
+  // |cof|_F^2 / |det J|.  Over T elements the reference's rounding could
+  // move its error integral G by up to T times the largest share
+  // err^(3/5); at 1e-7 of G (the size factor's stated error), or for a G
+  // that is zero or not finite, the pass is rounding-dominated (a constant
+  // field, one offset far above its variation): 1 here, else 0.  (max|u|
+  // from the prep kernel, the largest |cof|^2 / |det| once per mesh.  Another
+  // warp takes this power while thread 0 takes the factor's roots: the next
+  // kernel waits for both.)
+  if (threadIdx.x == 32) {
+    const double uf = (double)__int_as_float(umax);
+    const double en = 0x1p-84 / 6.0 * uf * uf * __longlong_as_double((long long)*qmax);
+    worst = (double)m.T * pow(en, 0.6);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     *done = 0;
-    // The reference forms an IP gradient as sum u_i grad N_i in FP64, whose
-    // rounding is about 2^-50 max|u| |J^-1|_F; 256 times that would give an
-    // element error (2^-42 max|u| |J^-1|_F)^2 |det J| / 6 = 2^-84 / 6 max|u|^2
-    // |cof|_F^2 / |det J|.  Over T elements the reference's rounding could
-    // move its error integral G by up to T times the largest share
-    // err^(3/5); at 1e-7 of G (the size factor's stated error), or for a G
-    // that is zero or not finite, the pass is rounding-dominated (a constant
-    // field, one offset far above its variation): 1 here, else 0.  (max|u|
-    // from the prep kernel, the largest |cof|^2 / |det| once per mesh.)
     const double G = out3[1];
-    const double uf = (double)__int_as_float(umax);
-    const double en = 0x1p-84 / 6.0 * uf * uf * __longlong_as_double((long long)*qmax);
-    const double worst = (double)m.T * pow(en, 0.6);
     *n_round = (!(worst <= 1e-7 * G) || !(G > 0.0)) ? 1 : 0;
   }
 }
@@ -1180,13 +1185,60 @@ __global__ void __launch_bounds__(kBlock) k_fast_average(DevMesh m, const float2
 // ---------------------------------------------------------------------------
 // measure: metric length with 2-point Gauss, h linearly interpolated
 // ---------------------------------------------------------------------------
+// a slot for every winning lane of the warp from one atomic on the shared
+// counter (all 32 lanes call it)
+__device__ __forceinline__ int warp_slot(bool win, int* counter) {
+  const unsigned mask = __ballot_sync(0xffffffffu, win);
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (mask) {
+    const int leader = __ffs(mask) - 1;
+    if (lane == leader) base = atomicAdd(counter, __popc(mask));
+    base = __shfl_sync(0xffffffffu, base, leader);
+  }
+  return base + __popc(mask & ((1u << lane) - 1));
+}
+
+// the guard's vertices at one end of a listed edge, by a warp: the distinct
+// vertices of the elements around it (lanes over the elements; a per-vertex
+// stamp de-duplicates across edges).  A kernel of its own for this waited on
+// the measure kernel and on three dependent loads of its own: 4 of a small
+// pass's 37 us, 12 of 160^3's.
+__device__ __forceinline__ void guard_collect(const DevMesh& m, int v, const GuardScratch& g, int* unresolved) {
+  const int stamp_id = *g.stamp_id, lane = threadIdx.x & 31;
+  const int b = m.a_off[v], cnt = min(m.a_off[v + 1] - b, kGuardMaxTets);
+  for (int r = 0; r < cnt; r += 32) {
+    const int j = r + lane;
+    const bool valid = j < cnt;
+    const int4 ev = valid ? __ldg(reinterpret_cast<const int4*>(m.ev) + m.a_el[b + j]) : make_int4(0, 0, 0, 0);
+    const int ws[4] = {ev.x, ev.y, ev.z, ev.w};
+    bool win[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) win[a] = valid && atomicExch(&g.stamp[ws[a]], stamp_id) != stamp_id;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int slot = warp_slot(win[a], g.fit_count);
+      if (win[a]) {
+        if (slot < g.fit_cap) g.fit_items[slot] = ws[a];
+        else atomicAdd(unresolved, 1);
+      }
+    }
+  }
+}
+
 // four edges per thread (e, e + 32, e + 64, e + 96 within the warp's 128-edge chunk), all
 // loads issued before use; the edge's half length is per-mesh data
-__global__ void __launch_bounds__(kBlock) k_fast_measure(DevMesh m, const float* __restrict__ half_len,
+constexpr int kMeasureBlock = 128;
+__global__ void __launch_bounds__(kMeasureBlock) k_fast_measure(const __grid_constant__ DevMesh m,
+                                                         const float* __restrict__ half_len,
                                                          const float2* __restrict__ sz2, uint32_t* __restrict__ split,
                                                          uint32_t* __restrict__ collapse, int* __restrict__ guard_items,
                                                          int* __restrict__ guard_count, int guard_cap,
-                                                         float guard_rel) {
+                                                         float guard_rel, const __grid_constant__ GuardScratch gs,
+                                                         int* __restrict__ unresolved) {
+  __shared__ int n_listed, list[4 * kMeasureBlock];  // the block's edges on the guard's list
+  if (threadIdx.x == 0) n_listed = 0;
+  __syncthreads();
   after_previous(sz2);
   const int lane = threadIdx.x & 31;
   const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
@@ -1247,7 +1299,10 @@ __global__ void __launch_bounds__(kBlock) k_fast_measure(DevMesh m, const float*
       }
       if (near || !(L == L)) {
         int slot = atomicAdd(guard_count, 1);
-        if (slot < guard_cap) guard_items[slot] = e;
+        if (slot < guard_cap) {
+          guard_items[slot] = e;
+          list[atomicAdd(&n_listed, 1)] = e;
+        }
       }
     }
     unsigned bs = __ballot_sync(0xffffffffu, s), bc = __ballot_sync(0xffffffffu, c);
@@ -1256,6 +1311,11 @@ __global__ void __launch_bounds__(kBlock) k_fast_measure(DevMesh m, const float*
       collapse[e >> 5] = bc;
     }
   }
+  // the block's listed edges' vertices, a warp per end
+  __syncthreads();
+  const int nl = 2 * n_listed;
+  for (int i = threadIdx.x >> 5; i < nl; i += kMeasureBlock / 32)
+    guard_collect(m, m.edv[2 * (size_t)list[i >> 1] + (i & 1)], gs, unresolved);
 }
 
 __global__ void k_size_to_f64(int V, const float2* __restrict__ s32, double* __restrict__ s64) {
@@ -1382,10 +1442,11 @@ void fast_average(const DevMesh& m, const float2* q, const double* out3, float2*
 }
 
 void fast_measure(const DevMesh& m, const float* half_len, const float2* sz2, uint32_t* split, uint32_t* collapse,
-                  int* guard_items, int* guard_count, int guard_cap, float guard_rel, cudaStream_t s) {
+                  int* guard_items, int* guard_count, int guard_cap, float guard_rel, const GuardScratch& gs,
+                  int* unresolved, cudaStream_t s) {
   if (m.E)
-    launch_after(m.early, k_fast_measure, nblk((m.E + 3) / 4), kBlock, s, m, half_len, sz2, split, collapse, guard_items,
-                 guard_count, guard_cap, guard_rel);
+    launch_after(m.early, k_fast_measure, nblk((m.E + 3) / 4, kMeasureBlock), kMeasureBlock, s, m, half_len, sz2, split, collapse, guard_items,
+                 guard_count, guard_cap, guard_rel, gs, unresolved);
 }
 
 void fast_size_to_f64(int V, const float2* sz2, double* s64, cudaStream_t s) {

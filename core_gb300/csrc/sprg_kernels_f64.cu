@@ -767,28 +767,27 @@ __device__ __forceinline__ double block_sum(double x, double* sh) {
 __global__ void __launch_bounds__(kBlock) k_size_factor(const double* __restrict__ partials, int nb, int mode,
                                                         double adapt_ratio, double target, int dim,
                                                         double* out3) {
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * (kBlock / 32)];
   rd_size_factor(partials, nb, mode, adapt_ratio, target, dim, out3, sh);
 }
 
 // one block per mesh of a batch: its segments' partials in a fixed order
 __global__ void __launch_bounds__(kBlock) k_size_factor_batch(const double* __restrict__ partials, BatchView bv,
                                                               double* __restrict__ out4) {
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * (kBlock / 32)];
   const int k = blockIdx.x;
   double a = 0, g = 0;
   for (int i = bv.segoff[k] + threadIdx.x; i < bv.segoff[k + 1]; i += blockDim.x) {
     a += partials[2 * i];
     g += partials[2 * i + 1];
   }
-  double snorm = block_sum(a, sh);
-  double gsum = block_sum(g, sh);
+  rd_block_sum2(a, g, sh);
   if (threadIdx.x == 0) {
     const double r = bv.ratios[k];
-    const double esn = sqrt(snorm);
-    out4[4 * k] = snorm;
-    out4[4 * k + 1] = gsum;
-    out4[4 * k + 2] = pow(r * r * esn * esn / gsum, 0.5);
+    const double esn = sqrt(a);
+    out4[4 * k] = a;
+    out4[4 * k + 1] = g;
+    out4[4 * k + 2] = sqrt(r * r * esn * esn / g);  // pow(b, 1 / (2 p)), p = 1
     out4[4 * k + 3] = 0;
   }
 }
@@ -967,8 +966,6 @@ __global__ void __launch_bounds__(kBlock) k_apply_marks(int E, const uint32_t* _
 // elements, element errors and sizes, the vertex averages) and re-decide the
 // edge's split/collapse bits.
 // ---------------------------------------------------------------------
-constexpr int kGuardMaxTets = 96;  // elements around one end vertex
-
 // FP64 gradient of the scalar field on tet t (cofactor inverse; FP64
 // accuracy, not the reference's rounding).  Every guard kernel that needs an
 // element's gradient evaluates it with this function, so all of them see the
@@ -991,10 +988,9 @@ __device__ __forceinline__ void tet_grad_f64(const DevMesh& m, int t, const doub
   for (int k = 0; k < 3; ++k) g[k] = fma(c1.v[k], d1, fma(c2.v[k], d2, c3.v[k] * d3)) * inv;
 }
 
-// Guard pipeline, three kernels over all listed edges at once:
-//   collect  thread per (edge, end, element around the end): the distinct
-//            vertices of those elements (a per-vertex stamp de-duplicates
-//            across edges)
+// Guard pipeline over all listed edges at once; the FP32 measure kernel lists
+// the edges and collects the distinct vertices of the elements around their
+// ends, then two kernels:
 //   fit      warp per collected vertex, lanes over its patch: the FP64
 //            element gradients, weighted with the per-mesh FP64 SPR weights
 //            (fixed reduction tree), the recovered value
@@ -1007,52 +1003,6 @@ __device__ __forceinline__ void tet_grad_f64(const DevMesh& m, int t, const doub
 // listing the distinct elements and one evaluating them took 12 + 14 us and
 // saved 19 us in the fit and decide stages: these small kernels wait on
 // their chains of dependent loads, not on the FP64 rate).
-// a slot for every winning lane of the warp from one atomic on the shared
-// counter (all 32 lanes call it)
-__device__ __forceinline__ int warp_slot(bool win, int* counter) {
-  const unsigned mask = __ballot_sync(0xffffffffu, win);
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (mask) {
-    const int leader = __ffs(mask) - 1;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-  }
-  return base + __popc(mask & ((1u << lane) - 1));
-}
-
-__global__ void k_guard_collect(DevMesh m, const int* __restrict__ items, const int* __restrict__ count, int cap,
-                                const int* __restrict__ stamp_id_ptr, int* __restrict__ stamp,
-                                int* __restrict__ fit_items,
-                                int* __restrict__ fit_count, int fit_cap, int* __restrict__ unresolved) {
-  after_previous(items, count, stamp_id_ptr);
-  // warp per (edge, end): lanes over the end's elements in rounds of 32
-  const int n = min(*count, cap);
-  const int stamp_id = *stamp_id_ptr;
-  const long total = (long)n * 2 * 32;
-  const int lane = threadIdx.x & 31;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int it = (int)(i >> 6);
-    const int s = (int)((i >> 5) & 1);
-    const int v = m.edv[2 * (size_t)items[it] + s];
-    const int b = m.a_off[v], cnt = min(m.a_off[v + 1] - b, kGuardMaxTets);
-    for (int r = 0; r < cnt; r += 32) {
-      const int j = r + lane;
-      const bool valid = j < cnt;
-      const int* ev = valid ? m.ev + 4 * (size_t)m.a_el[b + j] : nullptr;
-      for (int a = 0; a < 4; ++a) {
-        const int w = valid ? ev[a] : 0;
-        const bool win = valid && atomicExch(&stamp[w], stamp_id) != stamp_id;
-        const int slot = warp_slot(win, fit_count);
-        if (win) {
-          if (slot < fit_cap) fit_items[slot] = w;
-          else atomicAdd(unresolved, 1);
-        }
-      }
-    }
-  }
-}
-
 // eps*(w) = sum_t w_wt eps_t with the per-mesh FP64 SPR weights, warp per
 // collected vertex (lanes over the patch, fixed reduction tree); listed
 // patches take their FP64 reference (QR, grown patch) result
@@ -1074,9 +1024,9 @@ __global__ void k_guard_fit(DevMesh m, const double* __restrict__ u, const int* 
       double gt[3];
       tet_grad_f64(m, m.p_el[beg + k], u, gt);
       const double wk = g.w64[beg + k];
-      r0 += wk * gt[0];
-      r1 += wk * gt[1];
-      r2 += wk * gt[2];
+      r0 = fma(wk, gt[0], r0);
+      r1 = fma(wk, gt[1], r1);
+      r2 = fma(wk, gt[2], r2);
     }
     for (int o = 16; o > 0; o >>= 1) {
       r0 += __shfl_xor_sync(0xffffffffu, r0, o);
@@ -1106,7 +1056,7 @@ __global__ void __launch_bounds__(128) k_guard_decide(DevMesh m, const double* _
     const int next = *g.stamp_id + 1;
     *g.stamp_id = next > 0 ? next : 1;
   }
-  __shared__ double esz[2][2 * kGuardMaxTets];
+  __shared__ double esz[2][2 * kGuardMaxTets], size[2][2];
   const int half = threadIdx.x >> 6, j0 = threadIdx.x & 63;
   const int n = min(*count, cap);
   // every thread of the block runs the same number of rounds (the barriers)
@@ -1133,22 +1083,31 @@ __global__ void __launch_bounds__(128) k_guard_decide(DevMesh m, const double* _
           const int* ev = m.ev + 4 * (size_t)t;
           double gt[3];
           tet_grad_f64(m, t, u, gt);
-          double v2[3] = {0, 0, 0};
+          double v4[3] = {0, 0, 0};  // four times the recovered value at the integration point
           for (int k = 0; k < 4; ++k)
-            for (int c = 0; c < 3; ++c) v2[c] += g.rec64[3 * (size_t)ev[k] + c] * 0.25;
+            for (int c = 0; c < 3; ++c) v4[c] += g.rec64[3 * (size_t)ev[k] + c];
           const double2 dh = g.geo64[t];  // det J, h_max
           double dd = 0;
-          for (int c = 0; c < 3; ++c) dd += (gt[c] - v2[c]) * (gt[c] - v2[c]);
-          esz[half][j] = dh.y * pow(dd * (1.0 / 6.0) * dh.x, -0.2) * sf;
+          for (int c = 0; c < 3; ++c) {
+            const double d = fma(-0.25, v4[c], gt[c]);
+            dd = fma(d, d, dd);
+          }
+          double q, g5;
+          error_powers<3>(dd * (1.0 / 6.0) * dh.x, q, g5);
+          esz[half][j] = dh.y * q * sf;
         }
     }
     __syncthreads();
+    // the ends' averages, in adjacency order, by a thread of each warp
+    if (live && !bad && (j0 & 31) == 0) {
+      const int s = j0 >> 5;
+      double x = 0;
+      for (int i = 0; i < cnt[s]; ++i) x += esz[half][(s ? cnt[0] : 0) + i];
+      size[half][s] = x / (double)cnt[s];
+    }
+    __syncthreads();
     if (live && j0 == 0) {
-      double sz[2] = {0, 0};
-      for (int s = 0; s < 2 && !bad; ++s) {
-        for (int i = 0; i < cnt[s]; ++i) sz[s] += esz[half][(s ? cnt[0] : 0) + i];
-        sz[s] /= (double)cnt[s];
-      }
+      const double sz[2] = {size[half][0], size[half][1]};
       if (bad || !(sz[0] == sz[0]) || !(sz[1] == sz[1])) {  // too many elements, or a NaN size
         atomicAdd(unresolved, 1);
       } else {
@@ -2616,17 +2575,16 @@ void launch_apply_marks(int E, const uint32_t* split_bits, const uint32_t* colla
 void launch_guard_stage(int stage, const DevMesh& m, const double* u, const double* out3, const int* items,
                         const int* count, int cap, uint32_t* split, uint32_t* collapse, int* unresolved,
                         GuardScratch g, BatchView bv, cudaStream_t s) {
-  switch (stage) {
-    case 0:
-      launch_after(m.early, k_guard_collect, 152 * 4, 256, s, m, items, count, cap, g.stamp_id, g.stamp, g.fit_items, g.fit_count,
-                   g.fit_cap, unresolved);
-      break;
-    case 1:
-      launch_after(m.early, k_guard_fit, 152 * 8, 256, s, m, u, g.fit_items, g.fit_count, g.fit_cap, g);
-      break;
-    default:
-      launch_after(m.early, k_guard_decide, 152 * 4, 128, s, m, u, out3, g, items, count, cap, split, collapse, unresolved, bv);
-  }
+  // Blocks for a fraction of what the mesh could list (the listed edges are
+  // commonly a few per thousand), up to four and eight per SM: on a small mesh
+  // a full grid of idle blocks waiting for the kernel before took the slots of
+  // other streams' passes.
+  if (stage == 0)
+    launch_after(m.early, k_guard_fit, std::min(152 * 8, nblk(m.V, 32)), 256, s, m, u, g.fit_items, g.fit_count, g.fit_cap,
+                 g);
+  else
+    launch_after(m.early, k_guard_decide, std::min(152 * 4, nblk(m.E, 32)), 128, s, m, u, out3, g, items, count, cap, split,
+                 collapse, unresolved, bv);
 }
 
 void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double hmin, double hmax, double* sizes,

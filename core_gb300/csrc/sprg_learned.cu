@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(kBlock) k_lerror(DevMesh m, const float4* __re
   __syncthreads();
   if (!last) return;
   __threadfence();
-  __shared__ double shr[kBlock / 32];
+  __shared__ double shr[2 * (kBlock / 32)];
   rd_size_factor(partials, gridDim.x, 0, adapt_ratio, 0.0, m.dim, out3, shr);
   if (threadIdx.x == 0) *done = 0;
 }

@@ -1,9 +1,52 @@
-// FP64 metric edge lengths (MetricSizeField::measure, ma/maSize.cc:158-214),
-// shared by the FP64 translation units (-fmad=false).
+// The powers of an element error and FP64 metric edge lengths
+// (MetricSizeField::measure, ma/maSize.cc:158-214), shared by the FP64
+// translation units (-fmad=false).
 #pragma once
 #include "sprg_refmath.cuh"
 
 namespace sprg {
+
+// err to the exponents the size field needs in D dimensions (p = 1):
+//   q = (sqrt err)^(-2 / (2 + D))  = err^(-1/(D+2))
+//   g = (sqrt err)^(2 D / (2 + D)) = err q^2
+// Reduced to err = 2^(P k) m with m in [1, 2^P), P = D + 2: the hardware
+// log2 / exp2 give m^(-1/P) to 2^-21, one step of the cubically convergent
+// Householder iteration on 1 - m r^P squares that twice over, 2^-k goes into
+// the exponent.  9 FP64 operations, within 2 ulps; pow(sqrt(err)) took about
+// 110 for each of the two.  Zero, subnormal, negative and not finite errors
+// take the sequence itself.
+template <int D>
+static __device__ __noinline__ void error_powers_ref(double err, double* q, double* g) {
+  const double t = sqrt(err), p = 1, d = D;
+  *q = pow(t, -(2 / (2 * p + d)));
+  *g = pow(t, (2 * d) / (2 * p + d));
+}
+
+template <int D>
+__device__ __forceinline__ void error_powers(double err, double& q, double& g) {
+  constexpr int P = D + 2;
+  const int hi = __double2hiint(err), lo = __double2loint(err);
+  if (hi < 0x00100000 || hi >= 0x7ff00000) {
+    error_powers_ref<D>(err, &q, &g);
+    return;
+  }
+  const int e = (hi >> 20) - 1023;
+  const int k = (e + 300 * P) / P - 300;  // floor(e / P)
+  const int r = e - P * k, mant = hi & 0xfffff;
+  const double m = __hiloint2double(mant | ((r + 1023) << 20), lo);
+  float l, sf = __int_as_float((mant << 3) | (int)((unsigned)lo >> 29) | ((r + 127) << 23));
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(sf));
+  l *= -1.0f / P;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(sf) : "f"(l));
+  const int b = __float_as_int(sf);
+  const double r0 = __hiloint2double((b >> 3) + (896 << 20), b << 29);
+  const double r2 = r0 * r0, r4 = r2 * r2;
+  const double h = fma(-m, P == 5 ? r4 * r0 : r4, 1.0);
+  const double c = P == 5 ? fma(h, 3.0 / 25.0, 0.2) : fma(h, 5.0 / 32.0, 0.25);
+  const double y = fma(r0 * h, c, r0);
+  q = __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y));
+  g = err * (q * q);
+}
 
 __device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 

@@ -12,17 +12,24 @@ __device__ __forceinline__ double rd_warp_sum(double x) {
   return x;
 }
 
-// block total, in warp order, valid in thread 0 (every thread calls it)
-__device__ __forceinline__ double rd_block_sum(double x, double* sh) {
+// block totals of x and y, in warp order, valid in thread 0 (every thread
+// calls it; sh holds two values per warp)
+__device__ __forceinline__ void rd_block_sum2(double& x, double& y, double* sh) {
   x = rd_warp_sum(x);
+  y = rd_warp_sum(y);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) {
+    sh[2 * w] = x;
+    sh[2 * w + 1] = y;
+  }
   __syncthreads();
-  if (lane == 0) sh[w] = x;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
-  return t;
+  if (threadIdx.x == 0) {
+    x = y = 0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+      x += sh[2 * i];
+      y += sh[2 * i + 1];
+    }
+  }
 }
 
 // the two integrals from per-block partials (thread i sums blocks i, i +
@@ -36,9 +43,9 @@ __device__ __forceinline__ void rd_size_factor(const double* partials, int nb, i
     a += __ldcg(partials + 2 * i);
     g += __ldcg(partials + 2 * i + 1);
   }
-  const double snorm = rd_block_sum(a, sh);
-  const double gsum = rd_block_sum(g, sh);
+  rd_block_sum2(a, g, sh);
   if (threadIdx.x == 0) {
+    const double snorm = a, gsum = g;
     double sf;
     if (mode == 0) {
       const double esn = sqrt(snorm);

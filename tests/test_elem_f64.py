@@ -427,3 +427,27 @@ def test_resident_passes_back_to_back(gpu_lib, precision, n, graph):
         flags = want[i % 3]
         assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, flags & 1), i
         assert np.array_equal((b[1][e >> 5] >> (e & 31)) & 1, (flags >> 2) & 1), i
+
+
+@pytest.mark.parametrize("n,far", [(2, 3e-7), (7, 3e-7), (7, 1e-3), (24, 3e-7)])
+@pytest.mark.parametrize("threshold", [0.5, 1.5])
+def test_blocks_with_many_guarded_edges(gpu_lib, n, far, threshold):
+    """A quadratic on a regular box gives the interior equal sizes; the ratio puts
+    the commonest length at a relative distance `far` of a threshold, so whole
+    blocks of the FP32 measure kernel list their edges (or none).  The marks are
+    the FP64 form's: the distance is far above FP64 rounding."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m = workload.box(n)
+    u = (m.coords ** 2).sum(axis=1)
+    with cg.Context(m) as c:
+        size = c.estimate_and_mark(u, 0.1)[0]
+        L = c.makeSizeField(size).measure()
+        ratio = 0.1 * np.median(L) / (threshold * (1.0 + far))
+        want = c.estimate_and_mark(u, ratio)[1]
+    with cg.Context(m, precision="fp32") as c:
+        _, flags, _, _, info = c.estimate_and_mark(u, ratio)
+    assert info["n_guard_unresolved"] == 0
+    if n == 24 and far < 1e-6:
+        assert info["n_guard_edges"] > m.n_edges // 20
+    assert np.array_equal(flags, want)
