@@ -500,46 +500,48 @@ constexpr int kSmW3 = kSmW2 + 2 * kMlpHidden * kMlpHidden;
 constexpr int kSmBias = kSmW3 + 2 * 16 * kMlpHidden;  // b1 [64], b2 [64], b3 [16] FP32
 static_assert(kSmBias + 4 * 144 == kMlpPackedBytes, "packed parameter layout");
 
-// Inference shared memory for tiles of at most KMAX inputs: parameters, two
-// feature tiles (double buffer between producer and consumer warps), the
-// hidden tile, two auxiliary records, barriers, the CDF table.
+// Inference shared memory for tiles of at most KMAX inputs: parameters, a
+// feature tile and a hidden tile per consumer group, four auxiliary records,
+// barriers, the CDF table.
 template <int KMAX>
 struct InferSmem {
   static constexpr int kA1 = 27 * 1024;
   static constexpr int kA1Bytes = 2 * 128 * KMAX;
   static constexpr int kA2 = kA1 + 2 * kA1Bytes;
-  static constexpr int kAux = kA2 + 2 * 128 * kMlpHidden;
-  static constexpr int kAuxBytes = 128 * 5 * 4 + 16;  // g_c [128][3], scale [128], flag [128], K flag
-  // mma, full[2], empty[2], (unused), stall (8 B each); tmem slot at +40, abort flag at +56
-  static constexpr int kBar = kAux + 2 * kAuxBytes;
+  static constexpr int kA2Bytes = 2 * 128 * kMlpHidden;
+  static constexpr int kAux = kA2 + 2 * kA2Bytes;
+  static constexpr int kAuxBytes = 128 * 4 * 4 + 128 + 16;  // g_c [128][3], scale [128], flag [128] (bytes), K flag
+  // mma[2], full[2], empty[2], stall (8 B each); tmem slot at +56, abort flag at +60
+  static constexpr int kBar = kAux + 4 * kAuxBytes;
   static constexpr int kGelu = kBar + 64;
   static constexpr int kTotal = kGelu + 8 * kGeluN;
   static_assert(kA1 >= kMlpPackedBytes, "operand tiles after the parameters");
 };
 
-constexpr int kInferThreads = 512;  // warps 0-7 consume, warps 8-15 produce
-constexpr int kConsumers = 256;
-constexpr int kTmemCols = 128;      // D1 / D2 in columns 0..63, D3 in 64..79
+constexpr int kInferThreads = 512;  // warps 0-3 and 4-7 consume, warps 8-15 produce
+constexpr int kConsumers = 128;     // threads of a consumer group
+constexpr int kTmemCols = 256;      // group g: D1 / D2 in columns 128 g + 0..63, D3 in 128 g + 64..79
 
-// hidden layer epilogue by the 8 consumer warps: bias + GELU of a 128 x 64
+// hidden layer epilogue by a group's 4 warps: bias + GELU of a 128 x 64
 // accumulator into the next layer's A operand; warp w reads lanes
-// 32 (w % 4) .. + 31 and columns 32 (w / 4) .. + 31
+// 32 (w % 4) .. + 31
 __device__ __forceinline__ void hidden_epilogue(uint32_t tbase, const float* __restrict__ bias,
                                                 const float2* __restrict__ tab, __nv_bfloat16* __restrict__ A,
                                                 int warp, int lane) {
-  const int lq = warp & 3, ch = warp >> 2;
+  const int lq = warp & 3;
   const int row = 32 * lq + lane;
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int c0 = 32 * ch + 16 * half;
+  for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
     float z[16];
     tmem_ld16(tbase + ((uint32_t)(32 * lq) << 16) + c0, z);
     uint32_t h[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      __nv_bfloat162 p = __floats2bfloat162_rn(gelu_tab(tab, z[2 * i] + bias[c0 + 2 * i]),
-                                               gelu_tab(tab, z[2 * i + 1] + bias[c0 + 2 * i + 1]));
-      h[i] = *reinterpret_cast<uint32_t*>(&p);
+    for (int i = 0; i < 4; ++i) {
+      const float4 b = reinterpret_cast<const float4*>(bias + c0)[i];
+      __nv_bfloat162 p = __floats2bfloat162_rn(gelu_tab(tab, z[4 * i] + b.x), gelu_tab(tab, z[4 * i + 1] + b.y));
+      h[2 * i] = *reinterpret_cast<uint32_t*>(&p);
+      p = __floats2bfloat162_rn(gelu_tab(tab, z[4 * i + 2] + b.z), gelu_tab(tab, z[4 * i + 3] + b.w));
+      h[2 * i + 1] = *reinterpret_cast<uint32_t*>(&p);
     }
     *reinterpret_cast<uint4*>(A + tile_off(row, c0, kMlpHidden)) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(A + tile_off(row, c0 + 8, kMlpHidden)) = make_uint4(h[4], h[5], h[6], h[7]);
@@ -562,30 +564,46 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// named barrier `id` over n threads, AND of v
-__device__ __forceinline__ bool bar_and(int id, int n, bool v) {
+// consumer group g's named barrier (1 + g, over its threads), AND of v; the ids
+// are literals: with an id in a register every barrier of the SM is reserved
+__device__ __forceinline__ bool group_and(int g, bool v) {
   uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, %3, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(id), "r"(n)
-      : "memory");
+  if (g == 0)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "n"(kConsumers)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 2, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "n"(kConsumers)
+        : "memory");
   return r != 0;
 }
 
 constexpr int kWaitLimit = 1 << 22;
 
 // Warp-specialised persistent inference.  Producers (warps 8-15) compute the
-// features of a block's k-th tile into buffer k % 2 and arrive on full[b];
-// consumers (warps 0-7) wait on full[b], issue the three layers (thread 0)
-// and run the epilogues, then arrive on empty[b], which the producers wait on
-// before refilling the buffer.  Every wait is bounded; a wait that runs out
-// sets *err and both groups leave their loops (the consumers raise a shared
-// abort flag the producers' waits watch).  stall_polls > 0 (a test of that
-// path) replaces the first layer-1 completion wait by a wait of that many
-// polls on a barrier nothing completes: it runs out with the layer's MMAs in
-// flight, which are drained before the tensor memory is freed.
+// features of a block's k-th tile into buffer k % 2 and auxiliary record k % 4
+// and arrive on full[k % 2]; consumer group g (warps 4 g .. 4 g + 3) takes the
+// tiles k % 2 = g: it waits on full[g], its first thread issues the three
+// layers, its warps run the epilogues.  The buffer is free once layer 1 has
+// read it (empty[g]), so the next features are written under the rest of the
+// tile; the record is written again two of the group's tiles later.  While one
+// group waits for its matrix products or its barrier, the other's epilogue
+// runs (one group of 8 warps idled at six points a tile: 173 us at the 0.9M
+// vertices of a 96^3 box, 155 here; 85 % of the shared memory's cycles, most of
+// them the CDF table's look-ups at six a warp, bound it).
+// Every wait is bounded; a wait that runs out sets *err and raises a shared
+// abort flag that the others' waits watch, so all leave their loops.
+// stall_polls > 0 (a test of that path) replaces the first layer-1 completion
+// wait by a wait of that many polls on a barrier nothing completes: it runs
+// out with the layer's MMAs in flight, which are drained before the tensor
+// memory is freed.
 template <int KMAX>
 __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
     k_mlp_infer(int V, LearnMesh lm, const float4* __restrict__ vr, const float* __restrict__ lsc,
@@ -595,10 +613,10 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
   extern __shared__ __align__(1024) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* bias = reinterpret_cast<const float*>(sm + kSmBias);
-  __nv_bfloat16* A2 = reinterpret_cast<__nv_bfloat16*>(sm + S::kA2);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + S::kBar);  // [0] mma, [1..2] full, [3..4] empty
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S::kBar + 40);
-  volatile int* abort = reinterpret_cast<volatile int*>(sm + S::kBar + 56);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + S::kBar);
+  uint64_t *const mma = bars, *const full = bars + 2, *const empty = bars + 4, *const stall = bars + 6;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S::kBar + 56);
+  volatile int* abort = reinterpret_cast<volatile int*>(sm + S::kBar + 60);
   float2* gtab = reinterpret_cast<float2*>(sm + S::kGelu);
 
   for (int i = tid; i < kMlpPackedBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(sm)[i] = packed[i];
@@ -609,12 +627,12 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(bars, 1);
     for (int b = 0; b < 2; ++b) {
-      mbar_init(bars + 1 + b, kInferThreads - kConsumers);
-      mbar_init(bars + 3 + b, kConsumers);
+      mbar_init(mma + b, 1);
+      mbar_init(full + b, kInferThreads - 2 * kConsumers);
+      mbar_init(empty + b, 1);
     }
-    mbar_init(bars + 6, 1);
+    mbar_init(stall, 1);
     *abort = 0;
   }
   tc_fence_before();
@@ -627,21 +645,21 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
 
   if (warp >= 8) {
     // ---- producers: 256 threads, four lanes per vertex, two passes of 64
-    const int ptid = tid - kConsumers;
+    const int ptid = tid - 2 * kConsumers;
     const float cs = __ldg(lsc), cu = __ldg(lsc + 1);
     for (int k = 0;; ++k) {
       const int tile = blockIdx.x + k * gridDim.x;
       if (tile >= ntiles) break;
       const int b = k & 1;
-      if (k >= 2 && !mbar_wait_unless(bars + 3 + b, ((k - 2) >> 1) & 1, kWaitLimit, abort)) {
+      if (k >= 2 && !mbar_wait_unless(empty + b, ((k - 2) >> 1) & 1, kWaitLimit, abort)) {
         ok = false;
         break;
       }
       __nv_bfloat16* A1 = reinterpret_cast<__nv_bfloat16*>(sm + S::kA1 + b * S::kA1Bytes);
-      float* gcs = reinterpret_cast<float*>(sm + S::kAux + b * S::kAuxBytes);
+      float* gcs = reinterpret_cast<float*>(sm + S::kAux + (k & 3) * S::kAuxBytes);
       float* scls = gcs + 3 * 128;
-      int* flags = reinterpret_cast<int*>(scls + 128);
-      int* kflag = flags + 128;
+      unsigned char* flags = reinterpret_cast<unsigned char*>(scls + 128);
+      int* kflag = reinterpret_cast<int*>(flags + 128);
       const int half = KMAX == 64 ? 1 : lm.tile_half[tile];
       for (int pass = 0; pass < 2; ++pass) {
         const int r = 64 * pass + (ptid >> 2), q = ptid & 3;
@@ -653,7 +671,7 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
           if (q == 0) {
             gcs[3 * r] = f.gc[0]; gcs[3 * r + 1] = f.gc[1]; gcs[3 * r + 2] = f.gc[2];
             scls[r] = f.scl;
-            flags[r] = f.flag;
+            flags[r] = (unsigned char)f.flag;
           }
         } else if (KMAX == 128) {
           VFeat<8> f = vertex_features<8>(lm, vr, V, tile * 128 + r, q, cs, cu);
@@ -663,90 +681,91 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
           if (q == 0) {
             gcs[3 * r] = f.gc[0]; gcs[3 * r + 1] = f.gc[1]; gcs[3 * r + 2] = f.gc[2];
             scls[r] = f.scl;
-            flags[r] = f.flag;
+            flags[r] = (unsigned char)f.flag;
           }
         }
       }
       if (ptid == 0) *kflag = half;
       fence_async_smem();
-      mbar_arrive(bars + 1 + b);
+      mbar_arrive(full + b);
     }
   } else {
-    // ---- consumers: 256 threads; thread 0 issues the MMAs
-    const uint32_t sA2 = smem_u32(A2), sW1 = smem_u32(sm + kSmW1), sW2 = smem_u32(sm + kSmW2),
-                   sW3 = smem_u32(sm + kSmW3);
+    // ---- consumers: two groups of 128 threads; a group's first issues its MMAs
+    const int g = tid / kConsumers;
+    const bool first = tid == g * kConsumers;
+    const uint32_t td = tbase + 128u * g;
+    __nv_bfloat16* A2 = reinterpret_cast<__nv_bfloat16*>(sm + S::kA2 + g * S::kA2Bytes);
+    const uint32_t sA1 = smem_u32(sm + S::kA1 + g * S::kA1Bytes), sA2 = smem_u32(A2), sW1 = smem_u32(sm + kSmW1),
+                   sW2 = smem_u32(sm + kSmW2), sW3 = smem_u32(sm + kSmW3);
     constexpr uint32_t id64 = idesc_bf16(128, 64), id16 = idesc_bf16(128, 16);
     uint32_t mph = 0;
-    bool mma_pending = false;  // thread 0: MMAs committed whose completion was not yet seen
-    for (int k = 0;; ++k) {
+    bool mma_pending = false;  // first thread: MMAs committed whose completion was not yet seen
+    for (int k = g;; k += 2) {
       const int tile = blockIdx.x + k * gridDim.x;
       if (tile >= ntiles) break;
-      const int b = k & 1;
-      ok = bar_and(1, kConsumers, mbar_wait(bars + 1 + b, (k >> 1) & 1, kWaitLimit));
+      ok = group_and(g, mbar_wait_unless(full + g, (k >> 1) & 1, kWaitLimit, abort));
       if (!ok) break;
-      const float* gcs = reinterpret_cast<const float*>(sm + S::kAux + b * S::kAuxBytes);
+      const float* gcs = reinterpret_cast<const float*>(sm + S::kAux + (k & 3) * S::kAuxBytes);
       const float* scls = gcs + 3 * 128;
-      const int* flags = reinterpret_cast<const int*>(scls + 128);
-      const int half = flags[128];
-      const uint32_t sA1 = smem_u32(sm + S::kA1 + b * S::kA1Bytes);
+      const unsigned char* flags = reinterpret_cast<const unsigned char*>(scls + 128);
       tc_fence_after();
       // layer 1: D[0:64) = A1 W1^T (K = 64 for tiles of <= 16 neighbours)
-      if (tid == 0) {
-        const int nk = half ? 4 : KMAX / 16;
+      if (first) {
+        const int nk = *reinterpret_cast<const int*>(flags + 128) ? 4 : KMAX / 16;
         for (int kk = 0; kk < nk; ++kk)
-          mma_bf16(tbase, sdesc(sA1 + 256 * kk, 128, 16 * KMAX), sdesc(sW1 + 256 * kk, 128, 16 * kMlpIn), id64,
-                   kk > 0);
-        mma_commit(bars);
+          mma_bf16(td, sdesc(sA1 + 256 * kk, 128, 16 * KMAX), sdesc(sW1 + 256 * kk, 128, 16 * kMlpIn), id64, kk > 0);
+        mma_commit(mma + g);
         mma_pending = true;
       }
-      ok = bar_and(1, kConsumers,
-                   tid == 0 ? (stall_polls > 0 && k == 0 ? mbar_wait(bars + 6, 0, stall_polls)
-                                                         : mbar_wait(bars, mph, kWaitLimit))
-                            : true);
+      ok = group_and(g,
+                   first ? (stall_polls > 0 && k == 0 ? mbar_wait(stall, 0, stall_polls)
+                                                      : mbar_wait(mma + g, mph, kWaitLimit))
+                         : true);
       if (!ok) break;
+      if (first) mbar_arrive(empty + g);  // the layer has read the features
       mma_pending = false;
       mph ^= 1;
       tc_fence_after();
-      hidden_epilogue(tbase, bias, gtab, A2, warp, lane);
+      hidden_epilogue(td, bias, gtab, A2, warp, lane);
       fence_async_smem();
       tc_fence_before();
-      bar_and(1, kConsumers, true);
+      group_and(g, true);
       // layer 2: D[0:64) = H1 W2^T
-      if (tid == 0) {
+      if (first) {
         tc_fence_after();
         for (int kk = 0; kk < kMlpHidden / 16; ++kk)
-          mma_bf16(tbase, sdesc(sA2 + 256 * kk, 128, 16 * kMlpHidden), sdesc(sW2 + 256 * kk, 128, 16 * kMlpHidden),
-                   id64, kk > 0);
-        mma_commit(bars);
+          mma_bf16(td, sdesc(sA2 + 256 * kk, 128, 16 * kMlpHidden), sdesc(sW2 + 256 * kk, 128, 16 * kMlpHidden), id64,
+                   kk > 0);
+        mma_commit(mma + g);
         mma_pending = true;
       }
-      ok = bar_and(1, kConsumers, tid == 0 ? mbar_wait(bars, mph, kWaitLimit) : true);
+      ok = group_and(g, first ? mbar_wait(mma + g, mph, kWaitLimit) : true);
       if (!ok) break;
       mma_pending = false;
       mph ^= 1;
       tc_fence_after();
-      hidden_epilogue(tbase, bias + kMlpHidden, gtab, A2, warp, lane);
+      hidden_epilogue(td, bias + kMlpHidden, gtab, A2, warp, lane);
       fence_async_smem();
       tc_fence_before();
-      bar_and(1, kConsumers, true);
+      group_and(g, true);
       // layer 3: D[64:80) = H2 W3^T (rows 3..15 of W3 are zero)
-      if (tid == 0) {
+      if (first) {
         tc_fence_after();
         for (int kk = 0; kk < kMlpHidden / 16; ++kk)
-          mma_bf16(tbase + 64, sdesc(sA2 + 256 * kk, 128, 16 * kMlpHidden),
-                   sdesc(sW3 + 256 * kk, 128, 16 * kMlpHidden), id16, kk > 0);
-        mma_commit(bars);
+          mma_bf16(td + 64, sdesc(sA2 + 256 * kk, 128, 16 * kMlpHidden), sdesc(sW3 + 256 * kk, 128, 16 * kMlpHidden),
+                   id16, kk > 0);
+        mma_commit(mma + g);
         mma_pending = true;
       }
-      ok = bar_and(1, kConsumers, tid == 0 ? mbar_wait(bars, mph, kWaitLimit) : true);
+      ok = group_and(g, first ? mbar_wait(mma + g, mph, kWaitLimit) : true);
       if (!ok) break;
       mma_pending = false;
       mph ^= 1;
       tc_fence_after();
-      if (warp < 4) {
+      {
         float z[16];
-        tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + 64, z);
-        const int r = 32 * warp + lane, v = tile * 128 + r;
+        const int r = 32 * (warp & 3) + lane, v = tile * 128 + r;
+        tmem_ld16(td + ((uint32_t)(32 * (warp & 3)) << 16) + 64, z);
         const float* b3 = bias + 2 * kMlpHidden;
         float z0 = z[0] + b3[0], z1 = z[1] + b3[1], z2 = z[2] + b3[2];
         const bool in = v < V;
@@ -761,15 +780,13 @@ __global__ void __launch_bounds__(kInferThreads, KMAX == 64 ? 2 : 1)
         const int slot = warp_slot(fb, fb_count);
         if (fb && slot < V) fb_items[slot] = v;
       }
-      // buffer b (features and auxiliary record) is free again
-      tc_fence_before();
-      mbar_arrive(bars + 3 + b);
+      tc_fence_before();  // D3's reads before the next tile's products
     }
     // MMAs in flight finish before the memory is freed (a full-length bounded
     // wait, whatever limit the pass's waits had)
-    if (!ok && tid == 0) {
+    if (!ok && first) {
       *abort = 1;
-      if (mma_pending) mbar_wait(bars, mph, kWaitLimit);
+      if (mma_pending) mbar_wait(mma + g, mph, kWaitLimit);
     }
   }
   if (!ok) atomicExch(err, 1);
@@ -869,7 +886,9 @@ __global__ void k_lfallback(DevMesh m, LearnMesh lm, const float4* __restrict__ 
 // ---------------------------------------------------------------------------
 // error, average, measure in plain FP32
 // ---------------------------------------------------------------------------
-// two elements per iteration, all loads issued before use; w dV and h_max
+// one element per iteration (two, 80 registers: three blocks per SM, 74 us at
+// the 5.3M tets of a 96^3 box; 57 here, the 1216 blocks in two full waves; five
+// blocks at 48 registers 69); w dV and h_max
 // are the per-mesh element geometry
 __global__ void __launch_bounds__(kBlock) k_lerror(DevMesh m, const float4* __restrict__ rec,
                                                    const float* __restrict__ lsc, const float2* __restrict__ geo,
@@ -881,41 +900,39 @@ __global__ void __launch_bounds__(kBlock) k_lerror(DevMesh m, const float4* __re
   const float cs = __ldg(lsc), cu = __ldg(lsc + 1);
   float self = 0.f, gsum = 0.f;
   const int stride = gridDim.x * blockDim.x;
-  for (int t0 = blockIdx.x * blockDim.x + threadIdx.x; t0 < m.T; t0 += 2 * stride) {
-    const int ts[2] = {t0, t0 + stride};
-    int4 tv[2];
-    float2 gm[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const bool in = ts[i] < m.T;
-      tv[i] = in ? __ldg(reinterpret_cast<const int4*>(m.ev) + ts[i]) : make_int4(0, 0, 0, 0);
-      gm[i] = in ? __ldg(geo + ts[i]) : make_float2(0.f, 0.f);
-    }
+  // the next element's ids and geometry are loaded one iteration ahead: only
+  // the record gathers stay on the dependent chain
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  int4 ntv = make_int4(0, 0, 0, 0);
+  float2 ngm = make_float2(0.f, 0.f);
+  if (t < m.T) {
+    ntv = __ldg(reinterpret_cast<const int4*>(m.ev) + t);
+    ngm = __ldg(geo + t);
+  }
+  for (; t < m.T; t += stride) {
+    const int vs[4] = {ntv.x, ntv.y, ntv.z, ntv.w};
+    const float2 gm = ngm;
     // one 32-byte record per vertex: {X, Y, Z, U}, {eps*, 0}
-    float4 P[2][4], E[2][4];
+    float4 P[4], E[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int vs[4] = {tv[i].x, tv[i].y, tv[i].z, tv[i].w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ld_record(rec + 2 * (size_t)vs[k], P[i][k], E[i][k]);
+    for (int k = 0; k < 4; ++k) ld_record(rec + 2 * (size_t)vs[k], P[k], E[k]);
+    if (t < m.T - stride) {
+      ntv = __ldg(reinterpret_cast<const int4*>(m.ev) + t + stride);
+      ngm = __ldg(geo + t + stride);
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (ts[i] >= m.T) continue;
-      const float3 g = tet_grad_rec(P[i][0], P[i][1], P[i][2], P[i][3], cs, cu);
-      const float ex = 0.25f * ((E[i][0].x + E[i][1].x) + (E[i][2].x + E[i][3].x));
-      const float ey = 0.25f * ((E[i][0].y + E[i][1].y) + (E[i][2].y + E[i][3].y));
-      const float ez = 0.25f * ((E[i][0].z + E[i][1].z) + (E[i][2].z + E[i][3].z));
-      const float dx = g.x - ex, dy = g.y - ey, dz = g.z - ez;
-      const float wdv = gm[i].x;
-      const float err = (dx * dx + dy * dy + dz * dz) * wdv;
-      self = fmaf(ex * ex + ey * ey + ez * ez, wdv, self);
-      // err^(-1/5) through the hardware log2 / exp2 (the learned form is
-      // stated to 1e-2; these are good to a few 1e-7)
-      const float rr = err > 0.f ? exp2f(-0.2f * __log2f(err)) : __int_as_float(0x7f800000);
-      gsum += err > 0.f ? err * (rr * rr) : 0.f;
-      q[ts[i]] = gm[i].y * rr;
-    }
+    const float3 g = tet_grad_rec(P[0], P[1], P[2], P[3], cs, cu);
+    const float ex = 0.25f * ((E[0].x + E[1].x) + (E[2].x + E[3].x));
+    const float ey = 0.25f * ((E[0].y + E[1].y) + (E[2].y + E[3].y));
+    const float ez = 0.25f * ((E[0].z + E[1].z) + (E[2].z + E[3].z));
+    const float dx = g.x - ex, dy = g.y - ey, dz = g.z - ez;
+    const float wdv = gm.x;
+    const float err = (dx * dx + dy * dy + dz * dz) * wdv;
+    self = fmaf(ex * ex + ey * ey + ez * ez, wdv, self);
+    // err^(-1/5) through the hardware log2 / exp2 (the learned form is
+    // stated to 1e-2; these are good to a few 1e-7)
+    const float rr = err > 0.f ? exp2f(-0.2f * __log2f(err)) : __int_as_float(0x7f800000);
+    gsum += err > 0.f ? err * (rr * rr) : 0.f;
+    q[t] = gm.y * rr;
   }
   double s1 = self, s2 = gsum;
 #pragma unroll

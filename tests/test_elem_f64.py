@@ -451,3 +451,36 @@ def test_blocks_with_many_guarded_edges(gpu_lib, n, far, threshold):
     if n == 24 and far < 1e-6:
         assert info["n_guard_edges"] > m.n_edges // 20
     assert np.array_equal(flags, want)
+
+
+@pytest.mark.parametrize("n,extra", [(2, 0), (33, 0), (34, 0), (43, 0), (55, 0), (67, 0), (7, 2), (27, 2), (41, 2)])
+def test_network_tiles_of_both_consumer_groups(gpu_lib, n, extra):
+    """The inference kernel's answers from one tile in all (n = 2) to about eight
+    per block, so each consumer group takes none, one or several; with more than
+    sixteen neighbours for half of the vertices (extra edges) its wide form.
+    Against the training kernel's forward pass: both accumulate BF16 products in
+    FP32 and round each hidden activation to BF16 once, so an activation may
+    differ by one BF16 unit (2^-8) where the sums' last bits straddle a boundary."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import learned, workload
+    m = workload.box(n, jitter=0.2, seed=13)
+    v = np.arange(m.n_verts // 2)
+    for d in range(2, 2 + extra):
+        m.edge_verts = np.concatenate([m.edge_verts, np.stack([v, v + d], 1).astype(np.int32)])
+    u = workload.bump_field(m.coords, seed=13)
+    with cg.Context(m, precision="fp32") as c:
+        x_bits, aux = learned.features(c, u)
+        p = learned.init_params(21)
+        c.set_mlp_params(p)
+        c.set_precision("learned")
+        c.set_learned_options(True, 1e30)
+        c.estimate_and_mark(u, 0.05 / n)
+        rec = c.debug_read("rec16", np.float32, 8 * m.n_verts).reshape(-1, 8)[:, 4:7].astype(np.float64)
+    tr = learned.Trainer(p, 64)
+    z = tr.forward(torch.from_numpy(x_bits.view(np.int16)).cuda()).cpu().numpy().astype(np.float64)
+    ok = aux[:, 4] == 0
+    assert ok.any() or n == 2
+    want = aux[ok, :3] + z[ok] * aux[ok, 3:4]
+    scale = np.abs(z[ok] * aux[ok, 3:4]).max(initial=0.0) * 2e-2 + 1e-6 * np.abs(want).max(initial=0.0)
+    assert np.abs(rec[ok] - want).max(initial=0.0) <= scale
