@@ -1483,7 +1483,7 @@ static int fast_setup(sprg_ctx* c, ExpandList xl) {
   ENSURE(c->elen, 4 * (size_t)m.E);
   CK(cudaMemsetAsync(c->fcnt.p, 0, 8 * sizeof(int), c->stream));
   PB("setup_coords");
-  fast_prep_coords(m, c->frame, P<float4>(c->crec), c->stream);
+  fast_prep_coords(m, c->frame, false, P<float4>(c->crec), c->stream);
   PE();
   c->crec_ready = true;
   PB("setup_geometry");
@@ -2442,12 +2442,12 @@ static int hessian_operator_2d(sprg_ctx* c, double eps, double h_min, double h_m
   const PatchWeights ls = patch_weights(c, pc);
   PB("recover_grad_op_f64");
   launch_apply_operator(m, 1, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
-                        P<int>(c->klen), P<double>(c->f), P<double>(c->rec), ls, 0, 0, 0, nullptr, nullptr, c->stream);
+                        P<int>(c->klen), P<double>(c->f), P<double>(c->rec), ls, 0, 0, 0, nullptr, nullptr, nullptr, c->stream);
   PE();
   PB("hessian_metric_op_f64");
   launch_apply_operator(m, 3, c->op_kc, P<unsigned char>(c->twlisted), P<int>(c->kidx), P<double>(c->kval),
                         P<int>(c->klen), P<double>(c->rec), P<double>(c->rec9), ls, eps, h_min, h_max, P<float>(c->met32),
-                        c->qrec32.p, c->stream);
+                        c->qrec32.p, P<float4>(c->crec), c->stream);
   PE();
   c->launches += 2;
   return check_launch(c, "triangle operator");
@@ -2463,6 +2463,13 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
   const double* H;
   ENSURE(c->met32, sizeof(float) * 12 * (size_t)(m.V > 0 ? m.V : 1));
   ENSURE(c->qrec32, (size_t)quality_rec_bytes() * (size_t)(m.V > 0 ? m.V : 1));
+  const bool flat = m.dim == 2 && c->planar;
+  if (!c->crec_ready) {  // the coordinate records of the edge and element Jacobians (per mesh)
+    ENSURE(c->crec, 32 * (size_t)(m.V > 0 ? m.V : 1));
+    fast_prep_coords(m, c->frame, flat, P<float4>(c->crec), c->stream);
+    c->launches += 1;
+    c->crec_ready = true;
+  }
   if (m.dim == 2) {
     if ((rc = hessian_operator_2d(c, eps, h_min, h_max))) return rc;
     H = P<double>(c->rec9);
@@ -2471,12 +2478,6 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
     CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
     if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = step_recover(c))) return rc;
     H = P<double>(c->rec);
-  }
-  if (!c->crec_ready) {  // the coordinate records of the edge and element Jacobians (per mesh)
-    ENSURE(c->crec, 32 * (size_t)(m.V > 0 ? m.V : 1));
-    fast_prep_coords(m, c->frame, P<float4>(c->crec), c->stream);
-    c->launches += 1;
-    c->crec_ready = true;
   }
   ENSURE(c->agitems, sizeof(int) * (size_t)(m.E > 0 ? m.E : 1));
   ENSURE(c->agcount, sizeof(int));
@@ -2498,8 +2499,8 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
     frames64 = P<double>(c->frames9);
   }
   PB("measure_aniso_f32");
-  launch_measure_aniso_f32(m, P<float>(c->met32), P<float4>(c->crec), c->frame[3], d_split_bits, d_collapse_bits,
-                           P<int>(c->agitems), P<int>(c->agcount), m.E, c->stream);
+  launch_measure_aniso_f32(m, flat, flat ? P<float>(c->qrec32) : P<float>(c->met32), P<float4>(c->crec), c->frame[3],
+                           d_split_bits, d_collapse_bits, P<int>(c->agitems), P<int>(c->agcount), m.E, c->stream);
   PE();
   PB("guard_measure_f64");
   launch_measure_guard_f64(m, sizes64, frames64, H, eps, h_min, h_max, P<int>(c->agitems), P<int>(c->agcount), m.E,
@@ -2510,7 +2511,7 @@ static int aniso_pass_mixed(sprg_ctx* c, double eps, double h_min, double h_max,
     PB("quality_f32");
     ENSURE(c->cj64, sizeof(double) * (size_t)(m.V > 0 ? m.V : 1));
     ENSURE(c->qties, sizeof(int) * ((size_t)m.T + 1));
-    launch_quality_aniso_f32(m, c->qrec32.p, P<float4>(c->crec), c->frame[3], sizes64, frames64, H, eps, h_min,
+    launch_quality_aniso_f32(m, flat, c->qrec32.p, P<float4>(c->crec), c->frame[3], sizes64, frames64, H, eps, h_min,
                              h_max, P<double>(c->cj64), P<int>(c->qties) + 1, P<int>(c->qties), d_quality, c->stream);
     PE();
     c->launches += 2;

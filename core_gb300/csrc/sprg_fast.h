@@ -8,7 +8,7 @@ int fast_error_blocks(int T);
 // packed double-float coordinate records {x,y,z,0}_hi, {x,y,z,0}_lo (2 float4 per
 // vertex) of the coordinates mapped into [1, 2]: x' = (x - c) s + 1 with
 // frame = {c_x, c_y, c_z, s}, s a power of two
-void fast_prep_coords(const DevMesh& m, const double* frame, float4* vrec, cudaStream_t s);
+void fast_prep_coords(const DevMesh& m, const double* frame, bool flat, float4* vrec, cudaStream_t s);
 // once per mesh: per tet {w dV, h_max} (FP32) and {det J, h_max} (FP64), per
 // edge half its length
 // cent: 3 doubles per element, four times the integration point (once per mesh, read by

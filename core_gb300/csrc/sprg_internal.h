@@ -245,8 +245,9 @@ void launch_metric_f32(int V, int dim, const double* sizes, const double* frames
                        cudaStream_t s);
 int quality_rec_bytes();
 // crec: the FP32 path's coordinate records in the frame x' = (x - c) s + 1
-// (frame_scale = s)
-void launch_measure_aniso_f32(const DevMesh& m, const float* met, const float4* crec, double frame_scale,
+// (frame_scale = s); flat (a mesh in the z = 0 plane, the operator's two-row
+// form): met and crec are that form's flat_met and flat_rec
+void launch_measure_aniso_f32(const DevMesh& m, bool flat, const float* met, const float4* crec, double frame_scale,
                               uint32_t* split, uint32_t* collapse, int* guard, int* gcount, int gcap, cudaStream_t s);
 // sizes / frames: the FP64 metric, or null to rebuild the guarded edges'
 // ends from the Hessian H (hessian_metric_vertex, the FP64 pass's bits)
@@ -257,7 +258,7 @@ void launch_measure_guard_f64(const DevMesh& m, const double* sizes, const doubl
 // two launches: FP32 qualities (listing the elements whose vertex pick the
 // FP32 determinants leave open), then the FP64 tie-breaks; cj64: V doubles,
 // tie_items: T ints, tie_count: one int (scratch, cleared here)
-void launch_quality_aniso_f32(const DevMesh& m, const void* qrec, const float4* crec, double frame_scale,
+void launch_quality_aniso_f32(const DevMesh& m, bool flat, const void* qrec, const float4* crec, double frame_scale,
                               const double* sizes, const double* frames, const double* H, double eps, double hmin,
                               double hmax, double* cj64, int* tie_items, int* tie_count, double* q, cudaStream_t s);
 // Triangle recovery-of-gradient operator (per mesh, FP64): K_va over the
@@ -274,7 +275,7 @@ void launch_tri_operator(const DevMesh& m, int kc, const double* w, unsigned cha
 // through their patches' weights
 void launch_apply_operator(const DevMesh& m, int ncin, int kc, const unsigned char* listed, const int* kidx,
                            const double* kval, const int* klen, const double* f, double* out, const PatchWeights& ls,
-                           double eps, double hmin, double hmax, float* met, void* qrec, cudaStream_t s);
+                           double eps, double hmin, double hmax, float* met, void* qrec, float4* flat_rec, cudaStream_t s);
 // incremental mesh update: dst[ids[r] * width + j] = vals[r * width + j];
 // the coordinates' bounding box as order keys (3 minima, 3 maxima)
 void launch_scatter_rows_f64(long long n, int width, const int* ids, const double* vals, double* dst, cudaStream_t s);

@@ -198,12 +198,16 @@ __device__ __forceinline__ Grad rec_grad(const float4& h, const float4& l) {
 // two): differences of the high words of two records are then exact (Sterbenz)
 // and gradients scale back exactly (du/dx = s du/dx').
 __global__ void __launch_bounds__(kBlock) k_prep_coords(int V, const double* __restrict__ xyz, double cx, double cy,
-                                                        double cz, double cs, float4* __restrict__ rec) {
+                                                        double cz, double cs, bool flat, float4* __restrict__ rec) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= V) return;
   double x = (xyz[3 * (size_t)v] - cx) * cs + 1.0, y = (xyz[3 * (size_t)v + 1] - cy) * cs + 1.0,
          z = (xyz[3 * (size_t)v + 2] - cz) * cs + 1.0;
   float xh = (float)x, yh = (float)y, zh = (float)z;
+  if (flat) {  // a planar mesh's anisotropic pass writes the rest of the record
+    rec[2 * (size_t)v] = make_float4(xh, yh, (float)(x - xh), (float)(y - yh));
+    return;
+  }
   rec[2 * (size_t)v] = make_float4(xh, yh, zh, 0.f);
   rec[2 * (size_t)v + 1] = make_float4((float)(x - xh), (float)(y - yh), (float)(z - zh), 0.f);
 }
@@ -1358,8 +1362,8 @@ int fast_error_blocks(int T) {
   return nb < g ? nb : g;
 }
 
-void fast_prep_coords(const DevMesh& m, const double* frame, float4* vrec, cudaStream_t s) {
-  if (m.V) k_prep_coords<<<nblk(m.V), kBlock, 0, s>>>(m.V, m.xyz, frame[0], frame[1], frame[2], frame[3], vrec);
+void fast_prep_coords(const DevMesh& m, const double* frame, bool flat, float4* vrec, cudaStream_t s) {
+  if (m.V) k_prep_coords<<<nblk(m.V), kBlock, 0, s>>>(m.V, m.xyz, frame[0], frame[1], frame[2], frame[3], flat, vrec);
 }
 
 void fast_geometry(const DevMesh& m, float2* geo, double2* geo64, double* cent, unsigned long long* qmax,

@@ -484,3 +484,38 @@ def test_network_tiles_of_both_consumer_groups(gpu_lib, n, extra):
     want = aux[ok, :3] + z[ok] * aux[ok, 3:4]
     scale = np.abs(z[ok] * aux[ok, 3:4]).max(initial=0.0) * 2e-2 + 1e-6 * np.abs(want).max(initial=0.0)
     assert np.abs(rec[ok] - want).max(initial=0.0) <= scale
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 33, 130])
+@pytest.mark.parametrize("kind", ["layer", "odd", "nan"])
+def test_flat_records_against_the_general_form(gpu_lib, n, kind):
+    """The mixed anisotropic pass of a mesh in the z = 0 plane (compact records)
+    and of the same mesh at z = 1/4 (the general records and products): the same
+    qualities to the bit (only products of exact zeros differ), the same marks."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    from core_gb300.mesh import makeMdsBox
+    m = makeMdsBox(n, n, 0)
+    rng = np.random.default_rng(n)
+    inner = np.all((m.coords[:, :2] > 0) & (m.coords[:, :2] < 1), axis=1)
+    m.coords[inner, :2] += rng.uniform(-0.2, 0.2, (int(inner.sum()), 2)) / n
+    u = workload.boundary_layer_field(m.coords)
+    if kind == "odd":  # flat pieces (zero Hessians), values over many orders of magnitude
+        u = np.where(m.coords[:, 0] < 0.5, 0.0, u * 10.0 ** rng.integers(-200, 100, m.n_verts))
+    elif kind == "nan":
+        u[m.n_verts // 2] = np.nan
+    got = []
+    for z in (0.0, 0.25):
+        m.coords[:, 2] = z
+        with cg.Context(m, precision="fp32") as c:
+            bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+            q = torch.zeros(m.n_elems, dtype=torch.float64, device="cuda")
+            d_u = torch.from_numpy(u).cuda()
+            torch.cuda.synchronize()
+            c.aniso_estimate_and_mark_resident(d_u.data_ptr(), 2.0 / n ** 2, 0.05 / n, 4.0 / n, bits[0].data_ptr(),
+                                               bits[1].data_ptr(), q.data_ptr())
+            torch.cuda.synchronize()
+            got.append((bits.cpu().numpy(), q.cpu().numpy()))
+    assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
+    assert np.array_equal(got[0][0], got[1][0])
