@@ -803,9 +803,11 @@ __device__ __forceinline__ double edge_measure(const V3& x0, const V3& x1) {
   return r;
 }
 
-// AnisoSizeField lengths, with the predicate bitmaps where they are asked for.
-// FP64-rate bound: 1.35 ms for the 3.1M edges of a 1024^2 square (2.77 ms with
-// the general 3 x 3 sequence, plus 0.02 ms for marking from the stored lengths).
+// AnisoSizeField lengths, with the predicate bitmaps where they are asked for
+// (the passes; their frames are rotations on a triangle mesh, the lengths good
+// to a few ulps and the marks those of the bitwise lengths).  FP64-rate bound:
+// 0.42 ms for the 3.1M edges of a 1024^2 square, 1.35 with the planar
+// sequence, 2.77 with the general 3 x 3 one.
 template <bool MARK>
 __global__ void __launch_bounds__(kBlock) k_measure_aniso(DevMesh m, const double* __restrict__ sizes,
                                                           const double* __restrict__ frames, double* __restrict__ L,
@@ -826,7 +828,9 @@ __global__ void __launch_bounds__(kBlock) k_measure_aniso(DevMesh m, const doubl
       Rv[k] = __ldg(frames + 9 * (size_t)vv.x + k);
       Rv[9 + k] = __ldg(frames + 9 * (size_t)vv.y + k);
     }
-    const double l = aniso_length(load_xyz(m.xyz, vv.x), load_xyz(m.xyz, vv.y), hv, Rv);
+    const V3 x0 = load_xyz(m.xyz, vv.x), x1 = load_xyz(m.xyz, vv.y);
+    double l;
+    if (!MARK || !rotated_length(ref::sub(x1, x0), hv, Rv, &l)) l = aniso_length(x0, x1, hv, Rv);
     L[e] = l;
     sp = l > 1.5;
     co = l < .5;

@@ -223,6 +223,48 @@ __device__ __forceinline__ double aniso_length(const ref::V3& x0, const ref::V3&
   return L;
 }
 
+// The same length where both ends' frames are rotations about z and the edge
+// lies in a z = const plane (what the Hessian's metric gives on a triangle
+// mesh): the interpolated second column is the first's +90 degree rotation, so
+// with c the first column, a = d . c, b = d x c and h0, h1 the interpolated sizes
+//   |e Q| = sqrt((a / h0)^2 + (b / h1)^2) / |c|
+//         = n / sqrt(n |c|^2 (h0 h1)^2),   n = (a h1)^2 + (b h0)^2:
+// about 75 FP64 operations an edge against 250.  The two agree to a few ulps
+// times the sizes' ratio (the cancellation in a and b), so a length within
+// 2^24 ulps of a threshold is left to the sequence, as are ratios past 2^19,
+// sizes, lengths or columns outside the ordinary range.  False: not taken.
+__device__ __forceinline__ bool rotated_length(const ref::V3& d, const double* hv, const double* Rv, double* L) {
+  const unsigned long long sign = 0x8000000000000000ull;
+  auto bits = [](double x) { return (unsigned long long)__double_as_longlong(x); };
+  auto turned = [&](const double* R) {  // {c, -s, 0; s, c, 0; 0, 0, .}
+    return all_zero(R[2], R[5], R[6], R[7]) && bits(R[4]) == bits(R[0]) &&
+           (bits(R[1]) == (bits(R[3]) ^ sign) || ((bits(R[1]) | bits(R[3])) << 1) == 0);
+  };
+  auto size = [](double h) { return (unsigned)((__double2hiint(h) >> 20) - 923) <= 200u; };  // (0, 2^+-100)
+  const int spread = max(max(bexp(hv[0]), bexp(hv[1])), max(bexp(hv[3]), bexp(hv[4]))) -
+                     min(min(bexp(hv[0]), bexp(hv[1])), min(bexp(hv[3]), bexp(hv[4])));
+  if (!(turned(Rv) && turned(Rv + 9) && (bits(d.v[2]) << 1) == 0 && spread <= 19)) return false;
+  if (!(size(hv[0]) && size(hv[1]) && size(hv[2]) && size(hv[3]) && size(hv[4]) && size(hv[5]))) return false;
+  const double N0 = (1.0 - 0.577350269189626) / 2.0, N1 = (1.0 + 0.577350269189626) / 2.0;
+  double s[2];
+  bool fine = true;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const double w0 = p ? N1 : N0, w1 = p ? N0 : N1;
+    const double h0 = fma(hv[0], w0, hv[3] * w1), h1 = fma(hv[1], w0, hv[4] * w1);
+    const double cx = fma(Rv[0], w0, Rv[9] * w1), cy = fma(Rv[3], w0, Rv[12] * w1);
+    const double a = fma(d.v[0], cx, d.v[1] * cy), b = fma(d.v[1], cx, -(d.v[0] * cy));
+    const double ah = a * h1, bh = b * h0, hh = h0 * h1;
+    const double n = fma(ah, ah, bh * bh), c2 = fma(cx, cx, cy * cy);
+    fine = fine && bexp(c2) >= 1003 && bexp(c2) <= 1033 && (unsigned)(bexp(n) - 523) <= 1000u;
+    s[p] = n * rsqrt(n * (c2 * (hh * hh)));
+  }
+  *L = 0.5 * (s[0] + s[1]);
+  const long long l = (long long)bits(*L);
+  auto away = [&](double t) { return llabs(l - __double_as_longlong(t)) > (1ll << 24); };
+  return fine && bexp(*L) >= 923 && bexp(*L) <= 1123 && away(1.5) && away(0.5);
+}
+
 // ---- log-interpolated transforms (LogAnisoSizeField) ------------------------
 // |e Q|^2 at one point, e the edge vector and Q = R diag(sqrt(exp(lambda))) of
 // the interpolated log-metric A = R diag(lambda) R^T (a: rows 0 and 1 from

@@ -519,3 +519,42 @@ def test_flat_records_against_the_general_form(gpu_lib, n, kind):
             got.append((bits.cpu().numpy(), q.cpu().numpy()))
     assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
     assert np.array_equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("n", [2, 3, 16, 33])
+@pytest.mark.parametrize("ratio", [1.0, 30.0, 1e5, 1e7])
+@pytest.mark.parametrize("scale", [1.0, 1e40])
+def test_rotated_frames_lengths(gpu_lib, n, ratio, scale):
+    """The FP64 anisotropic pass's lengths (rotation frames on a plane) against the
+    bitwise lengths of the same metric, sizes' ratios up to and past the line
+    (2^19) where the sequence itself is taken, lengths inside and outside the
+    ordinary range: each form's dot products round to 8 ulps of |d|, which
+    counts at most `ratio` times in the length.  Marks: the bitwise lengths'."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    from core_gb300.mesh import makeMdsBox
+    m = makeMdsBox(n, n, 0)
+    m.coords *= scale
+    x = m.coords / scale
+    u = workload.boundary_layer_field(x)
+    hmin = 0.3 * scale / n
+    eps = 0.1 * np.abs(u).max()  # h = sqrt(eps / |lambda|), lambda up to about |u| n^2 / scale^2
+    with cg.Context(m) as c:
+        bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        d_u = torch.from_numpy(u).cuda()
+        torch.cuda.synchronize()
+        c.aniso_estimate_and_mark_resident(d_u.data_ptr(), eps, hmin, hmin * ratio, bits[0].data_ptr(),
+                                           bits[1].data_ptr(), 0)
+        torch.cuda.synchronize()
+        L = c.debug_read("L", np.float64, m.n_edges)
+        sizes = c.debug_read("sizes3", np.float64, 3 * m.n_verts).reshape(-1, 3)
+        frames = c.debug_read("frames9", np.float64, 9 * m.n_verts).reshape(-1, 9)
+        want = c.makeSizeField(sizes=sizes, frames=frames).measure()
+    aspect = (sizes[:, :2].max(axis=1) / sizes[:, :2].min(axis=1)).max()
+    spread = max(aspect, sizes[:, :2].max() / sizes[:, :2].min())
+    assert np.all(np.abs(L - want) <= (32 + 16 * spread) * 2.0 ** -53 * want)
+    e = np.arange(m.n_edges)
+    b = bits.cpu().numpy().view(np.uint32)
+    assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, want > 1.5)
+    assert np.array_equal((b[1][e >> 5] >> (e & 31)) & 1, want < 0.5)
