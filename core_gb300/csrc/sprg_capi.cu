@@ -649,7 +649,7 @@ int fill_info(sprg_ctx* c, sprg_size_info* info) {
 // FP64 qualities into q on the context stream; the vertices' transforms need
 // 81 bytes a vertex, without which they are computed per element
 int step_quality(sprg_ctx* c, const double* size, const double* sizes, const double* frames, const double* logm,
-                 double* q) {
+                 double* q, bool pass = false) {
   DevMesh& m = c->m;
   double* xf = nullptr;
   if (!size) {
@@ -659,7 +659,8 @@ int step_quality(sprg_ctx* c, const double* size, const double* sizes, const dou
     else if (rc != SPRG_ENOMEM) return rc;
     else cudaGetLastError();  // the failed allocation is no error of this call
   }
-  launch_quality_f64(m, size, sizes, frames, logm, xf, P<unsigned char>(c->vbad), q, P<DevStatus>(c->status), c->stream);
+  launch_quality_f64(m, size, sizes, frames, logm, xf, P<unsigned char>(c->vbad), pass, q, P<DevStatus>(c->status),
+                     c->stream);
   c->launches += xf ? 2 : 1;
   return check_launch(c, "quality");
 }
@@ -2551,7 +2552,7 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   c->launches += 2;
   if (d_quality) {
     PB("quality_f64");
-    if ((rc = step_quality(c, nullptr, P<double>(c->sizes3), P<double>(c->frames9), nullptr, d_quality))) return rc;
+    if ((rc = step_quality(c, nullptr, P<double>(c->sizes3), P<double>(c->frames9), nullptr, d_quality, true))) return rc;
     PE();
   }
   c->L_valid = true;

@@ -318,7 +318,7 @@ void launch_size_factor_batch(const double* partials, BatchView bv, int dim, dou
 // transforms (null: computed per element), not used for the isotropic field
 size_t vertex_transform_bytes(int V);
 void launch_quality_f64(const DevMesh& m, const double* size, const double* sizes, const double* frames,
-                        const double* logm, double* xf, unsigned char* bad, double* q, DevStatus* st, cudaStream_t s);
+                        const double* logm, double* xf, unsigned char* bad, bool pass, double* q, DevStatus* st, cudaStream_t s);
 // anisotropic metric (sizes V x 3, frames V x 9) from a nodal Hessian (V x 9)
 void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double hmin, double hmax, double* sizes,
                            double* frames, cudaStream_t s);

@@ -153,24 +153,34 @@ __device__ __forceinline__ double quality_of(const V3* e, const V3* o, double* s
   return ratio_of<D>((D == 3 ? 1.0 / 6.0 : 1.0 / 2.0) * dV, acc);
 }
 
-template <int D>
+// PASS: the anisotropic passes' qualities, good to a few ulps: the squared
+// lengths as they are, without the reference's root and square of each, and
+// fused products (about 55 FP64 operations a triangle of 115)
+template <int D, bool PASS>
 __device__ __forceinline__ double element_quality(const V3* x, const M3& Q) {
   double s, r;
-  if (D == 2 && all_zero(Q.m[0][2], Q.m[1][2], Q.m[2][0], Q.m[2][1]) && x[1].v[2] == x[0].v[2] &&
-      x[2].v[2] == x[0].v[2]) {
+  auto same = [](double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); };
+  if (D == 2 && all_zero(Q.m[0][2], Q.m[1][2], Q.m[2][0], Q.m[2][1]) && same(x[1].v[2], x[0].v[2]) &&
+      same(x[2].v[2], x[0].v[2])) {
     // an element and frames in a z = const plane: the 2 x 2 block alone
     double acc = 0, ex[3], ey[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {  // edges 0-1, 1-2, 0-2
       const int p = i == 1 ? 1 : 0, q = i == 0 ? 1 : 2;
       const double dx = x[q].v[0] - x[p].v[0], dy = x[q].v[1] - x[p].v[1];
-      ex[i] = dx * Q.m[0][0] + dy * Q.m[1][0];
-      ey[i] = dx * Q.m[0][1] + dy * Q.m[1][1];
-      const double l = sqrt(ex[i] * ex[i] + ey[i] * ey[i]);
-      acc += l * l;
+      if (PASS) {
+        ex[i] = fma(dx, Q.m[0][0], dy * Q.m[1][0]);
+        ey[i] = fma(dx, Q.m[0][1], dy * Q.m[1][1]);
+        acc = fma(ex[i], ex[i], fma(ey[i], ey[i], acc));
+      } else {
+        ex[i] = dx * Q.m[0][0] + dy * Q.m[1][0];
+        ey[i] = dx * Q.m[0][1] + dy * Q.m[1][1];
+        const double l = sqrt(ex[i] * ex[i] + ey[i] * ey[i]);
+        acc += l * l;
+      }
     }
     s = acc;
-    const double z = ex[0] * ey[2] - ey[0] * ex[2];
+    const double z = PASS ? fma(ex[0], ey[2], -(ey[0] * ex[2])) : ex[0] * ey[2] - ey[0] * ex[2];
     // |z| = sqrt(z^2) while the square neither under- nor overflows
     const double dV = (unsigned)(bexp(z) - 623) <= 800u ? fabs(z) : sqrt(z * z);
     r = ratio_of<2>(0.5 * dV, acc);
@@ -192,9 +202,10 @@ __device__ __forceinline__ double element_quality(const V3* x, const M3& Q) {
 // Anisotropic and log-interpolated fields: the element takes the transform of
 // its vertex with the largest determinant (the first such).  PRE: from the
 // vertices' records, else (no memory for them) computed in place.
-// FP64-rate bound: 1024^2 square, both kernels 0.58 ms against 3.25 ms with
-// every transform computed per element and the full 3 x 3 products.
-template <int D, bool LOG, bool PRE>
+// FP64-rate bound: 1024^2 square, both kernels 0.40 ms in the pass and 0.58 in
+// the calls, against 3.25 ms with every transform computed per element and the
+// full 3 x 3 products.
+template <int D, bool LOG, bool PRE, bool PASS = false>
 __global__ void __launch_bounds__(kBlock) k_quality(DevMesh m, const double* __restrict__ sizes,
                                                     const double* __restrict__ frames,
                                                     const double* __restrict__ logm, const double* __restrict__ xf,
@@ -215,7 +226,14 @@ __global__ void __launch_bounds__(kBlock) k_quality(DevMesh m, const double* __r
   for (int a = 0; a <= D; ++a) {
     if constexpr (PRE) {
       const double cj = __ldg(xf + kXf * (size_t)id[a] + 9);
-      if (cj > maxJ) {
+      bool larger;
+      if constexpr (D == 2) {  // a length: not negative, ordered as its bits (a NaN is past infinity's)
+        const long long b = __double_as_longlong(cj);
+        larger = (unsigned long long)b <= 0x7ff0000000000000ull && (pick < 0 || b > __double_as_longlong(maxJ));
+      } else {
+        larger = cj > maxJ;
+      }
+      if (larger) {
         maxJ = cj;
         pick = id[a];
       }
@@ -239,7 +257,7 @@ __global__ void __launch_bounds__(kBlock) k_quality(DevMesh m, const double* __r
   V3 x[D + 1];
 #pragma unroll
   for (int a = 0; a <= D; ++a) x[a] = load_xyz(m.xyz, id[a]);
-  q[e] = element_quality<D>(x, Q);
+  q[e] = element_quality<D, PASS>(x, Q);
 }
 
 template <int D>
@@ -316,7 +334,7 @@ __global__ void __launch_bounds__(kBlock) k_quality_iso(DevMesh m, const double*
 size_t vertex_transform_bytes(int V) { return sizeof(double) * kXf * (size_t)V; }
 
 void launch_quality_f64(const DevMesh& m, const double* size, const double* sizes, const double* frames,
-                        const double* logm, double* xf, unsigned char* bad, double* q, DevStatus* st,
+                        const double* logm, double* xf, unsigned char* bad, bool pass, double* q, DevStatus* st,
                         cudaStream_t s) {
   if (!m.T) return;
   const int ge = nblk(m.T), gv = nblk(m.V);
@@ -334,7 +352,7 @@ void launch_quality_f64(const DevMesh& m, const double* size, const double* size
   } else {
     if (xf) transforms(logm ? k_vertex_transforms<2, true> : k_vertex_transforms<2, false>);
     if (logm) quality(xf ? k_quality<2, true, true> : k_quality<2, true, false>);
-    else quality(xf ? k_quality<2, false, true> : k_quality<2, false, false>);
+    else quality(!xf ? k_quality<2, false, false> : pass ? k_quality<2, false, true, true> : k_quality<2, false, true>);
   }
 }
 

@@ -544,16 +544,21 @@ def test_rotated_frames_lengths(gpu_lib, n, ratio, scale):
         bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
         d_u = torch.from_numpy(u).cuda()
         torch.cuda.synchronize()
+        q = torch.zeros(m.n_elems, dtype=torch.float64, device="cuda")
         c.aniso_estimate_and_mark_resident(d_u.data_ptr(), eps, hmin, hmin * ratio, bits[0].data_ptr(),
-                                           bits[1].data_ptr(), 0)
+                                           bits[1].data_ptr(), q.data_ptr())
         torch.cuda.synchronize()
         L = c.debug_read("L", np.float64, m.n_edges)
         sizes = c.debug_read("sizes3", np.float64, 3 * m.n_verts).reshape(-1, 3)
         frames = c.debug_read("frames9", np.float64, 9 * m.n_verts).reshape(-1, 9)
         want = c.makeSizeField(sizes=sizes, frames=frames).measure()
+        want_q = c.measureQuality(sizes=sizes, frames=frames)
     aspect = (sizes[:, :2].max(axis=1) / sizes[:, :2].min(axis=1)).max()
     spread = max(aspect, sizes[:, :2].max() / sizes[:, :2].min())
     assert np.all(np.abs(L - want) <= (32 + 16 * spread) * 2.0 ** -53 * want)
+    # a metric edge vector is off by delta = 4 spread ulps of its length at most,
+    # 48 A^2 / s^2 <= 1 by 8 delta
+    assert np.all(np.abs(q.cpu().numpy() - want_q) <= (32 + 32 * spread) * 2.0 ** -53)
     e = np.arange(m.n_edges)
     b = bits.cpu().numpy().view(np.uint32)
     assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, want > 1.5)
