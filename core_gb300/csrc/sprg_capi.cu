@@ -81,6 +81,11 @@ struct sprg_ctx {
   bool qw_ready = false;
   // mixed-precision anisotropic pass: triangle patch weights and their
   // listed vertices (per mesh), FP32 metric records, guarded edges
+  // triangles' refined patch weights (the FP64 passes) and the number of patches
+  // too large for them
+  bool rw_ready = false;
+  int n_rw_big = 0;
+  DevBuf rw, rwlisted, rwitems, rwcount;
   DevBuf tw, twlisted, twitems, twcount, met32, qrec32, agitems, agcount, kidx, kval, klen, rec9, cj64, qties;
   bool tw_ready = false;
   int op_kc = 3;  // operator components per slot (2 on a mesh in the z = 0 plane)
@@ -161,7 +166,7 @@ struct sprg_ctx {
   double frame[4] = {0, 0, 0, 1};  // coordinate records: x' = (x - c) s + 1 in [1, 2]
   bool planar = false;             // every vertex has z = 0
   int n_listed = 0, n_refit = 0;
-  PatchCache cache64, cache32, cache2d;
+  PatchCache cache64, cache32, cache2d, cache2r;
   static constexpr int kGuardCap = 1 << 20;
   static constexpr float kGuardRel = 2e-6f;
   std::string err_msg;
@@ -839,12 +844,13 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   // the tuned launch shape stays: every choice gives bitwise the same result,
   // and an adapt iteration changes the patch-size mix little
   c->tw_ready = false;
+  c->rw_ready = false;
   c->qw_ready = false;
   c->tfac_ready = c->tfac_none = false;
   c->egeo_ready = c->egeo_none = c->elen64_ready = c->elen64_none = false;
   c->vv_ready = false;
-  c->cache64.valid = c->cache32.valid = c->cache2d.valid = false;
-  c->cache64.w_ready = c->cache32.w_ready = c->cache2d.w_ready = false;
+  c->cache64.valid = c->cache32.valid = c->cache2d.valid = c->cache2r.valid = false;
+  c->cache64.w_ready = c->cache32.w_ready = c->cache2d.w_ready = c->cache2r.w_ready = false;
   c->batch_n = 0;
   c->batch_nseg = 0;
   c->gstamp_ready = false;  // zeroed again at the next guard pass
@@ -1021,7 +1027,7 @@ int sprg_destroy(sprg_ctx* c) {
   DevBuf* bufs[] = {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
                     &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
-                    &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->cache2d.woff, &c->cache2d.w, &c->cache2d.wn, &c->agitems, &c->agcount,
+                    &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->rw, &c->rwlisted, &c->rwitems, &c->rwcount, &c->cache2r.v, &c->cache2r.n, &c->cache2r.el, &c->cache2r.woff, &c->cache2r.w, &c->cache2r.wn, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->cache2d.woff, &c->cache2d.w, &c->cache2d.wn, &c->agitems, &c->agcount,
                     &c->crec,  &c->vrec,    &c->rec32, &c->q32, &c->sz2,  &c->fcnt,   &c->guard, &c->tetd,
                     &c->wts,   &c->w64,     &c->listed, &c->geo, &c->geo64, &c->elen, &c->fitems, &c->gstamp, &c->gfit, &c->grec, &c->tnext, &c->edone,
                     &c->hess, &c->pcls, &c->bverts, &c->btiles, &c->bnext, &c->bvoff, &c->bseg, &c->bsegoff, &c->bratios, &c->vvoff, &c->vv, &c->vtile, &c->vr16, &c->rec16,
@@ -1943,6 +1949,56 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
   return check_launch(c, "learned pass");
 }
 
+// the triangles' refined patch weights (once per mesh) and the patches they
+// leave out
+static int ensure_pass_weights(sprg_ctx* c) {
+  DevMesh& m = c->m;
+  int rc;
+  ENSURE(c->rwitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
+  ENSURE(c->rwcount, 2 * sizeof(int));  // listed patches, patches too large
+  const ExpandList lst{P<int>(c->rwitems), P<int>(c->rwcount), m.V};
+  if (!c->rw_ready) {
+    ENSURE(c->rw, sizeof(double) * (size_t)m.T * m.nn);
+    ENSURE(c->rwlisted, (size_t)(m.V > 0 ? m.V : 1));
+    CK(cudaMemsetAsync(c->rwcount.p, 0, 2 * sizeof(int), c->stream));
+    PB("tri_weights_f64");
+    launch_tri_weights(m, P<double>(c->rw), P<unsigned char>(c->rwlisted), lst, P<int>(c->rwcount) + 1, c->stream);
+    PE();
+    c->launches += 1;
+    CK(cudaMemcpyAsync(&c->n_rw_big, P<int>(c->rwcount) + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if ((rc = check_launch(c, "triangle weights"))) return rc;
+    c->rw_ready = true;
+  }
+  return c->n_rw_big ? SPRG_OK : ensure_listed(c, c->cache2r, lst, -1);
+}
+
+// The recovery of the FP64 passes.  On triangles weighted sums, as on tets,
+// instead of applying the factors to every component (both recoveries of a
+// 1024^2 square's anisotropic pass: 152 us against 744); the recovery calls
+// keep the factors, whose bits are the reference's.  Without memory for the
+// weights, or with a patch of more elements than they take (the factors' warp
+// path has no limit), the factors here too.
+static int pass_recover(sprg_ctx* c) {
+  DevMesh& m = c->m;
+  if (m.dim == 3) return step_recover(c);
+  const int nc = c->ip_nc;
+  ENSURE(c->rec, sizeof(double) * (size_t)m.V * nc);
+  ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + nc + 1));
+  const int rc = ensure_pass_weights(c);
+  if (rc && rc != SPRG_ENOMEM) return rc;
+  if (rc || c->n_rw_big) {
+    if (rc) cudaGetLastError();  // the failed allocation is no error of this call
+    return step_recover(c);
+  }
+  PB("recover_f64");
+  launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->rw), P<unsigned char>(c->rwlisted),
+                     patch_weights(c, c->cache2r), P<double>(c->rec), c->stream);
+  PE();
+  c->launches += 1;
+  return check_launch(c, "recover");
+}
+
 // the pass on a device field (read in place, in stream order)
 static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
   int rc;
@@ -1955,7 +2011,7 @@ static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uin
   }
   if (c->precision == SPRG_FP32) return pass_fast(c, d_u, adapt_ratio, d_split, d_collapse);
   if (c->precision == SPRG_LEARNED) return pass_learned(c, d_u, adapt_ratio, d_split, d_collapse);
-  if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = step_recover(c)) ||
+  if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = pass_recover(c)) ||
       (rc = step_size(c, 0, adapt_ratio, 0, 0, 0)))
     return rc;
   return step_measure_mark(c, d_split, d_collapse);
@@ -2425,7 +2481,7 @@ static int hessian_operator_2d(sprg_ctx* c, double eps, double h_min, double h_m
     ENSURE(c->klen, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
     CK(cudaMemsetAsync(c->twcount.p, 0, sizeof(int), c->stream));
     PB("tri_weights_f64");
-    launch_tri_weights(m, P<double>(c->tw), P<unsigned char>(c->twlisted), lst, c->stream);
+    launch_tri_weights(m, P<double>(c->tw), P<unsigned char>(c->twlisted), lst, nullptr, c->stream);
     PE();
     PB("tri_operator_f64");
     launch_tri_operator(m, c->op_kc, P<double>(c->tw), P<unsigned char>(c->twlisted), lst, P<int>(c->kidx),
@@ -2538,9 +2594,9 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
   if (c->precision == SPRG_FP32) return aniso_pass_mixed(c, eps, h_min, h_max, d_split_bits, d_collapse_bits, d_quality);
   // recovered gradient, then the recovered gradient of it (nodal Hessian)
-  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = step_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = pass_recover(c))) return rc;
   CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
-  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = step_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = pass_recover(c))) return rc;
   PB("hessian_metric");
   launch_hessian_metric(m, P<double>(c->rec), eps, h_min, h_max, P<double>(c->sizes3), P<double>(c->frames9),
                         c->stream);

@@ -1571,9 +1571,17 @@ __global__ void __launch_bounds__(kBlock) k_mark_quality(int T, const double* __
 // is the reference's (as in k_recover_tri); listed: patches the weights do
 // not cover (fewer than NT or more than MAXM elements, rank deficient),
 // which take the FP64 fit paths every pass.
-template <int MAXM>
+//
+// REFINED (the FP64 passes): one step of correction with the moments Sum w = 1,
+// Sum w (p - x_v) = 0 in coordinates about the vertex.  The QR's are absolute,
+// which costs both the factors and these weights digits: over patches of 4 to 7
+// elements 1/1024 wide, values about 1, the rms error of the recovered value is
+// 4.5e-16 with the factors, 4.3e-16 with the weights, 1.0e-16 with refined ones.
+// n_big counts the patches of more elements than the weights take.
+template <int MAXM, bool REFINED>
 __global__ void __launch_bounds__(128) k_tri_weights(DevMesh m, double* __restrict__ w,
-                                                     unsigned char* __restrict__ listed, ExpandList lst) {
+                                                     unsigned char* __restrict__ listed, ExpandList lst,
+                                                     int* __restrict__ n_big) {
   constexpr int NT = 3;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= m.V) return;
@@ -1585,6 +1593,7 @@ __global__ void __launch_bounds__(128) k_tri_weights(DevMesh m, double* __restri
     if (slot < lst.cap) lst.items[slot] = v;
   };
   if (cnt < NT || cnt > MAXM) {
+    if (REFINED && cnt > MAXM) atomicAdd(n_big, 1);
     give_up();
     return;
   }
@@ -1658,6 +1667,38 @@ __global__ void __launch_bounds__(128) k_tri_weights(DevMesh m, double* __restri
     w[beg + r] = q[0] * z[0] + q[1] * z[1] + q[2] * z[2];
   }
   listed[v] = 0;
+  if constexpr (REFINED) {
+    double px[MAXM], py[MAXM], wr[MAXM];
+    double sx = 0, sy = 0, sxx = 0, sxy = 0, syy = 0, r0 = 1, rx = 0, ry = 0;
+#pragma unroll
+    for (int r = 0; r < MAXM; ++r) {
+      if (r >= cnt) break;
+      const V3 p = elem_ip_point(m, m.p_el[beg + r]);
+      const double x = p.v[0] - xv.v[0], y = p.v[1] - xv.v[1], wk = w[beg + r];
+      px[r] = x;
+      py[r] = y;
+      wr[r] = wk;
+      sx += x;
+      sy += y;
+      sxx = fma(x, x, sxx);
+      sxy = fma(x, y, sxy);
+      syy = fma(y, y, syy);
+      r0 -= wk;
+      rx = fma(-wk, x, rx);
+      ry = fma(-wk, y, ry);
+    }
+    const double mx = sx / cnt, my = sy / cnt;
+    const double a = fma(-mx, sx, sxx), b = fma(-mx, sy, sxy), c = fma(-my, sy, syy);
+    const double b1 = fma(-mx, r0, rx), b2 = fma(-my, r0, ry), det = fma(a, c, -(b * b));
+    if (!(det > 1e-8 * (a * c))) return;  // nearly collinear: the QR's weights
+    const double z1 = fma(b1, c, -(b2 * b)) / det, z2 = fma(a, b2, -(b * b1)) / det;
+    const double z0 = (r0 - fma(sx, z1, sy * z2)) / cnt;
+#pragma unroll
+    for (int r = 0; r < MAXM; ++r) {
+      if (r >= cnt) break;
+      w[beg + r] = wr[r] + fma(z1, px[r], fma(z2, py[r], z0));
+    }
+  }
 }
 
 // Per vertex: the FP32 metric record h (3), frame (9, row-major) for the
@@ -2765,8 +2806,10 @@ void launch_mark_quality(int T, const double* q, double good, int* flags, unsign
                          cudaStream_t s) {
   if (T) k_mark_quality<<<count_grid(T), kBlock, 0, s>>>(T, q, good, flags, count, st);
 }
-void launch_tri_weights(const DevMesh& m, double* w, unsigned char* listed, ExpandList lst, cudaStream_t s) {
-  if (m.V) k_tri_weights<kTriThreadRows><<<(m.V + 127) / 128, 128, 0, s>>>(m, w, listed, lst);
+void launch_tri_weights(const DevMesh& m, double* w, unsigned char* listed, ExpandList lst, int* n_big, cudaStream_t s) {
+  if (!m.V) return;
+  auto k = n_big ? k_tri_weights<kTriThreadRows, true> : k_tri_weights<kTriThreadRows, false>;
+  k<<<(m.V + 127) / 128, 128, 0, s>>>(m, w, listed, lst, n_big);
 }
 
 void launch_metric_f32(int V, int dim, const double* sizes, const double* frames, float* out, void* qrec,

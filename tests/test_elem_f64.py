@@ -563,3 +563,54 @@ def test_rotated_frames_lengths(gpu_lib, n, ratio, scale):
     b = bits.cpu().numpy().view(np.uint32)
     assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, want > 1.5)
     assert np.array_equal((b[1][e >> 5] >> (e & 31)) & 1, want < 0.5)
+
+
+@pytest.mark.parametrize("n,kind", [(2, "plain"), (3, "plain"), (16, "plain"), (33, "warped"), (9, "fan"), (9, "no memory")])
+def test_pass_recovery_on_triangles(gpu_lib, n, kind):
+    """The FP64 pass's recovered gradient (refined weights) against the recovery
+    call's (the factors, in absolute coordinates: good to about cond(patch) ulps,
+    the vertices' distance from the origin over an element's width, below 4 n, a
+    few times over); with a patch too large for the weights, or without memory for
+    them, the factors' bits."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    from core_gb300.mesh import Mesh, makeMdsBox
+    m = makeMdsBox(n, n, 0)
+    rng = np.random.default_rng(n)
+    inner = np.all((m.coords[:, :2] > 0) & (m.coords[:, :2] < 1), axis=1)
+    m.coords[inner, :2] += rng.uniform(-0.2, 0.2, (int(inner.sum()), 2)) / n
+    if kind == "warped":
+        m.coords[:, 2] = 0.1 * np.sin(3 * m.coords[:, 0])
+    elif kind == "fan":  # a wheel of twelve triangles beside the square
+        k, V = 12, m.n_verts
+        t = np.arange(k) * 2 * np.pi / k
+        x = np.zeros((k + 1, 3))
+        x[1:, 0], x[1:, 1] = np.cos(t), np.sin(t)
+        x[:, 0] += 3.0
+        ring = V + 1 + np.arange(k)
+        hub = np.full(k, V)
+        ev = np.stack([hub, ring, np.roll(ring, -1)], 1)
+        ed = np.concatenate([np.stack([hub, ring], 1), np.stack([ring, np.roll(ring, -1)], 1)])
+        m = Mesh(2, np.concatenate([m.coords, x]), np.concatenate([m.elem_verts, ev]).astype(np.int32),
+                 np.concatenate([m.edge_verts, ed]).astype(np.int32))
+    u = workload.boundary_layer_field(m.coords)
+    with cg.Context(m) as c:
+        ip = c.getGradIPField(u)
+        want = c.recoverField(ip)
+    with cg.Context(m) as c:
+        if kind == "no memory":
+            c.test_hooks(alloc_fail_after=3)
+        bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        d_u = torch.from_numpy(u).cuda()
+        torch.cuda.synchronize()
+        try:
+            c.estimate_and_mark_resident(d_u.data_ptr(), 0.1, bits[0].data_ptr(), bits[1].data_ptr())
+        except cg.SprgError:
+            assert kind == "no memory"  # the failed allocation was one the pass needs
+            return
+        torch.cuda.synchronize()
+        got = c.debug_read("rec", np.float64, 3 * m.n_verts).reshape(-1, 3)
+    if kind == "fan":
+        assert np.array_equal(got, want)
+    assert np.abs(got - want).max() <= 64 * 4 * n * 2.0 ** -53 * np.abs(ip).max()
