@@ -2603,10 +2603,14 @@ __global__ void __launch_bounds__(kBlock) k_qr_weights(DevMesh m, double* __rest
   if (lane == 0) listed[v] = 0;
 }
 
-// FP64 recovery from the weights: thread per vertex, NC components (fused
-// multiply-adds: the sum's order is this method's own, and the FP64 pipe, at
-// 73 % with separate products and sums, bounds the kernel)
-template <int NC>
+// FP64 recovery from the weights: LANES consecutive lanes per vertex, NC
+// components (fused multiply-adds: the sum's order is this method's own, and
+// the FP64 pipe, at 73 % with separate products and sums, bounds the kernel).
+// Tets two lanes: a warp's ids and weights come from half as many patches, and
+// the extra sums are 3 of 72; 96^3 box: 134 us, 197 with one lane, 159 with four.
+// Triangles one: six elements hide no sum (1024^2 square, both recoveries: 152
+// us, 192 with two).
+template <int NC, int LANES>
 __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double* __restrict__ ip,
                                                         const double* __restrict__ w,
                                                         const unsigned char* __restrict__ listed,
@@ -2618,18 +2622,24 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
     if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
     return;
   }
-  const int v = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
-  if (v >= m.V || listed[v]) return;
-  const int beg = m.p_off[v], end = m.p_off[v + 1];
+  const int i = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
+  const int v = i / LANES, l = i % LANES;
+  const bool mine = v < m.V && !listed[v];
+  const int beg = mine ? m.p_off[v] : 0, end = mine ? m.p_off[v + 1] : 0;
   double acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c] = 0;
-  for (int k = beg; k < end; ++k) {
+  for (int k = beg + l; k < end; k += LANES) {
     const double wk = w[k];
     const double* b = ip + (size_t)m.p_el[k] * NC;
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] = fma(wk, b[c], acc[c]);
   }
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+  if (!mine || l) return;
 #pragma unroll
   for (int c = 0; c < NC; ++c) rec[(size_t)v * NC + c] = acc[c];
 }
@@ -2906,8 +2916,11 @@ void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double
                         const PatchWeights& pw, double* rec, cudaStream_t s) {
   if (!m.V) return;
   const int nl = nblk((long)pw.n * 32);
-  launch_after(m.early, nc == 3 ? k_recover_w64<3> : k_recover_w64<9>, nl + nblk(m.V), kBlock, s, m, ip, w, listed, nl,
-               pw, rec);
+  auto go = [&](int lanes, auto kernel) {
+    launch_after(m.early, kernel, nl + nblk((long)m.V * lanes), kBlock, s, m, ip, w, listed, nl, pw, rec);
+  };
+  if (m.dim == 3) go(2, nc == 3 ? k_recover_w64<3, 2> : k_recover_w64<9, 2>);  // lanes: see the kernel
+  else go(1, nc == 3 ? k_recover_w64<3, 1> : k_recover_w64<9, 1>);
 }
 
 }  // namespace sprg
