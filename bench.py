@@ -102,12 +102,13 @@ def pass_bytes(V, T, E):
 def algorithmic_bytes(kernel, V, T, E, vb=8):
     ib = 4
     table = {
-        "grad_ip_f64": 4 * ib * T + 3 * vb * V + vb * V + 3 * vb * T,
+        # FP64 path: per-mesh element records (J^-1, det J, h_max), edge lengths
+        "grad_ip_f64": 4 * ib * T + 9 * vb * T + vb * V + 3 * vb * T,
         "recover_f64": ib * (V + 1) + 4 * ib * T + 4 * ib * T + 3 * vb * V + 3 * vb * T + 3 * vb * V,
-        "error_f64": 4 * ib * T + 3 * vb * V + 3 * vb * T + 3 * vb * V + vb * T,
-        "esize_f64": 4 * ib * T + 3 * vb * V + vb * T + vb * T,
+        "error_f64": 4 * ib * T + 2 * vb * T + 3 * vb * T + 3 * vb * V + 2 * vb * T,
+        "esize_f64": 2 * vb * T,
         "average_f64": ib * (V + 1) + 4 * ib * T + vb * T + vb * V,
-        "measure_f64": 2 * ib * E + 3 * vb * V + vb * V + vb * E,
+        "measure_f64": 2 * ib * E + 2 * vb * E + vb * V + E // 4,
         "mark_bits": vb * E + E // 4,
         # FP32 path: 32-byte vertex records (coordinates + field pair), 16-byte
         # packed element gradients and recovered values, per-mesh geometry

@@ -25,9 +25,10 @@
 // half its length (FP64, rounded).
 //
 // Phases of a pass:
-//   prep      four vertices per thread: the field pairs
-//   tet       thread per tet: its gradient as 16 bytes, the FP32 value s
-//             and the packed correction r (exact = s + r, see pack_corr)
+//   prep      four vertices per thread: the field pairs; the pass's counters
+//   tet       the listed patches' FP64 sums, a warp each, then a thread per
+//             tet: its gradient as 16 bytes, the FP32 value s and the packed
+//             correction r (exact = s + r, see pack_corr)
 //   recover   1, 2 or 4 lanes per vertex (tuned per patch-size bin):
 //             eps*(v) = g_ref + sum w_vt (eps_t - g_ref)
 //   error     thread per tet: element error, SelfProduct and Error terms
@@ -37,7 +38,8 @@
 //             (compensated) and the size's error bound, packed as a pair
 //   measure   thread per edge: metric length, split/collapse bitmaps, and the
 //             list of edges whose distance to 0.5 / 1.5 is within the error
-//             bound (re-decided in FP64 by the guard kernels)
+//             bound, with the vertices around them (re-decided in FP64 by the
+//             guard kernels)
 #include <algorithm>
 
 #include "sprg_fast.h"
