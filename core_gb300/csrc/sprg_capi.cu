@@ -81,7 +81,7 @@ struct sprg_ctx {
   bool qw_ready = false;
   // mixed-precision anisotropic pass: triangle patch weights and their
   // listed vertices (per mesh), FP32 metric records, guarded edges
-  // triangles' refined patch weights (the FP64 passes) and the number of patches
+  // triangles' refined patch weights (the FP64 anisotropic pass) and the number of patches
   // too large for them
   bool rw_ready = false;
   int n_rw_big = 0;
@@ -1951,7 +1951,7 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
 
 // the triangles' refined patch weights (once per mesh) and the patches they
 // leave out
-static int ensure_pass_weights(sprg_ctx* c) {
+static int ensure_aniso_weights(sprg_ctx* c) {
   DevMesh& m = c->m;
   int rc;
   ENSURE(c->rwitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
@@ -1973,19 +1973,21 @@ static int ensure_pass_weights(sprg_ctx* c) {
   return c->n_rw_big ? SPRG_OK : ensure_listed(c, c->cache2r, lst, -1);
 }
 
-// The recovery of the FP64 passes.  On triangles weighted sums, as on tets,
-// instead of applying the factors to every component (both recoveries of a
-// 1024^2 square's anisotropic pass: 152 us against 744); the recovery calls
-// keep the factors, whose bits are the reference's.  Without memory for the
-// weights, or with a patch of more elements than they take (the factors' warp
-// path has no limit), the factors here too.
-static int pass_recover(sprg_ctx* c) {
+// The recoveries of the FP64 anisotropic pass.  On triangles weighted sums, as
+// on tets, instead of applying the factors to every component (both recoveries
+// of a 1024^2 square: 152 us against 744).  The recovery calls and the
+// isotropic pass keep the factors: their bits are the reference's, and on a
+// linear field, whose deviations are rounding alone, they decide the sizes
+// (here such a field's sizes are the largest whatever the rounding).  Without
+// memory for the weights, or with a patch of more elements than they take (the
+// factors' warp path has no limit), the factors here too.
+static int aniso_recover(sprg_ctx* c) {
   DevMesh& m = c->m;
   if (m.dim == 3) return step_recover(c);
   const int nc = c->ip_nc;
   ENSURE(c->rec, sizeof(double) * (size_t)m.V * nc);
   ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + nc + 1));
-  const int rc = ensure_pass_weights(c);
+  const int rc = ensure_aniso_weights(c);
   if (rc && rc != SPRG_ENOMEM) return rc;
   if (rc || c->n_rw_big) {
     if (rc) cudaGetLastError();  // the failed allocation is no error of this call
@@ -2011,7 +2013,7 @@ static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uin
   }
   if (c->precision == SPRG_FP32) return pass_fast(c, d_u, adapt_ratio, d_split, d_collapse);
   if (c->precision == SPRG_LEARNED) return pass_learned(c, d_u, adapt_ratio, d_split, d_collapse);
-  if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = pass_recover(c)) ||
+  if ((rc = reset_status(c)) || (rc = step_grad(c, d_u, 1)) || (rc = step_recover(c)) ||
       (rc = step_size(c, 0, adapt_ratio, 0, 0, 0)))
     return rc;
   return step_measure_mark(c, d_split, d_collapse);
@@ -2594,9 +2596,9 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
   if (c->precision == SPRG_FP32) return aniso_pass_mixed(c, eps, h_min, h_max, d_split_bits, d_collapse_bits, d_quality);
   // recovered gradient, then the recovered gradient of it (nodal Hessian)
-  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = pass_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = aniso_recover(c))) return rc;
   CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
-  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = pass_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = aniso_recover(c))) return rc;
   PB("hessian_metric");
   launch_hessian_metric(m, P<double>(c->rec), eps, h_min, h_max, P<double>(c->sizes3), P<double>(c->frames9),
                         c->stream);

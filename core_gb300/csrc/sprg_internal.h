@@ -239,7 +239,7 @@ void launch_mark_quality(int T, const double* q, double good, int* flags, unsign
 // FP32 edge measure writing the mark bitmaps and the
 // edges within their error bound of 0.5 / 1.5 (guard); the guard's FP64
 // re-measure fixing those bits; FP32 qualities.
-// n_big (zero before): the refined weights of the FP64 passes, with the count of
+// n_big (zero before): the refined weights of the FP64 anisotropic pass, with the count of
 // the patches of more elements than the weights take; null: the mixed pass's
 void launch_tri_weights(const DevMesh& m, double* w, unsigned char* listed, ExpandList lst, int* n_big, cudaStream_t s);
 // qrec: quality_rec_bytes() per vertex

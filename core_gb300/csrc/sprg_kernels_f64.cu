@@ -1572,7 +1572,7 @@ __global__ void __launch_bounds__(kBlock) k_mark_quality(int T, const double* __
 // not cover (fewer than NT or more than MAXM elements, rank deficient),
 // which take the FP64 fit paths every pass.
 //
-// REFINED (the FP64 passes): one step of correction with the moments Sum w = 1,
+// REFINED (the FP64 anisotropic pass): one step of correction with the moments Sum w = 1,
 // Sum w (p - x_v) = 0 in coordinates about the vertex.  The QR's are absolute,
 // which costs both the factors and these weights digits: over patches of 4 to 7
 // elements 1/1024 wide, values about 1, the rms error of the recovered value is

@@ -567,11 +567,12 @@ def test_rotated_frames_lengths(gpu_lib, n, ratio, scale):
 
 @pytest.mark.parametrize("n,kind", [(2, "plain"), (3, "plain"), (16, "plain"), (33, "warped"), (9, "fan"), (9, "no memory")])
 def test_pass_recovery_on_triangles(gpu_lib, n, kind):
-    """The FP64 pass's recovered gradient (refined weights) against the recovery
-    call's (the factors, in absolute coordinates: good to about cond(patch) ulps,
-    the vertices' distance from the origin over an element's width, below 4 n, a
-    few times over); with a patch too large for the weights, or without memory for
-    them, the factors' bits."""
+    """The FP64 anisotropic pass's Hessian (refined weights) against the calls'
+    (the factors, in absolute coordinates: a recovered value is good to about
+    cond(patch) ulps, the vertices' distance from the origin over an element's
+    width, below 4 n, a few times over, and the second gradient divides the first
+    recovery's error by the width); with a patch too large for the weights, the
+    factors' bits."""
     import torch
     import core_gb300 as cg
     from core_gb300 import workload
@@ -597,7 +598,8 @@ def test_pass_recovery_on_triangles(gpu_lib, n, kind):
     u = workload.boundary_layer_field(m.coords)
     with cg.Context(m) as c:
         ip = c.getGradIPField(u)
-        want = c.recoverField(ip)
+        ip2 = c.getGradIPField(c.recoverField(ip))
+        want = c.recoverField(ip2)
     with cg.Context(m) as c:
         if kind == "no memory":
             c.test_hooks(alloc_fail_after=3)
@@ -605,12 +607,13 @@ def test_pass_recovery_on_triangles(gpu_lib, n, kind):
         d_u = torch.from_numpy(u).cuda()
         torch.cuda.synchronize()
         try:
-            c.estimate_and_mark_resident(d_u.data_ptr(), 0.1, bits[0].data_ptr(), bits[1].data_ptr())
+            c.aniso_estimate_and_mark_resident(d_u.data_ptr(), 0.1, 0.1 / n, 1.0, bits[0].data_ptr(), bits[1].data_ptr())
         except cg.SprgError:
             assert kind == "no memory"  # the failed allocation was one the pass needs
             return
         torch.cuda.synchronize()
-        got = c.debug_read("rec", np.float64, 3 * m.n_verts).reshape(-1, 3)
+        got = c.debug_read("rec", np.float64, 9 * m.n_verts).reshape(-1, 9)
     if kind == "fan":
         assert np.array_equal(got, want)
-    assert np.abs(got - want).max() <= 64 * 4 * n * 2.0 ** -53 * np.abs(ip).max()
+    one = 64 * 4 * n * 2.0 ** -53
+    assert np.abs(got - want).max() <= one * (np.abs(ip2).max() + 4 * n * np.abs(ip).max())
