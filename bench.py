@@ -103,7 +103,7 @@ def algorithmic_bytes(kernel, V, T, E, vb=8):
     ib = 4
     table = {
         # FP64 path: per-mesh element records (J^-1, det J, h_max), edge lengths
-        "grad_ip_f64": 4 * ib * T + 9 * vb * T + vb * V + 3 * vb * T,
+        "grad_ip_f64": 4 * ib * T + 12 * vb * T + vb * V + 3 * vb * T,
         "recover_f64": ib * (V + 1) + 4 * ib * T + 4 * ib * T + 3 * vb * V + 3 * vb * T + 3 * vb * V,
         "error_f64": 4 * ib * T + 2 * vb * T + 3 * vb * T + 3 * vb * V + 2 * vb * T,
         "esize_f64": 2 * vb * T,

@@ -74,7 +74,7 @@ struct sprg_ctx {
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
   // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
   // egeo_none: there was no memory for them, the kernels compute in place
-  DevBuf egeo, elen64;  // elen64: the edges' lengths
+  DevBuf egeo, elen64;  // elen64: half the edges' lengths
   bool egeo_ready = false, egeo_none = false, elen64_ready = false, elen64_none = false;
   // FP64 recovery on tets: per-mesh QR weights and the listed patches
   DevBuf qw, qwlisted, qwitems, qwcount;

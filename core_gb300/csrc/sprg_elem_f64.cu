@@ -37,11 +37,12 @@ __device__ __forceinline__ void load_ids(const int* __restrict__ ev, int e, int*
 
 // One element's geometry: the rows of J^-1 (D columns each; the third column
 // of a triangle's pseudo-inverse is 0), dV = det J, and the longest edge
-// (apf::measure).  Record planes: J^-1 row-major (3 D planes), dV, h; plane
-// k of element e at k T + e.
+// (apf::measure).  Record planes: J^-1 row-major (3 D planes), dV, h, and on
+// tets the first vertex's shape gradient (the negated row sums); plane k of
+// element e at k T + e.
 template <int D>
 struct ElemRec {
-  static constexpr int kPlanes = 3 * D + 2;
+  static constexpr int kPlanes = 3 * D + (D == 3 ? 5 : 2);
   double v[kPlanes];
 };
 
@@ -134,8 +135,13 @@ __device__ __forceinline__ void elem_record_of(const DevMesh& m, const int* id, 
   V3 x[D + 1];
 #pragma unroll
   for (int a = 0; a <= D; ++a) x[a] = load_xyz(m.xyz, id[a]);
-  if constexpr (D == 3) tet_record(x, out);
-  else elem_record_ref<D>(x, out);
+  if constexpr (D == 3) {
+    tet_record(x, out);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) out[11 + r] = -out[3 * r] - out[3 * r + 1] - out[3 * r + 2];
+  } else {
+    elem_record_ref<D>(x, out);
+  }
 }
 
 // per mesh; FP64-rate bound (the operations above), 8 kPlanes bytes written
@@ -156,9 +162,9 @@ __global__ void __launch_bounds__(kBlock) k_elem_records(DevMesh m, double* __re
 // shape functions are J^-1's columns and, for the first vertex, the negated
 // sum of each row (the reference's products with 1, 0 and -1); the sums over
 // the vertices keep its order.  With the per-mesh records a scalar field
-// costs 27 FP64 operations and 112 bytes a tet, 0.28 ms for the 5.3M tets of
-// a 96^3 box (2.2 TB/s, FP64 pipe about 80 % busy) against 2.76 ms with the
-// sequence written out; without them (no memory for the records) they are
+// costs 21 FP64 operations and 136 bytes a tet, 0.22 ms for the 5.3M tets of
+// a 96^3 box (3.3 TB/s; 0.28 ms with the first vertex's gradients summed here,
+// 27 operations and 112 bytes) against 2.76 ms with the sequence written out; without them (no memory for the records) they are
 // computed in place.
 // ---------------------------------------------------------------------
 template <int D, int NC, bool REC>
@@ -172,6 +178,9 @@ __global__ void __launch_bounds__(kBlock) k_grad_ip(DevMesh m, const double* __r
   if constexpr (REC) {
 #pragma unroll
     for (int k = 0; k < 3 * D; ++k) j[k] = __ldcs(geo + (size_t)k * m.T + e);
+    if (D == 3)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) j[ElemRec<D>::kPlanes - 3 + k] = __ldcs(geo + (size_t)(11 + k) * m.T + e);
   } else {
     elem_record_of<D>(m, id, j);
   }
@@ -197,9 +206,7 @@ __global__ void __launch_bounds__(kBlock) k_grad_ip(DevMesh m, const double* __r
       break;
     }
     if (D == 2 && r == 2) asm volatile("");  // a branch, not selects
-    double g0 = -j[D * r];
-#pragma unroll
-    for (int k = 1; k < D; ++k) g0 -= j[D * r + k];
+    const double g0 = D == 3 ? j[ElemRec<D>::kPlanes - 3 + r] : -j[D * r] - j[D * r + 1];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       double g = g0 * u[0][c];
@@ -219,7 +226,7 @@ __global__ void __launch_bounds__(kBlock) k_grad_ip(DevMesh m, const double* __r
 // power alone (mode 1).  The two integrals are summed per thread over a fixed
 // grid, then per block in a fixed order; with `done` (zero between launches)
 // the last block also reduces the blocks' partials and computes the size
-// factor.  FP64-rate bound: about 36 operations a tet, 0.37 ms at 5.3M tets
+// factor.  FP64-rate bound: about 34 operations a tet, 0.34 ms at 5.3M tets
 // (2.36 ms with pow, the Jacobian and one tree reduction per 256 elements).
 template <int D, int NC, bool REC>
 __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __restrict__ geo,
@@ -266,8 +273,8 @@ __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, const double* __res
       vv = fma(v2, v2, vv);
       dd = fma(dv, dv, dd);
     }
-    self_sum += vv * w * dV;
-    const double er = dd * w * dV;
+    const double wdv = w * dV, er = dd * wdv;
+    self_sum = fma(vv, wdv, self_sum);
     err[e] = er;
     double q, g;
     error_powers<D>(er, q, g);
@@ -348,23 +355,23 @@ __global__ void __launch_bounds__(kBlock) k_measure_iso(DevMesh m, const double*
   L[e] = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), __ldg(size + v.x), __ldg(size + v.y));
 }
 
-// per mesh: the edges' Euclidean lengths
+// per mesh: half the edges' Euclidean lengths
 __global__ void __launch_bounds__(kBlock) k_edge_records(DevMesh m, double* __restrict__ len) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.E) return;
   const int2 v = __ldg(reinterpret_cast<const int2*>(m.edv) + e);
-  len[e] = ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
+  len[e] = 0.5 * ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
 }
 
 // The pass's lengths and marks.  The sizes it computed are good to about
 // 1e-10 of the reference's, so the lengths need no particular rounding:
-// |d| / 2 (1 / h0 + 1 / h1) = |d| (h0 + h1) / (2 h0 h1), about 20 FP64
-// operations with the per-mesh edge lengths against 55.  Lengths within 1e-6
+// |d| / 2 (1 / h0 + 1 / h1) = (|d| / 2) (h0 + h1) / (h0 h1), about 17 FP64
+// operations with the per-mesh half lengths against 55.  Lengths within 1e-6
 // of 0.5 or 1.5, and those iso_length hands to the reference's sequence, take
 // iso_length, so every mark is that of the bitwise length.  The comparisons
 // and windows are integer ones on the bits (FP64 comparisons use the FP64
 // pipe).  96^3 box, 6.3M edges: 0.99 ms for the reference's sequence plus
-// 0.03 ms for marking from the stored lengths, 0.24 ms here.
+// 0.03 ms for marking from the stored lengths, 0.18 ms here.
 template <bool REC>
 __global__ void __launch_bounds__(kBlock) k_measure_mark(DevMesh m, const double* __restrict__ len,
                                                          const double* __restrict__ size, double* __restrict__ L,
@@ -378,19 +385,23 @@ __global__ void __launch_bounds__(kBlock) k_measure_mark(DevMesh m, const double
     const double sa = __ldg(size + v.x), sb = __ldg(size + v.y);
     double d;
     if constexpr (REC) d = __ldcs(len + e);
-    else d = ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
-    double h[2];
-    gauss_sizes(sa, sb, h);
-    double l = 0.5 * ((d * (h[0] + h[1])) / (h[0] * h[1]));
-    const int e0 = __double2hiint(h[0]) >> 20, e1 = __double2hiint(h[1]) >> 20, hl = __double2hiint(l);
+    else d = 0.5 * ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
+    const double N0 = (1.0 - 0.577350269189626) / 2.0, N1 = (1.0 + 0.577350269189626) / 2.0;
+    const double h0 = fma(sa, N0, sb * N1), h1 = fma(sa, N1, sb * N0);
+    double l = (d * (h0 + h1)) / (h0 * h1);
+    const int e0 = __double2hiint(h0) >> 20, e1 = __double2hiint(h1) >> 20, hl = __double2hiint(l);
     // hl >> 20 is the biased exponent of a positive length, negative for a
     // negative one; 0x3ff80000 is 1.5's high word, 0x3fe00000 0.5's
     if (min(min(e0, e1), hl >> 20) < 623 || max(max(e0, e1), hl >> 20) > 1423 ||
-        (unsigned)(hl - 0x3ff7ffff) < 2u || (unsigned)(hl - 0x3fdfffff) < 2u)
+        (unsigned)(hl - 0x3ff7ffff) < 2u || (unsigned)(hl - 0x3fdfffff) < 2u) {
       l = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), sa, sb);
+      sp = l > 1.5;
+      co = l < .5;
+    } else {
+      sp = hl > 0x3ff80000;
+      co = hl < 0x3fdfffff;
+    }
     L[e] = l;
-    sp = l > 1.5;
-    co = l < .5;
   }
   const unsigned bs = __ballot_sync(0xffffffffu, sp), bc = __ballot_sync(0xffffffffu, co);
   if ((threadIdx.x & 31) == 0 && e < m.E) {

@@ -128,7 +128,8 @@ struct ExpandList {
 
 // ---- FP64 element kernels (sprg_elem_f64.cu) --------------------------
 // per-mesh element records: elem_record_planes(dim) planes of T doubles
-// (J^-1 row-major, D columns a row; det J; the longest edge)
+// (J^-1 row-major, D columns a row; det J; the longest edge; tets: the first
+// vertex's shape gradient)
 int elem_record_planes(int dim);
 void launch_elem_records(const DevMesh& m, double* geo, cudaStream_t s);
 // geo: the records, or null to compute them in place
