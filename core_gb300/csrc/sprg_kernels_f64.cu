@@ -1,13 +1,15 @@
 // FP64 ("parity") kernels of the estimate-and-mark pass.
 //
 // Compiled with -fmad=false: element and edge arithmetic follows the
-// reference's operation order (sprg_refmath.cuh), so gradients, element
-// errors, sizes, lengths and qualities round like PUMI's apf/spr/ma code.
-// Two places differ by design and are stated in the parity tests: the
-// patch QR uses warp-tree reductions and applies the reflectors to the
-// right-hand side instead of forming Q (mth/mthQR.cc builds an explicit
-// m x m Q), and the two global integrals are summed by a fixed tree instead
-// of sequentially.  Both move results by a few ulps only.
+// reference's operation order (sprg_refmath.cuh), so the calls' gradients,
+// element errors, lengths and qualities round like PUMI's apf/spr/ma code.
+// What differs by design is stated in the parity tests: the recovery of tets
+// (and of triangles in the anisotropic pass) is a weighted sum with per-mesh
+// weights from the reference's QR instead of the QR applied to the samples
+// (mth/mthQR.cc builds an explicit m x m Q), the powers of the errors come from
+// a root iteration, the global integrals are summed in a fixed order of
+// their own, and the passes' lengths and qualities, away from the thresholds,
+// take fewer operations.  All move results by a few ulps only.
 #include <cub/cub.cuh>
 #include <cstring>
 
