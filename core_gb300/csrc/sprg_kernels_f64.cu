@@ -11,6 +11,7 @@
 // their own, and the passes' lengths and qualities, away from the thresholds,
 // take fewer operations.  All move results by a few ulps only.
 #include <cub/cub.cuh>
+#include <algorithm>
 #include <cstring>
 
 #include "sprg_internal.h"
@@ -2742,12 +2743,13 @@ void launch_guard_stage(int stage, const DevMesh& m, const double* u, const doub
   // commonly a few per thousand), up to four and eight per SM: on a small mesh
   // a full grid of idle blocks waiting for the kernel before took the slots of
   // other streams' passes.
-  if (stage == 0)
-    launch_after(m.early, k_guard_fit, std::min(152 * 8, nblk(m.V, 32)), 256, s, m, u, g.fit_items, g.fit_count, g.fit_cap,
-                 g);
-  else
-    launch_after(m.early, k_guard_decide, std::min(152 * 4, nblk(m.E, 32)), 128, s, m, u, out3, g, items, count, cap, split,
-                 collapse, unresolved, bv);
+  if (stage == 0) {
+    const int grid = std::max(1, std::min(152 * 8, nblk(m.V, 32)));
+    launch_after(m.early, k_guard_fit, grid, 256, s, m, u, g.fit_items, g.fit_count, g.fit_cap, g);
+  } else {
+    const int grid = std::max(1, std::min(152 * 4, nblk(m.E, 32)));
+    launch_after(m.early, k_guard_decide, grid, 128, s, m, u, out3, g, items, count, cap, split, collapse, unresolved, bv);
+  }
 }
 
 void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double hmin, double hmax, double* sizes,
