@@ -134,7 +134,9 @@ struct sprg_ctx {
   int use_mlp = 1;
   float z_max = 8.f;
   int stall_polls = 0;      // test hook: network-kernel wait on a barrier nothing completes (0: off)
-  int alloc_fail_in = -1;   // test hook: device allocations left before one fails (-1: off)
+  // test hooks: device allocations left before one fails (-1: off), and how
+  // many attempts fail from there on (-1: all)
+  int alloc_fail_in = -1, alloc_fail_n = -1;
   // copy stream of the host entry point: the flags upload and (FP32) the size
   // download run beside the pass
   cudaStream_t copy = nullptr;
@@ -206,27 +208,35 @@ void release(DevBuf& b) {
   b.bytes = 0;
 }
 
+// one attempt at device memory; the test hooks' failures are made here, on the
+// host, and look like cudaMalloc's own
+cudaError_t device_alloc(sprg_ctx* c, void** p, size_t bytes) {
+  *p = nullptr;
+  if (c->alloc_fail_in == 0) {
+    if (c->alloc_fail_n > 0 && --c->alloc_fail_n == 0) c->alloc_fail_in = -1;
+    return cudaErrorMemoryAllocation;
+  }
+  if (c->alloc_fail_in > 0) --c->alloc_fail_in;
+  return cudaMalloc(p, bytes);
+}
+
 // grow-only device buffer
 int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (b.bytes >= bytes) return SPRG_OK;
-  if (c->alloc_fail_in == 0) return fail(c, SPRG_ENOMEM, "device allocation failed (injected)");
-  if (c->alloc_fail_in > 0) --c->alloc_fail_in;
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.bytes = 0;
-  cudaError_t e = cudaMalloc(&b.p, bytes);
-  if (e == cudaErrorMemoryAllocation) {
+  release(b);
+  cudaError_t e = device_alloc(c, &b.p, bytes);
+  if (e == cudaErrorMemoryAllocation && !c->updating) {
     // the spare mesh arrays are only kept while there is room for them
     bool freed = false;
-    for (DevBuf* sp : {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage})
-      if (sp != &b && sp->p && !c->updating) {
+    for (DevBuf* sp : {&c->sxyz, &c->sev, &c->sedv, &c->ustage})
+      if (sp->p) {
         release(*sp);
         freed = true;
       }
     if (freed) {
       cudaGetLastError();
-      e = cudaMalloc(&b.p, bytes);
+      e = device_alloc(c, &b.p, bytes);
     }
   }
   if (e != cudaSuccess) {
@@ -2369,7 +2379,8 @@ int sprg_set_mlp_params(sprg_ctx* c, const float* params, int n_params) {
 int sprg_test_hooks(sprg_ctx* c, int wait_polls, int alloc_fail_after) {
   if (!c || wait_polls < 0 || alloc_fail_after < -1) return SPRG_EINVAL;
   c->stall_polls = wait_polls;
-  c->alloc_fail_in = alloc_fail_after;
+  c->alloc_fail_in = alloc_fail_after < 0 ? -1 : alloc_fail_after & 0xffffff;
+  c->alloc_fail_n = alloc_fail_after >> 24 > 0 ? alloc_fail_after >> 24 : -1;
   drop_e2e_graph(c);
   return SPRG_OK;
 }

@@ -364,7 +364,10 @@ const char* sprg_e2e_timing_report(sprg_ctx* ctx);
    that bounded wait runs out and the pass returns SPRG_ECUDA ("a tensor-core
    wait ran out of time") after the kernel has drained the matrix multiplies
    in flight and freed its tensor memory; the context stays usable.  alloc_fail_after >= 0 makes the context's device
-   allocation after that many more succeed fail with SPRG_ENOMEM (-1: off). */
+   allocation after that many more succeed fail with SPRG_ENOMEM (-1: off):
+   every one from there on, or, with a count in bits 24 to 30, that many
+   attempts (a call that gives back what it can spare and tries again makes a
+   second attempt). */
 int sprg_test_hooks(sprg_ctx* ctx, int wait_polls, int alloc_fail_after);
 
 /* ---- size field without device allocation ------------------------------- */
