@@ -220,11 +220,20 @@ cudaError_t device_alloc(sprg_ctx* c, void** p, size_t bytes) {
   return cudaMalloc(p, bytes);
 }
 
-// grow-only device buffer
+// a buffer that goes takes the result it held along
+void discard(sprg_ctx* c, DevBuf& b) {
+  if (&b == &c->ip) c->ip_valid = false;
+  if (&b == &c->size) c->size_valid = false;
+  if (&b == &c->L) c->L_valid = false;
+  if (&b == &c->q) c->q_valid = false;
+  release(b);
+}
+
+// grow-only device buffer (its contents are not kept)
 int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (b.bytes >= bytes) return SPRG_OK;
-  release(b);
+  discard(c, b);
   cudaError_t e = device_alloc(c, &b.p, bytes);
   if (e == cudaErrorMemoryAllocation && !c->updating) {
     // the spare mesh arrays are only kept while there is room for them

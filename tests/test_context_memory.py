@@ -42,3 +42,24 @@ def test_spare_arrays_given_back(gpu_lib, precision):
             fail(c, k)
             assert same(c.estimate_and_mark(u1, 0.1)[:4], want), k
             assert same(c.estimate_and_mark(u1, 0.1)[:4], want), k
+
+
+def test_results_go_with_their_buffers(gpu_lib):
+    """A scalar field's gradients are resident; the vector field's do not fit, and
+    the smaller buffer is gone: no resident field any more, then a new one."""
+    import core_gb300 as cg
+    from core_gb300 import _lib
+    m, u = box(4)
+    v = np.stack([u, u * u, 1 - u], 1)
+    out = np.empty((m.n_verts, 3))
+    with cg.Context(m) as c:
+        ip = c.getGradIPField(u)
+        want = c.recoverField(ip)
+        fail(c, 1)  # f grows, then ip
+        with pytest.raises(cg.SprgError) as e:
+            c.getGradIPField(v)
+        assert e.value.code == _lib.SPRG_ENOMEM
+        assert gpu_lib.sprg_recover_field(c.h, None, 3, out.ctypes.data) == _lib.SPRG_ESTATE
+        assert np.array_equal(c.getGradIPField(u), ip)
+        assert gpu_lib.sprg_recover_field(c.h, None, 3, out.ctypes.data) == _lib.SPRG_OK
+        assert np.array_equal(out, want)
