@@ -57,6 +57,10 @@ struct sprg_ctx {
   // the next one builds (given back when an allocation fails), and its staging
   DevBuf sxyz, sev, sedv, ustage, ubad;
   bool updating = false;  // an update is filling the spare arrays
+  // the end of the last update's work, for a stream set afterwards, and
+  // whether an earlier stream may still hold work of this context
+  cudaEvent_t updated = nullptr;
+  bool update_pending = false, switched = false;
   // fields
   DevBuf f, ip, rec, err, esize, size, L, flags, q, sizes3, frames9;
   int ip_nc = 0;
@@ -914,7 +918,12 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   int rc = set_device(c);
   if (rc) return rc;
   c->launches = 0;
-  CK(cudaStreamSynchronize(c->stream));
+  if (!c->updated) CK(cudaEventCreateWithFlags(&c->updated, cudaEventDisableTiming));
+  // passes on this mesh are done before its arrays change, on whatever stream
+  // they run (an earlier stream's handle may be gone, so the device is asked)
+  if (c->switched) CK(cudaDeviceSynchronize());
+  else CK(cudaStreamSynchronize(c->stream));
+  c->switched = false;
   // ---- the new arrays, in the spare buffers: kept rows copied, listed rows
   // scattered from one staging buffer (each kind its own part, so that
   // nothing waits in between)
@@ -1034,8 +1043,15 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   m.p_off = P<int>(c->poff);
   m.p_el = P<int>(c->pel);
   c->launches += 5;
-  if ((rc = check_launch(c, "mesh update"))) return rc;
-  if (d->vert_elem_offsets) CK(cudaStreamSynchronize(c->stream));  // the caller's CSR is read
+  c->update_pending = false;
+  rc = check_launch(c, "mesh update");
+  if (d->vert_elem_offsets || rc) {
+    CK(cudaStreamSynchronize(c->stream));  // the caller's CSR is read
+    return rc;
+  }
+  // the adjacency is still being built: sprg_set_stream orders a new stream behind it
+  CK(cudaEventRecord(c->updated, c->stream));
+  c->update_pending = true;
   return SPRG_OK;
 }
 
@@ -1067,6 +1083,7 @@ int sprg_destroy(sprg_ctx* c) {
   for (auto& e : c->e2e_ev)
     if (e) cudaEventDestroy(e);
   if (c->stage) cudaFreeHost(c->stage);
+  if (c->updated) cudaEventDestroy(c->updated);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->e2e_exec) cudaGraphExecDestroy(c->e2e_exec);
   if (c->own) cudaStreamDestroy(c->own);
@@ -1089,7 +1106,18 @@ int sprg_set_precision(sprg_ctx* c, int precision) {
 
 int sprg_set_stream(sprg_ctx* c, void* stream) {
   if (!c) return SPRG_EINVAL;
-  c->stream = stream ? static_cast<cudaStream_t>(stream) : c->own;
+  const cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->own;
+  if (s != c->stream && c->update_pending) {
+    int rc = set_device(c);
+    if (rc) return rc;
+    // a stream that is being captured cannot wait on work outside the capture
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamWaitEvent(s, c->updated, 0));
+    else CK(cudaEventSynchronize(c->updated));
+  }
+  if (s != c->stream) c->switched = true;
+  c->stream = s;
   drop_e2e_graph(c);
   return SPRG_OK;
 }

@@ -110,7 +110,8 @@ int sprg_destroy(sprg_ctx* ctx);
 const char* sprg_last_error(const sprg_ctx* ctx);
 /* SPRG_FP64 (default), SPRG_FP32 or SPRG_LEARNED. */
 int sprg_set_precision(sprg_ctx* ctx, int precision);
-/* Run on this CUDA stream (cudaStream_t, NULL = the context's own). */
+/* Run on this CUDA stream (cudaStream_t, NULL = the context's own).  A mesh
+   update may still run on the stream before it: the new one waits for that. */
 int sprg_set_stream(sprg_ctx* ctx, void* stream);
 
 /* ---- spr ------------------------------------------------------------- */
