@@ -52,7 +52,7 @@ struct sprg_ctx {
   int precision = SPRG_FP64;
   DevMesh m{};
   // mesh
-  DevBuf xyz, xyzq, ev, edv, poff, pel, aoff, ael, tmp;
+  DevBuf xyz, xyzq, ev, edv, poff, pel, aoff, ael, tmp, vscan;
   // sprg_update_mesh: the arrays of the mesh before the last update, into which
   // the next one builds (given back when an allocation fails), and its staging
   DevBuf sxyz, sev, sedv, ustage, ubad;
@@ -793,6 +793,7 @@ int sprg_create(const sprg_mesh_view* mv, int device, sprg_ctx** out) {
   ENSUREC(c->poff, sizeof(int) * ((size_t)m.V + 1));
   ENSUREC(c->pel, sizeof(int) * nel);
   ENSUREC(c->tmp, sizeof(int) * (size_t)m.V);
+  ENSUREC(c->vscan, offset_scan_bytes(m.V));
   ENSUREC(c->status, sizeof(DevStatus));
   ENSUREC(c->count, sizeof(unsigned long long));
   CKC(cudaMemsetAsync(c->status.p, 0, sizeof(DevStatus), c->stream));
@@ -828,7 +829,7 @@ int sprg_create(const sprg_mesh_view* mv, int device, sprg_ctx** out) {
     m.a_off = P<int>(c->aoff);
     m.a_el = P<int>(c->ael);
   } else {
-    launch_build_v2e(m, P<int>(c->poff), P<int>(c->pel), P<int>(c->tmp), c->stream);
+    CKC(launch_build_v2e(m, P<int>(c->poff), P<int>(c->pel), P<int>(c->tmp), c->vscan.p, c->vscan.bytes, c->stream));
     launch_sort_segments(m.V, P<int>(c->poff), P<int>(c->pel), c->stream);
     m.a_off = P<int>(c->poff);
     m.a_el = P<int>(c->pel);
@@ -989,6 +990,7 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   grow.push_back({c->poff, sizeof(int) * ((size_t)V1 + 1), {}});
   grow.push_back({c->pel, sizeof(int) * nel, {}});
   grow.push_back({c->tmp, sizeof(int) * (size_t)V1, {}});
+  grow.push_back({c->vscan, offset_scan_bytes((int)V1), {}});
   if (d->vert_elem_offsets) {
     grow.push_back({c->aoff, sizeof(int) * ((size_t)V1 + 1), {}});
     grow.push_back({c->ael, sizeof(int) * nel, {}});
@@ -1035,7 +1037,7 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
     m.a_off = P<int>(c->aoff);
     m.a_el = P<int>(c->ael);
   } else {
-    launch_build_v2e(m, P<int>(c->poff), P<int>(c->pel), P<int>(c->tmp), c->stream);
+    CK(launch_build_v2e(m, P<int>(c->poff), P<int>(c->pel), P<int>(c->tmp), c->vscan.p, c->vscan.bytes, c->stream));
     launch_sort_segments(m.V, P<int>(c->poff), P<int>(c->pel), c->stream);
     m.a_off = P<int>(c->poff);
     m.a_el = P<int>(c->pel);
@@ -1060,7 +1062,7 @@ int sprg_destroy(sprg_ctx* c) {
   cudaSetDevice(c->device);
   if (c->own) cudaStreamSynchronize(c->own);
   DevBuf* bufs[] = {&c->umaxp, &c->sxyz, &c->sev, &c->sedv, &c->ustage, &c->ubad, &c->vxf, &c->vbad, &c->tqc, &c->trr, &c->tcode, &c->txcount, &c->egeo, &c->elen64, &c->soff, &c->sel, &c->sw, &c->qmax, &c->bcnt, &c->cent, &c->xyz,   &c->xyzq,   &c->ev,   &c->edv,   &c->poff,    &c->pel,    &c->aoff,
-                    &c->ael,   &c->tmp,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
+                    &c->ael,   &c->tmp, &c->vscan,     &c->f,    &c->ip,    &c->rec,     &c->err,    &c->esize,
                     &c->size,  &c->L,       &c->flags, &c->q,    &c->sizes3,  &c->frames9, &c->partials,
                     &c->out3,  &c->status,  &c->count, &c->mcount, &c->xitems, &c->xcount, &c->slab, &c->bits, &c->titems, &c->tcountb, &c->Lx, &c->pairs, &c->red, &c->eflags, &c->logm, &c->qw, &c->qwlisted, &c->qwitems, &c->qwcount, &c->rw, &c->rwlisted, &c->rwitems, &c->rwcount, &c->cache2r.v, &c->cache2r.n, &c->cache2r.el, &c->cache2r.woff, &c->cache2r.w, &c->cache2r.wn, &c->tw, &c->twlisted, &c->twitems, &c->twcount, &c->met32, &c->qrec32, &c->cj64, &c->qties, &c->kidx, &c->kval, &c->klen, &c->rec9, &c->cache2d.v, &c->cache2d.n, &c->cache2d.el, &c->cache2d.woff, &c->cache2d.w, &c->cache2d.wn, &c->agitems, &c->agcount,
                     &c->crec,  &c->vrec,    &c->rec32, &c->q32, &c->sz2,  &c->fcnt,   &c->guard, &c->tetd,
@@ -1954,8 +1956,8 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
     ENSURE(c->vv, sizeof(int) * 2 * (size_t)m.E);
     ENSURE(c->tmp, sizeof(int) * (size_t)m.V);
     ENSURE(c->vtile, ((size_t)m.V + 127) / 128);
-    learned_build_v2v(m, P<int>(c->vvoff), P<int>(c->vv), P<int>(c->tmp), P<unsigned char>(c->vtile),
-                      P<int>(c->fcnt) + 6, c->stream);
+    CK(learned_build_v2v(m, P<int>(c->vvoff), P<int>(c->vv), P<int>(c->tmp), P<unsigned char>(c->vtile),
+                         P<int>(c->fcnt) + 6, c->vscan.p, c->vscan.bytes, c->stream));
     CK(cudaMemcpyAsync(&c->max_degree, P<int>(c->fcnt) + 6, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaMemsetAsync(c->mlp_err.p, 0, sizeof(int), c->stream));
@@ -2448,8 +2450,8 @@ int sprg_learned_features(sprg_ctx* c, const double* d_u, uint16_t* d_x, float* 
     ENSURE(c->tmp, sizeof(int) * (size_t)m.V);
     ENSURE(c->mlp_err, sizeof(int));
     ENSURE(c->vtile, ((size_t)m.V + 127) / 128);
-    learned_build_v2v(m, P<int>(c->vvoff), P<int>(c->vv), P<int>(c->tmp), P<unsigned char>(c->vtile),
-                      P<int>(c->fcnt) + 6, c->stream);
+    CK(learned_build_v2v(m, P<int>(c->vvoff), P<int>(c->vv), P<int>(c->tmp), P<unsigned char>(c->vtile),
+                         P<int>(c->fcnt) + 6, c->vscan.p, c->vscan.bytes, c->stream));
     CK(cudaMemcpyAsync(&c->max_degree, P<int>(c->fcnt) + 6, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaMemsetAsync(c->mlp_err.p, 0, sizeof(int), c->stream));

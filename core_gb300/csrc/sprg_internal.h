@@ -328,8 +328,14 @@ void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double
 
 // ---- adjacency builders (sprg_kernels_f64.cu) ---------------------------
 // Ascending vertex->element CSR via counting sort on the device.
-// off must hold V + 1 ints, el T * nn ints, tmp V ints.
-void launch_build_v2e(const DevMesh& m, int* off, int* el, int* tmp, cudaStream_t s);
+// off must hold V + 1 ints, el T * nn ints, tmp V ints, scan
+// offset_scan_bytes(V) (taken before a mesh is given up: the offsets are
+// built by the scan, and counts left in their place would be read as offsets).
+cudaError_t launch_build_v2e(const DevMesh& m, int* off, int* el, int* tmp, void* scan, size_t scan_bytes,
+                             cudaStream_t s);
+// V counts and a zero -> V + 1 offsets, in place
+size_t offset_scan_bytes(int V);
+cudaError_t launch_offset_scan(int V, int* off, void* scan, size_t scan_bytes, cudaStream_t s);
 // Sort each CSR segment ascending (segments are short).
 void launch_sort_segments(int V, const int* off, int* el, cudaStream_t s);
 // X = rint((x - c) s 2^30) per coordinate (c the frame's corner, s its scale)

@@ -2757,18 +2757,27 @@ void launch_hessian_metric(const DevMesh& m, const double* H, double eps, double
   if (m.V) k_hessian_metric<<<nblk(m.V), kBlock, 0, s>>>(m.V, m.dim, H, eps, hmin, hmax, sizes, frames);
 }
 
-void launch_build_v2e(const DevMesh& m, int* off, int* el, int* tmp, cudaStream_t s) {
+size_t offset_scan_bytes(int V) {
+  size_t bytes = 0;
+  int* off = nullptr;
+  cub::DeviceScan::ExclusiveSum(nullptr, bytes, off, off, V + 1);
+  return bytes;
+}
+
+cudaError_t launch_offset_scan(int V, int* off, void* scan, size_t scan_bytes, cudaStream_t s) {
+  return cub::DeviceScan::ExclusiveSum(scan, scan_bytes, off, off, V + 1, s);
+}
+
+cudaError_t launch_build_v2e(const DevMesh& m, int* off, int* el, int* tmp, void* scan, size_t scan_bytes,
+                             cudaStream_t s) {
   cudaMemsetAsync(tmp, 0, sizeof(int) * (size_t)m.V, s);
   cudaMemsetAsync(off, 0, sizeof(int) * ((size_t)m.V + 1), s);
   if (m.T) k_count_v2e<<<nblk(m.T), kBlock, 0, s>>>(m, off);
   // exclusive scan of the V+1 counts (last is 0) -> offsets
-  size_t bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes, off, off, m.V + 1, s);
-  void* scratch = nullptr;
-  cudaMallocAsync(&scratch, bytes, s);
-  cub::DeviceScan::ExclusiveSum(scratch, bytes, off, off, m.V + 1, s);
-  cudaFreeAsync(scratch, s);
+  const cudaError_t e = launch_offset_scan(m.V, off, scan, scan_bytes, s);
+  if (e != cudaSuccess) return e;  // counts are no offsets: nothing is filled
   if (m.T) k_fill_v2e<<<nblk(m.T), kBlock, 0, s>>>(m, off, tmp, el);
+  return cudaSuccess;
 }
 
 void launch_sort_segments(int V, const int* off, int* el, cudaStream_t s) {

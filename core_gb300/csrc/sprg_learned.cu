@@ -22,7 +22,6 @@
 // where they are needed, and no per-element gradient array is stored.
 #include <algorithm>
 #include <cuda_bf16.h>
-#include <cub/cub.cuh>
 
 #include "sprg_ld.cuh"
 #include "sprg_listed.cuh"
@@ -1318,21 +1317,18 @@ constexpr int kLErrorGrid = 152 * 8;
 
 }  // namespace
 
-void learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned char* tile_half, int* max_deg,
-                       cudaStream_t s) {
+cudaError_t learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned char* tile_half, int* max_deg,
+                              void* scan, size_t scan_bytes, cudaStream_t s) {
   cudaMemsetAsync(off, 0, sizeof(int) * ((size_t)m.V + 1), s);
   cudaMemsetAsync(tmp, 0, sizeof(int) * (size_t)m.V, s);
   if (m.E) k_v2v_count<<<nblk(m.E), kBlock, 0, s>>>(m.E, m.edv, off);
-  size_t bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes, off, off, m.V + 1, s);
-  void* scratch = nullptr;
-  cudaMallocAsync(&scratch, bytes, s);
-  cub::DeviceScan::ExclusiveSum(scratch, bytes, off, off, m.V + 1, s);
-  cudaFreeAsync(scratch, s);
+  const cudaError_t e = launch_offset_scan(m.V, off, scan, scan_bytes, s);
+  if (e != cudaSuccess) return e;  // counts are no offsets: nothing is filled
   if (m.E) k_v2v_fill<<<nblk(m.E), kBlock, 0, s>>>(m.E, m.edv, off, tmp, nb);
   if (m.V) k_v2v_sort<<<nblk(m.V), kBlock, 0, s>>>(m.V, off, nb);
   cudaMemsetAsync(max_deg, 0, sizeof(int), s);
   if (m.V) k_tile_half<<<(m.V + 127) / 128, 128, 0, s>>>(m.V, off, tile_half, max_deg);
+  return cudaSuccess;
 }
 
 size_t learned_range_bytes() { return sizeof(double) * (3 * kRangeGrid + 2); }

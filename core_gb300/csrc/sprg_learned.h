@@ -34,10 +34,11 @@ struct LearnMesh {
   const unsigned char* tile_half;   // per 128-vertex tile: all degrees <= 16
 };
 
-// vertex -> vertex CSR from the edge list (off: V + 1, nb: 2E, tmp: V ints),
-// the per-tile degree flags (ceil(V / 128) bytes) and the largest degree
-void learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned char* tile_half, int* max_deg,
-                       cudaStream_t s);
+// vertex -> vertex CSR from the edge list (off: V + 1, nb: 2E, tmp: V ints;
+// scan: offset_scan_bytes(V)), the per-tile degree flags (ceil(V / 128) bytes)
+// and the largest degree
+cudaError_t learned_build_v2v(const DevMesh& m, int* off, int* nb, int* tmp, unsigned char* tile_half, int* max_deg,
+                              void* scan, size_t scan_bytes, cudaStream_t s);
 // device words the pass's first kernel clears for the kernels after it
 struct LearnCounters {
   static constexpr int kCount = 4;

@@ -63,3 +63,35 @@ def test_results_go_with_their_buffers(gpu_lib):
         assert np.array_equal(c.getGradIPField(u), ip)
         assert gpu_lib.sprg_recover_field(c.h, None, 3, out.ctypes.data) == _lib.SPRG_OK
         assert np.array_equal(out, want)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "learned"])
+@pytest.mark.parametrize("csr", [False, True])
+def test_update_fails_before_the_old_mesh_goes(gpu_lib, oracle_lib, precision, csr):
+    """Whichever of an update's allocations fails, the scan of its offsets
+    included, the context still holds the old mesh; the next update holds."""
+    import core_gb300 as cg
+    (m0, u0), (m1, u1) = box(5), box(7, 2)
+    if csr:
+        o = oracle_lib.OracleMesh.box(7, 7, 7)
+        m1.v2e_off, m1.v2e = o.v2e_off, o.v2e
+    want = [fresh(m, u, precision) for m, u in ((m0, u0), (m1, u1))]
+    failed = 0
+    for k in range(32):
+        with cg.Context(m0, precision=precision) as c:
+            c.estimate_and_mark(u0, 0.1)
+            fail(c, k, 100)
+            try:
+                c.update_mesh(m1)
+            except cg.SprgError as e:
+                assert e.code == 4
+                failed += 1
+                c.test_hooks()
+                assert same(c.estimate_and_mark(u0, 0.1)[:4], want[0]), k
+                c.update_mesh(m1)
+            c.test_hooks()
+            assert same(c.estimate_and_mark(u1, 0.1)[:4], want[1]), k
+    # three arrays, staging, the out-of-range count, the box keys, and what
+    # derives from the arrays: fixed-point coordinates, offsets, elements,
+    # counters, the scan (as large as the old mesh's here) and the caller's order
+    assert failed >= (12 if csr else 10)
