@@ -119,11 +119,22 @@ struct sprg_ctx {
   int tile_mode = -1;  // the lane mode every tile shares, or -1
   std::string tune_json;
   // CUDA graph of the resident pass (sprg_graph_capture / sprg_graph_replay)
+  // and what it was captured with; stale: one of the context's buffers has
+  // moved since, the next replay runs the pass and captures it again
   cudaGraphExec_t graph_exec = nullptr;
+  struct CapturedPass {
+    const double* u = nullptr;
+    double ratio = 0;
+    uint32_t *split = nullptr, *collapse = nullptr;
+    int precision = SPRG_FP64, use_mlp = 1, batch_n = 0, batch_nseg = 0;
+    float z_max = 8.f;
+  } graph_of;
+  bool graph_stale = false;
   // the host entry point's own graph of the resident pass: captured on the
   // third call in a row with the same adapt ratio, form, stream and size
   // download (per-mesh setup is done by then), replayed after that; any
-  // setter or mesh change drops it, a failed capture turns it off
+  // setter or mesh change, or a buffer that moves, drops it, a failed capture
+  // turns it off
   cudaGraphExec_t e2e_exec = nullptr;
   int e2e_calls = 0;
   int64_t e2e_launches = 0;
@@ -224,8 +235,24 @@ cudaError_t device_alloc(sprg_ctx* c, void** p, size_t bytes) {
   return cudaMalloc(p, bytes);
 }
 
-// a buffer that goes takes the result it held along
+void drop_e2e_graph(sprg_ctx* c) {
+  if (c->e2e_exec) cudaGraphExecDestroy(c->e2e_exec);
+  c->e2e_exec = nullptr;
+  c->e2e_calls = 0;
+}
+
+// the captured passes hold the addresses of the context's buffers
+void graphs_stale(sprg_ctx* c) {
+  drop_e2e_graph(c);
+  if (!c->graph_exec) return;
+  cudaGraphExecDestroy(c->graph_exec);
+  c->graph_exec = nullptr;
+  c->graph_stale = true;
+}
+
+// a buffer that goes takes the result it held along, and the graphs
 void discard(sprg_ctx* c, DevBuf& b) {
+  if (b.p) graphs_stale(c);
   if (&b == &c->ip) c->ip_valid = false;
   if (&b == &c->size) c->size_valid = false;
   if (&b == &c->L) c->L_valid = false;
@@ -853,12 +880,6 @@ int sprg_create(const sprg_mesh_view* mv, int device, sprg_ctx** out) {
 }
 
 // every per-mesh result, cache and derived structure, after the mesh changed
-static void drop_e2e_graph(sprg_ctx* c) {
-  if (c->e2e_exec) cudaGraphExecDestroy(c->e2e_exec);
-  c->e2e_exec = nullptr;
-  c->e2e_calls = 0;
-}
-
 static void invalidate_mesh_state(sprg_ctx* c) {
   drop_e2e_graph(c);
   c->ip_valid = c->size_valid = c->L_valid = c->q_valid = false;
@@ -882,6 +903,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
     cudaGraphExecDestroy(c->graph_exec);
     c->graph_exec = nullptr;
   }
+  c->graph_stale = false;
 }
 
 int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
@@ -2744,16 +2766,10 @@ const char* sprg_tuning_report(sprg_ctx* c) {
   return c->tune_json.c_str();
 }
 
-int sprg_graph_capture(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split_bits,
-                       uint32_t* d_collapse_bits) {
-  if (!c || !d_u || !d_split_bits || !d_collapse_bits) return SPRG_EINVAL;
-  int rc = set_device(c);
-  if (rc) return rc;
-  if (c->stream == c->own || c->stream == nullptr)
-    return fail(c, SPRG_ESTATE, "graph capture needs a caller stream (sprg_set_stream)");
-  // one ordinary pass first: buffers, per-mesh setup, patch cache and tuning
-  if ((rc = sprg_estimate_and_mark_resident(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits))) return rc;
-  CK(cudaStreamSynchronize(c->stream));
+// the pass into graph_exec (no replay left in flight, buffers and setup made by
+// an ordinary pass)
+static int capture_pass(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split_bits,
+                        uint32_t* d_collapse_bits) {
   const bool prof = c->prof;
   c->prof = false;
   if (c->graph_exec) {
@@ -2761,7 +2777,7 @@ int sprg_graph_capture(sprg_ctx* c, const double* d_u, double adapt_ratio, uint3
     c->graph_exec = nullptr;
   }
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  rc = sprg_estimate_and_mark_resident(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits);
+  const int rc = sprg_estimate_and_mark_resident(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits);
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
   c->prof = prof;
@@ -2773,14 +2789,57 @@ int sprg_graph_capture(sprg_ctx* c, const double* d_u, double adapt_ratio, uint3
   e = cudaGraphInstantiate(&c->graph_exec, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphInstantiate");
+  c->graph_of = {d_u, adapt_ratio, d_split_bits, d_collapse_bits, c->precision, c->use_mlp, c->batch_n, c->batch_nseg,
+                 c->z_max};
+  c->graph_stale = false;
   return SPRG_OK;
+}
+
+int sprg_graph_capture(sprg_ctx* c, const double* d_u, double adapt_ratio, uint32_t* d_split_bits,
+                       uint32_t* d_collapse_bits) {
+  if (!c || !d_u || !d_split_bits || !d_collapse_bits) return SPRG_EINVAL;
+  int rc = set_device(c);
+  if (rc) return rc;
+  if (c->stream == c->own || c->stream == nullptr)
+    return fail(c, SPRG_ESTATE, "graph capture needs a caller stream (sprg_set_stream)");
+  // one ordinary pass first: buffers, per-mesh setup, patch cache and tuning
+  if ((rc = sprg_estimate_and_mark_resident(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits))) return rc;
+  CK(cudaStreamSynchronize(c->stream));
+  return capture_pass(c, d_u, adapt_ratio, d_split_bits, d_collapse_bits);
+}
+
+// A replay whose graph lost a buffer: the pass itself, with the settings it was
+// captured with, then the capture again (left for the next replay where the
+// stream cannot be captured now).
+static int replay_stale(sprg_ctx* c) {
+  const sprg_ctx::CapturedPass g = c->graph_of;
+  const sprg_ctx::CapturedPass now = {nullptr,    0,          nullptr,       nullptr, c->precision,
+                                      c->use_mlp, c->batch_n, c->batch_nseg, c->z_max};
+  auto settings = [c](const sprg_ctx::CapturedPass& s) {
+    c->precision = s.precision;
+    c->use_mlp = s.use_mlp;
+    c->batch_n = s.batch_n;
+    c->batch_nseg = s.batch_nseg;
+    c->z_max = s.z_max;
+  };
+  settings(g);
+  int rc = sprg_estimate_and_mark_resident(c, g.u, g.ratio, g.split, g.collapse);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (rc == SPRG_OK && c->stream != c->own && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess &&
+      cap == cudaStreamCaptureStatusNone) {
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    rc = e == cudaSuccess ? capture_pass(c, g.u, g.ratio, g.split, g.collapse) : cuda_fail(c, e, "graph replay");
+  }
+  settings(now);
+  return rc;
 }
 
 int sprg_graph_replay(sprg_ctx* c) {
   if (!c) return SPRG_EINVAL;
-  if (!c->graph_exec) return fail(c, SPRG_ESTATE, "no captured graph (sprg_graph_capture)");
+  if (!c->graph_exec && !c->graph_stale) return fail(c, SPRG_ESTATE, "no captured graph (sprg_graph_capture)");
   int rc = set_device(c);
   if (rc) return rc;
+  if (c->graph_stale) return replay_stale(c);
   CK(cudaGraphLaunch(c->graph_exec, c->stream));
   return SPRG_OK;
 }
