@@ -2113,6 +2113,13 @@ int sprg_rounding_dominated(sprg_ctx* c, int* out) {
   return SPRG_OK;
 }
 
+// a replayed FP64 pass leaves its gradients, sizes and lengths as a direct one does
+static void replayed(sprg_ctx* c, int precision) {
+  if (precision != SPRG_FP64) return;
+  c->ip_nc = 3;
+  c->ip_valid = c->size_valid = c->L_valid = true;
+}
+
 // the resident pass of the host entry point: direct launches for the first
 // two calls with a key, a captured graph from the third on
 static int e2e_pass(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t* d_collapse) {
@@ -2121,6 +2128,7 @@ static int e2e_pass(sprg_ctx* c, double adapt_ratio, uint32_t* d_split, uint32_t
   if (c->e2e_exec) {
     CK(cudaGraphLaunch(c->e2e_exec, c->stream));
     c->launches += c->e2e_launches;
+    replayed(c, c->precision);
     return SPRG_OK;
   }
   if (call < 2) return pass_resident(c, P<double>(c->f), adapt_ratio, d_split, d_collapse);
@@ -2841,6 +2849,7 @@ int sprg_graph_replay(sprg_ctx* c) {
   if (rc) return rc;
   if (c->graph_stale) return replay_stale(c);
   CK(cudaGraphLaunch(c->graph_exec, c->stream));
+  replayed(c, c->graph_of.precision);
   return SPRG_OK;
 }
 

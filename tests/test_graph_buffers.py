@@ -86,3 +86,37 @@ def test_user_graph_around_a_call_that_moves_buffers(gpu_lib, precision, moved_b
         c.graph_replay()
         c.getGradIPField(us[0])  # waits
         assert np.array_equal(bits.cpu().numpy().view(np.uint32), b)
+
+
+@pytest.mark.parametrize("user_graph", [False, True])
+def test_resident_gradients_after_a_replay(gpu_lib, user_graph):
+    """The resident integration-point field after a replayed pass is the pass's
+    (3 components), as after a direct one."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import _lib
+    m, us = box(5)
+    v = np.stack([np.sin(3 * m.coords[:, k]) for k in range(3)], 1)
+    stream = torch.cuda.Stream()
+    with cg.Context(m) as c:
+        c.recoverField(c.getGradIPField(v))
+        want = c.recoverField(c.getGradIPField(us[0]))
+        if user_graph:
+            c.set_stream(stream.cuda_stream)
+            d_u = torch.from_numpy(us[0]).cuda()
+            bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            c.graph_capture(d_u.data_ptr(), RATIO, bits[0].data_ptr(), bits[1].data_ptr())
+        else:
+            for _ in range(4):
+                c.estimate_and_mark(us[0], RATIO)
+        c.getGradIPField(v)
+        if user_graph:
+            c.graph_replay()
+        else:
+            c.estimate_and_mark(us[0], RATIO)
+        out = np.empty((m.n_verts, 9))
+        assert gpu_lib.sprg_recover_field(c.h, None, 9, out.ctypes.data) == _lib.SPRG_EINVAL
+        out = np.empty((m.n_verts, 3))
+        assert gpu_lib.sprg_recover_field(c.h, None, 3, out.ctypes.data) == _lib.SPRG_OK
+        assert np.array_equal(out, want)
