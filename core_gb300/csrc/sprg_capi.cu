@@ -1685,6 +1685,10 @@ static int build_tiles(sprg_ctx* c, int only = -1) {
     }
     first += c->bin_count[b];
   }
+  // a captured pass has the old list's length and lane mode, a pass in flight
+  // still reads the old list
+  if (c->e2e_exec || c->graph_exec) graphs_stale(c);
+  CK(cudaStreamSynchronize(c->stream));
   ENSURE(c->btiles, sizeof(int4) * (tiles.empty() ? 1 : tiles.size()));
   if (!tiles.empty())
     CK(cudaMemcpy(c->btiles.p, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
@@ -2728,6 +2732,16 @@ int sprg_set_batch(sprg_ctx* c, int n_meshes, const int64_t* vert_offsets, const
   }
   voff[n_meshes] = m.V;
   segoff[n_meshes] = (int)seg.size();
+  // A captured batch pass reads these arrays: it follows the new batch, captured
+  // again where the counts that its launches hold differ.
+  const bool captured = (c->graph_exec || c->graph_stale) && c->graph_of.batch_n;
+  const bool recapture = captured && (c->graph_of.batch_n != n_meshes || c->graph_of.batch_nseg != (int)seg.size());
+  CK(cudaStreamSynchronize(c->stream));  // a pass in flight
+  c->batch_n = 0;                        // none until all of it is in place
+  if (recapture) {
+    graphs_stale(c);
+    c->graph_stale = false;
+  }
   ENSURE(c->bvoff, sizeof(int) * voff.size());
   ENSURE(c->bsegoff, sizeof(int) * segoff.size());
   ENSURE(c->bseg, sizeof(int2) * seg.size());
@@ -2738,6 +2752,11 @@ int sprg_set_batch(sprg_ctx* c, int n_meshes, const int64_t* vert_offsets, const
   CK(cudaMemcpy(c->bratios.p, adapt_ratios, sizeof(double) * n_meshes, cudaMemcpyHostToDevice));
   c->batch_n = n_meshes;
   c->batch_nseg = (int)seg.size();
+  if (recapture) {
+    c->graph_of.batch_n = c->batch_n;
+    c->graph_of.batch_nseg = c->batch_nseg;
+    c->graph_stale = true;
+  }
   return SPRG_OK;
 }
 

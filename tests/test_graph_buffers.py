@@ -120,3 +120,75 @@ def test_resident_gradients_after_a_replay(gpu_lib, user_graph):
         out = np.empty((m.n_verts, 3))
         assert gpu_lib.sprg_recover_field(c.h, None, 3, out.ctypes.data) == _lib.SPRG_OK
         assert np.array_equal(out, want)
+
+
+def marks(bits, E):
+    b, e = bits.cpu().numpy().view(np.uint32), np.arange(E)
+    return np.stack([(b[k][e >> 5] >> (e & 31)) & 1 for k in range(2)])
+
+
+@pytest.mark.parametrize("first,then", [(([0, 0, 0, 0], 64, 8), ([4, 1, 2, 1], 48, 4)),
+                                        (([4, 4, 4, 4], 1024, 8), ([4, 4, 4, 4], 64, 8)),
+                                        (([1, 1, 1, 1], 64, 4), ([0, 0, 0, 0], 1024, 8))])
+def test_user_graph_after_a_tiling_change(gpu_lib, first, then):
+    """The captured recovery holds the tile list's length and lane mode."""
+    import torch
+    import core_gb300 as cg
+    m, us = box(14)
+    stream = torch.cuda.Stream()
+    with cg.Context(m, precision="fp32") as c, torch.cuda.stream(stream):
+        c.set_stream(stream.cuda_stream)
+        c.set_tiling(*first)
+        d_u = torch.from_numpy(us[0]).cuda()
+        bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        c.graph_capture(d_u.data_ptr(), RATIO, bits[0].data_ptr(), bits[1].data_ptr())
+        c.graph_replay()
+        c.set_tiling(*then)  # a replay may still be in flight
+        for u in us:
+            d_u.copy_(torch.from_numpy(u))
+            c.graph_replay()
+            stream.synchronize()
+            flags = fresh(m, u, "fp32")[1]
+            assert np.array_equal(marks(bits, m.n_edges), [flags & 1, (flags >> 2) & 1])
+        c.set_stream(0)
+
+
+def test_user_graph_follows_the_batch(gpu_lib):
+    """Other ratios for the captured batch, then another partition of the same
+    meshes into batches (two boxes each, then three), then the batch cleared:
+    the replay is the pass of the batch that was set last."""
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m, u, voff, eoff, doff, ns = workload.batch_boxes(12, seed=7, lo=4, hi=12)
+    K = len(ns)
+    sets = [(voff, eoff, np.full(K, 0.1)), (voff, eoff, np.linspace(0.05, 0.2, K)),
+            (voff[::2], eoff[::2], np.full(K // 2, 0.1)), (voff[::3], eoff[::3], np.full(K // 3, 0.07)),
+            (voff, eoff, np.full(K, 0.2))]
+    want = []
+    for s in sets:
+        with cg.Context(m, precision="fp32") as c:
+            c.set_batch(*s)
+            flags = c.estimate_and_mark(u, 1.0)[1]
+        want.append([flags & 1, (flags >> 2) & 1])
+    assert not np.array_equal(want[0], want[2])
+    stream = torch.cuda.Stream()
+    with cg.Context(m, precision="fp32") as c, torch.cuda.stream(stream):
+        c.set_stream(stream.cuda_stream)
+        d_u = torch.from_numpy(u).cuda()
+        bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        c.set_batch(*sets[0])
+        c.graph_capture(d_u.data_ptr(), 1.0, bits[0].data_ptr(), bits[1].data_ptr())
+        for s, w in zip(sets[1:], want[1:]):
+            c.set_batch(*s)
+            for _ in range(2):
+                bits.zero_()
+                c.graph_replay()
+                stream.synchronize()
+                assert np.array_equal(marks(bits, m.n_edges), w)
+        c.set_batch([], [], [])
+        bits.zero_()
+        c.graph_replay()
+        stream.synchronize()
+        assert np.array_equal(marks(bits, m.n_edges), want[-1])
+        c.set_stream(0)
