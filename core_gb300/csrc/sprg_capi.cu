@@ -68,6 +68,11 @@ struct sprg_ctx {
   // scratch
   DevBuf partials, out3, status, count, xitems, xcount, slab, bits;
   DevBuf titems, tcountb;  // triangle patches above the thread-per-vertex size
+  // What a form computes in place where there is no memory for it (the element
+  // records, edge lengths, triangle factors, refined weights, vertex transforms
+  // below).  Taken with an Optional on the frame, given back when a buffer that
+  // a call must have does not fit; *_none: not tried again on this mesh.
+  int optional = 0;  // Optionals on the frame
   // per mesh: the triangle patches' factors (33 doubles a vertex) and the
   // lengths of the two lists; tfac_none: no memory, each recovery factors in place
   DevBuf tqc, trr, tcode, txcount;
@@ -76,7 +81,7 @@ struct sprg_ctx {
   DevBuf Lx, pairs, red, eflags;  // MA sweeps: lengths, vertex pairs, reduction scratch, element flags
   DevBuf vxf, vbad;               // the vertices' metric transforms of the quality kernels
   DevBuf logm;                    // LogAnisoSizeField: per-vertex log-metrics (V x 9)
-  // FP64 form: per-mesh element records (88 bytes a tet, 64 a triangle);
+  // FP64 form: per-mesh element records (112 bytes a tet, 64 a triangle);
   // egeo_none: there was no memory for them, the kernels compute in place
   DevBuf egeo, elen64;  // elen64: half the edges' lengths
   bool egeo_ready = false, egeo_none = false, elen64_ready = false, elen64_none = false;
@@ -87,7 +92,7 @@ struct sprg_ctx {
   // listed vertices (per mesh), FP32 metric records, guarded edges
   // triangles' refined patch weights (the FP64 anisotropic pass) and the number of patches
   // too large for them
-  bool rw_ready = false;
+  bool rw_ready = false, rw_none = false;
   int n_rw_big = 0;
   DevBuf rw, rwlisted, rwitems, rwcount;
   DevBuf tw, twlisted, twitems, twcount, met32, qrec32, agitems, agcount, kidx, kval, klen, rec9, cj64, qties;
@@ -260,6 +265,54 @@ void discard(sprg_ctx* c, DevBuf& b) {
   release(b);
 }
 
+struct Optional {
+  sprg_ctx* c;
+  explicit Optional(sprg_ctx* x) : c(x) { ++c->optional; }
+  ~Optional() { --c->optional; }
+};
+
+bool discard_all(sprg_ctx* c, std::initializer_list<DevBuf*> bufs) {
+  bool any = false;
+  for (DevBuf* b : bufs) {
+    any = any || b->p;
+    discard(c, *b);
+  }
+  return any;
+}
+
+// Each optional group with its flags; freeing waits for kernels that still read
+// it.  A caller holds no pointer into one across an allocation.
+bool drop_tri_factors(sprg_ctx* c) {
+  c->tfac_ready = false;
+  c->tfac_none = true;
+  return discard_all(c, {&c->tqc, &c->trr, &c->tcode});
+}
+
+bool drop_refined_weights(sprg_ctx* c) {
+  c->rw_ready = false;
+  c->rw_none = true;
+  PatchCache& pc = c->cache2r;
+  pc.valid = pc.w_ready = false;
+  return discard_all(c, {&c->rw, &c->rwlisted, &pc.v, &pc.n, &pc.el, &pc.woff, &pc.w, &pc.wn});
+}
+
+bool give_back_optional(sprg_ctx* c) {
+  bool any = discard_all(c, {&c->vxf, &c->vbad});
+  if (c->egeo.p) {
+    c->egeo_ready = false;
+    c->egeo_none = true;
+    any |= discard_all(c, {&c->egeo});
+  }
+  if (c->elen64.p) {
+    c->elen64_ready = false;
+    c->elen64_none = true;
+    any |= discard_all(c, {&c->elen64});
+  }
+  if (c->tqc.p || c->trr.p || c->tcode.p) any |= drop_tri_factors(c);
+  if (c->rw.p || c->rwlisted.p || c->cache2r.el.p) any |= drop_refined_weights(c);
+  return any;
+}
+
 // grow-only device buffer (its contents are not kept)
 int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -278,6 +331,10 @@ int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
       cudaGetLastError();
       e = device_alloc(c, &b.p, bytes);
     }
+  }
+  if (e == cudaErrorMemoryAllocation && !c->optional && give_back_optional(c)) {
+    cudaGetLastError();
+    e = device_alloc(c, &b.p, bytes);
   }
   if (e != cudaSuccess) {
     b.p = nullptr;
@@ -453,6 +510,7 @@ int listed_fits(sprg_ctx* c, PatchCache& pc, const double* ip, int nc, double* r
 int ensure_elem_records(sprg_ctx* c) {
   if (c->egeo_ready || c->egeo_none) return SPRG_OK;
   DevMesh& m = c->m;
+  Optional opt(c);
   int rc = ensure(c, c->egeo, sizeof(double) * (size_t)elem_record_planes(m.dim) * m.T);
   if (rc == SPRG_ENOMEM) {
     cudaGetLastError();  // the failed allocation is no error of this call
@@ -530,6 +588,7 @@ int step_recover(sprg_ctx* c) {
     CK(cudaMemsetAsync(c->xcount.p, 0, sizeof(int), c->stream));
     CK(cudaMemsetAsync(c->tcountb.p, 0, sizeof(int), c->stream));
     if (!c->tfac_none) {
+      Optional opt(c);
       struct { DevBuf& b; size_t bytes; } need[] = {{c->tqc, sizeof(double) * tri_factor_planes() * (size_t)m.V},
                                                     {c->trr, sizeof(double) * tri_r_planes() * (size_t)m.V},
                                                     {c->tcode, (size_t)m.V}};
@@ -537,7 +596,7 @@ int step_recover(sprg_ctx* c) {
         if (!c->tfac_none && (rc = ensure(c, n.b, n.bytes))) {
           if (rc != SPRG_ENOMEM) return rc;
           cudaGetLastError();  // the failed allocation is no error of this call
-          c->tfac_none = true;
+          drop_tri_factors(c);
         }
       }
     }
@@ -557,12 +616,13 @@ int step_recover(sprg_ctx* c) {
     // the warp path appends its own growth patches behind the factors' ones
     CK(cudaMemcpyAsync(c->xcount.p, c->txcount.p, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
   }
-  const TriFactor tf{c->tfac_ready ? P<double>(c->tqc) : nullptr, P<double>(c->trr), P<unsigned char>(c->tcode)};
   // with the lists complete (no patch on the warp path, which may add to
   // them), the growth patches too are weighted sums inside the recovery
   PatchCache& pc = c->cache64;
   const bool complete = c->tfac_ready && !c->n_tri_big;
   if (complete && (rc = ensure_listed(c, pc, xl, -1))) return rc;
+  if (complete && !c->tfac_ready) return step_recover(c);  // the factors were given back for the patches
+  const TriFactor tf{c->tfac_ready ? P<double>(c->tqc) : nullptr, P<double>(c->trr), P<unsigned char>(c->tcode)};
   const PatchWeights none{};
   PB("recover_f64");
   launch_recover_f64(m, P<double>(c->ip), nc, P<double>(c->rec), tf, xl, big, !c->tfac_ready || c->n_tri_big > 0,
@@ -622,6 +682,7 @@ int step_measure_mark(sprg_ctx* c, uint32_t* d_split, uint32_t* d_collapse) {
   DevMesh& m = c->m;
   ENSURE(c->L, sizeof(double) * (size_t)m.E);
   if (!c->elen64_ready && !c->elen64_none) {
+    Optional opt(c);
     int rc = ensure(c, c->elen64, sizeof(double) * (size_t)m.E);
     if (rc == SPRG_ENOMEM) {
       cudaGetLastError();
@@ -708,11 +769,12 @@ int step_quality(sprg_ctx* c, const double* size, const double* sizes, const dou
   DevMesh& m = c->m;
   double* xf = nullptr;
   if (!size) {
+    Optional opt(c);
     int rc = ensure(c, c->vxf, vertex_transform_bytes(m.V));
     if (rc == SPRG_OK) rc = ensure(c, c->vbad, (size_t)m.V);
     if (rc == SPRG_OK) xf = P<double>(c->vxf);
     else if (rc != SPRG_ENOMEM) return rc;
-    else cudaGetLastError();  // the failed allocation is no error of this call
+    else discard_all(c, {&c->vxf, &c->vbad}), cudaGetLastError();  // the failed allocation is no error of this call
   }
   launch_quality_f64(m, size, sizes, frames, logm, xf, P<unsigned char>(c->vbad), pass, q, P<DevStatus>(c->status),
                      c->stream);
@@ -889,7 +951,7 @@ static void invalidate_mesh_state(sprg_ctx* c) {
   // the tuned launch shape stays: every choice gives bitwise the same result,
   // and an adapt iteration changes the patch-size mix little
   c->tw_ready = false;
-  c->rw_ready = false;
+  c->rw_ready = c->rw_none = false;
   c->qw_ready = false;
   c->tfac_ready = c->tfac_none = false;
   c->egeo_ready = c->egeo_none = c->elen64_ready = c->elen64_none = false;
@@ -2027,7 +2089,9 @@ static int pass_learned(sprg_ctx* c, const double* d_u, double adapt_ratio, uint
 // the triangles' refined patch weights (once per mesh) and the patches they
 // leave out
 static int ensure_aniso_weights(sprg_ctx* c) {
+  if (c->rw_none) return SPRG_ENOMEM;
   DevMesh& m = c->m;
+  Optional opt(c);
   int rc;
   ENSURE(c->rwitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
   ENSURE(c->rwcount, 2 * sizeof(int));  // listed patches, patches too large
@@ -2066,6 +2130,7 @@ static int aniso_recover(sprg_ctx* c) {
   if (rc && rc != SPRG_ENOMEM) return rc;
   if (rc || c->n_rw_big) {
     if (rc) cudaGetLastError();  // the failed allocation is no error of this call
+    if (!c->rw_none) drop_refined_weights(c);
     return step_recover(c);
   }
   PB("recover_f64");
@@ -2679,6 +2744,13 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   if ((rc = reset_status(c))) return rc;
   CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
   if (c->precision == SPRG_FP32) return aniso_pass_mixed(c, eps, h_min, h_max, d_split_bits, d_collapse_bits, d_quality);
+  if (m.dim == 2) {
+    // both recoveries' buffers before the weights: if these have to go for a
+    // buffer, they go before either recovery
+    ENSURE(c->ip, sizeof(double) * 9 * (size_t)m.T);
+    ENSURE(c->rec, sizeof(double) * 9 * (size_t)m.V);
+    ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + 9 + 1));
+  }
   // recovered gradient, then the recovered gradient of it (nodal Hessian)
   if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = aniso_recover(c))) return rc;
   CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
