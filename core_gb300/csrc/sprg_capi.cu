@@ -313,6 +313,23 @@ bool give_back_optional(sprg_ctx* c) {
   return any;
 }
 
+// What a mesh's passes derived from it, before an update that needs the room:
+// after it all of this is made anew in any case, and if the update fails the
+// old mesh's next pass does so.
+bool give_back_setup(sprg_ctx* c) {
+  c->vrec_ready = c->crec_ready = c->bins_ready = c->vv_ready = false;
+  c->tw_ready = c->qw_ready = c->gstamp_ready = false;
+  bool any = discard_all(
+      c, {&c->crec, &c->wts, &c->w64, &c->listed, &c->geo, &c->geo64, &c->cent, &c->elen, &c->pcls, &c->bverts, &c->bcnt,
+          &c->soff, &c->sel, &c->sw, &c->vvoff, &c->vv, &c->vtile, &c->gstamp, &c->tw, &c->twlisted, &c->kidx, &c->kval,
+          &c->klen, &c->qw, &c->qwlisted});
+  for (PatchCache* pc : {&c->cache64, &c->cache32, &c->cache2d, &c->cache2r}) {
+    pc->valid = pc->w_ready = false;
+    any |= discard_all(c, {&pc->v, &pc->n, &pc->el, &pc->woff, &pc->w, &pc->wn});
+  }
+  return any;
+}
+
 // grow-only device buffer (its contents are not kept)
 int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -333,6 +350,10 @@ int ensure(sprg_ctx* c, DevBuf& b, size_t bytes) {
     }
   }
   if (e == cudaErrorMemoryAllocation && !c->optional && give_back_optional(c)) {
+    cudaGetLastError();
+    e = device_alloc(c, &b.p, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && c->updating && give_back_setup(c)) {
     cudaGetLastError();
     e = device_alloc(c, &b.p, bytes);
   }

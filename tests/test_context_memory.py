@@ -213,3 +213,51 @@ def test_refined_weights_without_memory(gpu_lib, n):
             assert np.array_equal(got, refined) or np.array_equal(got, calls), k
         with_factors += np.array_equal(first, calls)
     assert with_factors >= 2  # the weights and their flags
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "learned"])
+def test_update_with_little_memory(gpu_lib, precision):
+    """An update needs room beside the old mesh: what the old mesh's passes
+    derived from it is given back for that, whichever allocation fails."""
+    import core_gb300 as cg
+    (m0, u0), (m1, u1) = box(6), box(9, 2)
+    want = fresh(m1, u1, precision)
+    # the records go first, then the rest: two attempts fail where there are both
+    for count in (1, 2) if precision == "fp64" else (1,):
+        for k in range(16):
+            with cg.Context(m0, precision=precision) as c:
+                c.estimate_and_mark(u0, 0.1)
+                fail(c, k, count)
+                c.update_mesh(m1)
+                c.test_hooks()
+                assert same(c.estimate_and_mark(u1, 0.1)[:4], want), (count, k)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "learned"])
+def test_failed_update_after_everything_went(gpu_lib, precision):
+    """No memory at all: the old mesh's passes make their setup anew, a captured
+    one too."""
+    import torch
+    import core_gb300 as cg
+    (m0, u0), (m1, u1) = box(6), box(9, 2)
+    want = fresh(m0, u0, precision)
+    stream = torch.cuda.Stream()
+    with cg.Context(m0, precision=precision) as c, torch.cuda.stream(stream):
+        c.set_stream(stream.cuda_stream)
+        d_u = torch.from_numpy(u0).cuda()
+        bits = torch.zeros((2, (m0.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        c.graph_capture(d_u.data_ptr(), 0.1, bits[0].data_ptr(), bits[1].data_ptr())
+        fail(c, 3, 100)
+        with pytest.raises(cg.SprgError) as e:
+            c.update_mesh(m1)
+        assert e.value.code == 4
+        c.test_hooks()
+        bits.zero_()
+        c.graph_replay()
+        stream.synchronize()
+        b, e = bits.cpu().numpy().view(np.uint32), np.arange(m0.n_edges)
+        assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, want[1] & 1)
+        assert same(c.estimate_and_mark(u0, 0.1)[:4], want)
+        c.update_mesh(m1)
+        assert same(c.estimate_and_mark(u1, 0.1)[:4], fresh(m1, u1, precision))
+        c.set_stream(0)
