@@ -99,6 +99,19 @@ inline void launch_after(bool early, void (*kernel)(P...), int grid, int block, 
   launch_after_smem(early, kernel, grid, block, 0, s, std::forward<A>(args)...);
 }
 
+// The vertex and lane of a thread where LANES consecutive threads take a vertex.
+// 64 bits: a mesh may have 2^31 - 1 vertices, LANES times as many threads, and
+// threads past the last.
+struct VertexLane {
+  long v;
+  int lane;
+};
+template <int LANES>
+__host__ __device__ inline VertexLane vertex_lane(unsigned block, int threads, int thread) {
+  const long i = (long)block * threads + thread;
+  return VertexLane{i / LANES, (int)(i % LANES)};
+}
+
 // Device status word written by kernels (first error wins).
 struct DevStatus {
   int code;        // SPRG_OK or SPRG_E*

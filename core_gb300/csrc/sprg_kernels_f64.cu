@@ -1376,7 +1376,7 @@ __device__ __forceinline__ void sort_segment_warp(int* el, int b, int n, int lan
 __global__ void __launch_bounds__(kBlock) k_sort_segments(int V, const int* __restrict__ off, int* __restrict__ el) {
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (kBlock / 32);
-  for (int v = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); v < V; v += nw) {
+  for (long v = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); v < V; v += nw) {
     const int b = off[v], n = off[v + 1] - b;
     if (n <= 32) {
       sort_segment_lanes(el, b, n, lane);
@@ -2474,7 +2474,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter_rows(long long n, int width,
 __global__ void __launch_bounds__(kBlock) k_bbox(int V, const double* __restrict__ xyz,
                                                  unsigned long long* __restrict__ keys) {
   unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+  for (long v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
     for (int k = 0; k < 3; ++k) {
       const unsigned long long key = order_key(xyz[3 * (size_t)v + k]);
       lo[k] = key < lo[k] ? key : lo[k];
@@ -2625,9 +2625,9 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
     if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
     return;
   }
-  const int i = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
-  const int v = i / LANES, l = i % LANES;
-  const bool mine = v < m.V && !listed[v];
+  const VertexLane vl = vertex_lane<LANES>(blockIdx.x - n_list_blocks, kBlock, threadIdx.x);
+  const bool mine = vl.v < m.V && !listed[vl.v];
+  const int v = (int)vl.v, l = vl.lane;
   const int beg = mine ? m.p_off[v] : 0, end = mine ? m.p_off[v + 1] : 0;
   double acc[NC];
 #pragma unroll
