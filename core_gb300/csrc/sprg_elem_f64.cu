@@ -307,7 +307,7 @@ template <int D, bool REC>
 __global__ void __launch_bounds__(kBlock) k_esize(DevMesh m, const double* __restrict__ geo,
                                                   const double* __restrict__ out3, int mode, double alpha, double beta,
                                                   double* __restrict__ esize) {
-  after_previous(geo, out3);
+  after_previous(geo, out3, esize);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.T) return;
   const double sf = out3[2];
