@@ -2406,7 +2406,8 @@ int sprg_debug_read(sprg_ctx* c, const char* name, void* host, size_t bytes) {
       {"fcnt", &c->fcnt},   {"guard", &c->guard}, {"xitems", &c->xitems}, {"xcount", &c->xcount}, {"agcount", &c->agcount}, {"sizes3", &c->sizes3}, {"frames9", &c->frames9}, {"twcount", &c->twcount}, {"met32", &c->met32}, {"rec9", &c->rec9},
       {"wts", &c->wts},     {"geo", &c->geo},     {"elen", &c->elen},     {"rec16", &c->rec16},
       {"sizel", &c->sizel}, {"ql", &c->ql},       {"vr16", &c->vr16},     {"fbitems", &c->fbitems},
-      {"fbcount", &c->fbcount}, {"listed", &c->listed}, {"bverts", &c->bverts}, {"pcls", &c->pcls}};
+      {"fbcount", &c->fbcount}, {"listed", &c->listed}, {"bverts", &c->bverts}, {"pcls", &c->pcls},
+      {"qmax", &c->qmax}};
   for (auto& e : table) {
     if (strcmp(e.n, name) != 0) continue;
     if (!e.b->p) return fail(c, SPRG_ESTATE, std::string("buffer not allocated: ") + name);

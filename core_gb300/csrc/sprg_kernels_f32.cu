@@ -328,26 +328,11 @@ __global__ void __launch_bounds__(kBlock) k_fast_geo(DevMesh m, float2* __restri
     for (int k = 0; k < 3; ++k) cent[3 * (size_t)t + k] = ((x[0][k] + x[1][k]) + x[2][k]) + x[3][k];
     // |cof(J)|_F^2 / |det J| (= |J^-1|_F^2 |det J|): the element's share of the
     // reference's gradient rounding in the error integral scales with it; the
-    // largest over the mesh, for the rounding-dominance test (whose threshold
-    // is a factor 256 wide: the reciprocal is good to 2^-40)
+    // largest over the mesh, for the rounding-dominance test
     double c2 = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) c2 += c[i][0] * c[i][0] + c[i][1] * c[i][1] + c[i][2] * c[i][2];
-    const double ad = fabs(det);
-    const int ex = __double2hiint(ad) >> 20;
-    if (ex >= 100 && ex <= 1900) {
-      // 1 / det from the hardware's FP32 reciprocal of its mantissa in [1, 2)
-      // and one Newton step
-      const int hi = __double2hiint(ad), lo = __double2loint(ad);
-      float f = __int_as_float(((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29) | 0x3f800000);
-      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(f));
-      const int b = __float_as_int(f);
-      double r = __hiloint2double((b >> 3) + (896 << 20) - ((ex - 1023) << 20), b << 29);
-      r = r * (2.0 - ad * r);
-      qv = c2 * r;
-    } else {
-      qv = c2 / ad;  // inf for a flat element
-    }
+    qv = c2 / fabs(det);  // inf for a flat element
     if (!(qv == qv)) qv = INFINITY;
   }
   // non-negative doubles order as their bit patterns

@@ -1,0 +1,26 @@
+"""Per-mesh geometry of the FP32 form against extended precision."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [2, 3])
+def test_largest_cofactor_norm(gpu_lib, n):
+    """|cof J|_F^2 / |det J| of the worst element (the rounding-dominance test's
+    measure) to FP64 rounding: on these boxes |p||q| is below 8 times a cofactor
+    and the products' sum below 8 times the determinant, so the cofactors'
+    squares carry 2 x 2 x 8 units of rounding, the determinant 8 + 16 and the sums
+    and the quotient a few: 64."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    for seed in range(24):
+        m = workload.box(n, jitter=0.2, seed=seed)
+        x = m.coords.astype(np.longdouble)
+        e = [x[m.elem_verts[:, k]] - x[m.elem_verts[:, 0]] for k in (1, 2, 3)]
+        cof = [np.cross(e[(i + 1) % 3], e[(i + 2) % 3]) for i in range(3)]
+        q = sum((c * c).sum(1) for c in cof) / np.abs((e[0] * cof[0]).sum(1))
+        with cg.Context(m, precision="fp32") as c:
+            c.estimate_and_mark(workload.bump_field(m.coords, seed=1), 0.1)
+            got = c.debug_read("qmax", np.float64, 1)[0]
+        assert abs(got - q.max()) <= 64 * 2.0 ** -53 * q.max(), seed
