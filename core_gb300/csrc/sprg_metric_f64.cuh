@@ -8,7 +8,7 @@ namespace sprg {
 
 // err to the exponents the size field needs in D dimensions (p = 1):
 //   q = (sqrt err)^(-2 / (2 + D))  = err^(-1/(D+2))
-//   g = (sqrt err)^(2 D / (2 + D)) = err q^2
+//   g = (sqrt err)^(2 D / (2 + D)) = err q^2, on triangles the root itself
 // Reduced to err = 2^(P k) m with m in [1, 2^P), P = D + 2: the hardware
 // log2 / exp2 give m^(-1/P) to 2^-21, one step of the cubically convergent
 // Householder iteration on 1 - m r^P squares that twice over, 2^-k goes into
@@ -45,7 +45,7 @@ __device__ __forceinline__ void error_powers(double err, double& q, double& g) {
   const double c = P == 5 ? fma(h, 3.0 / 25.0, 0.2) : fma(h, 5.0 / 32.0, 0.25);
   const double y = fma(r0 * h, c, r0);
   q = __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y));
-  g = err * (q * q);
+  g = D == 2 ? sqrt(err) : err * (q * q);
 }
 
 __device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }

@@ -24,3 +24,21 @@ def test_largest_cofactor_norm(gpu_lib, n):
             c.estimate_and_mark(workload.bump_field(m.coords, seed=1), 0.1)
             got = c.debug_read("qmax", np.float64, 1)[0]
         assert abs(got - q.max()) <= 64 * 2.0 ** -53 * q.max(), seed
+
+
+def test_error_sum_on_triangles(gpu_lib):
+    """The power of an error in the sum of a triangle mesh is its square root,
+    correctly rounded, as the reference's pow(sqrt(err), 1); eight elements are
+    summed as a tree over the lanes."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    for seed in range(24):
+        m = workload.box(2, nz=0, jitter=0.2, seed=seed)
+        with cg.Context(m) as c:
+            _, info = c.getSPRSizeField(c.getGradIPField(workload.bump_field(m.coords, seed=seed)), 0.1)
+            err = c.debug_read("err", np.float64, m.n_elems)
+        assert m.n_elems == 8 and np.all(err > 0)
+        x = np.sqrt(err)
+        x = x[:4] + x[4:]
+        x = x[:2] + x[2:]
+        assert info["error_sum"] == x[0] + x[1], seed
