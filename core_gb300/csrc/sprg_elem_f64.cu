@@ -355,19 +355,30 @@ __global__ void __launch_bounds__(kBlock) k_measure_iso(DevMesh m, const double*
   L[e] = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), __ldg(size + v.x), __ldg(size + v.y));
 }
 
+// half an edge's Euclidean length
+__device__ __forceinline__ double half_length(const DevMesh& m, int2 v) {
+  const V3 d = ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x));
+  return 0.5 * sqrt(fma(d.v[0], d.v[0], fma(d.v[1], d.v[1], d.v[2] * d.v[2])));
+}
+
 // per mesh: half the edges' Euclidean lengths
 __global__ void __launch_bounds__(kBlock) k_edge_records(DevMesh m, double* __restrict__ len) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.E) return;
   const int2 v = __ldg(reinterpret_cast<const int2*>(m.edv) + e);
-  len[e] = 0.5 * ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
+  len[e] = half_length(m, v);
 }
 
-// The pass's lengths and marks.  The sizes it computed are good to about
-// 1e-10 of the reference's, so the lengths need no particular rounding:
-// |d| / 2 (1 / h0 + 1 / h1) = (|d| / 2) (h0 + h1) / (h0 h1), about 17 FP64
-// operations with the per-mesh half lengths against 55.  Lengths within 1e-6
-// of 0.5 or 1.5, and those iso_length hands to the reference's sequence, take
+// The pass's lengths and marks.  Only the marks leave the pass, so the lengths
+// need not be the sequence's bits, but they are as near the exact ones (0.83
+// units of 2^-53 rms, the sequence 0.83 to 0.84; (|d| / 2) (h0 + h1) / (h0 h1) as
+// it stands 1.09): with the ends' sizes a, b
+//   |d| / 2 (1 / h0 + 1 / h1) = |d| / 2 (a + b) / (a b + K (a - b)^2),  K = N0 N1,
+// the quotient from the hardware's reciprocal (2^-20 at least) and one Newton
+// step, its residual with the denominator's rounding corrected before the
+// product: 15 FP64 operations with the per-mesh half lengths, 55 for the sequence.
+// Sizes more than about 2.8 apart (K (a - b)^2 then carries two roundings of its
+// own), lengths within 1e-6 of 0.5 or 1.5, and exponents outside [-300, 300] take
 // iso_length, so every mark is that of the bitwise length.  The comparisons
 // and windows are integer ones on the bits (FP64 comparisons use the FP64
 // pipe).  96^3 box, 6.3M edges: 0.99 ms for the reference's sequence plus
@@ -385,14 +396,19 @@ __global__ void __launch_bounds__(kBlock) k_measure_mark(DevMesh m, const double
     const double sa = __ldg(size + v.x), sb = __ldg(size + v.y);
     double d;
     if constexpr (REC) d = __ldcs(len + e);
-    else d = 0.5 * ref::len(ref::sub(load_xyz(m.xyz, v.y), load_xyz(m.xyz, v.x)));
-    const double N0 = (1.0 - 0.577350269189626) / 2.0, N1 = (1.0 + 0.577350269189626) / 2.0;
-    const double h0 = fma(sa, N0, sb * N1), h1 = fma(sa, N1, sb * N0);
-    double l = (d * (h0 + h1)) / (h0 * h1);
-    const int e0 = __double2hiint(h0) >> 20, e1 = __double2hiint(h1) >> 20, hl = __double2hiint(l);
+    else d = half_length(m, v);
+    const double K = (1.0 - 0.577350269189626) / 2.0 * ((1.0 + 0.577350269189626) / 2.0);
+    const double sum = sa + sb, df = sa - sb, p = K * df * df, den = fma(sa, sb, p);
+    const double den_err = fma(sa, sb, -den) + p;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+    y = fma(y, fma(-den, y, 1.0), y);
+    const double q = sum * y, c = fma(-q, den_err, fma(-den, q, sum)) * y;
+    double l = fma(d, q, d * c);
+    const int ha = __double2hiint(sa), hb = __double2hiint(sb), e0 = ha >> 20, e1 = hb >> 20, hl = __double2hiint(l);
     // hl >> 20 is the biased exponent of a positive length, negative for a
     // negative one; 0x3ff80000 is 1.5's high word, 0x3fe00000 0.5's
-    if (min(min(e0, e1), hl >> 20) < 623 || max(max(e0, e1), hl >> 20) > 1423 ||
+    if (min(min(e0, e1), hl >> 20) < 723 || max(max(e0, e1), hl >> 20) > 1323 || abs(ha - hb) > 0x180000 ||
         (unsigned)(hl - 0x3ff7ffff) < 2u || (unsigned)(hl - 0x3fdfffff) < 2u) {
       l = iso_length(load_xyz(m.xyz, v.x), load_xyz(m.xyz, v.y), sa, sb);
       sp = l > 1.5;

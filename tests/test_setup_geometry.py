@@ -42,3 +42,28 @@ def test_error_sum_on_triangles(gpu_lib):
         x = x[:4] + x[4:]
         x = x[:2] + x[2:]
         assert info["error_sum"] == x[0] + x[1], seed
+
+
+@pytest.mark.parametrize("n", [12, 20])
+def test_pass_lengths_as_near_as_the_sequence(gpu_lib, n):
+    """The FP64 pass's lengths against extended precision are no farther off than
+    the reference's sequence (the measure call) on the same sizes: their rms
+    errors agree to the statistics of the edges, 3 / sqrt(2 E) of 0.84 units."""
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m = workload.box(n, jitter=0.2, seed=4)
+    with cg.Context(m) as c:
+        size = c.estimate_and_mark(workload.bump_field(m.coords, seed=4), 1.28 / n)[0]
+        L = c.debug_read("L", np.float64, m.n_edges)
+        seq = c.measure_edges(size)
+    Q = np.longdouble
+    a, b = m.edge_verts.T
+    d = m.coords.astype(Q)[b] - m.coords.astype(Q)[a]
+    half = np.sqrt((d * d).sum(1)) / 2
+    g = Q(0.577350269189626)
+    s = size.astype(Q)
+    exact = sum(half / (s[a] * ((1 - x) / 2) + s[b] * ((1 + x) / 2)) for x in (g, -g))
+
+    def rms(x):
+        return float(np.sqrt(np.mean(((x - exact) / exact * 2 ** 53) ** 2)))
+    assert rms(L) <= rms(seq) * (1 + 3 / np.sqrt(2 * m.n_edges))
