@@ -2167,6 +2167,12 @@ static int pass_resident(sprg_ctx* c, const double* d_u, double adapt_ratio, uin
   int rc;
   if (c->batch_n && c->precision != SPRG_FP32)
     return fail(c, SPRG_EINVAL, "a batch of meshes runs in SPRG_FP32 (per-mesh size factors)");
+  if (reinterpret_cast<uintptr_t>(d_u) % alignof(double)) {
+    // the kernels load doubles; a copy has no such rule
+    ENSURE(c->f, sizeof(double) * (size_t)c->m.V);
+    CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)c->m.V, cudaMemcpyDeviceToDevice, c->stream));
+    d_u = P<double>(c->f);
+  }
   {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->stream, &cap));
