@@ -33,6 +33,7 @@ struct PatchCache {
   // tets: per-mesh weights of the cached patches' fits (w_ready once built)
   bool w_ready = false;
   DevBuf woff, w, wn;
+  DevBuf g;  // optional: the elements' gradients beside the weights (PatchWeights::g)
 };
 
 // events of one timed host call: 0 call start, 1 field uploaded, 2 pass done,
@@ -308,6 +309,7 @@ bool give_back_optional(sprg_ctx* c) {
     c->elen64_none = true;
     any |= discard_all(c, {&c->elen64});
   }
+  any |= discard_all(c, {&c->cache32.g});
   if (c->tqc.p || c->trr.p || c->tcode.p) any |= drop_tri_factors(c);
   if (c->rw.p || c->rwlisted.p || c->cache2r.el.p) any |= drop_refined_weights(c);
   return any;
@@ -325,7 +327,7 @@ bool give_back_setup(sprg_ctx* c) {
           &c->klen, &c->qw, &c->qwlisted});
   for (PatchCache* pc : {&c->cache64, &c->cache32, &c->cache2d, &c->cache2r}) {
     pc->valid = pc->w_ready = false;
-    any |= discard_all(c, {&pc->v, &pc->n, &pc->el, &pc->woff, &pc->w, &pc->wn});
+    any |= discard_all(c, {&pc->v, &pc->n, &pc->el, &pc->woff, &pc->w, &pc->wn, &pc->g});
   }
   return any;
 }
@@ -441,6 +443,13 @@ void prof_end(sprg_ctx* c) {
 
 // ---- pipeline steps on resident buffers -------------------------------
 
+// their weights for the recovery kernels (none of them: n = 0)
+PatchWeights patch_weights(sprg_ctx* c, PatchCache& pc) {
+  return PatchWeights{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v),  P<int>(pc.el),
+                      P<long long>(pc.woff),     P<double>(pc.w),    P<int>(pc.wn), P<double>(pc.g),
+                      P<DevStatus>(c->status)};
+}
+
 // Listed patches: grow them on the first pass (recording the final element
 // sets), afterwards one QR fit per cached set.
 // Once a patch cache exists, the QR of each cached patch runs once (per mesh)
@@ -470,9 +479,21 @@ int ensure_cache_weights(sprg_ctx* c, PatchCache& pc) {
   c->launches += 1;
   int rc = check_launch(c, "cached patch weights");
   if (rc) return rc;
-  CK(cudaStreamSynchronize(c->stream));  // the host offsets stay alive until the copy is done
   pc.w_ready = true;
-  return SPRG_OK;
+  if (&pc == &c->cache32) {  // the FP32 and learned forms' patches
+    Optional opt(c);
+    rc = ensure(c, pc.g, sizeof(double) * 12 * (size_t)(total > 0 ? total : 1));
+    if (rc == SPRG_OK) {
+      launch_listed_records(c->m, patch_weights(c, pc), P<double>(pc.g), c->stream);
+      c->launches += 1;
+      rc = check_launch(c, "listed records");
+    } else if (rc == SPRG_ENOMEM) {
+      cudaGetLastError();  // the failed allocation is no error of this call
+      rc = SPRG_OK;
+    }
+  }
+  CK(cudaStreamSynchronize(c->stream));  // the host offsets stay alive until the copy is done
+  return rc;
 }
 
 // The growth of the listed patches (once per mesh), their final element sets
@@ -506,12 +527,6 @@ int ensure_listed(sprg_ctx* c, PatchCache& pc, ExpandList xl, int known) {
   int rc = SPRG_OK;
   if (!pc.valid && (rc = grow_patches(c, pc, nullptr, 0, nullptr, xl, known))) return rc;
   return ensure_cache_weights(c, pc);
-}
-
-// their weights for the recovery kernels (none of them: n = 0)
-PatchWeights patch_weights(sprg_ctx* c, PatchCache& pc) {
-  return PatchWeights{pc.w_ready ? pc.count : 0, expand_max_elems(), P<int>(pc.v),  P<int>(pc.el),
-                      P<long long>(pc.woff),     P<double>(pc.w),    P<int>(pc.wn), P<DevStatus>(c->status)};
 }
 
 // triangles with patches on the warp path: the listed vertices' QR fits, which
@@ -1175,7 +1190,7 @@ int sprg_destroy(sprg_ctx* c) {
                     &c->hess, &c->pcls, &c->bverts, &c->btiles, &c->bnext, &c->bvoff, &c->bseg, &c->bsegoff, &c->bratios, &c->vvoff, &c->vv, &c->vtile, &c->vr16, &c->rec16,
                     &c->ql,    &c->sizel,   &c->fbitems, &c->fbcount, &c->mlp_packed, &c->mlp_err, &c->mlp_tmp, &c->lrange, &c->ldone, &c->lsc,
                     &c->cache64.v, &c->cache64.n, &c->cache64.el, &c->cache32.v, &c->cache32.n, &c->cache32.el,
-                    &c->cache64.woff, &c->cache64.w, &c->cache64.wn, &c->cache32.woff, &c->cache32.w,
+                    &c->cache64.woff, &c->cache64.w, &c->cache64.wn, &c->cache32.woff, &c->cache32.w, &c->cache32.g,
                     &c->cache32.wn};
   for (DevBuf* b : bufs) release(*b);
   for (auto& e : c->ev_pool) cudaEventDestroy(e);

@@ -157,6 +157,23 @@ __global__ void __launch_bounds__(kBlock) k_elem_records(DevMesh m, double* __re
   for (int k = 0; k < ElemRec<D>::kPlanes; ++k) geo[(size_t)k * m.T + e] = r[k];
 }
 
+// per mesh: the gradients of the listed patches' elements, a warp per patch
+__global__ void __launch_bounds__(kBlock) k_listed_records(DevMesh m, PatchWeights pw, double* __restrict__ g) {
+  const int it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (it >= pw.n) return;
+  for (int i = lane; i < pw.wn[it]; i += 32) {
+    int id[4];
+    load_ids<3>(m.ev, pw.el[(size_t)it * pw.stride + i], id);
+    double r[ElemRec<3>::kPlanes];
+    elem_record_of<3>(m, id, r);
+    double* o = g + 12 * (pw.woff[it] + i);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[k] = r[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o[9 + k] = r[11 + k];
+  }
+}
+
 // ---------------------------------------------------------------------
 // spr::getGradIPField (spr/sprGetGradIPField.cc:15-65): the gradients of the
 // shape functions are J^-1's columns and, for the first vertex, the negated
@@ -438,6 +455,10 @@ void launch_elem_records(const DevMesh& m, double* geo, cudaStream_t s) {
   if (!m.T) return;
   if (m.dim == 3) k_elem_records<3><<<nblk(m.T), kBlock, 0, s>>>(m, geo);
   else k_elem_records<2><<<nblk(m.T), kBlock, 0, s>>>(m, geo);
+}
+
+void launch_listed_records(const DevMesh& m, const PatchWeights& pw, double* g, cudaStream_t s) {
+  if (pw.n) k_listed_records<<<nblk((long)pw.n * 32), kBlock, 0, s>>>(m, pw, g);
 }
 
 void launch_grad_ip_f64(const DevMesh& m, const double* geo, const double* f, int ncin, double* ip, cudaStream_t s) {

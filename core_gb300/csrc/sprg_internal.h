@@ -120,7 +120,9 @@ struct DevStatus {
 
 // The listed patches' per-mesh FP64 weights: n patches; patch it: vertex v[it],
 // elements el + it stride, wn[it] weights at w + woff[it], or -1 where the
-// growth or the rank test failed (SPRG_EPATCH in st)
+// growth or the rank test failed (SPRG_EPATCH in st).  g (tets, optional): with
+// each weight its element's gradient, 12 doubles (J^-1 by rows, then the first
+// vertex's shape gradient)
 struct PatchWeights {
   int n, stride;
   const int* v;
@@ -128,6 +130,7 @@ struct PatchWeights {
   const long long* woff;
   const double* w;
   const int* wn;
+  const double* g;
   DevStatus* st;
 };
 
@@ -145,6 +148,8 @@ struct ExpandList {
 // vertex's shape gradient)
 int elem_record_planes(int dim);
 void launch_elem_records(const DevMesh& m, double* geo, cudaStream_t s);
+// the gradients of the listed patches' elements into g (PatchWeights::g)
+void launch_listed_records(const DevMesh& m, const PatchWeights& pw, double* g, cudaStream_t s);
 // geo: the records, or null to compute them in place
 void launch_grad_ip_f64(const DevMesh& m, const double* geo, const double* f, int ncin, double* ip, cudaStream_t s);
 // per-element errors, their powers in esize (k_error) and deterministic block
