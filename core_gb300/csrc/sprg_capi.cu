@@ -413,8 +413,13 @@ int sync_and_status(sprg_ctx* c) {
   return SPRG_OK;
 }
 
+// the status word, and behind it the count of vertices a weighted recovery leaves
+// to the factors' sequence
+size_t status_bytes() { return sizeof(DevStatus) + sizeof(int); }
+int* redo_count(sprg_ctx* c) { return reinterpret_cast<int*>(P<DevStatus>(c->status) + 1); }
+
 int reset_status(sprg_ctx* c) {
-  CK(cudaMemsetAsync(c->status.p, 0, sizeof(DevStatus), c->stream));
+  CK(cudaMemsetAsync(c->status.p, 0, status_bytes(), c->stream));
   return SPRG_OK;
 }
 
@@ -607,7 +612,7 @@ int step_recover(sprg_ctx* c) {
     if ((rc = ensure_listed(c, pc, lst, -1))) return rc;
     PB("recover_f64");
     launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->qw), P<unsigned char>(c->qwlisted), patch_weights(c, pc),
-                       P<double>(c->rec), c->stream);
+                       P<double>(c->rec), ExpandList{}, c->stream);
     PE();
     c->launches += 1;
     return check_launch(c, "recover");
@@ -919,9 +924,9 @@ int sprg_create(const sprg_mesh_view* mv, int device, sprg_ctx** out) {
   ENSUREC(c->pel, sizeof(int) * nel);
   ENSUREC(c->tmp, sizeof(int) * (size_t)m.V);
   ENSUREC(c->vscan, offset_scan_bytes(m.V));
-  ENSUREC(c->status, sizeof(DevStatus));
+  ENSUREC(c->status, status_bytes());
   ENSUREC(c->count, sizeof(unsigned long long));
-  CKC(cudaMemsetAsync(c->status.p, 0, sizeof(DevStatus), c->stream));
+  CKC(cudaMemsetAsync(c->status.p, 0, status_bytes(), c->stream));
   CKC(cudaMemcpyAsync(c->xyz.p, mv->coords, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyHostToDevice, c->stream));
   CKC(cudaMemcpyAsync(c->ev.p, mv->elem_verts, sizeof(int) * nel, cudaMemcpyHostToDevice, c->stream));
   CKC(cudaMemcpyAsync(c->edv.p, mv->edge_verts, sizeof(int) * 2 * (size_t)m.E, cudaMemcpyHostToDevice, c->stream));
@@ -2162,6 +2167,8 @@ static int aniso_recover(sprg_ctx* c) {
   const int nc = c->ip_nc;
   ENSURE(c->rec, sizeof(double) * (size_t)m.V * nc);
   ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + nc + 1));
+  const int redo_cap = (int)std::min(2ll * m.V, (long long)INT32_MAX);  // both recoveries of a pass append
+  ENSURE(c->titems, sizeof(int) * (size_t)redo_cap);
   const int rc = ensure_aniso_weights(c);
   if (rc && rc != SPRG_ENOMEM) return rc;
   if (rc || c->n_rw_big) {
@@ -2171,9 +2178,10 @@ static int aniso_recover(sprg_ctx* c) {
   }
   PB("recover_f64");
   launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->rw), P<unsigned char>(c->rwlisted),
-                     patch_weights(c, c->cache2r), P<double>(c->rec), c->stream);
+                     patch_weights(c, c->cache2r), P<double>(c->rec),
+                     ExpandList{P<int>(c->titems), redo_count(c), redo_cap}, c->stream);
   PE();
-  c->launches += 1;
+  c->launches += 2;
   return check_launch(c, "recover");
 }
 

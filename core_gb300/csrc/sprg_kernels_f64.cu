@@ -341,7 +341,10 @@ __device__ __forceinline__ double tri_div(double a, double b, double y, bool pla
 // elements, fixed reduction tree.  The recovery kernels' first blocks run these
 // beside the other vertices (a launch of their own took 10 us of latency, the
 // triangles' QR fits 46).
-template <int NC>
+// TRI: on triangles a sum that is not finite is NaN, as the fit of such samples
+// (the reference's reflectors spread an infinite sample over all of them).
+__device__ __forceinline__ double fit_value(double a) { return a + (a - a); }
+template <int NC, bool TRI>
 __device__ __noinline__ void listed_ip_sum(const double* __restrict__ ip, const PatchWeights& pw, int it,
                                            double* __restrict__ rec) {
   const int lane = threadIdx.x & 31;
@@ -364,7 +367,7 @@ __device__ __noinline__ void listed_ip_sum(const double* __restrict__ ip, const 
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const double a = warp_sum(acc[c]);
-    if (lane == 0) rec[(size_t)v * NC + c] = a;
+    if (lane == 0) rec[(size_t)v * NC + c] = TRI ? fit_value(a) : a;
   }
 }
 
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(128) k_recover_tri(DevMesh m, const double* __
                                                      int n_list_blocks, const __grid_constant__ PatchWeights pw) {
   if ((int)blockIdx.x < n_list_blocks) {
     const int it = blockIdx.x * (128 / 32) + (threadIdx.x >> 5);
-    if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
+    if (it < pw.n) listed_ip_sum<NC, true>(ip, pw, it, rec);
     return;
   }
   const int v = (blockIdx.x - n_list_blocks) * blockDim.x + threadIdx.x;
@@ -2363,7 +2366,7 @@ __device__ __noinline__ bool tri_listed_sum(const DevMesh& m, const double* __re
       for (int c = 0; c < 3; ++c) acc[3 * r + c] += wk * (jinv.m[c][0] * d1 + jinv.m[c][1] * d2);
     }
   }
-  for (int k = 0; k < 3 * NCIN; ++k) acc[k] = warp_sum(acc[k]);
+  for (int k = 0; k < 3 * NCIN; ++k) acc[k] = fit_value(warp_sum(acc[k]));
   return true;
 }
 
@@ -2618,11 +2621,11 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
                                                         const double* __restrict__ w,
                                                         const unsigned char* __restrict__ listed,
                                                         int n_list_blocks, const __grid_constant__ PatchWeights pw,
-                                                        double* __restrict__ rec) {
+                                                        double* __restrict__ rec, ExpandList redo) {
   after_previous(ip, w, listed);
   if ((int)blockIdx.x < n_list_blocks) {
     const int it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
-    if (it < pw.n) listed_ip_sum<NC>(ip, pw, it, rec);
+    if (it < pw.n) listed_ip_sum<NC, LANES == 1>(ip, pw, it, rec);
     return;
   }
   const VertexLane vl = vertex_lane<LANES>(blockIdx.x - n_list_blocks, kBlock, threadIdx.x);
@@ -2643,8 +2646,33 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
   if (!mine || l) return;
+  if constexpr (LANES == 1) {
+    // values that are not finite, or near overflow: k_recover_redo's
+    bool big = false;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) big = big || bexp(acc[c]) >= 1923;
+    if (big) list_append(redo, v);
+  }
 #pragma unroll
   for (int c = 0; c < NC; ++c) rec[(size_t)v * NC + c] = acc[c];
+}
+
+// Triangles: the vertices whose weighted sums are not finite or near overflow, by
+// the sequence of the factors (their patches passed its rank tests).  A kernel
+// of its own: the call inside the recovery cost it 12 us of 152.
+template <int NC>
+__global__ void __launch_bounds__(128) k_recover_redo(DevMesh m, const double* __restrict__ ip,
+                                                      double* __restrict__ rec, const int* __restrict__ items,
+                                                      const int* __restrict__ count, int cap) {
+  after_previous(ip, items, count);
+  const int n = min(*count, cap);
+  for (long i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int v = items[i], beg = m.p_off[v], cnt = m.p_off[v + 1] - beg;
+    double Qc[kTriThreadRows][3], R[kTriR];
+    if (!tri_factor<kTriThreadRows>(m, beg, cnt, Qc, R)) continue;
+    R[6] = R[7] = R[8] = 0;
+    recover_tri_vertex<NC, kTriThreadRows, false, false>(m, v, beg, cnt, true, ip, nullptr, Qc, R, rec);
+  }
 }
 
 }  // namespace
@@ -2926,14 +2954,20 @@ void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, Expan
 }
 
 void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
-                        const PatchWeights& pw, double* rec, cudaStream_t s) {
+                        const PatchWeights& pw, double* rec, ExpandList redo, cudaStream_t s) {
   if (!m.V) return;
   const int nl = nblk((long)pw.n * 32);
   auto go = [&](int lanes, auto kernel) {
-    launch_after(m.early, kernel, nl + nblk((long)m.V * lanes), kBlock, s, m, ip, w, listed, nl, pw, rec);
+    launch_after(m.early, kernel, nl + nblk((long)m.V * lanes), kBlock, s, m, ip, w, listed, nl, pw, rec, redo);
   };
-  if (m.dim == 3) go(2, nc == 3 ? k_recover_w64<3, 2> : k_recover_w64<9, 2>);  // lanes: see the kernel
-  else go(1, nc == 3 ? k_recover_w64<3, 1> : k_recover_w64<9, 1>);
+  if (m.dim == 3) {
+    go(2, nc == 3 ? k_recover_w64<3, 2> : k_recover_w64<9, 2>);  // lanes: see the kernel
+    return;
+  }
+  go(1, nc == 3 ? k_recover_w64<3, 1> : k_recover_w64<9, 1>);
+  // set up early on any mesh: a block per SM, which as a rule finds nothing
+  launch_after(true, nc == 3 ? k_recover_redo<3> : k_recover_redo<9>, std::min(nblk(m.V, 128), 152), 128, s, m, ip, rec,
+               redo.items, redo.count, redo.cap);
 }
 
 }  // namespace sprg
