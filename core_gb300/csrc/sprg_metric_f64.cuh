@@ -359,8 +359,10 @@ static __device__ __noinline__ double log_point_ref(const ref::V3& x0, const ref
 // MetricSizeField::measure under LogAnisoSizeField (ma/maSize.cc:158-216,
 // 508-523): two Gauss points, the ends' log-metrics la, lb interpolated.
 // Entries above 200 in magnitude (sizes beyond e^-100: the absolute deflation
-// test is then near the rounding) or not finite, and a first column the
-// reduction would leave alone (below 1e-10, not 0), take the sequence itself.
+// test is then near the rounding) or not finite, a first column the
+// reduction would leave alone (below 1e-10, not 0), and squared lengths outside
+// [2^-600, 2^600] or not finite (edges with infinite, huge or equal ends) take
+// the sequence itself.
 __device__ __forceinline__ double log_metric_length(const ref::V3& x0, const ref::V3& x1,
                                                     const double* __restrict__ la, const double* __restrict__ lb,
                                                     bool* ok) {
@@ -382,8 +384,9 @@ __device__ __forceinline__ double log_metric_length(const ref::V3& x0, const ref
     const double col = fmax(fabs(a[1]), fabs(a[2]));
     const bool fast = big <= 200.0 && a[0] == a[0] && a[1] == a[1] && a[2] == a[2] && a[3] == a[3] && a[4] == a[4] &&
                       a[5] == a[5] && (a[2] == 0.0 || col >= 1e-10);
-    if (fast) {
-      if (log_length2(a, d, &s) != 1) *ok = false;
+    const int status = fast ? log_length2(a, d, &s) : 0;
+    if (fast && (unsigned)(bexp(s) - 423) <= 1200u) {
+      if (status != 1) *ok = false;
       L += 0.5 * sqrt(s);
     } else {
       L += log_point_ref(x0, x1, la, lb, gp[p], ok);
