@@ -89,13 +89,13 @@ struct sprg_ctx {
   // FP64 recovery on tets: per-mesh QR weights and the listed patches
   DevBuf qw, qwlisted, qwitems, qwcount;
   bool qw_ready = false;
-  // mixed-precision anisotropic pass: triangle patch weights and their
-  // listed vertices (per mesh), FP32 metric records, guarded edges
-  // triangles' refined patch weights (the FP64 anisotropic pass) and the number of patches
-  // too large for them
+  // triangles' refined patch weights (the FP64 anisotropic pass) and the number of
+  // patches too large for them
   bool rw_ready = false, rw_none = false;
   int n_rw_big = 0;
   DevBuf rw, rwlisted, rwitems, rwcount;
+  // mixed-precision anisotropic pass: triangle patch weights and their
+  // listed vertices (per mesh), FP32 metric records, guarded edges
   DevBuf tw, twlisted, twitems, twcount, met32, qrec32, agitems, agcount, kidx, kval, klen, rec9, cj64, qties;
   bool tw_ready = false;
   int op_kc = 3;  // operator components per slot (2 on a mesh in the z = 0 plane)
@@ -455,12 +455,11 @@ PatchWeights patch_weights(sprg_ctx* c, PatchCache& pc) {
                       P<DevStatus>(c->status)};
 }
 
-// Listed patches: grow them on the first pass (recording the final element
-// sets), afterwards one QR fit per cached set.
-// Once a patch cache exists, the QR of each cached patch runs once (per mesh)
-// into weights, and the passes on tets and the mixed one on triangles take
-// weighted sums.  Runs on
-// the context stream (it reads the patch sizes back).
+// Listed patches grow on the first pass (recording the final element sets);
+// the QR of each cached patch then runs once (per mesh) into weights, and every
+// pass takes weighted sums, but for triangle meshes with patches on the warp
+// path, which fit them (listed_fits).  Runs on the context stream (it reads the
+// patch sizes back).
 int ensure_cache_weights(sprg_ctx* c, PatchCache& pc) {
   if (!pc.valid || pc.w_ready || pc.count <= 0) return SPRG_OK;
   std::vector<int> n((size_t)pc.count);
@@ -591,7 +590,7 @@ int step_recover(sprg_ctx* c) {
   ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + nc + 1));
   if (m.dim == 3) {
     // tets: the per-mesh FP64 QR weights, a weighted sum per vertex; the
-    // listed patches (growth, size) through the slab fits
+    // listed patches (growth, size) through their own weights
     ENSURE(c->qwitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
     ENSURE(c->qwcount, sizeof(int));
     const ExpandList lst{P<int>(c->qwitems), P<int>(c->qwcount), m.V};
@@ -2793,7 +2792,10 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
   ENSURE(c->frames9, sizeof(double) * 9 * (size_t)m.V);
   ENSURE(c->L, sizeof(double) * (size_t)m.E);
   if ((rc = reset_status(c))) return rc;
-  CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
+  if (c->precision == SPRG_FP32 || reinterpret_cast<uintptr_t>(d_u) % alignof(double)) {
+    CK(cudaMemcpyAsync(c->f.p, d_u, sizeof(double) * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
+    d_u = P<double>(c->f);
+  }
   if (c->precision == SPRG_FP32) return aniso_pass_mixed(c, eps, h_min, h_max, d_split_bits, d_collapse_bits, d_quality);
   if (m.dim == 2) {
     // both recoveries' buffers before the weights: if these have to go for a
@@ -2803,9 +2805,10 @@ int sprg_aniso_estimate_and_mark_resident(sprg_ctx* c, const double* d_u, double
     ENSURE(c->slab, sizeof(double) * (size_t)expand_grid() * expand_max_elems() * (4 + 9 + 1));
   }
   // recovered gradient, then the recovered gradient of it (nodal Hessian)
-  if ((rc = step_grad(c, P<double>(c->f), 1)) || (rc = aniso_recover(c))) return rc;
-  CK(cudaMemcpyAsync(c->f.p, c->rec.p, sizeof(double) * 3 * (size_t)m.V, cudaMemcpyDeviceToDevice, c->stream));
-  if ((rc = step_grad(c, P<double>(c->f), 3)) || (rc = aniso_recover(c))) return rc;
+  // (field and gradient read where they stand: the second recovery overwrites
+  // the latter after that)
+  if ((rc = step_grad(c, d_u, 1)) || (rc = aniso_recover(c))) return rc;
+  if ((rc = step_grad(c, P<double>(c->rec), 3)) || (rc = aniso_recover(c))) return rc;
   PB("hessian_metric");
   launch_hessian_metric(m, P<double>(c->rec), eps, h_min, h_max, P<double>(c->sizes3), P<double>(c->frames9),
                         c->stream);

@@ -218,11 +218,12 @@ __global__ void __launch_bounds__(kBlock) k_recover_list(DevMesh m, const double
 constexpr int kTriR = 9;               // planes of R: 6 entries, 3 reciprocals
 constexpr unsigned char kTriPlain = 64;  // flag of a factor that takes plain divisions and sums
 
-template <int MAXM>
+// U: how far the loops are unrolled (1: arrays in local memory, few registers)
+template <int MAXM, int U = MAXM>
 __device__ __forceinline__ bool tri_factor(const DevMesh& m, int beg, int cnt, double Qc[MAXM][3], double* Rr) {
   constexpr int NT = 3;
   double R[MAXM][NT];
-#pragma unroll
+#pragma unroll U
   for (int i = 0; i < MAXM; ++i) {
     R[i][0] = R[i][1] = R[i][2] = 0;
     if (i < cnt) {
@@ -233,53 +234,53 @@ __device__ __forceinline__ bool tri_factor(const DevMesh& m, int beg, int cnt, d
     }
   }
   double H[NT][MAXM];  // the reflectors
-#pragma unroll
+#pragma unroll U
   for (int k = 0; k < NT; ++k) {
     double cn = 0;
-#pragma unroll
+#pragma unroll U
     for (int i = k; i < MAXM; ++i)
       if (i < cnt) cn += R[i][k] * R[i][k];
     cn = sqrt(cn);
     if (cn < 1e-10) return false;
-#pragma unroll
+#pragma unroll U
     for (int i = 0; i < MAXM; ++i) H[k][i] = (i >= k && i < cnt) ? R[i][k] : 0.0;
     H[k][k] += ((R[k][k] < 0) ? -1 : 1) * cn;
     double rn = 0;
-#pragma unroll
+#pragma unroll U
     for (int i = k; i < MAXM; ++i)
       if (i < cnt) rn += H[k][i] * H[k][i];
     rn = sqrt(rn);
-#pragma unroll
+#pragma unroll U
     for (int i = k; i < MAXM; ++i)
       if (i < cnt) H[k][i] /= rn;
-#pragma unroll
+#pragma unroll U
     for (int j = k; j < NT; ++j) {
       double dot = 0;
-#pragma unroll
+#pragma unroll U
       for (int i = k; i < MAXM; ++i)
         if (i < cnt) dot += R[i][j] * H[k][i];
-#pragma unroll
+#pragma unroll U
       for (int i = k; i < MAXM; ++i)
         if (i < cnt) R[i][j] -= 2 * dot * H[k][i];
     }
   }
   // the first NT columns of Q, row by row
-#pragma unroll
+#pragma unroll U
   for (int r = 0; r < MAXM; ++r) {
     double q[MAXM];
-#pragma unroll
+#pragma unroll U
     for (int j = 0; j < MAXM; ++j) q[j] = (j == r) ? 1.0 : 0.0;
-#pragma unroll
+#pragma unroll U
     for (int k = 0; k < NT; ++k) {
       double dot = 0;
-#pragma unroll
+#pragma unroll U
       for (int j = k; j < MAXM; ++j)
         if (j < cnt) dot += q[j] * H[k][j];
-#pragma unroll
+#pragma unroll U
       for (int j = k; j < MAXM; ++j)
         if (j < cnt) q[j] -= 2 * dot * H[k][j];
     }
-#pragma unroll
+#pragma unroll U
     for (int i = 0; i < NT; ++i) Qc[r][i] = q[i];
   }
   Rr[0] = R[0][0]; Rr[1] = R[0][1]; Rr[2] = R[0][2];
@@ -415,6 +416,33 @@ __device__ __forceinline__ void recover_tri_vertex(const DevMesh& m, int v, int 
     sres += x1 * xv.v[0];
     sres += x2 * xv.v[1];
     o[comp(c)] = sres;
+  }
+}
+
+// A vertex that the refined weights do not serve (its patch passed their rank
+// tests, which are the factors'), rolled up to stay out of its caller's registers.
+template <int NC>
+__device__ __noinline__ void recover_tri_in_place(const DevMesh& m, int v, int beg, int cnt,
+                                                  const double* __restrict__ ip, double* __restrict__ rec) {
+  double Qc[kTriThreadRows][3], R[6];
+  if (!tri_factor<kTriThreadRows, 1>(m, beg, cnt, Qc, R)) return;
+  const V3 xv = load_xyz(m.xyz, v);
+#pragma unroll 1
+  for (int c = 0; c < NC; ++c) {
+    double y0 = 0, y1 = 0, y2 = 0;
+#pragma unroll 1
+    for (int r = 0; r < cnt; ++r) {
+      const double b = ip[(size_t)m.p_el[beg + r] * NC + c];
+      y0 += Qc[r][0] * b;
+      y1 += Qc[r][1] * b;
+      y2 += Qc[r][2] * b;
+    }
+    const double x2 = y2 / R[5], x1 = (y1 - R[4] * x2) / R[3], x0 = (y0 - R[1] * x1 - R[2] * x2) / R[0];
+    double sres = 0;
+    sres += x0 * 1.0;
+    sres += x1 * xv.v[0];
+    sres += x2 * xv.v[1];
+    rec[(size_t)v * NC + c] = sres;
   }
 }
 
@@ -757,18 +785,6 @@ __global__ void __launch_bounds__(32) k_cached_weights(DevMesh m, int n_cached, 
 // ---------------------------------------------------------------------
 // Size factor
 // ---------------------------------------------------------------------
-__device__ __forceinline__ double block_sum(double x, double* sh) {
-  x = warp_sum(x);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = x;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[i];
-  return t;
-}
-
 // one block: fixed-order reduction of the partials, then the size factor
 // (the FP32 error kernel's last block runs the same function)
 __global__ void __launch_bounds__(kBlock) k_size_factor(const double* __restrict__ partials, int nb, int mode,
@@ -1576,7 +1592,7 @@ __global__ void __launch_bounds__(kBlock) k_mark_quality(int T, const double* __
 // w = Q_c R^-T t (Q_c the first NT columns of Q, t = [1, x_v, y_v]).  The QR
 // is the reference's (as in k_recover_tri); listed: patches the weights do
 // not cover (fewer than NT or more than MAXM elements, rank deficient),
-// which take the FP64 fit paths every pass.
+// which take the weights of their (grown) patches.
 //
 // REFINED (the FP64 anisotropic pass): one step of correction with the moments Sum w = 1,
 // Sum w (p - x_v) = 0 in coordinates about the vertex.  The QR's are absolute,
@@ -2528,7 +2544,7 @@ __global__ void __launch_bounds__(kBlock) k_count_out_of_range(long long n, cons
 // from R and [z; 0] taken through the reflectors in reverse order.  Every
 // later FP64 recovery of the mesh is a weighted sum per vertex.  Patches
 // with fewer than 4 or more than 32 elements or rank deficient are listed
-// (lst) for the FP64 slab fits.
+// (lst): their grown patches' weights come from k_cached_weights.
 // ---------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock) k_qr_weights(DevMesh m, double* __restrict__ w,
                                                        unsigned char* __restrict__ listed, ExpandList lst) {
@@ -2616,7 +2632,12 @@ __global__ void __launch_bounds__(kBlock) k_qr_weights(DevMesh m, double* __rest
 // the extra sums are 3 of 72; 96^3 box: 134 us, 197 with one lane, 159 with four.
 // Triangles one: six elements hide no sum (1024^2 square, both recoveries: 152
 // us, 192 with two).
-template <int NC, int LANES>
+// REDO (triangles): what becomes of values that are not finite or near overflow,
+// which are the factors' sequence's: in place (the call costs registers: 164 us
+// against 152 at 1024^2) or listed for k_recover_redo (a launch: 1 us of the 37 of a
+// 128^2 square's pass); see launch_recover_w64.
+enum Redo { kRedoNone, kRedoHere, kRedoList };
+template <int NC, int LANES, Redo REDO>
 __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double* __restrict__ ip,
                                                         const double* __restrict__ w,
                                                         const unsigned char* __restrict__ listed,
@@ -2646,20 +2667,21 @@ __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double*
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
   if (!mine || l) return;
-  if constexpr (LANES == 1) {
-    // values that are not finite, or near overflow: k_recover_redo's
+  if constexpr (REDO != kRedoNone) {
     bool big = false;
 #pragma unroll
     for (int c = 0; c < NC; ++c) big = big || bexp(acc[c]) >= 1923;
-    if (big) list_append(redo, v);
+    if (big && REDO == kRedoList) list_append(redo, v);
+    if (big && REDO == kRedoHere) {
+      recover_tri_in_place<NC>(m, v, beg, end - beg, ip, rec);
+      return;
+    }
   }
 #pragma unroll
   for (int c = 0; c < NC; ++c) rec[(size_t)v * NC + c] = acc[c];
 }
 
-// Triangles: the vertices whose weighted sums are not finite or near overflow, by
-// the sequence of the factors (their patches passed its rank tests).  A kernel
-// of its own: the call inside the recovery cost it 12 us of 152.
+// the vertices k_recover_w64 listed, by the sequence of the factors
 template <int NC>
 __global__ void __launch_bounds__(128) k_recover_redo(DevMesh m, const double* __restrict__ ip,
                                                       double* __restrict__ rec, const int* __restrict__ items,
@@ -2667,11 +2689,8 @@ __global__ void __launch_bounds__(128) k_recover_redo(DevMesh m, const double* _
   after_previous(ip, items, count);
   const int n = min(*count, cap);
   for (long i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int v = items[i], beg = m.p_off[v], cnt = m.p_off[v + 1] - beg;
-    double Qc[kTriThreadRows][3], R[kTriR];
-    if (!tri_factor<kTriThreadRows>(m, beg, cnt, Qc, R)) continue;
-    R[6] = R[7] = R[8] = 0;
-    recover_tri_vertex<NC, kTriThreadRows, false, false>(m, v, beg, cnt, true, ip, nullptr, Qc, R, rec);
+    const int v = items[i], beg = m.p_off[v];
+    recover_tri_in_place<NC>(m, v, beg, m.p_off[v + 1] - beg, ip, rec);
   }
 }
 
@@ -2961,10 +2980,14 @@ void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double
     launch_after(m.early, kernel, nl + nblk((long)m.V * lanes), kBlock, s, m, ip, w, listed, nl, pw, rec, redo);
   };
   if (m.dim == 3) {
-    go(2, nc == 3 ? k_recover_w64<3, 2> : k_recover_w64<9, 2>);  // lanes: see the kernel
+    go(2, nc == 3 ? k_recover_w64<3, 2, kRedoNone> : k_recover_w64<9, 2, kRedoNone>);  // lanes: see the kernel
     return;
   }
-  go(1, nc == 3 ? k_recover_w64<3, 1> : k_recover_w64<9, 1>);
+  if (m.V < 1 << 18) {  // less than two waves of blocks: registers cost nothing, a launch does
+    go(1, nc == 3 ? k_recover_w64<3, 1, kRedoHere> : k_recover_w64<9, 1, kRedoHere>);
+    return;
+  }
+  go(1, nc == 3 ? k_recover_w64<3, 1, kRedoList> : k_recover_w64<9, 1, kRedoList>);
   // set up early on any mesh: a block per SM, which as a rule finds nothing
   launch_after(true, nc == 3 ? k_recover_redo<3> : k_recover_redo<9>, std::min(nblk(m.V, 128), 152), 128, s, m, ip, rec,
                redo.items, redo.count, redo.cap);

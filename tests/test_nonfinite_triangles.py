@@ -64,3 +64,25 @@ def test_anisotropic_pass(gpu_lib, n, bad):
             sure = ~(np.abs(L - 1.5) < 1e-9) & ~(np.abs(L - 0.5) < 1e-9)
             assert np.array_equal(((b[0][e >> 5] >> (e & 31)) & 1)[sure], (L > 1.5)[sure]), v
             assert np.array_equal(((b[1][e >> 5] >> (e & 31)) & 1)[sure], (L < 0.5)[sure]), v
+
+
+@pytest.mark.parametrize("n", [520])
+def test_anisotropic_pass_on_a_large_square(gpu_lib, n):
+    """From 2^18 vertices on such vertices are listed for a kernel of their own."""
+    import torch
+    import core_gb300 as cg
+    m, u = square(n)
+    assert m.n_verts > 1 << 18
+    rng = np.random.default_rng(1)
+    u[rng.choice(m.n_verts, 300, replace=False)] = np.inf
+    u[rng.choice(m.n_verts, 300, replace=False)] = -1e306
+    bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+    d_u = torch.from_numpy(u).cuda()
+    torch.cuda.synchronize()
+    with cg.Context(m) as c:
+        want = c.recoverField(c.getGradIPField(c.recoverField(c.getGradIPField(u))))
+        c.aniso_estimate_and_mark_resident(d_u.data_ptr(), 0.1, 0.1 / n, 1.0, bits[0].data_ptr(), bits[1].data_ptr())
+        torch.cuda.synchronize()
+        got = c.debug_read("rec", np.float64, 9 * m.n_verts).reshape(-1, 9)
+    assert np.isnan(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))

@@ -39,3 +39,26 @@ def test_field_at_any_address(gpu_lib, precision, offset, graph):
             assert np.array_equal((b[0][e >> 5] >> (e & 31)) & 1, flags & 1)
             assert np.array_equal((b[1][e >> 5] >> (e & 31)) & 1, (flags >> 2) & 1)
         c.set_stream(0)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("offset", [0, 4, 8])
+def test_anisotropic_field_at_any_address(gpu_lib, precision, offset):
+    import torch
+    import core_gb300 as cg
+    from core_gb300 import workload
+    m, u, (eps, hmin, hmax) = workload.aniso2d(24)
+    out = []
+    for at in (0, offset):
+        raw = torch.zeros(8 * m.n_verts + 16, dtype=torch.uint8, device="cuda")
+        field = raw[at:at + 8 * m.n_verts]
+        field.copy_(torch.from_numpy(u.view(np.uint8)))
+        bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+        q = torch.zeros(m.n_elems, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        with cg.Context(m, precision=precision) as c:
+            c.aniso_estimate_and_mark_resident(field.data_ptr(), eps, hmin, hmax, bits[0].data_ptr(), bits[1].data_ptr(),
+                                               q.data_ptr())
+            torch.cuda.synchronize()
+        out.append((bits.cpu().numpy(), q.cpu().numpy()))
+    assert out[0][0].any() and np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
