@@ -1,11 +1,13 @@
-// FP64 element kernels of the parity form: the per-mesh element records and
-// the integration-point gradients taken from them.
+// FP64 element and edge kernels of the parity form: the per-mesh element records,
+// the integration-point gradients taken from them, errors and sizes, lengths.
 //
-// Compiled with -fmad=false; every result is bitwise the reference's
-// operation order (sprg_refmath.cuh).  Operations whose result the
-// reference's own sequence fixes in advance are left out (products with the
-// shape gradients' 0, 1 and -1, sums with 0), and quotients by one common
-// divisor come from its rounded reciprocal with exact residuals.
+// Compiled with -fmad=false.  Records, gradients and the lengths of given sizes
+// are bitwise the reference's operation order (sprg_refmath.cuh): operations
+// whose result the reference's own sequence fixes in advance are left out
+// (products with the shape gradients' 0, 1 and -1, sums with 0), and quotients by
+// one common divisor come from its rounded reciprocal with exact residuals.
+// Errors and their powers (k_error) and the pass's lengths (k_measure_mark) are
+// sums and quotients in an order of their own, with fused operations.
 #include "sprg_internal.h"
 #include "sprg_metric_f64.cuh"
 #include "sprg_reduce.cuh"

@@ -166,8 +166,9 @@ void launch_esize_f64(const DevMesh& m, const double* geo, const double* out3, i
 void launch_average(const DevMesh& m, const double* esize, double* size, cudaStream_t s);
 // isotropic lengths of given sizes, bitwise the reference's
 void launch_measure_iso_f64(const DevMesh& m, const double* size, double* L, cudaStream_t s);
-// per-mesh Euclidean edge lengths (E doubles); the pass's lengths (a few ulps,
-// bitwise near 0.5 and 1.5) with the predicate bitmaps, len null: in place
+// per mesh, half the Euclidean edge lengths (E doubles); the pass's lengths (not
+// the sequence's bits but near 0.5 and 1.5) with the predicate bitmaps, len null:
+// in place
 void launch_edge_records(const DevMesh& m, double* len, cudaStream_t s);
 void launch_measure_mark_f64(const DevMesh& m, const double* len, const double* size, double* L, uint32_t* split,
                              uint32_t* collapse, cudaStream_t s);

@@ -1305,8 +1305,8 @@ int infer_grid() {
     cudaFuncSetAttribute(k_mlp_infer<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, InferSmem<KMAX>::kTotal);
     cudaFuncSetAttribute(k_mlp_infer<KMAX>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mlp_infer<KMAX>, kInferThreads, InferSmem<KMAX>::kTotal);
-    // KMAX = 64: two blocks per SM (64 registers x 512 threads, ~92 KB of
-    // shared memory, 128 tensor-memory columns each)
+    // KMAX = 64: two blocks per SM (64 registers x 512 threads, 114 KB of
+    // shared memory, 256 tensor-memory columns each)
     grid = (sms > 0 ? sms : 152) * (per > 0 ? per : 1);
     if (KMAX == 64 && per < 2) grid = (sms > 0 ? sms : 152) * 2;
   }

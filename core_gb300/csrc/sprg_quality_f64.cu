@@ -1,7 +1,8 @@
 // FP64 mean-ratio qualities (measureTetQuality / measureTriQuality with
 // useMax = true, ma/maQuality.cc:83-167) under isotropic, anisotropic and
-// log-interpolated size fields.  Compiled with -fmad=false; every quality is
-// bitwise the reference's sequence.
+// log-interpolated size fields.  Compiled with -fmad=false; the calls' qualities
+// are bitwise the reference's sequence, the anisotropic pass's on triangles
+// (PASS) as near the exact values.
 #include "sprg_internal.h"
 #include "sprg_metric_f64.cuh"
 
@@ -153,10 +154,11 @@ __device__ __forceinline__ double quality_of(const V3* e, const V3* o, double* s
   return ratio_of<D>((D == 3 ? 1.0 / 6.0 : 1.0 / 2.0) * dV, acc);
 }
 
-// PASS: the anisotropic passes' qualities, good to a few ulps: the squared
-// lengths as they are, without the reference's root and square of each, the
-// third edge as a sum, fused products (about 40 FP64 operations a triangle of
-// 115)
+// PASS: the anisotropic passes' qualities: the squared lengths as they are,
+// without the reference's root and square of each, the third edge as a sum,
+// fused products (about 40 FP64 operations a triangle of 115).  Against extended
+// precision 2.2 to 2.5 units of 2^-53 off (rms; sizes 1:2 to 1:500000 apart), the
+// sequence 2.7 to 3.0.
 template <int D, bool PASS>
 __device__ __forceinline__ double element_quality(const V3* x, const M3& Q) {
   double s, r;
