@@ -449,7 +449,10 @@ const char* sprg_tuning_report(sprg_ctx* ctx);
 /* Capture the resident pass (sprg_estimate_and_mark_resident with these
    device buffers) into a CUDA graph, after one ordinary pass; needs a caller
    stream (sprg_set_stream).  sprg_graph_replay relaunches it on that stream:
-   the caller refreshes d_u in place between replays. */
+   the caller refreshes d_u in place between replays.  After a call that moved
+   one of the context's buffers (a larger field, memory given back, another
+   tiling or batch) the next replay runs the pass with these buffers and the
+   settings of the capture, waits for it and captures it again. */
 int sprg_graph_capture(sprg_ctx* ctx, const double* d_u, double adapt_ratio, uint32_t* d_split_bits,
                        uint32_t* d_collapse_bits);
 int sprg_graph_replay(sprg_ctx* ctx);
