@@ -213,6 +213,7 @@ int fail(sprg_ctx* c, int code, const std::string& msg) {
 
 int cuda_fail(sprg_ctx* c, cudaError_t e, const char* where) {
   std::string msg = std::string(where) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();  // reported here: no later call's check finds it
   int code = (e == cudaErrorMemoryAllocation) ? SPRG_ENOMEM : SPRG_ECUDA;
   return fail(c, code, msg);
 }
@@ -229,13 +230,13 @@ void release(DevBuf& b) {
   b.bytes = 0;
 }
 
-// one attempt at device memory; the test hooks' failures are made here, on the
-// host, and look like cudaMalloc's own
+// one attempt at device memory; the test hooks' failures are made here, by asking
+// for more than there can be, so that they leave behind what cudaMalloc's do
 cudaError_t device_alloc(sprg_ctx* c, void** p, size_t bytes) {
   *p = nullptr;
   if (c->alloc_fail_in == 0) {
     if (c->alloc_fail_n > 0 && --c->alloc_fail_n == 0) c->alloc_fail_in = -1;
-    return cudaErrorMemoryAllocation;
+    return cudaMalloc(p, (size_t)1 << 60);
   }
   if (c->alloc_fail_in > 0) --c->alloc_fail_in;
   return cudaMalloc(p, bytes);

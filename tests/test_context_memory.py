@@ -261,3 +261,25 @@ def test_failed_update_after_everything_went(gpu_lib, precision):
         c.update_mesh(m1)
         assert same(c.estimate_and_mark(u1, 0.1)[:4], fresh(m1, u1, precision))
         c.set_stream(0)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "learned"])
+def test_a_failed_call_leaves_no_error_behind(gpu_lib, precision):
+    """The error of a failed allocation is that call's alone: the next calls, on
+    this context and on another, do not report it."""
+    import core_gb300 as cg
+    m, u = box(5)
+    want = fresh(m, u, precision)
+    for k in (0, 2, 5):
+        with cg.Context(m, precision=precision) as c:
+            fail(c, k, 100)
+            with pytest.raises(cg.SprgError) as e:
+                c.estimate_and_mark(u, 0.1)
+            assert e.value.code == 4
+            with cg.Context(m, precision=precision) as other:
+                assert same(other.estimate_and_mark(u, 0.1)[:4], want)
+            with pytest.raises(cg.SprgError) as e:
+                c.estimate_and_mark(u, 0.1)
+            assert e.value.code == 4
+            c.test_hooks()
+            assert same(c.estimate_and_mark(u, 0.1)[:4], want)
