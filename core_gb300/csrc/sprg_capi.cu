@@ -1046,10 +1046,15 @@ int sprg_update_mesh(sprg_ctx* c, const sprg_mesh_delta* d) {
   c->launches = 0;
   if (!c->updated) CK(cudaEventCreateWithFlags(&c->updated, cudaEventDisableTiming));
   // passes on this mesh are done before its arrays change, on whatever stream
-  // they run (an earlier stream's handle may be gone, so the device is asked)
-  if (c->switched) CK(cudaDeviceSynchronize());
-  else CK(cudaStreamSynchronize(c->stream));
-  c->switched = false;
+  // they run.  An earlier stream's handle may be gone, and a device
+  // synchronisation is refused while another thread captures: freeing memory
+  // waits for all of the device's work and is not.
+  if (c->switched) {
+    ENSURE(c->ubad, sizeof(unsigned long long));
+    release(c->ubad);
+    c->switched = false;
+  }
+  CK(cudaStreamSynchronize(c->stream));
   // ---- the new arrays, in the spare buffers: kept rows copied, listed rows
   // scattered from one staging buffer (each kind its own part, so that
   // nothing waits in between)
