@@ -393,6 +393,14 @@ int ensure_stage(sprg_ctx* c) {
   return SPRG_OK;
 }
 
+// A host list of this call's frame to the device.  On the context's stream: the
+// default stream's blocking copy may return while its last part is still on the
+// way, and no kernel of another stream waits for that.
+cudaError_t upload_now(sprg_ctx* c, DevBuf& b, const void* host, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(b.p, host, bytes, cudaMemcpyHostToDevice, c->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
 // the device status word, read back with the stream's other results
 int sync_and_status(sprg_ctx* c) {
   int rc = ensure_stage(c);
@@ -1798,8 +1806,7 @@ static int build_tiles(sprg_ctx* c, int only = -1) {
   if (c->e2e_exec || c->graph_exec) graphs_stale(c);
   CK(cudaStreamSynchronize(c->stream));
   ENSURE(c->btiles, sizeof(int4) * (tiles.empty() ? 1 : tiles.size()));
-  if (!tiles.empty())
-    CK(cudaMemcpy(c->btiles.p, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
+  if (!tiles.empty()) CK(upload_now(c, c->btiles, tiles.data(), sizeof(int4) * tiles.size()));
   c->n_tiles = (int)tiles.size();
   return SPRG_OK;
 }
@@ -2878,10 +2885,10 @@ int sprg_set_batch(sprg_ctx* c, int n_meshes, const int64_t* vert_offsets, const
   ENSURE(c->bsegoff, sizeof(int) * segoff.size());
   ENSURE(c->bseg, sizeof(int2) * seg.size());
   ENSURE(c->bratios, sizeof(double) * n_meshes);
-  CK(cudaMemcpy(c->bvoff.p, voff.data(), sizeof(int) * voff.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->bsegoff.p, segoff.data(), sizeof(int) * segoff.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->bseg.p, seg.data(), sizeof(int2) * seg.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->bratios.p, adapt_ratios, sizeof(double) * n_meshes, cudaMemcpyHostToDevice));
+  CK(upload_now(c, c->bvoff, voff.data(), sizeof(int) * voff.size()));
+  CK(upload_now(c, c->bsegoff, segoff.data(), sizeof(int) * segoff.size()));
+  CK(upload_now(c, c->bseg, seg.data(), sizeof(int2) * seg.size()));
+  CK(upload_now(c, c->bratios, adapt_ratios, sizeof(double) * n_meshes));
   c->batch_n = n_meshes;
   c->batch_nseg = (int)seg.size();
   if (recapture) {
