@@ -123,6 +123,7 @@ struct sprg_ctx {
   int bin_lanes[4] = {4, 4, 4, 4};
   int tile_verts = 256, grid_per_sm = 8, n_tiles = 0, n_sms = 152;
   int tile_mode = -1;  // the lane mode every tile shares, or -1
+  std::vector<int4> tiles;  // host copy of btiles (its upload may still read it)
   std::string tune_json;
   // CUDA graph of the resident pass (sprg_graph_capture / sprg_graph_replay)
   // and what it was captured with; stale: one of the context's buffers has
@@ -393,12 +394,12 @@ int ensure_stage(sprg_ctx* c) {
   return SPRG_OK;
 }
 
-// A host list of this call's frame to the device.  On the context's stream: the
-// default stream's blocking copy may return while its last part is still on the
-// way, and no kernel of another stream waits for that.
-cudaError_t upload_now(sprg_ctx* c, DevBuf& b, const void* host, size_t bytes) {
-  const cudaError_t e = cudaMemcpyAsync(b.p, host, bytes, cudaMemcpyHostToDevice, c->stream);
-  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+// A host list to the device, on the context's stream: behind a pass in flight that
+// still reads the old one, before the next.  (The default stream's blocking copy
+// may return while its last part is still on the way, and no kernel of another
+// stream waits for that.)  The list stays until the stream was waited for.
+cudaError_t upload(sprg_ctx* c, DevBuf& b, const void* host, size_t bytes) {
+  return cudaMemcpyAsync(b.p, host, bytes, cudaMemcpyHostToDevice, c->stream);
 }
 
 // the device status word, read back with the stream's other results
@@ -1786,7 +1787,9 @@ static int build_bins(sprg_ctx* c) {
 // `only` >= 0 keeps one bin (autotuning).  A bin in the sliced mode without
 // the sliced copy, or with tiles that do not start on a slice, takes 1 lane.
 static int build_tiles(sprg_ctx* c, int only = -1) {
-  std::vector<int4> tiles;
+  std::vector<int4>& tiles = c->tiles;
+  CK(cudaStreamSynchronize(c->stream));  // the last upload
+  tiles.clear();
   int first = 0;
   c->tile_mode = -2;  // no tile yet
   for (int b = 0; b < 4; ++b) {
@@ -1801,12 +1804,10 @@ static int build_tiles(sprg_ctx* c, int only = -1) {
     }
     first += c->bin_count[b];
   }
-  // a captured pass has the old list's length and lane mode, a pass in flight
-  // still reads the old list
+  // a captured pass has the old list's length and lane mode
   if (c->e2e_exec || c->graph_exec) graphs_stale(c);
-  CK(cudaStreamSynchronize(c->stream));
   ENSURE(c->btiles, sizeof(int4) * (tiles.empty() ? 1 : tiles.size()));
-  if (!tiles.empty()) CK(upload_now(c, c->btiles, tiles.data(), sizeof(int4) * tiles.size()));
+  if (!tiles.empty()) CK(upload(c, c->btiles, tiles.data(), sizeof(int4) * tiles.size()));
   c->n_tiles = (int)tiles.size();
   return SPRG_OK;
 }
@@ -2875,8 +2876,7 @@ int sprg_set_batch(sprg_ctx* c, int n_meshes, const int64_t* vert_offsets, const
   // again where the counts that its launches hold differ.
   const bool captured = (c->graph_exec || c->graph_stale) && c->graph_of.batch_n;
   const bool recapture = captured && (c->graph_of.batch_n != n_meshes || c->graph_of.batch_nseg != (int)seg.size());
-  CK(cudaStreamSynchronize(c->stream));  // a pass in flight
-  c->batch_n = 0;                        // none until all of it is in place
+  c->batch_n = 0;  // none until all of it is in place
   if (recapture) {
     graphs_stale(c);
     c->graph_stale = false;
@@ -2885,10 +2885,11 @@ int sprg_set_batch(sprg_ctx* c, int n_meshes, const int64_t* vert_offsets, const
   ENSURE(c->bsegoff, sizeof(int) * segoff.size());
   ENSURE(c->bseg, sizeof(int2) * seg.size());
   ENSURE(c->bratios, sizeof(double) * n_meshes);
-  CK(upload_now(c, c->bvoff, voff.data(), sizeof(int) * voff.size()));
-  CK(upload_now(c, c->bsegoff, segoff.data(), sizeof(int) * segoff.size()));
-  CK(upload_now(c, c->bseg, seg.data(), sizeof(int2) * seg.size()));
-  CK(upload_now(c, c->bratios, adapt_ratios, sizeof(double) * n_meshes));
+  CK(upload(c, c->bvoff, voff.data(), sizeof(int) * voff.size()));
+  CK(upload(c, c->bsegoff, segoff.data(), sizeof(int) * segoff.size()));
+  CK(upload(c, c->bseg, seg.data(), sizeof(int2) * seg.size()));
+  CK(upload(c, c->bratios, adapt_ratios, sizeof(double) * n_meshes));
+  CK(cudaStreamSynchronize(c->stream));
   c->batch_n = n_meshes;
   c->batch_nseg = (int)seg.size();
   if (recapture) {
