@@ -620,10 +620,9 @@ int step_recover(sprg_ctx* c) {
     int rc;
     if ((rc = ensure_listed(c, pc, lst, -1))) return rc;
     PB("recover_f64");
-    launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->qw), P<unsigned char>(c->qwlisted), patch_weights(c, pc),
-                       P<double>(c->rec), ExpandList{}, c->stream);
+    c->launches += launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->qw), P<unsigned char>(c->qwlisted),
+                                      patch_weights(c, pc), P<double>(c->rec), ExpandList{}, c->stream);
     PE();
-    c->launches += 1;
     return check_launch(c, "recover");
   }
   ENSURE(c->xitems, sizeof(int) * (size_t)(m.V > 0 ? m.V : 1));
@@ -2190,11 +2189,10 @@ static int aniso_recover(sprg_ctx* c) {
     return step_recover(c);
   }
   PB("recover_f64");
-  launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->rw), P<unsigned char>(c->rwlisted),
-                     patch_weights(c, c->cache2r), P<double>(c->rec),
-                     ExpandList{P<int>(c->titems), redo_count(c), redo_cap}, c->stream);
+  c->launches += launch_recover_w64(m, P<double>(c->ip), nc, P<double>(c->rw), P<unsigned char>(c->rwlisted),
+                                    patch_weights(c, c->cache2r), P<double>(c->rec),
+                                    ExpandList{P<int>(c->titems), redo_count(c), redo_cap}, c->stream);
   PE();
-  c->launches += 2;
   return check_launch(c, "recover");
 }
 

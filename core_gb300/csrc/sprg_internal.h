@@ -310,8 +310,8 @@ double key_to_double(unsigned long long k);
 // patches in lst) and the FP64 recovery from them
 void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, ExpandList lst, cudaStream_t s);
 // (the listed ones through pw; redo, triangles: scratch for V items a recovery and a
-// count that is zero before a pass's first)
-void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
+// count that is zero before a pass's first); returns the number of launches
+int launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
                         const PatchWeights& pw, double* rec, ExpandList redo, cudaStream_t s);
 // FP64 guard band of the FP32 path: re-decide the listed edges' bits.
 struct GuardScratch {

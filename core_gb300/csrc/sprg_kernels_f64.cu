@@ -2633,9 +2633,9 @@ __global__ void __launch_bounds__(kBlock) k_qr_weights(DevMesh m, double* __rest
 // Triangles one: six elements hide no sum (1024^2 square, both recoveries: 152
 // us, 192 with two).
 // REDO (triangles): what becomes of values that are not finite or near overflow,
-// which are the factors' sequence's: in place (the call costs registers: 164 us
-// against 152 at 1024^2) or listed for k_recover_redo (a launch: 1 us of the 37 of a
-// 128^2 square's pass); see launch_recover_w64.
+// which are the factors' sequence's: in place (the call costs registers: both
+// recoveries of a 1024^2 square 164 us against 152) or listed for k_recover_redo
+// (another launch); see launch_recover_w64.
 enum Redo { kRedoNone, kRedoHere, kRedoList };
 template <int NC, int LANES, Redo REDO>
 __global__ void __launch_bounds__(kBlock) k_recover_w64(DevMesh m, const double* __restrict__ ip,
@@ -2972,25 +2972,29 @@ void launch_qr_weights(const DevMesh& m, double* w, unsigned char* listed, Expan
   if (m.V) k_qr_weights<<<nblk((long)m.V * 32), kBlock, 0, s>>>(m, w, listed, lst);
 }
 
-void launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
-                        const PatchWeights& pw, double* rec, ExpandList redo, cudaStream_t s) {
-  if (!m.V) return;
+int launch_recover_w64(const DevMesh& m, const double* ip, int nc, const double* w, const unsigned char* listed,
+                       const PatchWeights& pw, double* rec, ExpandList redo, cudaStream_t s) {
+  if (!m.V) return 0;
   const int nl = nblk((long)pw.n * 32);
   auto go = [&](int lanes, auto kernel) {
     launch_after(m.early, kernel, nl + nblk((long)m.V * lanes), kBlock, s, m, ip, w, listed, nl, pw, rec, redo);
   };
   if (m.dim == 3) {
     go(2, nc == 3 ? k_recover_w64<3, 2, kRedoNone> : k_recover_w64<9, 2, kRedoNone>);  // lanes: see the kernel
-    return;
+    return 1;
   }
-  if (m.V < 1 << 18) {  // less than two waves of blocks: registers cost nothing, a launch does
+  // less than a wave of blocks: registers cost nothing, a launch does (the pass of
+  // a 128^2 square 34.5 us in place, 38.0 listed, 400^2 187.7 and 188.7, 520^2 317 and
+  // 315, 1000^2 1156 and 1148)
+  if (m.V < 1 << 18) {
     go(1, nc == 3 ? k_recover_w64<3, 1, kRedoHere> : k_recover_w64<9, 1, kRedoHere>);
-    return;
+    return 1;
   }
   go(1, nc == 3 ? k_recover_w64<3, 1, kRedoList> : k_recover_w64<9, 1, kRedoList>);
   // set up early on any mesh: a block per SM, which as a rule finds nothing
   launch_after(true, nc == 3 ? k_recover_redo<3> : k_recover_redo<9>, std::min(nblk(m.V, 128), 152), 128, s, m, ip, rec,
                redo.items, redo.count, redo.cap);
+  return 2;
 }
 
 }  // namespace sprg

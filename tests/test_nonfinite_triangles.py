@@ -86,3 +86,19 @@ def test_anisotropic_pass_on_a_large_square(gpu_lib, n):
         got = c.debug_read("rec", np.float64, 9 * m.n_verts).reshape(-1, 9)
     assert np.isnan(want).any()
     assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+
+
+@pytest.mark.parametrize("n,recovery", [(9, 1), (520, 2)])
+def test_launches_counted(gpu_lib, n, recovery):
+    """Two gradients, two recoveries, the metric and the lengths."""
+    import torch
+    import core_gb300 as cg
+    m, u = square(n)
+    bits = torch.zeros((2, (m.n_edges + 31) // 32), dtype=torch.int32, device="cuda")
+    d_u = torch.from_numpy(u).cuda()
+    torch.cuda.synchronize()
+    with cg.Context(m) as c:
+        for _ in range(2):
+            c.aniso_estimate_and_mark_resident(d_u.data_ptr(), 0.1, 0.1 / n, 1.0, bits[0].data_ptr(), bits[1].data_ptr())
+        torch.cuda.synchronize()
+        assert c.last_launch_count == 2 + 2 * recovery + 2
